@@ -25,8 +25,13 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-pthread", "-shared",
 ]
 
+# the binding of the operators on torch tensors (csrc/torch_ops.cpp), an extension module of this package
+OPS_PATH = os.path.join(_HERE, "_torch_ops.so")
+OPS_SOURCE = os.path.join(CSRC, "torch_ops.cpp")
+
 _lock = threading.Lock()
 _lib = None
+_ops = None
 
 c_int_p = ctypes.POINTER(ctypes.c_int)
 _vp = ctypes.c_void_p
@@ -181,6 +186,39 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if out.returncode != 0:
             raise RuntimeError("nvcc failed building libani_b200.so:\n" + out.stderr)
         return LIB_PATH
+
+
+def build_ops(force: bool = False) -> str:
+    """Compile the torch binding into ``khan_b200/_torch_ops.so`` (host code only)."""
+    import sysconfig
+
+    from torch.utils import cpp_extension
+    with _lock:
+        if not force and os.path.exists(OPS_PATH) and os.path.getmtime(OPS_PATH) >= os.path.getmtime(OPS_SOURCE):
+            return OPS_PATH
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_torch_ops", OPS_SOURCE, "-o", OPS_PATH]
+        cmd += ["-I" + d for d in cpp_extension.include_paths("cuda") + [sysconfig.get_paths()["include"]]]
+        cmd += ["-L" + d for d in cpp_extension.library_paths("cuda")]
+        cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lcudart"]
+        out = subprocess.run(cmd, capture_output=True, text=True)
+        if out.returncode != 0:
+            raise RuntimeError("g++ failed building _torch_ops.so:\n" + out.stderr)
+        return OPS_PATH
+
+
+def torch_ops():
+    """The torch binding, bound to the library of :func:`lib`.  Raises if it is not built."""
+    global _ops
+    if _ops is None:
+        handle = lib()
+        import torch  # noqa: F401  (the extension links to torch's libraries)
+        if not os.path.exists(OPS_PATH):
+            raise RuntimeError(f"{OPS_PATH} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
+        from . import _torch_ops as mod
+        mod.bind(*(ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in (
+            "ani_sort", "ani_featurize_f32", "ani_featurize_f64", "ani_featurize_grad_f32", "ani_featurize_grad_f64")))
+        _ops = mod
+    return _ops
 
 
 def lib() -> ctypes.CDLL:

@@ -59,17 +59,21 @@ def _acs_ptr(acs: np.ndarray):
     return acs.ctypes.data_as(_lib.c_int_p)
 
 
+def _run(where: str, call, *args):
+    """The result of a function of the torch binding; a negative status raises."""
+    out = call(*args)
+    if type(out) is int:
+        _lib.check(out, where)
+    return out
+
+
 def ani_sort(atomic_numbers: torch.Tensor):
     """AniSort: returns ``(scatter_idxs, gather_idxs, atom_counts)`` as int32 CUDA tensors."""
-    a = _dev(atomic_numbers, torch.int32, "atomic_numbers")
-    n = a.numel()
-    with torch.cuda.device(a.device):
-        scatter = torch.empty(n, dtype=torch.int32, device=a.device)
-        gather = torch.empty(n, dtype=torch.int32, device=a.device)
-        counts = torch.empty(4, dtype=torch.int32, device=a.device)
-        _lib.check(_lib.lib().ani_sort(_p(a), n, _p(scatter), _p(gather), _p(counts), _stream()),
-                   "ani_sort")
-    return scatter, gather, counts
+    call = _lib.torch_ops().ani_sort
+    out = _run("ani_sort", call, atomic_numbers)
+    if out is None:
+        out = _run("ani_sort", call, _dev(atomic_numbers, torch.int32, "atomic_numbers"))
+    return out
 
 
 def _common(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs):
@@ -83,20 +87,29 @@ def _common(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_id
     return xs, ys, zs, a, mo, mac, si
 
 
+def _featurize_call(name: str, batch, acs, *rest):
+    """One call of the binding; where it does not take the arguments as they are, once more with them
+    converted (dtype, contiguity, counts on the host)."""
+    call = getattr(_lib.torch_ops(), name)
+    out = call(*batch, acs, *rest)
+    if out is None:
+        batch = _common(*batch)
+        _suffix(batch[0])
+        out = call(*batch, host_counts(acs), *rest)
+        if out is None:
+            _lib.same_device(batch[0].device, *batch, *(r for r in rest if isinstance(r, torch.Tensor)), where=name)
+            raise ValueError(f"{name}: the arrays do not fit the batch")
+    if type(out) is int:
+        _lib.check(out, f"ani_{name}")
+    return out
+
+
 def featurize_into(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs,
                    acs_host: np.ndarray, out: torch.Tensor):
     """Featurize into a caller-owned ``[n_atoms, 384]`` buffer laid out H rows, C rows, N rows,
     O rows (the element-sorted order ``gather_idxs`` indexes).  No allocation, no sync."""
-    xs, ys, zs, a, mo, mac, si = _common(xs, ys, zs, atomic_numbers, mol_offsets,
-                                         mol_atom_counts, scatter_idxs)
-    suf = _suffix(xs)
-    starts = np.concatenate([[0], np.cumsum(acs_host)])[:4] * FEATURE_SIZE
-    flat = out.view(-1)
-    ptrs = [ctypes.c_void_p(flat.data_ptr() + int(s) * flat.element_size()) for s in starts]
-    with torch.cuda.device(xs.device):
-        fn = getattr(_lib.lib(), "ani_featurize_" + suf)
-        _lib.check(fn(_p(xs), _p(ys), _p(zs), _p(a), _p(mo), _p(mac), mo.numel(), _p(si), *ptrs,
-                      _acs_ptr(acs_host), _stream()), "ani_featurize_" + suf)
+    _featurize_call("featurize_into", (xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs),
+                    acs_host, out)
     return out
 
 
@@ -104,15 +117,8 @@ def featurize(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_
     """Featurize: returns four flat tensors ``h, c, n, o`` of ``acs[t] * 384`` values
     (views of one allocation; reshape each to ``(-1, 384)`` as the reference trainer does,
     ``khan/training/trainer_multi_tower.py:324-327``)."""
-    acs_host = host_counts(acs)
-    n_atoms = int(acs_host.sum())
-    out = torch.empty((n_atoms, FEATURE_SIZE), dtype=xs.dtype, device=xs.device)
-    featurize_into(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs,
-                   acs_host, out)
-    flat = out.view(-1)
-    ends = np.cumsum(acs_host) * FEATURE_SIZE
-    starts = ends - acs_host * FEATURE_SIZE
-    return tuple(flat[int(s):int(e)] for s, e in zip(starts, ends))
+    return _featurize_call("featurize", (xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs),
+                           acs, True)
 
 
 def featurize_grad(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs, acs,
@@ -122,25 +128,20 @@ def featurize_grad(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, sca
     The arrays start as zeros, so an atom that no molecule range covers gets a zero gradient, as
     in the reference (gpu_featurizer/functor_op_cpu.cpp:70-72); the C entry point itself writes
     only the atoms of the molecules it is given."""
-    xs, ys, zs, a, mo, mac, si = _common(xs, ys, zs, atomic_numbers, mol_offsets,
-                                         mol_atom_counts, scatter_idxs)
-    suf = _suffix(xs)
-    acs_host = host_counts(acs)
-    n_atoms = int(acs_host.sum())
-    gs = []
-    for t, g in enumerate((h_grads, c_grads, n_grads, o_grads)):
-        g = _dev(g, xs.dtype, "grads").view(-1)
-        if g.numel() != int(acs_host[t]) * FEATURE_SIZE:
-            raise ValueError(f"upstream gradient {t} has {g.numel()} values, expected "
-                             f"{int(acs_host[t]) * FEATURE_SIZE}")
-        gs.append(g)
-    with torch.cuda.device(xs.device):
-        outs = torch.zeros((3, n_atoms), dtype=xs.dtype, device=xs.device)
-        fn = getattr(_lib.lib(), "ani_featurize_grad_" + suf)
-        _lib.check(fn(_p(xs), _p(ys), _p(zs), _p(a), _p(mo), _p(mac), mo.numel(), _p(si),
-                      *[_p(g) for g in gs], _p(outs[0]), _p(outs[1]), _p(outs[2]),
-                      _acs_ptr(acs_host), _stream()), "ani_featurize_grad_" + suf)
-    return outs[0], outs[1], outs[2]
+    batch = (xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs)
+    grads = (h_grads, c_grads, n_grads, o_grads)
+    out = _run("ani_featurize_grad", _lib.torch_ops().featurize_grad, *batch, acs, *grads)
+    if out is None:
+        batch = _common(*batch)
+        _suffix(batch[0])
+        acs = host_counts(acs)
+        grads = [_dev(g, batch[0].dtype, "grads") for g in grads]
+        for t, g in enumerate(grads):
+            if g.numel() != int(acs[t]) * FEATURE_SIZE:
+                raise ValueError(f"upstream gradient {t} has {g.numel()} values, expected "
+                                 f"{int(acs[t]) * FEATURE_SIZE}")
+        out = _featurize_call("featurize_grad", batch, acs, *grads)
+    return out
 
 
 def featurize_grad_inverse(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs,
@@ -172,10 +173,8 @@ def featurize_grad_inverse(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_cou
 def featurize_sorted(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs, acs):
     """Featurize into one ``[n_atoms, 384]`` tensor laid out H rows, C rows, N rows, O rows (the
     order ``gather_idxs`` indexes; the four outputs of :func:`featurize` are its slices)."""
-    acs_host = host_counts(acs)
-    out = torch.empty((int(acs_host.sum()), FEATURE_SIZE), dtype=xs.dtype, device=xs.device)
-    return featurize_into(xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs,
-                          acs_host, out)
+    return _featurize_call("featurize", (xs, ys, zs, atomic_numbers, mol_offsets, mol_atom_counts, scatter_idxs),
+                           acs, False)
 
 
 def _split(buf, acs_host):
