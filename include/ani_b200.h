@@ -461,6 +461,9 @@ int ani_host_pack_batch(const ani_host_pack_args* args);
 #define ANI_PASS_BACKWARD 16     /* ani_mlp_backward_f32 (feature_grads == NULL skips the products towards the features) */
 #define ANI_PASS_WEIGHT_GRAD 32  /* clear zero_ptr[0 .. zero_bytes), then ani_mlp_weight_grad_f32 */
 #define ANI_PASS_COORD_GRAD 64   /* ani_featurize_grad_f32 with feature_grads as its upstream */
+#define ANI_PASS_TRANSIENT 128   /* what the networks leave behind (act*, dact*, dz*) is not read after this call: only
+                                    what the call's own phases need is written, and a batch of few atoms may go
+                                    through one kernel that writes none of it */
 typedef struct ani_pass_args {
     int phases;
     int n_atoms, n_mols;
@@ -488,6 +491,27 @@ typedef struct ani_pass_args {
     size_t zero_bytes;
 } ani_pass_args;
 int ani_network_pass_f32(const ani_pass_args* args, void* stream);
+
+/* Energies, and energies + forces, in double precision (the precision the reference serves in,
+ * energy_server.py): the phases FEATURIZE, FORWARD, ENERGY, BACKWARD and COORD_GRAD of the above for
+ * the 384-128-128-64-1 networks (FORWARD and BACKWARD together are one kernel; BACKWARD alone is refused),
+ * dE_molecule/dE_atom = 1.  Launches only. */
+typedef struct ani_energy_args_f64 {
+    int phases;
+    int n_atoms, n_mols;
+    const int* acs_host;             /* HOST [4] */
+    int activation;
+    const double *xs, *ys, *zs;      /* [n_atoms] */
+    const int *atomic_numbers, *mol_offsets, *mol_atom_counts;
+    int *scatter_idxs, *gather_idxs, *atom_counts;
+    double* features;                /* [n_atoms][384] */
+    double* feature_grads;           /* [n_atoms][384] */
+    double *x_grads, *y_grads, *z_grads;
+    double* energy_sorted;           /* [n_atoms] */
+    double* mol_energy;              /* [n_mols] */
+    const double *w1[4], *b1[4], *w2[4], *b2[4], *w3[4], *b3[4], *w4[4], *b4[4];
+} ani_energy_args_f64;
+int ani_energy_pass_f64(const ani_energy_args_f64* args, void* stream);
 
 /*
  * The submitter thread of the batch feeder in native code (the reference: a Python thread that

@@ -18,7 +18,7 @@ CSRC = os.path.join(_HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(_HERE), "include")
 SOURCES = ["ani_b200.cu"]
 HEADERS = ["ani_params.h", "ani_common.cuh", "ani_device_math.cuh", "ani_feeder.h", "ani_peer.cuh", "ani_sort.cuh", "ani_featurize.cuh", "ani_featurize_mol.cuh", "ani_featurize_large.cuh", "ani_featurize_round_passes.inl", "ani_grad.cuh", "ani_grad_mol.cuh", "ani_grad_pair_pass.inl",
-           "ani_grad_inverse.cuh", "ani_mlp.cuh", "ani_mlp_pipe.cuh", "ani_mlp_forward.cuh", "ani_mlp_backward.cuh", "ani_mlp_wgrad.cuh", "ani_charge.cuh", "ani_optim.cuh", "ani_energy.cuh", "ani_host_pack.h"]
+           "ani_grad_inverse.cuh", "ani_mlp.cuh", "ani_mlp_pipe.cuh", "ani_mlp_forward.cuh", "ani_mlp_backward.cuh", "ani_mlp_wgrad.cuh", "ani_mlp_small.cuh", "ani_launch.cuh", "ani_charge.cuh", "ani_optim.cuh", "ani_energy.cuh", "ani_host_pack.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -91,8 +91,19 @@ class PassArgs(ctypes.Structure):
                 + [("zero_ptr", ctypes.c_void_p), ("zero_bytes", ctypes.c_size_t)])
 
 
-PASS_PACK, PASS_FEATURIZE, PASS_FORWARD, PASS_ENERGY, PASS_BACKWARD, PASS_WEIGHT_GRAD, PASS_COORD_GRAD = (
-    1, 2, 4, 8, 16, 32, 64)
+class EnergyArgs64(ctypes.Structure):
+    """``ani_energy_args_f64`` of include/ani_b200.h."""
+    _fields_ = ([("phases", ctypes.c_int), ("n_atoms", ctypes.c_int), ("n_mols", ctypes.c_int),
+                 ("acs_host", ctypes.c_void_p), ("activation", ctypes.c_int)]
+                + [(n, ctypes.c_void_p) for n in (
+                    "xs", "ys", "zs", "atomic_numbers", "mol_offsets", "mol_atom_counts", "scatter_idxs", "gather_idxs",
+                    "atom_counts", "features", "feature_grads", "x_grads", "y_grads", "z_grads", "energy_sorted",
+                    "mol_energy")]
+                + [(n, ctypes.c_void_p * 4) for n in ("w1", "b1", "w2", "b2", "w3", "b3", "w4", "b4")])
+
+
+PASS_PACK, PASS_FEATURIZE, PASS_FORWARD, PASS_ENERGY, PASS_BACKWARD, PASS_WEIGHT_GRAD, PASS_COORD_GRAD, PASS_TRANSIENT = (
+    1, 2, 4, 8, 16, 32, 64, 128)
 
 
 class MlpBackwardArgs(ctypes.Structure):
@@ -134,6 +145,7 @@ SIGNATURES = {
     "ani_scale_by_loss_f32": (_i, [_vp, ctypes.c_longlong, _vp, _i, _i, _vp, _vp]),
     "ani_host_pack_batch": (_i, [_vp]),
     "ani_network_pass_f32": (_i, [ctypes.POINTER(PassArgs), _vp]),
+    "ani_energy_pass_f64": (_i, [ctypes.POINTER(EnergyArgs64), _vp]),
     "ani_feeder_create": (_i, [_i, _vp, _i, ctypes.POINTER(_vp)]),
     "ani_feeder_begin": (_i, [_vp, _vp, ctypes.c_longlong, _i]),
     "ani_feeder_next": (_i, [_vp, ctypes.POINTER(FeederBatch)]),

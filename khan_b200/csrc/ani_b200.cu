@@ -24,6 +24,7 @@
 #include "ani_mlp_forward.cuh"
 #include "ani_mlp_backward.cuh"
 #include "ani_mlp_wgrad.cuh"
+#include "ani_mlp_small.cuh"
 #include "ani_charge.cuh"
 #include "ani_optim.cuh"
 #include "ani_energy.cuh"
@@ -241,10 +242,9 @@ int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, cons
     // central atoms
     if (small_molecules(n_atoms, n_mols) && all_aligned16({oh, oc, on, oo}) &&
         (long long)n_mols * kMolRounds <= 0x7fffffffLL) {
-        featurize_mol_kernel<T><<<n_mols * kMolRounds, kWarp, 0, (cudaStream_t)stream>>>(
-            xs, ys, zs, types, mos, macs, n_mols, (int)n_atoms, sis, oh, oc, on, oo, acs_host[0], acs_host[1],
-            acs_host[2], acs_host[3]);
-        ANI_CUDA(cudaGetLastError());
+        ANI_CUDA(launch_chain(featurize_mol_kernel<T>, n_mols * kMolRounds, kWarp, 0, (cudaStream_t)stream, 1, xs, ys, zs,
+                              types, mos, macs, n_mols, (int)n_atoms, sis, oh, oc, on, oo, acs_host[0], acs_host[1],
+                              acs_host[2], acs_host[3]));
         return ANI_OK;
     }
 
@@ -254,10 +254,9 @@ int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, cons
         const long long mean_rounds = (n_atoms / n_mols + kMolCentrals) / kMolCentrals;
         const int rounds_in_grid = (int)std::min<long long>(std::max<long long>(mean_rounds, kMolRounds), 64);
         if ((long long)n_mols * rounds_in_grid <= 0x7fffffffLL) {
-            featurize_large_kernel<T><<<n_mols * rounds_in_grid, kWarp, 0, (cudaStream_t)stream>>>(
-                xs, ys, zs, types, mos, macs, n_mols, (int)n_atoms, rounds_in_grid, sis, oh, oc, on, oo, acs_host[0],
-                acs_host[1], acs_host[2], acs_host[3]);
-            ANI_CUDA(cudaGetLastError());
+            ANI_CUDA(launch_chain(featurize_large_kernel<T>, n_mols * rounds_in_grid, kWarp, 0, (cudaStream_t)stream, 1,
+                                  xs, ys, zs, types, mos, macs, n_mols, (int)n_atoms, rounds_in_grid, sis, oh, oc, on, oo,
+                                  acs_host[0], acs_host[1], acs_host[2], acs_host[3]));
             return ANI_OK;
         }
     }
@@ -313,18 +312,16 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
             if (int rc = set_smem(mol_kernel, mol_smem)) return rc;
             mol_configured_dev = dev;
         }
-        mol_kernel<<<n_mols * kMolGradClasses, kMolGradWarps * kWarp, mol_smem, st>>>(xs, ys, zs, types, mos, macs, n_mols, (int)n_atoms, sis, gh,
-                                                          gc, gn, go, gx, gy, gz, acs_host[0], acs_host[1],
-                                                          acs_host[2], acs_host[3]);
-        ANI_CUDA(cudaGetLastError());
+        ANI_CUDA(launch_chain(mol_kernel, n_mols * kMolGradClasses, kMolGradWarps * kWarp, mol_smem, st, 1, xs, ys, zs, types,
+                              mos, macs, n_mols, (int)n_atoms, sis, gh, gc, gn, go, gx, gy, gz, acs_host[0], acs_host[1],
+                              acs_host[2], acs_host[3]));
         return ANI_OK;
     }
     {
         const int threads = 256;
         long long blocks = (n_atoms + threads - 1) / threads;
         if (blocks > 1184) blocks = 1184;
-        zero3_kernel<T><<<(int)blocks, threads, 0, st>>>(gx, gy, gz, (int)n_atoms);
-        ANI_CUDA(cudaGetLastError());
+        ANI_CUDA(launch_chain(zero3_kernel<T>, (int)blocks, threads, 0, st, 1, gx, gy, gz, (int)n_atoms));
     }
     if (n_mols == 0) return ANI_OK;
     if (!xs || !ys || !zs || !types || !mos || !macs || !sis) return ANI_ERR_NULL_POINTER;
@@ -348,10 +345,8 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
     const int slot_shift = pick_slot_shift(n_atoms, n_mols);
     const long long needed = (long long)n_mols * ((1 << (slot_shift & 31)) / kNW);
     const int grid = (int)(needed < cached_resident ? needed : cached_resident);
-    kernel<<<grid, kNW * kWarp, smem, st>>>(
-        xs, ys, zs, types, mos, macs, n_mols, (int)n_atoms, slot_shift, sis, gh, gc, gn, go, gx, gy, gz,
-        acs_host[0], acs_host[1], acs_host[2], acs_host[3]);
-    ANI_CUDA(cudaGetLastError());
+    ANI_CUDA(launch_chain(kernel, grid, kNW * kWarp, smem, st, 1, xs, ys, zs, types, mos, macs, n_mols, (int)n_atoms,
+                          slot_shift, sis, gh, gc, gn, go, gx, gy, gz, acs_host[0], acs_host[1], acs_host[2], acs_host[3]));
     return ANI_OK;
 }
 
@@ -449,8 +444,7 @@ template <int ACT, bool SPLIT> int mlp_launch(const MlpParams& p, int n_tiles, c
         if (int rc = set_smem(kernel, smem)) return rc;
         configured_dev = dev;
     }
-    kernel<<<n_tiles, kMlpAllThreads, smem, st>>>(p);
-    ANI_CUDA(cudaGetLastError());
+    ANI_CUDA(launch_chain(kernel, n_tiles, kMlpAllThreads, smem, st, 1, p));
     return ANI_OK;
 }
 
@@ -465,8 +459,7 @@ template <bool SPLIT> int mlp_backward_launch(const MlpBackwardParams& p, int n_
         if (int rc = set_smem(kernel, smem)) return rc;
         configured_dev = dev;
     }
-    kernel<<<n_tiles, kMlpAllThreads, smem, st>>>(p);
-    ANI_CUDA(cudaGetLastError());
+    ANI_CUDA(launch_chain(kernel, n_tiles, kMlpAllThreads, smem, st, 1, p));
     return ANI_OK;
 }
 
@@ -483,6 +476,90 @@ template <bool SPLIT> int mlp_wgrad_launch(const MlpWgradParams& p, int n_ranges
     }
     kernel<<<dim3(n_ranges, kWgradBlocks), kMlpAllThreads, smem, st>>>(p);
     ANI_CUDA(cudaGetLastError());
+    return ANI_OK;
+}
+
+int pack_params(const float* const* w1, const float* const* w2, const float* const* w3, void* const* packed, MlpPackParams* p,
+                bool* any)
+{
+    for (int t = 0; t < kTypes; t++) {
+        p->w1[t] = w1[t]; p->w2[t] = w2[t]; p->w3[t] = w3[t];
+        p->packed[t] = (unsigned char*)packed[t];
+        if (!packed[t]) continue;
+        if (!w1[t] || !w2[t] || !w3[t]) return ANI_ERR_NULL_POINTER;
+        if (reinterpret_cast<uintptr_t>(packed[t]) & 15) return ANI_ERR_MISALIGNED;
+        *any = true;
+    }
+    return ANI_OK;
+}
+int pack_launch(const MlpPackParams& p, cudaStream_t st)
+{
+    mlp_pack_kernel<<<dim3(kPackChunks, kTypes), kMlpThreads, 0, st>>>(p);
+    ANI_CUDA(cudaGetLastError());
+    return ANI_OK;
+}
+
+// Batches whose networks take mlp_small_kernel: every tile of 16 atoms is a cluster of 8 CTAs, and TODO_FEW
+constexpr int kFewTiles = 40;
+bool few_atoms(const int* acs)
+{
+    int tiles = 0;
+    for (int t = 0; t < kTypes; t++) tiles += (acs[t] + kSmallTile - 1) / kSmallTile;
+    return tiles <= kFewTiles;
+}
+
+template <typename T>
+int energy_launch(const T* atom_energy_sorted, const int* gather, const int* mos, const int* macs, int n_mols, int n_atoms,
+                  const T* labels, T grad_scale, T* mol_energy, T* l2s, T* grad_atom_energy_sorted, cudaStream_t st)
+{
+    int grid = 0;
+    if (int rc = charge_grid(n_mols, &grid)) return rc;
+    ANI_CUDA(launch_chain(molecule_energy_kernel<T, kNW>, grid, kNW * kWarp, 0, st, 1, atom_energy_sorted, gather, mos, macs,
+                          n_mols, n_atoms, labels, grad_scale, mol_energy, l2s, grad_atom_energy_sorted));
+    return ANI_OK;
+}
+
+// Networks of few atoms / of double precision: forward and (grad_feat != NULL) backward to the features.
+template <typename T>
+int mlp_small_launch(const T* feat, const int* acs, const T* const* w1, const T* const* b1, const T* const* w2,
+                     const T* const* b2, const T* const* w3, const T* const* b3, const T* const* w4, const T* const* b4,
+                     const T* grad_energy, T* energy, T* grad_feat, int activation, cudaStream_t st)
+{
+    if (activation < 0 || activation > 3) return ANI_ERR_BAD_SIZE;
+    MlpSmallParams<T> p;
+    p.feat = feat;
+    p.grad_energy = grad_energy;
+    p.energy = energy;
+    p.grad_feat = grad_feat;
+    p.activation = activation;
+    int tiles = 0, row = 0;
+    if (!feat || !energy) return ANI_ERR_NULL_POINTER;
+    if (!all_aligned16({feat, grad_feat})) return ANI_ERR_MISALIGNED;
+    for (int t = 0; t < kTypes; t++) {
+        p.tile_start[t] = tiles;
+        p.row_start[t] = row;
+        p.count[t] = acs[t];
+        tiles += (acs[t] + kSmallTile - 1) / kSmallTile;
+        row += acs[t];
+        if (acs[t] > 0) {
+            if (!w1[t] || !b1[t] || !w2[t] || !b2[t] || !w3[t] || !b3[t] || !w4[t] || !b4[t]) return ANI_ERR_NULL_POINTER;
+            if (!all_aligned16({w1[t], w2[t], w3[t]})) return ANI_ERR_MISALIGNED;
+        }
+        p.w1[t] = w1[t]; p.b1[t] = b1[t]; p.w2[t] = w2[t]; p.b2[t] = b2[t];
+        p.w3[t] = w3[t]; p.b3[t] = b3[t]; p.w4[t] = w4[t]; p.b4[t] = b4[t];
+    }
+    p.tile_start[kTypes] = tiles;
+    if (tiles == 0) return ANI_OK;
+    auto kernel = mlp_small_kernel<T>;
+    const size_t smem = sizeof(MlpSmallShared<T>);
+    static thread_local int configured_dev = -1;
+    int dev = 0;
+    ANI_CUDA(cudaGetDevice(&dev));
+    if (configured_dev != dev) {
+        if (int rc = set_smem(kernel, smem)) return rc;
+        configured_dev = dev;
+    }
+    ANI_CUDA(launch_chain(kernel, tiles * kSmallCtas, kSmallThreads, smem, st, kSmallCtas, p));
     return ANI_OK;
 }
 
@@ -544,9 +621,8 @@ int ani_sort(const int* atomic_numbers, int n_atoms, int* scatter_idxs, int* gat
     if (!atomic_numbers || !scatter_idxs || !gather_idxs) return ANI_ERR_NULL_POINTER;
     const int n_tiles = (n_atoms + kSortTile - 1) / kSortTile;
     if (n_atoms <= kSortSingleLaunchMax) {
-        sort_single_kernel<<<n_tiles, kSortThreads, 0, st>>>(atomic_numbers, n_atoms, scatter_idxs,
-                                                             gather_idxs, atom_counts);
-        ANI_CUDA(cudaGetLastError());
+        ANI_CUDA(launch_chain(sort_single_kernel, n_tiles, kSortThreads, 0, st, 1, atomic_numbers, n_atoms, scatter_idxs,
+                              gather_idxs, atom_counts));
         return ANI_OK;
     }
     int* scratch = nullptr;
@@ -708,18 +784,8 @@ int ani_mlp_pack_weights_f32(const ani_mlp_pack_args* a, void* stream)
     if (!a) return ANI_ERR_NULL_POINTER;
     MlpPackParams p;
     bool any = false;
-    for (int t = 0; t < kTypes; t++) {
-        p.w1[t] = a->w1[t]; p.w2[t] = a->w2[t]; p.w3[t] = a->w3[t];
-        p.packed[t] = (unsigned char*)a->packed[t];
-        if (!a->packed[t]) continue;
-        if (!a->w1[t] || !a->w2[t] || !a->w3[t]) return ANI_ERR_NULL_POINTER;
-        if (reinterpret_cast<uintptr_t>(a->packed[t]) & 15) return ANI_ERR_MISALIGNED;
-        any = true;
-    }
-    if (!any) return ANI_OK;
-    mlp_pack_kernel<<<dim3(kPackChunks, kTypes), kMlpThreads, 0, (cudaStream_t)stream>>>(p);
-    ANI_CUDA(cudaGetLastError());
-    return ANI_OK;
+    if (int rc = pack_params(a->w1, a->w2, a->w3, a->packed, &p, &any)) return rc;
+    return any ? pack_launch(p, (cudaStream_t)stream) : ANI_OK;
 }
 
 int ani_mlp_backward_f32(const ani_mlp_backward_args* a, const int* acs_host, int split_precision,
@@ -814,13 +880,8 @@ int ani_molecule_energy_f32(const float* atom_energy_sorted, const int* gather_i
     if (n_mols == 0) return ANI_OK;
     if (!mol_offsets || !mol_atom_counts || !mol_energy) return ANI_ERR_NULL_POINTER;
     if (n_atoms > 0 && (!atom_energy_sorted || !gather_idxs)) return ANI_ERR_NULL_POINTER;
-    int grid = 0;
-    if (int rc = charge_grid(n_mols, &grid)) return rc;
-    molecule_energy_kernel<kNW><<<grid, kNW * kWarp, 0, (cudaStream_t)stream>>>(
-        atom_energy_sorted, gather_idxs, mol_offsets, mol_atom_counts, n_mols, n_atoms, labels, grad_scale,
-        mol_energy, l2s, grad_atom_energy_sorted);
-    ANI_CUDA(cudaGetLastError());
-    return ANI_OK;
+    return energy_launch<float>(atom_energy_sorted, gather_idxs, mol_offsets, mol_atom_counts, n_mols, n_atoms, labels,
+                                grad_scale, mol_energy, l2s, grad_atom_energy_sorted, (cudaStream_t)stream);
 }
 
 int ani_nadam_step_f32(float* params, const float* grads, float* m, float* v, float* ema,
@@ -1108,33 +1169,60 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
     auto rows = [&](float* base, int t, int width) -> float* {
         return base && acs[t] > 0 ? base + start[t] * (size_t)width : nullptr;
     };
+    bool sorted = false;
     if (a->phases & ANI_PASS_PACK) {
-        ani_mlp_pack_args p;
-        for (int t = 0; t < kTypes; t++) {
-            p.w1[t] = a->w1[t]; p.w2[t] = a->w2[t]; p.w3[t] = a->w3[t];
-            p.packed[t] = a->packed[t];
+        MlpPackParams p;
+        bool any = false;
+        if (int rc = pack_params(a->w1, a->w2, a->w3, a->packed, &p, &any)) return rc;
+        // with a sort of one launch in the same pass: both in one kernel
+        if (any && (a->phases & ANI_PASS_FEATURIZE) && n_atoms > 0 && n_atoms <= kSortSingleLaunchMax) {
+            if (!a->atomic_numbers || !a->scatter_idxs || !a->gather_idxs || !a->atom_counts) return ANI_ERR_NULL_POINTER;
+            const int n_tiles = (int)((n_atoms + kSortTile - 1) / kSortTile);
+            ANI_CUDA(launch_chain(sort_and_pack_kernel, n_tiles + kPackChunks * kTypes, kSortThreads, 0, (cudaStream_t)stream,
+                                  1, a->atomic_numbers, (int)n_atoms, n_tiles, a->scatter_idxs, a->gather_idxs,
+                                  a->atom_counts, p));
+            sorted = true;
+        } else if (any) {
+            if (int rc = pack_launch(p, (cudaStream_t)stream)) return rc;
         }
-        if (int rc = ani_mlp_pack_weights_f32(&p, stream)) return rc;
     }
     if (a->phases & ANI_PASS_FEATURIZE) {
-        if (int rc = ani_sort(a->atomic_numbers, a->n_atoms, a->scatter_idxs, a->gather_idxs, a->atom_counts, stream))
-            return rc;
+        if (!sorted)
+            if (int rc = ani_sort(a->atomic_numbers, a->n_atoms, a->scatter_idxs, a->gather_idxs, a->atom_counts, stream))
+                return rc;
         if (int rc = ani_featurize_f32(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
                                        a->n_mols, a->scatter_idxs, rows(a->features, 0, kTotal),
                                        rows(a->features, 1, kTotal), rows(a->features, 2, kTotal),
                                        rows(a->features, 3, kTotal), acs, stream))
             return rc;
     }
-    if (a->phases & ANI_PASS_FORWARD) {
+    const bool transient = (a->phases & ANI_PASS_TRANSIENT) != 0;
+    bool backward_done = false;
+    if ((a->phases & ANI_PASS_FORWARD) && transient && few_atoms(acs) && !(a->phases & ANI_PASS_WEIGHT_GRAD) && !a->labels) {
+        const bool backward = (a->phases & ANI_PASS_BACKWARD) && a->feature_grads;
+        if (n_atoms > 0)
+            if (int rc = mlp_small_launch<float>(a->features, acs, a->w1, a->b1, a->w2, a->b2, a->w3, a->b3, a->w4, a->b4,
+                                                 a->grad_energy_sorted, a->energy_sorted,
+                                                 backward ? a->feature_grads : nullptr, a->activation,
+                                                 (cudaStream_t)stream))
+                return rc;
+        backward_done = true;
+    } else if (a->phases & ANI_PASS_FORWARD) {
+        // what only the backward steps read is not written when they do not follow
+        const bool save = !transient || (a->phases & (ANI_PASS_BACKWARD | ANI_PASS_WEIGHT_GRAD));
+        const bool save_act = save && (!transient || (a->phases & ANI_PASS_WEIGHT_GRAD));
         ani_mlp_args f;
         for (int t = 0; t < kTypes; t++) {
             f.features[t] = rows(a->features, t, kTotal);
             f.w1[t] = a->w1[t]; f.b1[t] = a->b1[t]; f.w2[t] = a->w2[t]; f.b2[t] = a->b2[t];
             f.w3[t] = a->w3[t]; f.b3[t] = a->b3[t]; f.w4[t] = a->w4[t]; f.b4[t] = a->b4[t];
             f.energy[t] = rows(a->energy_sorted, t, 1);
-            f.act1[t] = rows(a->act1, t, kMlpH1); f.act2[t] = rows(a->act2, t, kMlpH2); f.act3[t] = rows(a->act3, t, kMlpH3);
-            f.dact1[t] = rows(a->dact1, t, kMlpH1); f.dact2[t] = rows(a->dact2, t, kMlpH2);
-            f.dact3[t] = rows(a->dact3, t, kMlpH3);
+            f.act1[t] = save_act ? rows(a->act1, t, kMlpH1) : nullptr;
+            f.act2[t] = save_act ? rows(a->act2, t, kMlpH2) : nullptr;
+            f.act3[t] = save_act ? rows(a->act3, t, kMlpH3) : nullptr;
+            f.dact1[t] = save ? rows(a->dact1, t, kMlpH1) : nullptr;
+            f.dact2[t] = save ? rows(a->dact2, t, kMlpH2) : nullptr;
+            f.dact3[t] = save ? rows(a->dact3, t, kMlpH3) : nullptr;
             f.packed[t] = a->packed[t];
         }
         if (int rc = ani_mlp_forward_f32(&f, acs, a->activation, a->split_precision, stream)) return rc;
@@ -1146,7 +1234,7 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
                                              a->labels ? a->grad_energy_sorted : nullptr, stream))
             return rc;
     }
-    if (a->phases & ANI_PASS_BACKWARD) {
+    if ((a->phases & ANI_PASS_BACKWARD) && !backward_done) {
         ani_mlp_backward_args b;
         for (int t = 0; t < kTypes; t++) {
             b.grad_energy[t] = rows(a->grad_energy_sorted, t, 1);
@@ -1179,6 +1267,52 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
                                             rows(a->feature_grads, 1, kTotal), rows(a->feature_grads, 2, kTotal),
                                             rows(a->feature_grads, 3, kTotal), a->x_grads, a->y_grads, a->z_grads,
                                             acs, stream))
+            return rc;
+    }
+    return ANI_OK;
+}
+
+int ani_energy_pass_f64(const ani_energy_args_f64* a, void* stream)
+{
+    if (!a) return ANI_ERR_NULL_POINTER;
+    long long n_atoms = 0;
+    if (int rc = check_acs(a->acs_host, &n_atoms)) return rc;
+    if (a->n_atoms < 0 || a->n_mols < 0 || n_atoms != a->n_atoms) return ANI_ERR_BAD_SIZE;
+    if ((a->phases & ANI_PASS_BACKWARD) && !(a->phases & ANI_PASS_FORWARD)) return ANI_ERR_BAD_SIZE;
+    const int* acs = a->acs_host;
+    double *rows[kTypes], *grad_rows[kTypes];
+    size_t at = 0;
+    for (int t = 0; t < kTypes; t++) {
+        rows[t] = a->features && acs[t] > 0 ? a->features + at * kTotal : nullptr;
+        grad_rows[t] = a->feature_grads && acs[t] > 0 ? a->feature_grads + at * kTotal : nullptr;
+        at += (size_t)acs[t];
+    }
+    if (a->phases & ANI_PASS_FEATURIZE) {
+        if (int rc = ani_sort(a->atomic_numbers, a->n_atoms, a->scatter_idxs, a->gather_idxs, a->atom_counts, stream))
+            return rc;
+        if (int rc = ani_featurize_f64(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts, a->n_mols,
+                                       a->scatter_idxs, rows[0], rows[1], rows[2], rows[3], acs, stream))
+            return rc;
+    }
+    if ((a->phases & ANI_PASS_FORWARD) && n_atoms > 0) {
+        const bool backward = (a->phases & ANI_PASS_BACKWARD) != 0;
+        if (backward && !a->feature_grads) return ANI_ERR_NULL_POINTER;
+        if (int rc = mlp_small_launch<double>(a->features, acs, a->w1, a->b1, a->w2, a->b2, a->w3, a->b3, a->w4, a->b4,
+                                              nullptr, a->energy_sorted, backward ? a->feature_grads : nullptr,
+                                              a->activation, (cudaStream_t)stream))
+            return rc;
+    }
+    if ((a->phases & ANI_PASS_ENERGY) && a->n_mols > 0) {
+        if (!a->mol_offsets || !a->mol_atom_counts || !a->mol_energy) return ANI_ERR_NULL_POINTER;
+        if (n_atoms > 0 && (!a->energy_sorted || !a->gather_idxs)) return ANI_ERR_NULL_POINTER;
+        if (int rc = energy_launch<double>(a->energy_sorted, a->gather_idxs, a->mol_offsets, a->mol_atom_counts, a->n_mols,
+                                           a->n_atoms, nullptr, 0.0, a->mol_energy, nullptr, nullptr, (cudaStream_t)stream))
+            return rc;
+    }
+    if (a->phases & ANI_PASS_COORD_GRAD) {
+        if (int rc = ani_featurize_grad_f64(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
+                                            a->n_mols, a->scatter_idxs, grad_rows[0], grad_rows[1], grad_rows[2],
+                                            grad_rows[3], a->x_grads, a->y_grads, a->z_grads, acs, stream))
             return rc;
     }
     return ANI_OK;

@@ -11,22 +11,25 @@
 #pragma once
 
 #include "ani_common.cuh"
+#include "ani_launch.cuh"
 
 namespace ani {
 
-template <int NW>
+template <typename T, int NW>
 __global__ void __launch_bounds__(NW* kWarp)
-    molecule_energy_kernel(const float* __restrict__ atom_energy_sorted, const int* __restrict__ gather,
+    molecule_energy_kernel(const T* __restrict__ atom_energy_sorted, const int* __restrict__ gather,
                            const int* __restrict__ mol_offsets, const int* __restrict__ mol_counts,
-                           int n_mols, int n_atoms, const float* __restrict__ labels, float grad_scale,
-                           float* __restrict__ mol_energy, float* __restrict__ l2s,
-                           float* __restrict__ grad_atom_energy_sorted)
+                           int n_mols, int n_atoms, const T* __restrict__ labels, T grad_scale,
+                           T* __restrict__ mol_energy, T* __restrict__ l2s,
+                           T* __restrict__ grad_atom_energy_sorted)
 {
+    pdl_wait();
+    pdl_trigger();
     const int lane = lane_id();
     const int grid_warps = gridDim.x * NW;
     for (int m = blockIdx.x * NW + warp_id(); m < n_mols; m += grid_warps) {
         MolRange mol;
-        float e = 0.0f;
+        T e = (T)0;
         const bool ok = load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol);
         if (ok) {
             for (int i = lane; i < mol.n; i += kWarp) {
@@ -39,10 +42,10 @@ __global__ void __launch_bounds__(NW* kWarp)
         }
         if (lane == 0) mol_energy[m] = e;
         if (labels) {
-            const float diff = e - labels[m];
+            const T diff = e - labels[m];
             if (lane == 0 && l2s) l2s[m] = diff * diff;
             if (ok && grad_atom_energy_sorted) {
-                const float g_mol = grad_scale * 2.0f * diff;
+                const T g_mol = grad_scale * (T)2 * diff;
                 for (int i = lane; i < mol.n; i += kWarp) {
                     const int g = gather[mol.base + i];
                     if (g >= 0 && g < n_atoms) grad_atom_energy_sorted[g] = g_mol;

@@ -51,6 +51,8 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
     using Granule = Vec4<float>;
     constexpr int kPerGranule = 16 / (int)sizeof(T);
     const int lane = lane_id();
+    pdl_wait();
+    pdl_trigger();
 
     // round-major grid, as in featurize_mol_kernel: the first rounds of all molecules start first
     const int round0 = blockIdx.x / n_mols, m = blockIdx.x - round0 * n_mols;

@@ -40,6 +40,7 @@
 #include "ani_common.cuh"
 #include "ani_device_math.cuh"
 #include "ani_featurize.cuh"
+#include "ani_launch.cuh"
 
 namespace ani {
 
@@ -174,6 +175,8 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     using Granule = Vec4<float>;                      // 16 bytes of zeros, whatever T is
     constexpr int kPerGranule = 16 / (int)sizeof(T);  // values in a granule
     const int lane = lane_id();
+    pdl_wait();
+    pdl_trigger();
 
     // Round-major order of the grid: all first rounds (every molecule has one), then all second rounds, ...
     // so the work that exists starts first and is spread evenly over the SMs, and the CTAs of rounds that

@@ -25,6 +25,7 @@
 #pragma once
 
 #include "ani_common.cuh"
+#include "ani_launch.cuh"
 #include "ani_device_math.cuh"
 
 namespace ani {
@@ -141,6 +142,8 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? ANI_GRAD_MIN_CTAS 
     __shared__ int cta_next_item;
     if (threadIdx.x == 0) cta_next_item = 0;
     __syncthreads();
+    pdl_wait();
+    pdl_trigger();
     for (;;) {
         int m, slot;
         if (!next_work<NW>(&cta_next_item, n_mols, slot_shift & 31, (slot_shift & 32) != 0, &m, &slot)) break;
@@ -310,6 +313,8 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? ANI_GRAD_MIN_CTAS 
 // them; the reference zero-fills in its functor, gpu_featurizer/functor_op_cpu.cpp:70-72).
 template <typename T> __global__ void zero3_kernel(T* a, T* b, T* c, int n)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         a[i] = (T)0;
         b[i] = (T)0;

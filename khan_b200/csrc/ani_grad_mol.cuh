@@ -135,6 +135,8 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     using WarpShared = MolGradWarpShared<T>;
     const int lane = lane_id(), warp = warp_id();
+    pdl_wait();
+    pdl_trigger();
     WarpShared& ws = reinterpret_cast<WarpShared*>(smem_raw)[warp];
     T* part = reinterpret_cast<T*>(smem_raw + NW * sizeof(WarpShared));
     auto part_at = [part](int plane, int c, int j) -> T& {

@@ -22,6 +22,7 @@
 #pragma once
 
 #include "ani_common.cuh"
+#include "ani_launch.cuh"
 
 namespace ani {
 

@@ -68,6 +68,8 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_backward_kernel(const M
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
+    pdl_trigger();
     const unsigned tmem = sh.tmem_base;
     const int step_k[2] = {kMlpH3, kMlpH2};
     const bool want_feat = p.grad_feat[e] != nullptr;

@@ -43,6 +43,8 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_forward_kernel(const Ml
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
+    pdl_trigger();
     const unsigned tmem = sh.tmem_base;
     const int layer_k[3] = {kMlpIn, kMlpH1, kMlpH2};
     const int layer_n[3] = {kMlpH1, kMlpH2, kMlpH3};

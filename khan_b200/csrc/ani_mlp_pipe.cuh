@@ -261,16 +261,18 @@ __device__ __forceinline__ void pipe_produce(MlpShared& sh, int nchunks, PipeSta
 
 // Packs the weights of the four elements into the stage layout (both products that read them:
 // forward B[n = out][k = in] = W[k][n], backward B[n = in][k = out] = W[n][k]), high and low tf32
-// parts.  grid = (kPackChunks, 4 elements); run once per weight update.
+// parts; one CTA per (chunk, element), once per weight update.  2.4 MB read, 4.9 MB written: bound by
+// latency, so a thread moves four values of K at a time with 16-byte stores (a core matrix per 8 lanes);
+// reads are rows of 128 consecutive values (forward) or 64-byte pieces of rows (backward).  One value at a
+// time along K, with 512 bytes between the lanes of a read, took 8.7 us.
 struct MlpPackParams {
     const float* w1[kTypes];   // [384][128]
     const float* w2[kTypes];   // [128][128]
     const float* w3[kTypes];   // [128][64]
     unsigned char* packed[kTypes];
 };
-__global__ void __launch_bounds__(kMlpThreads) mlp_pack_kernel(const MlpPackParams p)
+__device__ __forceinline__ void pack_chunk(const MlpPackParams& p, int chunk, int e)
 {
-    const int e = blockIdx.y, chunk = blockIdx.x;
     if (!p.packed[e]) return;
     const float* w;
     int ld, k0, n0, rows;
@@ -286,16 +288,25 @@ __global__ void __launch_bounds__(kMlpThreads) mlp_pack_kernel(const MlpPackPara
     }
     unsigned char* hi = p.packed[e] + (size_t)chunk * kPackedChunkBytes;
     unsigned char* lo = hi + kPipeOperandBytes;
-    for (int idx = threadIdx.x; idx < kMlpTile * kPipeK; idx += kMlpThreads) {
-        const int n = idx / kPipeK, k = idx % kPipeK;
-        float v = 0.0f;
-        if (n < rows) v = transposed ? w[(size_t)(k0 + k) * ld + n0 + n] : w[(size_t)(n0 + n) * ld + k0 + k];
-        const float h = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
-        const int off = pipe_offset(n, k);
-        *reinterpret_cast<float*>(hi + off) = h;
-        *reinterpret_cast<float*>(lo + off) = v - h;
+    const bool aligned = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+    for (int idx = threadIdx.x; idx < kMlpTile * kPipeK / 4; idx += blockDim.x) {
+        // transposed: consecutive lanes = consecutive n; else 8 rows x 4 groups of K per warp
+        const int n = transposed ? idx & 127 : (idx >> 6) * 8 + (idx & 7);
+        const int k = 4 * (transposed ? idx >> 7 : (idx >> 3) & 7);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (n < rows) {
+            if (transposed) {
+                const float* s = w + (size_t)(k0 + k) * ld + n0 + n;
+                v = make_float4(s[0], s[ld], s[2 * ld], s[3 * ld]);
+            } else {
+                const float* s = w + (size_t)(n0 + n) * ld + k0 + k;
+                v = aligned ? *reinterpret_cast<const float4*>(s) : make_float4(s[0], s[1], s[2], s[3]);
+            }
+        }
+        pipe_store4<true>(hi, lo, pipe_offset(n, k), v);
     }
 }
+__global__ void __launch_bounds__(kMlpThreads) mlp_pack_kernel(const MlpPackParams p) { pack_chunk(p, blockIdx.x, blockIdx.y); }
 
 // MMA-warp side of the same product: waits (bounded) for each filled stage, issues its MMAs and
 // commits them to the stage's barrier.  `fresh` = overwrite the accumulator with the first chunk.

@@ -17,6 +17,8 @@
 #pragma once
 
 #include "ani_common.cuh"
+#include "ani_launch.cuh"
+#include "ani_mlp_pipe.cuh"
 
 namespace ani {
 
@@ -141,13 +143,10 @@ __device__ __forceinline__ void rank_tile(const int* __restrict__ types, int n_a
     }
 }
 
-// Single launch: grid = number of tiles.
-__global__ void __launch_bounds__(kSortThreads)
-    sort_single_kernel(const int* __restrict__ types, int n_atoms, int* __restrict__ scatter,
-                       int* __restrict__ gather, int* __restrict__ counts)
+// Tile `tile` of a single-launch sort.
+__device__ __forceinline__ void sort_tile(const int* __restrict__ types, int n_atoms, int tile, int* __restrict__ scatter,
+                                          int* __restrict__ gather, int* __restrict__ counts, int (*red)[kTypes])
 {
-    __shared__ int red[kSortWarps][kTypes];
-    const int tile = blockIdx.x;
     Count4 vb, vt;
     count_two_ranges(types, n_atoms, tile * kSortTile, &vb, &vt);
     const Count4 before = block_sum(vb, red);
@@ -157,6 +156,33 @@ __global__ void __launch_bounds__(kSortThreads)
         for (int g = 0; g < kTypes; g++) counts[g] = total.c[g];
     }
     rank_tile(types, n_atoms, tile, before, total, scatter, gather, red);
+}
+
+// Single launch: grid = number of tiles.
+__global__ void __launch_bounds__(kSortThreads)
+    sort_single_kernel(const int* __restrict__ types, int n_atoms, int* __restrict__ scatter,
+                       int* __restrict__ gather, int* __restrict__ counts)
+{
+    __shared__ int red[kSortWarps][kTypes];
+    pdl_wait();
+    pdl_trigger();
+    sort_tile(types, n_atoms, blockIdx.x, scatter, gather, counts, red);
+}
+
+// The same with the weight packing of a pass in the CTAs behind the tiles: the two have nothing to do with
+// one another, either is bound by latency (5 us and 3 us) and together they fill a wave of the device.
+__global__ void __launch_bounds__(kSortThreads)
+    sort_and_pack_kernel(const int* __restrict__ types, int n_atoms, int n_tiles, int* __restrict__ scatter,
+                         int* __restrict__ gather, int* __restrict__ counts, const MlpPackParams pack)
+{
+    __shared__ int red[kSortWarps][kTypes];
+    pdl_wait();     // no early trigger: the kernel writes weights
+    if ((int)blockIdx.x >= n_tiles) {
+        const int c = (int)blockIdx.x - n_tiles;
+        pack_chunk(pack, c % kPackChunks, c / kPackChunks);
+        return;
+    }
+    sort_tile(types, n_atoms, blockIdx.x, scatter, gather, counts, red);
 }
 
 // Large batches, first: per-tile element counts into scratch[tile][4].

@@ -8,8 +8,9 @@ atomic self energies, the gradient flattened atom by atom (x, y, z) in Hartree/B
 connection serves requests until the client closes it.
 
 The reference evaluates each request with a float64 CPU trainer through ``predict`` and
-``coordinate_gradients``; here the evaluator is any object with those two methods -- a
-``TrainerMultiTower`` on one GPU by default -- so the protocol can be tested without a GPU.
+``coordinate_gradients``; here the evaluator is any object with those two methods, so that the protocol can
+be tested without a GPU, or with ``energy_and_gradient``, which gives both from one evaluation -- a
+``TrainerMultiTower`` on one GPU by default.
 """
 from __future__ import annotations
 
@@ -39,9 +40,13 @@ def evaluate(evaluator, X) -> dict:
     types = arr[:, 0].astype(np.int64)
     if np.any(types != arr[:, 0]) or types.min() < 0 or types.max() > 3:
         raise ValueError("element ids must be 0 (H), 1 (C), 2 (N) or 3 (O)")
-    rd = RawDataset([arr], [0.0])
-    energy = float(evaluator.predict(rd)[0]) + float(sum(SELF_ENERGY[t] for t in types))
-    gradient = np.asarray(list(evaluator.coordinate_gradients(rd))[0], dtype=np.float64).reshape(-1)
+    if hasattr(evaluator, "energy_and_gradient"):
+        energy, gradient = evaluator.energy_and_gradient(arr)
+    else:
+        rd = RawDataset([arr], [0.0])
+        energy, gradient = evaluator.predict(rd)[0], list(evaluator.coordinate_gradients(rd))[0]
+    energy = float(energy) + float(sum(SELF_ENERGY[t] for t in types))
+    gradient = np.asarray(gradient, dtype=np.float64).reshape(-1)
     return {"energy": energy, "gradient": [float(g) * BOHR for g in gradient]}
 
 

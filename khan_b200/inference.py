@@ -16,61 +16,59 @@ import torch
 
 from . import _lib
 from .model import activations
-from .staged import FEATURE_SIZE, StagedBatch
-
-
-def _ptr(t: torch.Tensor, offset_elems: int = 0):
-    return ctypes.c_void_p(t.data_ptr() + offset_elems * t.element_size())
+from .staged import StagedBatch
 
 
 class EnergyForces:
-    """Pre-allocated evaluator for one model (float32, the fused 384-128-128-64-1 networks)."""
+    """Pre-allocated evaluator for one model (the 384-128-128-64-1 networks, float32 or float64)."""
 
     def __init__(self, model, n_atoms: int, n_mols: int, device="cuda:0"):
-        if not model.fused:
-            raise ValueError("EnergyForces needs the fused float32 384-128-128-64-1 networks")
+        if not model.has_kernels:
+            raise ValueError("EnergyForces needs the fused 384-128-128-64-1 networks")
         self.model = model
         self.device = torch.device(device)
+        self.dtype = model.precision
+        self.f64 = self.dtype == torch.float64
         _lib.same_device(self.device, *model.get_parameters(), where="EnergyForces")
         self.act_id = activations.KERNEL_ID[model.activation_fn]
         self.split = bool(model.split_precision)
-        f32 = dict(dtype=torch.float32, device=self.device)
-        self.energy_sorted = torch.empty(n_atoms, **f32)
-        self.ones = torch.ones(n_atoms, **f32)
-        self.acts = [torch.empty((n_atoms, w), **f32) for w in (128, 128, 64)]
-        self.dacts = [torch.empty((n_atoms, w), **f32) for w in (128, 128, 64)]
-        self.dzs = [torch.empty((n_atoms, w), **f32) for w in (128, 128, 64)]
-        self.mol_energy = torch.zeros(n_mols, **f32)
+        real = dict(dtype=self.dtype, device=self.device)
+        self.energy_sorted = torch.empty(n_atoms, **real)
+        self.mol_energy = torch.zeros(n_mols, **real)
+        if not self.f64:      # what the tensor-core kernels hand from one to the next
+            self.ones = torch.ones(n_atoms, **real)
+            self.dacts = [torch.empty((n_atoms, w), **real) for w in (128, 128, 64)]
+            self.dzs = [torch.empty((n_atoms, w), **real) for w in (128, 128, 64)]
         self.n_atoms_cap, self.n_mols_cap = n_atoms, n_mols
 
-    def _weights(self, t: int):
-        ann = self.model.anns[t]
-        return [w.detach() for w in ann.Ws], [b.detach() for b in ann.bs]
-
-    def _pass_args(self, sb: StagedBatch):
-        """The argument block of ``ani_network_pass_f32``: everything that does not change from batch to batch
-        is filled once (and again when the model's weights have moved), the batch's own fields per call."""
-        first = self.model.anns[0].Ws[0]
-        packed = self.model.packed_weights()
-        key = (first.data_ptr(), None if packed is None else packed.data_ptr())
-        if getattr(self, "_pa_key", None) != key:
-            a = _lib.PassArgs()
-            a.activation, a.split_precision = self.act_id, int(self.split)
-            a.energy_sorted, a.grad_energy_sorted = self.energy_sorted.data_ptr(), self.ones.data_ptr()
-            for name, bufs in (("act", self.acts), ("dact", self.dacts), ("dz", self.dzs)):
+    def _fixed_args(self, packed):
+        """A new argument block with everything that does not change from batch to batch."""
+        a = _lib.EnergyArgs64() if self.f64 else _lib.PassArgs()
+        a.activation = self.act_id
+        a.energy_sorted, a.mol_energy = self.energy_sorted.data_ptr(), self.mol_energy.data_ptr()
+        if not self.f64:
+            a.split_precision = int(self.split)
+            a.grad_energy_sorted = self.ones.data_ptr()
+            for name, bufs in (("dact", self.dacts), ("dz", self.dzs)):
                 for k, t in enumerate(bufs):
                     setattr(a, f"{name}{k + 1}", t.data_ptr())
-            a.mol_energy = self.mol_energy.data_ptr()
-            for t in range(4):
-                (w1, w2, w3, w4), (b1, b2, b3, b4) = self._weights(t)
-                for name, v in (("w1", w1), ("w2", w2), ("w3", w3), ("w4", w4), ("b1", b1), ("b2", b2), ("b3", b3),
-                                ("b4", b4)):
-                    getattr(a, name)[t] = v.data_ptr()
-                if packed is not None:
-                    a.packed[t] = packed[t].data_ptr()
-            self._pa, self._pa_key = a, key
+        for t, ann in enumerate(self.model.anns):
+            for k, (w, b) in enumerate(zip(ann.Ws, ann.bs)):
+                getattr(a, f"w{k + 1}")[t], getattr(a, f"b{k + 1}")[t] = w.data_ptr(), b.data_ptr()
+            if packed is not None:
+                a.packed[t] = packed[t].data_ptr()
+        return a
+
+    def _pass_args(self, sb: StagedBatch):
+        """The argument block of the pass: everything that does not change from batch to batch is filled once
+        (and again when the model's weights have moved), the batch's own fields per call."""
+        first = self.model.anns[0].Ws[0]
+        packed = None if self.f64 else self.model.packed_weights()
+        key = (first.data_ptr(), None if packed is None else packed.data_ptr())
+        if getattr(self, "_pa_key", None) != key:
+            self._pa, self._pa_key = self._fixed_args(packed), key
         a = self._pa
-        a.n_atoms, a.n_mols, a.acs_host = sb.n_atoms, sb.n_mols, sb.acs_host.ctypes.data
+        a.n_atoms, a.n_mols, a.acs_host = sb.n_atoms, sb.n_mols, sb.acs_ptr
         a.xs, a.ys, a.zs = sb.x.data_ptr(), sb.y.data_ptr(), sb.z.data_ptr()
         a.atomic_numbers, a.mol_offsets, a.mol_atom_counts = (sb.types.data_ptr(), sb.mol_offsets.data_ptr(),
                                                               sb.mol_counts.data_ptr())
@@ -80,39 +78,89 @@ class EnergyForces:
         a.x_grads, a.y_grads, a.z_grads = g, g + cap * esz, g + 2 * cap * esz
         return a
 
+    def _call(self, sb: StagedBatch, phases: int, stream, where: str) -> None:
+        if sb.n_atoms > self.n_atoms_cap or sb.n_mols > self.n_mols_cap or sb.dtype != self.dtype:
+            raise ValueError("batch does not fit this evaluator")
+        _lib.same_device(self.device, sb.features, sb.x, where=where)
+        if stream is None:
+            stream = torch.cuda.current_stream(self.device).cuda_stream
+        if self.f64:
+            phases &= ~_lib.PASS_PACK
+        elif self.model.packed_weights() is None:
+            self.model.pack_weights(ctypes.c_void_p(stream) if isinstance(stream, int) else stream)   # allocates the packed copy (first use)
+            phases &= ~_lib.PASS_PACK
+        a = self._pass_args(sb)
+        a.phases = phases
+        if self.f64:
+            _lib.check(_lib.lib().ani_energy_pass_f64(ctypes.byref(a), stream), "ani_energy_pass_f64")
+        else:
+            _lib.check(_lib.lib().ani_network_pass_f32(ctypes.byref(a), stream), "ani_network_pass_f32")
+
     def featurize(self, sb: StagedBatch, stream: ctypes.c_void_p | None = None) -> None:
         """Sort + featurize of the batch staged in ``sb`` only (one C-ABI call): they need nothing but the
         coordinates, so a caller may run them for the NEXT batch on another stream beside the network kernels
         of this one and then call ``run(..., featurized=True)``."""
-        if sb.n_atoms > self.n_atoms_cap or sb.n_mols > self.n_mols_cap or sb.dtype != torch.float32:
-            raise ValueError("batch does not fit this evaluator")
-        _lib.same_device(self.device, sb.features, sb.x, where="EnergyForces.featurize")
-        if stream is None:
-            stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
-        a = self._pass_args(sb)
-        a.phases = _lib.PASS_FEATURIZE
-        _lib.check(_lib.lib().ani_network_pass_f32(ctypes.byref(a), stream), "ani_network_pass_f32")
+        self._call(sb, _lib.PASS_FEATURIZE, stream, "EnergyForces.featurize")
 
     def run(self, sb: StagedBatch, stream: ctypes.c_void_p | None = None, pack: bool = True,
             forces: bool = True, featurized: bool = False) -> None:
-        """One pass over the batch staged in ``sb`` -- one C-ABI call (``ani_network_pass_f32``).  Afterwards
+        """One pass over the batch staged in ``sb`` -- one C-ABI call (``ani_network_pass_f32`` or
+        ``ani_energy_pass_f64``).  Afterwards
         ``self.mol_energy[:sb.n_mols]`` holds the molecule energies and ``sb.grads[:, :sb.n_atoms]`` dE/dx,
         dE/dy, dE/dz (forces are their negatives).  ``pack=False`` skips the refresh of the pre-packed
         weights: for a caller that packed them (``model.pack_weights``) after the last change of the
         weights, e.g. once before a series of passes that run side by side on several streams.
         ``forces=False`` stops after the molecule energies (``predict``); ``featurized=True`` leaves sort +
         featurize out (``featurize`` has run for this batch)."""
-        if sb.n_atoms > self.n_atoms_cap or sb.n_mols > self.n_mols_cap or sb.dtype != torch.float32:
-            raise ValueError("batch does not fit this evaluator")
-        _lib.same_device(self.device, sb.features, sb.x, where="EnergyForces.run")
-        if stream is None:
-            stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
-        if self.model.packed_weights() is None:
-            self.model.pack_weights(stream)          # allocates the packed copy (first use)
-            pack = False
-        a = self._pass_args(sb)
-        a.phases = ((_lib.PASS_PACK if pack else 0) | (0 if featurized else _lib.PASS_FEATURIZE) | _lib.PASS_FORWARD
-                    | _lib.PASS_ENERGY | ((_lib.PASS_BACKWARD | _lib.PASS_COORD_GRAD) if forces else 0))
-        _lib.check(_lib.lib().ani_network_pass_f32(ctypes.byref(a), stream), "ani_network_pass_f32")
+        self._call(sb, (_lib.PASS_PACK if pack else 0) | (0 if featurized else _lib.PASS_FEATURIZE) | _lib.PASS_FORWARD
+                   | _lib.PASS_ENERGY | _lib.PASS_TRANSIENT
+                   | ((_lib.PASS_BACKWARD | _lib.PASS_COORD_GRAD) if forces else 0), stream, "EnergyForces.run")
 
     KERNELS_PER_PASS = 7   # weight packing (unless pack=False), sort, featurize, mlp forward, molecule sums, mlp backward, featurize_grad
+
+
+class SingleGeometry:
+    """Energy and gradient of one geometry at a time (the energy server's request): the inputs cross in one
+    copy from a pinned arena, the results in one copy back, and nothing is allocated per call.  Calls must not
+    overlap."""
+
+    def __init__(self, model, capacity: int, device):
+        self.capacity = capacity
+        self.batch = StagedBatch(capacity, 1, model.precision, device=device)
+        self.evaluator = EnergyForces(model, capacity, 1, device=device)
+        size = self.batch.xyz.element_size()
+        nbytes = 3 * capacity * size + 4 * capacity + 8      # x, y, z | elements | offset, count of the molecule
+        self.host_in = torch.zeros(nbytes, dtype=torch.uint8).pin_memory()
+        self.dev_in = torch.zeros(nbytes, dtype=torch.uint8, device=device)
+
+        def views(arena):
+            ints = arena[3 * capacity * size:].view(torch.int32)
+            return arena[:3 * capacity * size].view(model.precision).view(3, capacity), ints[:capacity], ints[capacity:]
+
+        xyz, types, table = views(self.host_in)
+        self._xyz, self._types, self._table = xyz.numpy(), types.numpy(), table.numpy()
+        b = self.batch
+        b.xyz, b.types, table = views(self.dev_in)
+        b.x, b.y, b.z = b.xyz[0], b.xyz[1], b.xyz[2]
+        b.mol_offsets, b.mol_counts = table[:1], table[1:]
+        # the gradient (padded to the capacity) and the energy in one array each side
+        self.dev_out = torch.zeros(3 * capacity + 1, dtype=model.precision, device=device)
+        self.host_out = torch.zeros(3 * capacity + 1, dtype=model.precision).pin_memory()
+        self._out = self.host_out.numpy()
+        b.grads = self.dev_out[:3 * capacity].view(3, capacity)
+        self.evaluator.mol_energy = self.dev_out[3 * capacity:]
+
+    def evaluate(self, arr):
+        """``arr``: float64 ``(n, 4)`` array, n up to the capacity.  Returns (energy, (n, 3) gradient)."""
+        n, b = len(arr), self.batch
+        self._xyz[:, :n] = arr[:, 1:].T
+        self._types[:n] = arr[:, 0]
+        self._table[1] = n
+        b.set_shape(n, 1, np.bincount(self._types[:n], minlength=4))
+        with torch.cuda.device(b.device):
+            stream = torch.cuda.current_stream()
+            self.dev_in.copy_(self.host_in, non_blocking=True)
+            self.evaluator.run(b, stream=stream.cuda_stream)
+            self.host_out.copy_(self.dev_out, non_blocking=True)
+            stream.synchronize()
+        return float(self._out[-1]), self._out[:-1].reshape(3, self.capacity)[:, :n].T.copy()

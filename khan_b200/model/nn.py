@@ -291,9 +291,15 @@ class MoleculeNN:
         return getattr(self, "_packed", None)
 
     @property
+    def has_kernels(self) -> bool:
+        """The architecture of the hand-written network kernels: in float32 all of them, in float64 the one
+        that evaluates energies and their gradient (``ani_energy_pass_f64``)."""
+        return (self.layer_sizes == FUSED_LAYERS and len(self.anns) == 4
+                and self.activation_fn in activations.KERNEL_ID)
+
+    @property
     def fused(self) -> bool:
-        return (self.precision == torch.float32 and self.layer_sizes == FUSED_LAYERS
-                and len(self.anns) == 4 and self.activation_fn in activations.KERNEL_ID)
+        return self.precision == torch.float32 and self.has_kernels
 
     def atom_energies_sorted(self, features: torch.Tensor, acs) -> torch.Tensor:
         """Energies in element-sorted order from the ``[n_atoms, F]`` feature buffer laid out H

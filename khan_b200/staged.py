@@ -49,6 +49,7 @@ class StagedBatch:
         self.grads = torch.empty((3, n_atoms), dtype=dtype, device=d)
         self.acs_host = np.zeros(4, np.int32)
         self._acs_ptr = self.acs_host.ctypes.data_as(_lib.c_int_p)
+        self.acs_ptr = self.acs_host.ctypes.data      # the same as a plain address
 
     # -- host -> device --------------------------------------------------------------------
     def set_shape(self, n_atoms: int, n_mols: int, acs_host) -> None:

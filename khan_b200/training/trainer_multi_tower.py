@@ -18,12 +18,14 @@ from __future__ import annotations
 import ctypes
 import itertools
 import os
+import threading
 import time
 
 import numpy as np
 import torch
 
 from .. import _lib, ani_mod
+from ..data.dataset import RawDataset
 from ..data.feeder import BatchFeeder, PackedDataset
 from ..model import activations
 from ..model.nn import MoleculeNN
@@ -166,6 +168,7 @@ class TrainerMultiTower:
         self.train_op_forces = _Op("train_op_forces")  # exp(force rmse)
         self.max_norm_ops = _Op("max_norm_ops")
         self._device_l2s = _Op("_device_l2s")          # squared errors left on the device (no host wait)
+        self._single, self._single_lock = None, threading.Lock()   # evaluator of energy_and_gradient
         self._fused = None                              # (capacity, StagedBatch, FusedTrainStep) of the fused path
 
     # ------------------------------------------------------------------ bookkeeping
@@ -573,7 +576,7 @@ class TrainerMultiTower:
 
     def coordinate_gradients(self, dataset, batch_size=1024, use_evaluator=True):
         """Per-molecule ``(n, 3)`` gradients of the predicted energy
-        (``trainer_multi_tower.py:580-614``).  On one float32 tower with the fused networks the
+        (``trainer_multi_tower.py:580-614``).  On one tower with the networks that have kernels the
         batches go through the allocation-free evaluator (``khan_b200.inference.EnergyForces``: C-ABI
         calls only, no host wait per batch); ``use_evaluator=False`` forces the autograd path."""
         # an iterator, as in the reference; the per-batch lists are chained in C, so a molecule costs no
@@ -591,10 +594,13 @@ class TrainerMultiTower:
                 yield _split_rows(np.stack(grads[k], axis=1), mos[k])
 
     def _evaluator_usable(self, dataset) -> bool:
-        """One float32 CUDA tower with the fused networks: batches can go through the
+        """One CUDA tower with the networks that have kernels: batches can go through the
         allocation-free evaluator (``khan_b200.inference.EnergyForces``)."""
-        return (self.num_towers == 1 and self.precision == torch.float32 and self.model.fused
-                and self.towers[0].type == "cuda" and dataset.num_mols() > 0)
+        return (self.num_towers == 1 and self.model.has_kernels and self.towers[0].type == "cuda"
+                and dataset.num_mols() > 0)
+
+    def _np_dtype(self):
+        return np.float32 if self.precision == torch.float32 else np.float64
 
     def _evaluator(self, packed, batch_size):
         from ..inference import EnergyForces
@@ -603,21 +609,22 @@ class TrainerMultiTower:
         dev = self.towers[0]
         cached = getattr(self, "_infer", None)
         if cached is None or cached[0][0] < cap_atoms or cached[0][1] < cap_mols:
-            self._infer = cached = ((cap_atoms, cap_mols), StagedBatch(cap_atoms, cap_mols, device=dev),
+            self._infer = cached = ((cap_atoms, cap_mols), StagedBatch(cap_atoms, cap_mols, self.precision, device=dev),
                                     EnergyForces(self.model, cap_atoms, cap_mols, device=dev))
         return cached[1], cached[2]
 
     def _evaluator_predictions(self, dataset, batch_size):
         """``_device_predictions`` through the evaluator: sort, featurize, networks forward and the
         molecule sums as four C-ABI calls per batch, the weights packed once."""
-        packed = PackedDataset.from_raw(dataset, np.float32)
+        packed = PackedDataset.from_raw(dataset, self._np_dtype())
         sb, ev = self._evaluator(packed, batch_size)
         dev = self.towers[0]
         # two batches at a time: sort + featurize of the next one on a side stream beside the networks of this one
         twin = getattr(self, "_infer_twin", None)
         if twin is None or twin[0].n_atoms_cap < sb.n_atoms_cap or twin[0].n_mols_cap < sb.n_mols_cap:
             from ..staged import StagedBatch
-            twin = self._infer_twin = (StagedBatch(sb.n_atoms_cap, sb.n_mols_cap, device=dev), torch.cuda.Stream(device=dev))
+            twin = self._infer_twin = (StagedBatch(sb.n_atoms_cap, sb.n_mols_cap, self.precision, device=dev),
+                                       torch.cuda.Stream(device=dev))
         sbs, side = (sb, twin[0]), twin[1]
         it = BatchFeeder(packed, batch_size, False, None, devices=self.towers, depth=3, hold=2)
         preds, l2s = [], []
@@ -653,12 +660,12 @@ class TrainerMultiTower:
         """Gradients of all molecules through the evaluator, one list per batch.  The result of a batch is copied to a pinned
         host buffer behind its kernels, and the host cuts the PREVIOUS batch into per-molecule arrays while
         the GPU works on this one (cutting 32,768 molecules takes as long as computing them)."""
-        packed = PackedDataset.from_raw(dataset, np.float32)
+        packed = PackedDataset.from_raw(dataset, self._np_dtype())
         sb, ev = self._evaluator(packed, batch_size)
         cap = sb.n_atoms_cap
         ring = getattr(self, "_grad_ring", None)
         if ring is None or ring[0].shape[0] < cap:
-            ring = self._grad_ring = [torch.empty((cap, 3), dtype=torch.float32).pin_memory() for _ in range(3)]
+            ring = self._grad_ring = [torch.empty((cap, 3), dtype=self.precision).pin_memory() for _ in range(3)]
         it = BatchFeeder(packed, batch_size, False, None, devices=self.towers, depth=2, hold=1)
         pending = []      # (host buffer, event, n_atoms, batch index) of batches whose copy is in flight
         slices = packed.batch_slices(batch_size)
@@ -686,6 +693,20 @@ class TrainerMultiTower:
             it.close()
         for entry in pending:
             yield finished(entry)
+
+    def energy_and_gradient(self, X):
+        """Energy and ``(n, 3)`` gradient of ONE geometry ``[[type, x, y, z], ...]``: what ``predict`` and
+        ``coordinate_gradients`` give for a data set of that molecule, from one evaluation.  With the networks
+        that have kernels it is one copy in, one C-ABI call and one copy out."""
+        arr = np.asarray(X, dtype=np.float64)
+        rd = RawDataset([arr], [0.0])
+        if not self._evaluator_usable(rd) or not len(arr):
+            return float(self.predict(rd)[0]), np.asarray(next(iter(self.coordinate_gradients(rd))))
+        with self._single_lock:
+            if self._single is None or self._single.capacity < len(arr):
+                from ..inference import SingleGeometry
+                self._single = SingleGeometry(self.model, 1 << max(6, (len(arr) - 1).bit_length()), self.towers[0])
+            return self._single.evaluate(arr)
 
     def eval_abs_rmse(self, dataset, batch_size=1024):
         """Absolute RMSE of the energies in kcal/mol (``trainer_multi_tower.py:560-578``)."""

@@ -173,3 +173,34 @@ def test_packed_and_unpacked_weight_paths_agree(monkeypatch):
     assert torch.equal(f0, f1)
     for a, b in zip(g0, g1):
         assert (a - b).abs().max().item() <= 1e-5 * b.abs().max().item()
+
+
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+@pytest.mark.parametrize("n_mols,heavy", [(1, 1), (1, 8), (7, 2), (40, 8), (90, 8)])
+def test_few_atom_networks_match_the_autograd_path(precision, n_mols, heavy):
+    """The 16-atom-tile kernel (float64: any size; float32: up to a limit that 90 molecules exceed): energies
+    and coordinate gradients against the dense differentiable path, tiles of 1 to 16 atoms, absent elements."""
+    import torch
+    from khan_b200 import RawDataset, TrainerMultiTower
+    from khan_b200.model import activations
+    from khan_b200.data import synthetic as syn
+    mols = syn.gdb_like_batch(n_mols, seed=n_mols, heavy_min=heavy, heavy_max=heavy).molecules()
+    ds = RawDataset(mols)
+    for act in (activations.celu, activations.gaussian, activations.normal, activations.softplus):
+        tr = TrainerMultiTower(None, [torch.device("cuda", 0)], precision=precision, layer_sizes=(128, 128, 64, 1),
+                               activation_fn=act, seed=3)
+        got_e, got_g = np.array(tr.predict(ds)), np.concatenate(list(tr.coordinate_gradients(ds)))
+        dense = TrainerMultiTower(None, [torch.device("cuda", 0)], precision="float64", layer_sizes=(128, 128, 64, 1),
+                                  activation_fn=act, seed=3)
+        with torch.no_grad():      # the same (float32) weights in the dense double-precision path
+            for a, b in zip(dense.parameters, tr.parameters):
+                a.copy_(b)
+        dense._evaluator_usable = lambda dataset: False
+        want_e = np.array(dense.predict(ds))
+        want_g = np.concatenate(list(dense.coordinate_gradients(ds, use_evaluator=False)))
+        tol = 1e-4 if precision == "float32" else 1e-10
+        assert np.abs(got_e - want_e).max() <= tol * np.abs(want_e).max()
+        assert np.abs(got_g - want_g).max() <= tol * np.abs(want_g).max()
+        e1, g1 = tr.energy_and_gradient(mols[0])
+        assert abs(e1 - want_e[0]) <= tol * np.abs(want_e).max()
+        assert np.abs(g1 - want_g[:len(mols[0])]).max() <= tol * np.abs(want_g).max()
