@@ -14,8 +14,8 @@
 //      pass T needs; the per-element counts fall out of the same ballots;
 //   R. radial features of the whole round, lane = (central atom, pair of shifts): every lane walks
 //      the radial list of its central atom and adds to the sum of the neighbour's element.
-// A central atom with more than 32 angular or 64 radial neighbours goes through the streaming
-// routine of ani_featurize.cuh.  A CTA takes the rounds r, r + R0, r + 2 R0, ... of its molecule
+// When a radial list is full (64 entries), pass R works it off and the scan goes on; a central atom with more
+// than 32 angular neighbours goes through the streaming routine of ani_featurize.cuh.  A CTA takes the rounds r, r + R0, r + 2 R0, ... of its molecule
 // (R0 rounds per molecule in the grid, chosen by the host from the mean molecule size), so molecules
 // of any size are covered.  Nothing is accumulated with atomics; rows need no zero fill by the caller.
 //
@@ -33,7 +33,7 @@ constexpr int kLargeCapR = 64;   // radial neighbours kept per central atom
 constexpr int kLargeCapA = 32;   // angular neighbours kept per central atom (one ballot sort covers 32 entries)
 
 template <typename T> struct LargeFwdWarpShared {
-    MolAngularShared<T, kLargeCapA, kLargeCapR> ang;   // its radial lists are in arrival order
+    MolAngularShared<T, kMolCentrals * kLargeCapA, kLargeCapA, kLargeCapR> ang;   // its radial lists are in arrival order
     unsigned char rad_t[kMolCentrals][kLargeCapR];   // element of that neighbour
     unsigned char ang_t[kMolCentrals * kLargeCapA];    // element of each angular neighbour before the sort
     int cnt_r[kMolCentrals];
@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
             ws.ang.ang_fc[0] = (T)0;
         }
         if (lane < kMolCentrals * kTypes) ws.ang.cnt_a[lane] = 0;
+        if (lane < kMolCentrals) ws.ang.list_base[lane] = lane * kLargeCapA;
 
         // ---- the central atoms: coordinates to all lanes, rows, zero fill of the angular blocks ----
         T xi[kMolCentrals], yi[kMolCentrals], zi[kMolCentrals];
@@ -103,14 +104,19 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
 
         // ---- A: scan, 32 candidates at a time against all central atoms of the round ----
         int cA[kMolCentrals] = {0, 0, 0, 0}, cR[kMolCentrals] = {0, 0, 0, 0};
+        int j0 = 0;
+        bool again = false;   // pass R has written the rows once: it adds from now on
+        do {
         T qx, qy, qz;   // the next 32 candidates are requested before this chunk's arithmetic
         int qt;
         {
-            const int gj = base + (lane < n ? lane : 0);
+            const int gj = base + (j0 + lane < n ? j0 + lane : 0);
             qx = xs[gj]; qy = ys[gj]; qz = zs[gj];
             qt = types[gj];
         }
-        for (int j0 = 0; j0 < n; j0 += kWarp) {
+        for (; j0 < n; j0 += kWarp) {
+            const int had_r[kMolCentrals] = {cR[0], cR[1], cR[2], cR[3]};
+            const int had_a[kMolCentrals] = {cA[0], cA[1], cA[2], cA[3]};
             const int j = j0 + lane;
             const bool live = j < n;
             const T px = qx, py = qy, pz = qz;
@@ -150,38 +156,17 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
                 cR[g] += __popc(mR);
                 cA[g] += __popc(mA);
             }
+            if (max(max(cR[0], cR[1]), max(cR[2], cR[3])) > kLargeCapR) {   // this chunk comes again after pass R
+#pragma unroll
+                for (int g = 0; g < kMolCentrals; g++) {
+                    cR[g] = had_r[g];
+                    cA[g] = had_a[g];
+                }
+                break;
+            }
         }
         __syncwarp();
 
-        // ---- S: each angular list into element order; denser neighbourhoods stream ----
-#pragma unroll
-        for (int g = 0; g < kMolCentrals; g++) {
-            if ((skip >> g) & 1u) continue;
-            if (cA[g] > kLargeCapA || cR[g] > kLargeCapR) {
-                featurize_atom_streaming<T>(xs, ys, zs, types, base, n, ci[g], ws.ang.row[g]);
-                skip |= 1u << g;
-                __syncwarp();
-                continue;
-            }
-            const bool have = lane < cA[g];
-            const int p = g * kLargeCapA + (have ? lane : 0);
-            const Vec4<T> u = ws.ang.ang_u[p];
-            const T fc = ws.ang.ang_fc[p];
-            const int t = have ? ws.ang_t[p] : kTypes;
-            const unsigned m0 = __ballot_sync(kFull, t == 0), m1 = __ballot_sync(kFull, t == 1),
-                           m2 = __ballot_sync(kFull, t == 2), m3 = __ballot_sync(kFull, t == 3);
-            const int c0 = __popc(m0), c1 = __popc(m1), c2 = __popc(m2);
-            const unsigned mine = t == 0 ? m0 : (t == 1 ? m1 : (t == 2 ? m2 : m3));
-            const int start = t == 0 ? 0 : (t == 1 ? c0 : (t == 2 ? c0 + c1 : c0 + c1 + c2));
-            __syncwarp();   // every entry has been read
-            if (have) {
-                const int q = g * kLargeCapA + start + __popc(mine & lanemask_lt());
-                ws.ang.ang_u[q] = u;
-                ws.ang.ang_fc[q] = fc;
-            }
-            if (lane == 0)
-                *reinterpret_cast<int4*>(&ws.ang.cnt_a[g * kTypes]) = make_int4(c0, c1, c2, __popc(m3));
-        }
         if (lane < kMolCentrals) ws.cnt_r[lane] = 0;
         __syncwarp();
 #pragma unroll
@@ -212,13 +197,50 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
             if (!((skip >> g) & 1u)) {
                 T* row = ws.ang.row[g];
 #pragma unroll
-                for (int t = 0; t < kTypes; t++)
-                    *reinterpret_cast<Vec2<T>*>(row + t * kNumRs + 2 * sp) = Vec2<T>{acc[t].x, acc[t].y};
+                for (int t = 0; t < kTypes; t++) {
+                    Vec2<T>* at = reinterpret_cast<Vec2<T>*>(row + t * kNumRs + 2 * sp);
+                    const Vec2<T> had = again ? *at : Vec2<T>{(T)0, (T)0};
+                    *at = Vec2<T>{had.x + acc[t].x, had.y + acc[t].y};
+                }
             }
+        }
+        again = true;
+#pragma unroll
+        for (int g = 0; g < kMolCentrals; g++) cR[g] = 0;
+        __syncwarp();
+        } while (j0 < n);
+
+        // ---- S: each angular list into element order; denser neighbourhoods stream ----
+#pragma unroll
+        for (int g = 0; g < kMolCentrals; g++) {
+            if ((skip >> g) & 1u) continue;
+            if (cA[g] > kLargeCapA) {
+                featurize_atom_streaming<T>(xs, ys, zs, types, base, n, ci[g], ws.ang.row[g]);
+                skip |= 1u << g;
+                __syncwarp();
+                continue;
+            }
+            const bool have = lane < cA[g];
+            const int p = g * kLargeCapA + (have ? lane : 0);
+            const Vec4<T> u = ws.ang.ang_u[p];
+            const T fc = ws.ang.ang_fc[p];
+            const int t = have ? ws.ang_t[p] : kTypes;
+            const unsigned m0 = __ballot_sync(kFull, t == 0), m1 = __ballot_sync(kFull, t == 1),
+                           m2 = __ballot_sync(kFull, t == 2), m3 = __ballot_sync(kFull, t == 3);
+            const int c0 = __popc(m0), c1 = __popc(m1), c2 = __popc(m2);
+            const unsigned mine = t == 0 ? m0 : (t == 1 ? m1 : (t == 2 ? m2 : m3));
+            const int start = t == 0 ? 0 : (t == 1 ? c0 : (t == 2 ? c0 + c1 : c0 + c1 + c2));
+            __syncwarp();   // every entry has been read
+            if (have) {
+                const int q = g * kLargeCapA + start + __popc(mine & lanemask_lt());
+                ws.ang.ang_u[q] = u;
+                ws.ang.ang_fc[q] = fc;
+            }
+            if (lane == 0)
+                *reinterpret_cast<int4*>(&ws.ang.cnt_a[g * kTypes]) = make_int4(c0, c1, c2, __popc(m3));
         }
         __syncwarp();
 
-        constexpr int kRoundCapA = kLargeCapA;
 #include "ani_featurize_round_passes.inl"
     }
 }

@@ -12,7 +12,9 @@
 //      is compacted in lane order comes out sorted by element for free;
 //   A. per central atom of the round (coordinates by shuffle): one distance per lane; (r, f_C)
 //      of every atom of the molecule goes to a table (f_C = 0 beyond R_Rc), and the neighbours
-//      within A_Rc, compacted by a ballot, to the list (unit vector, r, f_C) of this central atom;
+//      within A_Rc, compacted by a ballot, to the list (unit vector, r, f_C) of this central atom.  The
+//      lists of the round share 96 entries: an atom whose list does not fit any more waits until T, B
+//      and C have worked off the ones before it (31 neighbours of one atom always fit);
 //   R. the radial features of all central atoms of the round at once: lane = (central atom,
 //      pair of radial shifts) walks the table of its central atom.  The table is in element
 //      order for every central atom alike, so the loops over the four element runs are uniform
@@ -31,8 +33,10 @@
 // not depend on the launch shape.
 //
 // A molecule with more than 32 atoms met by this kernel (the host picks it from the MEAN
-// molecule size) and a central atom with more than 24 neighbours within A_Rc go through the
-// streaming routine of ani_featurize.cuh.
+// molecule size) goes through the streaming routine of ani_featurize.cuh.  (With 24 fixed entries per
+// central atom a denser atom streamed too.  One in a few batches of 1024 molecules has such an atom, and a
+// lone warp then worked on it for 30 us (float) to 140 us (double) after everything else had ended: the
+// three operators on 1024 molecules took 104 / 317 us with one, 70 / 178 us without.)
 //
 // Computes what featurize_cpu of the reference computes (gpu_featurizer/kernel_cpu.cpp:406-537).
 #pragma once
@@ -46,17 +50,20 @@ namespace ani {
 
 constexpr int kMolMaxAtoms = 32;       // molecules up to this size take the fast path
 constexpr int kMolCentrals = 4;        // central atoms per round
-constexpr int kMolCapA = 24;           // angular neighbours kept per central atom
+constexpr int kMolPool = 96;           // angular neighbours of the central atoms worked on together
 constexpr int kMolGroupStride = 16;    // group id = central slot * 16 + element-pair bucket
 constexpr int kMolNoGroup = 0xff;      // id of the quads behind the last group
 constexpr int kMolSlotsPerLane = 1;    // slots a lane evaluates per pass B (2 was measured: no gain)
 constexpr int kMolChunk = kMolSlotsPerLane * kWarp;   // slots per pass B / C
 constexpr int kMolChunkStride = kMolChunk + 4;        // + 4 words: keeps the 16-byte reads of pass C conflict-free
 constexpr int kMolRounds = kMolMaxAtoms / kMolCentrals;   // rounds of the largest molecule of the fast path
-// padded slots of one central atom: at most CapA (CapA - 1) / 2 pairs + 3 per bucket, in quads
-constexpr int mol_quad_bytes(int cap_a)
+// padded slots of the central atoms worked on together, in quads: at most n (n - 1) / 2 pairs for n neighbours
+// and 3 per bucket, n <= cap each and <= pool in all (most pairs: as many lists of `cap` as fit)
+constexpr int mol_quad_bytes(int cap, int pool)
 {
-    return ((kMolCentrals * ((cap_a * (cap_a - 1) / 2 + 3 * kPairBuckets) / 4 + 1) + 2 * (kMolChunk / 4) + 7) / 8) * 8;
+    const int full = pool / cap < kMolCentrals ? pool / cap : kMolCentrals, rest = full < kMolCentrals ? pool - full * cap : 0;
+    const int pairs = full * (cap * (cap - 1) / 2) + rest * (rest - 1) / 2;
+    return (((pairs + 3 * kPairBuckets * kMolCentrals) / 4 + kMolCentrals + 2 * (kMolChunk / 4) + 7) / 8) * 8;
 }
 
 struct alignas(16) MolGroupInfo {
@@ -76,22 +83,22 @@ struct MolSortShared {
 
 // What the angular passes (T, B, C) of a round work on: the angular neighbour lists of the round's
 // central atoms (element order inside each list), the group table, the factor chunks and the rows.
-// CAPA = angular neighbours kept per central atom (at most 32: list indices are packed into 8 bits).
-template <typename T, int CAPA, int CAPR> struct MolAngularShared {
-    static constexpr int kCapA = CAPA;
-    Vec4<T> ang_u[kMolCentrals * CAPA];   // (x_i - x_j) / r_ij and r_ij, element order, per central atom
-    T ang_fc[kMolCentrals * CAPA];        // f_C(r_ij, A_Rc)
+// POOL = entries of the lists together, MAXA = longest list (list indices are packed into 8 bits).
+template <typename T, int POOL, int MAXA, int CAPR> struct MolAngularShared {
+    Vec4<T> ang_u[POOL];                  // (x_i - x_j) / r_ij and r_ij, element order, per central atom
+    T ang_fc[POOL];                       // f_C(r_ij, A_Rc)
     Vec2<T> rad[kMolCentrals][CAPR];      // (r_ij, f_C(r_ij, R_Rc)) per central atom: the radial pass reads it, not T / B / C
     alignas(16) T A[kNumThetas][kMolChunkStride];
     alignas(16) T BF[kNumARs][kMolChunkStride];
     MolGroupInfo tab[kMolCentrals * kMolGroupStride];
     T* row[kMolCentrals];                     // feature row of each central atom of the round
     alignas(16) int cnt_a[kMolCentrals * kTypes];   // angular neighbours per element, per central atom
-    alignas(8) unsigned char quad_gid[mol_quad_bytes(CAPA)];
+    int list_base[kMolCentrals];              // first entry of each central atom's list
+    alignas(8) unsigned char quad_gid[mol_quad_bytes(MAXA, POOL)];
 };
 
 template <typename T> struct MolFwdWarpShared {
-    MolAngularShared<T, kMolCapA, kMolMaxAtoms> ang;   // its radial table: every atom j of the molecule, f_C = 0 out of range
+    MolAngularShared<T, kMolPool, kMolMaxAtoms - 1, kMolMaxAtoms> ang;   // its radial table: every atom j of the molecule, f_C = 0 out of range
     MolSortShared sort;
 };
 
@@ -217,12 +224,15 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
         ws.ang.ang_u[0] = Vec4<T>{(T)1, (T)0, (T)0, (T)1};
         ws.ang.ang_fc[0] = (T)0;
     }
+    unsigned skip = 0;   // central atoms that are refused
+    int g = 0;
+    do {
     if (lane < kMolCentrals * kTypes) ws.ang.cnt_a[lane] = 0;
     __syncwarp();
 
-    // ---- A: scan, one central atom after another ----
-    unsigned skip = 0;   // central atoms that are finished (streaming routine) or refused
-    for (int g = 0; g < G; g++) {
+    // ---- A: scan, one central atom after another, as many as the lists have room for ----
+    int used = 0;
+    for (; g < G; g++) {
         const int c = round + g * n_rounds;
         const T xi = __shfl_sync(kFull, ml.x, c), yi = __shfl_sync(kFull, ml.y, c), zi = __shfl_sync(kFull, ml.z, c);
         const int ti = __shfl_sync(kFull, ml.type, c);
@@ -242,12 +252,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
         const bool in_rad = lane < n && lane != c && r < (T)kR_Rc;
         const bool in_ang = in_rad && r < (T)kA_Rc;
         const unsigned mA = __ballot_sync(kFull, in_ang);
-        if (__popc(mA) > kMolCapA) {   // denser than the list: the streaming routine does the whole row
-            featurize_atom_streaming<T>(xs, ys, zs, types, base, n, ws.sort.src[c], row);
-            skip |= 1u << g;
-            __syncwarp();
-            continue;
-        }
+        if (used + __popc(mA) > kMolPool) break;   // this central atom opens the next pass
         // the angular blocks start as zeros (16-byte stores: 2.5 per lane); pass C writes the blocks of
         // the element pairs that occur, after a __syncwarp, so the order of the two is fixed
         {
@@ -259,13 +264,18 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
         }
         ws.ang.rad[g][lane] = Vec2<T>{r, in_rad ? cutoff_value<T>(r, (T)kR_Rc) : (T)0};
         if (in_ang) {
-            const int p = g * kMolCapA + __popc(mA & lanemask_lt());
+            const int p = used + __popc(mA & lanemask_lt());
             ws.ang.ang_u[p] = Vec4<T>{dx * inv, dy * inv, dz * inv, r};
             ws.ang.ang_fc[p] = cutoff_value<T>(r, (T)kA_Rc);
         }
         if (lane < kTypes) ws.ang.cnt_a[g * kTypes + lane] = __popc(mA & ws.sort.tmask[lane]);
+        if (lane == 0) ws.ang.list_base[g] = used;
+        used += __popc(mA);
     }
     __syncwarp();
+
+#include "ani_featurize_round_passes.inl"
+    } while (g < G);
 
     // ---- R: radial features of the whole round, lane = (central atom, pair of shifts) ----
     {
@@ -294,9 +304,6 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
                 *reinterpret_cast<Vec2<T>*>(row + t * kNumRs + 2 * sp) = Vec2<T>{acc[t].x, acc[t].y};
         }
     }
-
-    constexpr int kRoundCapA = kMolCapA;
-#include "ani_featurize_round_passes.inl"
 }
 
 }  // namespace ani

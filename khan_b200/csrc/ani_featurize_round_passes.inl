@@ -2,7 +2,7 @@
 // shared state: from the angular lists and the per-element counts (ws.ang.cnt_a) of the round's central
 // atoms to the angular blocks of their feature rows.  A central atom with all counts zero contributes
 // nothing (its blocks keep the zeros written before).  Expects in scope: T, `ws` (a __shared__ object
-// with a MolAngularShared member `ang`), `lane`, and the constant kRoundCapA (the CAPA of ws.ang).
+// with a MolAngularShared member `ang`) and `lane`.
 // It is a fragment and not a function because the function form, although inlined, compiled to a
 // kernel that was 6 % slower (measured: 25.6 -> 27.3 us on a 1024-molecule batch).
 {
@@ -33,7 +33,8 @@
             MolGroupInfo e;
             e.off = off;
             e.cnt = cnt;
-            e.packed = (g * kRoundCapA + pick4(stv, ta)) | ((g * kRoundCapA + pick4(stv, tb)) << 8) | (nb << 16) |
+            const int first = ws.ang.list_base[g];
+            e.packed = (first + pick4(stv, ta)) | ((first + pick4(stv, tb)) << 8) | (nb << 16) |
                        ((ta == tb ? 1 : 0) << 24);
             e.recip = (unsigned)(65536.0f * __frcp_rn((float)nb)) + 1u;   // in [2^16 / nb, 2^16 / nb + 1.01)
             const int gid = g * kMolGroupStride + bk;
