@@ -492,6 +492,32 @@ typedef struct ani_pass_args {
 } ani_pass_args;
 int ani_network_pass_f32(const ani_pass_args* args, void* stream);
 
+/* One batch of force training: weight gradients of exp(sum over x, y, z of rmse(forces, targets)), the
+ * loss behind the reference's train_op_forces (khan/training/trainer_multi_tower.py:377-399, there a
+ * tf.gradients of a tf.gradients through FeaturizeGrad and FeaturizeGradInverse).  In order: the phases
+ * PACK and FEATURIZE of `pass` as requested, networks forward, backward to the features (from
+ * grad_energy_sorted = ones), coordinate gradients; the loss and its derivative v with respect to them;
+ * feature rates J v; the second-order pass through the networks; zero_ptr cleared; weight gradients added.
+ * Every buffer named below is required; packed weights are, too.  Launches only. */
+typedef struct ani_force_fit_args {
+    ani_pass_args pass;
+    const float *fx, *fy, *fz;       /* [n_atoms] target forces */
+    float *vx, *vy, *vz;             /* [n_atoms] */
+    float* feature_rates;            /* [n_atoms][384] */
+    float *r1, *r2;                  /* [n_atoms][128] */
+    float *adot1, *adot2, *adot3;    /* [n_atoms][128], [128], [64] */
+    float *q1, *q2, *q3;             /* [n_atoms][128], [128], [64] */
+    double* partial;                 /* [192] */
+    float* rmse;                     /* [1]: sum of the three rmses */
+    const float *z1, *z2, *z3;       /* pre-activations in plain float32 ([n_atoms][128], [128], [64], element-sorted), or
+                                        NULL: whose sign decides about celu's second derivative (other activations: unused) */
+    void* z_ready;                   /* cudaEvent_t after which they may be read, or NULL */
+} ani_force_fit_args;
+int ani_force_fit_pass_f32(const ani_force_fit_args* args, void* stream);
+/* Between two dense layers: z[rows][width] += the bias of the row's element (rows element-sorted, acs_host of
+ * each), a = celu(z) unless a is NULL.  width a multiple of 4. */
+int ani_bias_celu_f32(float* z, float* a, const float* const* bias_host4, const int* acs_host, int width, void* stream);
+
 /* Energies, and energies + forces, in double precision (the precision the reference serves in,
  * energy_server.py): the phases FEATURIZE, FORWARD, ENERGY, BACKWARD and COORD_GRAD of the above for
  * the 384-128-128-64-1 networks (FORWARD and BACKWARD together are one kernel; BACKWARD alone is refused),

@@ -18,7 +18,7 @@ CSRC = os.path.join(_HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(_HERE), "include")
 SOURCES = ["ani_b200.cu"]
 HEADERS = ["ani_params.h", "ani_common.cuh", "ani_device_math.cuh", "ani_feeder.h", "ani_peer.cuh", "ani_sort.cuh", "ani_featurize.cuh", "ani_featurize_mol.cuh", "ani_featurize_large.cuh", "ani_featurize_round_passes.inl", "ani_grad.cuh", "ani_grad_mol.cuh", "ani_grad_pair_pass.inl",
-           "ani_grad_inverse.cuh", "ani_mlp.cuh", "ani_mlp_pipe.cuh", "ani_mlp_forward.cuh", "ani_mlp_backward.cuh", "ani_mlp_wgrad.cuh", "ani_mlp_small.cuh", "ani_launch.cuh", "ani_charge.cuh", "ani_optim.cuh", "ani_energy.cuh", "ani_host_pack.h"]
+           "ani_grad_inverse.cuh", "ani_tangent_mol.cuh", "ani_mlp.cuh", "ani_mlp_pipe.cuh", "ani_mlp_forward.cuh", "ani_mlp_backward.cuh", "ani_mlp_wgrad.cuh", "ani_mlp_small.cuh", "ani_mlp_tangent.cuh", "ani_launch.cuh", "ani_charge.cuh", "ani_optim.cuh", "ani_energy.cuh", "ani_host_pack.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -91,6 +91,13 @@ class PassArgs(ctypes.Structure):
                 + [("zero_ptr", ctypes.c_void_p), ("zero_bytes", ctypes.c_size_t)])
 
 
+class ForceFitArgs(ctypes.Structure):
+    """``ani_force_fit_args`` of include/ani_b200.h."""
+    _fields_ = ([("pass_", PassArgs)]
+                + [(n, ctypes.c_void_p) for n in ("fx", "fy", "fz", "vx", "vy", "vz", "feature_rates", "r1", "r2", "adot1",
+                                                  "adot2", "adot3", "q1", "q2", "q3", "partial", "rmse", "z1", "z2", "z3", "z_ready")])
+
+
 class EnergyArgs64(ctypes.Structure):
     """``ani_energy_args_f64`` of include/ani_b200.h."""
     _fields_ = ([("phases", ctypes.c_int), ("n_atoms", ctypes.c_int), ("n_mols", ctypes.c_int),
@@ -145,6 +152,8 @@ SIGNATURES = {
     "ani_scale_by_loss_f32": (_i, [_vp, ctypes.c_longlong, _vp, _i, _i, _vp, _vp]),
     "ani_host_pack_batch": (_i, [_vp]),
     "ani_network_pass_f32": (_i, [ctypes.POINTER(PassArgs), _vp]),
+    "ani_force_fit_pass_f32": (_i, [ctypes.POINTER(ForceFitArgs), _vp]),
+    "ani_bias_celu_f32": (_i, [_vp, _vp, _vp, c_int_p, _i, _vp]),
     "ani_energy_pass_f64": (_i, [ctypes.POINTER(EnergyArgs64), _vp]),
     "ani_feeder_create": (_i, [_i, _vp, _i, ctypes.POINTER(_vp)]),
     "ani_feeder_begin": (_i, [_vp, _vp, ctypes.c_longlong, _i]),
@@ -211,7 +220,7 @@ def build_ops(force: bool = False) -> str:
         cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_torch_ops", OPS_SOURCE, "-o", OPS_PATH]
         cmd += ["-I" + d for d in cpp_extension.include_paths("cuda") + [sysconfig.get_paths()["include"]]]
         cmd += ["-L" + d for d in cpp_extension.library_paths("cuda")]
-        cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lcudart"]
+        cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lcudart", "-lcublas"]
         out = subprocess.run(cmd, capture_output=True, text=True)
         if out.returncode != 0:
             raise RuntimeError("g++ failed building _torch_ops.so:\n" + out.stderr)
@@ -228,7 +237,8 @@ def torch_ops():
             raise RuntimeError(f"{OPS_PATH} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
         from . import _torch_ops as mod
         mod.bind(*(ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in (
-            "ani_sort", "ani_featurize_f32", "ani_featurize_f64", "ani_featurize_grad_f32", "ani_featurize_grad_f64")))
+            "ani_sort", "ani_featurize_f32", "ani_featurize_f64", "ani_featurize_grad_f32", "ani_featurize_grad_f64",
+            "ani_bias_celu_f32")))
         _ops = mod
     return _ops
 

@@ -21,10 +21,12 @@
 #include "ani_grad.cuh"
 #include "ani_grad_mol.cuh"
 #include "ani_grad_inverse.cuh"
+#include "ani_tangent_mol.cuh"
 #include "ani_mlp_forward.cuh"
 #include "ani_mlp_backward.cuh"
 #include "ani_mlp_wgrad.cuh"
 #include "ani_mlp_small.cuh"
+#include "ani_mlp_tangent.cuh"
 #include "ani_charge.cuh"
 #include "ani_optim.cuh"
 #include "ani_energy.cuh"
@@ -366,6 +368,15 @@ int featurize_grad_inverse_impl(const T* xs, const T* ys, const T* zs, const int
     for (int t = 0; t < kTypes; t++)
         if (acs_host[t] > 0 && !outs[t]) return ANI_ERR_NULL_POINTER;
 
+    // small molecules with outputs that take 16-byte stores: rounds of four central atoms per warp
+    if (small_molecules(n_atoms, n_mols) && all_aligned16({oh, oc, on, oo}) &&
+        (long long)n_mols * kMolRounds <= 0x7fffffffLL) {
+        ANI_CUDA(launch_chain(featurize_tangent_mol_kernel<T>, n_mols * kMolRounds, kWarp, 0, (cudaStream_t)stream, 1, xs, ys,
+                              zs, types, mos, macs, n_mols, (int)n_atoms, sis, vx, vy, vz, oh, oc, on, oo, acs_host[0],
+                              acs_host[1], acs_host[2], acs_host[3]));
+        return ANI_OK;
+    }
+
     auto kernel = featurize_grad_inverse_kernel<T, kNW>;
     const size_t smem = kNW * sizeof(JvpWarpShared<T>);
     static thread_local int configured_dev = -1, cached_resident = 0;
@@ -474,8 +485,7 @@ template <bool SPLIT> int mlp_wgrad_launch(const MlpWgradParams& p, int n_ranges
         if (int rc = set_smem(kernel, smem)) return rc;
         configured_dev = dev;
     }
-    kernel<<<dim3(n_ranges, kWgradBlocks), kMlpAllThreads, smem, st>>>(p);
-    ANI_CUDA(cudaGetLastError());
+    ANI_CUDA(launch_chain(kernel, dim3(n_ranges, kWgradBlocks), kMlpAllThreads, smem, st, 1, p));
     return ANI_OK;
 }
 
@@ -561,6 +571,85 @@ int mlp_small_launch(const T* feat, const int* acs, const T* const* w1, const T*
     }
     ANI_CUDA(launch_chain(kernel, tiles * kSmallCtas, kSmallThreads, smem, st, kSmallCtas, p));
     return ANI_OK;
+}
+
+// Adds the weight gradients described by p (range fields are set here).
+int wgrad_call(MlpWgradParams& p, int split_precision, cudaStream_t st)
+{
+    // atoms per CTA: the smallest multiple of 64 for which the grid fits the SMs once (the
+    // kernels run one CTA per SM, so a second partial wave would double the time)
+    int dev = 0, sms = 0;
+    ANI_CUDA(cudaGetDevice(&dev));
+    ANI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int range = 256;
+    for (;; range += 64) {
+        long long ctas = 0;
+        for (int t = 0; t < kTypes; t++) ctas += (p.count[t] + range - 1) / range;
+        if (ctas * kWgradBlocks <= sms || range >= (1 << 20)) break;
+    }
+    p.range = range;
+    int ranges = 0;
+    for (int t = 0; t < kTypes; t++) {
+        p.range_start[t] = ranges;
+        ranges += (p.count[t] + range - 1) / range;
+    }
+    p.range_start[kTypes] = ranges;
+    return split_precision ? mlp_wgrad_launch<true>(p, ranges, st) : mlp_wgrad_launch<false>(p, ranges, st);
+}
+
+template <int ACT, bool SPLIT> int mlp_tangent_launch(const MlpTangentParams& p, int n_tiles, cudaStream_t st)
+{
+    auto kernel = mlp_tangent_kernel<ACT, SPLIT>;
+    const size_t smem = sizeof(MlpShared) + 1024;
+    static thread_local int configured_dev = -1;
+    int dev = 0;
+    ANI_CUDA(cudaGetDevice(&dev));
+    if (configured_dev != dev) {
+        if (int rc = set_smem(kernel, smem)) return rc;
+        configured_dev = dev;
+    }
+    ANI_CUDA(launch_chain(kernel, n_tiles, kMlpAllThreads, smem, st, 1, p));
+    return ANI_OK;
+}
+template <int ACT> int mlp_tangent_act(const MlpTangentParams& p, int n_tiles, bool split, cudaStream_t st)
+{
+    return split ? mlp_tangent_launch<ACT, true>(p, n_tiles, st) : mlp_tangent_launch<ACT, false>(p, n_tiles, st);
+}
+
+// ani_mlp_backward_f32, with dL/dA_l of the two inner layers in r1 and r2 (element-sorted rows) when given.
+int backward_call(const ani_mlp_backward_args* a, const int* acs_host, int split_precision, float* r1, float* r2,
+                  cudaStream_t st)
+{
+    long long n_atoms = 0;
+    if (!a) return ANI_ERR_NULL_POINTER;
+    if (int rc = check_acs(acs_host, &n_atoms)) return rc;
+    if (n_atoms == 0) return ANI_OK;
+    MlpBackwardParams p;
+    int tiles = 0, row = 0;
+    for (int t = 0; t < kTypes; t++) {
+        p.tile_start[t] = tiles;
+        p.count[t] = acs_host[t];
+        tiles += (acs_host[t] + kMlpTile - 1) / kMlpTile;
+        if (acs_host[t] > 0 && (!a->grad_energy[t] || !a->w1[t] || !a->w2[t] || !a->w3[t] || !a->w4[t] ||
+                                !a->dact1[t] || !a->dact2[t] || !a->dact3[t] || !a->dz1[t] || !a->dz2[t] ||
+                                !a->dz3[t]))
+            return ANI_ERR_NULL_POINTER;
+        if (acs_host[t] > 0 && !all_aligned16({a->w1[t], a->w2[t], a->w3[t], a->dact1[t], a->dact2[t], a->dact3[t],
+                                               a->dz1[t], a->dz2[t], a->dz3[t], a->grad_features[t]}))
+            return ANI_ERR_MISALIGNED;
+        p.grad_energy[t] = a->grad_energy[t];
+        p.w1[t] = a->w1[t]; p.w2[t] = a->w2[t]; p.w3[t] = a->w3[t]; p.w4[t] = a->w4[t];
+        p.dact1[t] = a->dact1[t]; p.dact2[t] = a->dact2[t]; p.dact3[t] = a->dact3[t];
+        p.dz1[t] = a->dz1[t]; p.dz2[t] = a->dz2[t]; p.dz3[t] = a->dz3[t];
+        p.grad_feat[t] = a->grad_features[t];
+        p.packed[t] = (const unsigned char*)a->packed[t];
+        p.r1[t] = r1 && acs_host[t] > 0 ? r1 + (size_t)row * kMlpH1 : nullptr;
+        p.r2[t] = r2 && acs_host[t] > 0 ? r2 + (size_t)row * kMlpH2 : nullptr;
+        row += acs_host[t];
+        if (reinterpret_cast<uintptr_t>(a->packed[t]) & 15) return ANI_ERR_MISALIGNED;
+    }
+    p.tile_start[kTypes] = tiles;
+    return split_precision ? mlp_backward_launch<true>(p, tiles, st) : mlp_backward_launch<false>(p, tiles, st);
 }
 
 template <int ACT> int mlp_launch_act(const MlpParams& p, int n_tiles, bool split, cudaStream_t st)
@@ -791,36 +880,8 @@ int ani_mlp_pack_weights_f32(const ani_mlp_pack_args* a, void* stream)
 int ani_mlp_backward_f32(const ani_mlp_backward_args* a, const int* acs_host, int split_precision,
                          void* stream)
 {
-    long long n_atoms = 0;
-    if (!a) return ANI_ERR_NULL_POINTER;
-    if (int rc = check_acs(acs_host, &n_atoms)) return rc;
-    if (n_atoms == 0) return ANI_OK;
-    MlpBackwardParams p;
-    int tiles = 0;
-    for (int t = 0; t < kTypes; t++) {
-        p.tile_start[t] = tiles;
-        p.count[t] = acs_host[t];
-        tiles += (acs_host[t] + kMlpTile - 1) / kMlpTile;
-        if (acs_host[t] > 0 && (!a->grad_energy[t] || !a->w1[t] || !a->w2[t] || !a->w3[t] || !a->w4[t] ||
-                                !a->dact1[t] || !a->dact2[t] || !a->dact3[t] || !a->dz1[t] || !a->dz2[t] ||
-                                !a->dz3[t]))
-            return ANI_ERR_NULL_POINTER;
-        if (acs_host[t] > 0 && !all_aligned16({a->w1[t], a->w2[t], a->w3[t], a->dact1[t], a->dact2[t], a->dact3[t],
-                                               a->dz1[t], a->dz2[t], a->dz3[t], a->grad_features[t]}))
-            return ANI_ERR_MISALIGNED;
-        p.grad_energy[t] = a->grad_energy[t];
-        p.w1[t] = a->w1[t]; p.w2[t] = a->w2[t]; p.w3[t] = a->w3[t]; p.w4[t] = a->w4[t];
-        p.dact1[t] = a->dact1[t]; p.dact2[t] = a->dact2[t]; p.dact3[t] = a->dact3[t];
-        p.dz1[t] = a->dz1[t]; p.dz2[t] = a->dz2[t]; p.dz3[t] = a->dz3[t];
-        p.grad_feat[t] = a->grad_features[t];
-        p.packed[t] = (const unsigned char*)a->packed[t];
-        if (reinterpret_cast<uintptr_t>(a->packed[t]) & 15) return ANI_ERR_MISALIGNED;
-    }
-    p.tile_start[kTypes] = tiles;
-    cudaStream_t st = (cudaStream_t)stream;
-    return split_precision ? mlp_backward_launch<true>(p, tiles, st) : mlp_backward_launch<false>(p, tiles, st);
+    return backward_call(a, acs_host, split_precision, nullptr, nullptr, (cudaStream_t)stream);
 }
-
 int ani_mlp_weight_grad_f32(const ani_mlp_weight_grad_args* a, const int* acs_host, int split_precision,
                             void* stream)
 {
@@ -849,26 +910,7 @@ int ani_mlp_weight_grad_f32(const ani_mlp_weight_grad_args* a, const int* acs_ho
         p.act3[t] = a->act3[t]; p.grad_energy[t] = a->grad_energy[t];
         p.dw4[t] = a->dw4[t]; p.db4[t] = a->db4[t];
     }
-    // atoms per CTA: the smallest multiple of 64 for which the grid fits the SMs once (the
-    // kernels run one CTA per SM, so a second partial wave would double the time)
-    int dev = 0, sms = 0;
-    ANI_CUDA(cudaGetDevice(&dev));
-    ANI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    int range = 256;
-    for (;; range += 64) {
-        long long ctas = 0;
-        for (int t = 0; t < kTypes; t++) ctas += (acs_host[t] + range - 1) / range;
-        if (ctas * kWgradBlocks <= sms || range >= (1 << 20)) break;
-    }
-    p.range = range;
-    int ranges = 0;
-    for (int t = 0; t < kTypes; t++) {
-        p.range_start[t] = ranges;
-        ranges += (acs_host[t] + range - 1) / range;
-    }
-    p.range_start[kTypes] = ranges;
-    cudaStream_t st = (cudaStream_t)stream;
-    return split_precision ? mlp_wgrad_launch<true>(p, ranges, st) : mlp_wgrad_launch<false>(p, ranges, st);
+    return wgrad_call(p, split_precision, (cudaStream_t)stream);
 }
 
 int ani_molecule_energy_f32(const float* atom_energy_sorted, const int* gather_idxs, const int* mol_offsets,
@@ -1316,6 +1358,140 @@ int ani_energy_pass_f64(const ani_energy_args_f64* a, void* stream)
             return rc;
     }
     return ANI_OK;
+}
+
+int ani_bias_celu_f32(float* z, float* a, const float* const* bias, const int* acs_host, int width, void* stream)
+{
+    long long n_atoms = 0;
+    if (int rc = check_acs(acs_host, &n_atoms)) return rc;
+    if (width <= 0 || (width & 3) || n_atoms * width > 0x7fffffffLL) return ANI_ERR_BAD_SIZE;
+    if (n_atoms == 0) return ANI_OK;
+    if (!z || !bias) return ANI_ERR_NULL_POINTER;
+    BiasCeluParams p;
+    p.z = z;
+    p.a = a;
+    p.rows = (int)n_atoms;
+    p.width = width;
+    int row = 0;
+    for (int t = 0; t < kTypes; t++) {
+        if (acs_host[t] > 0 && !bias[t]) return ANI_ERR_NULL_POINTER;
+        if (!all_aligned16({bias[t]})) return ANI_ERR_MISALIGNED;
+        p.bias[t] = bias[t];
+        row += acs_host[t];
+        p.row_end[t] = row;
+    }
+    if (!all_aligned16({z, a})) return ANI_ERR_MISALIGNED;
+    ANI_CUDA(launch_chain(bias_celu_kernel, (int)((n_atoms * (width / 4) + 255) / 256), 256, 0, (cudaStream_t)stream, 1, p));
+    return ANI_OK;
+}
+
+int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
+{
+    if (!f) return ANI_ERR_NULL_POINTER;
+    const ani_pass_args* a = &f->pass;
+    const int* acs = a->acs_host;
+    long long n_atoms = 0;
+    if (int rc = check_acs(acs, &n_atoms)) return rc;
+    if (n_atoms == 0) return ANI_OK;
+    if (!f->fx || !f->fy || !f->fz || !f->vx || !f->vy || !f->vz || !f->feature_rates || !f->r1 || !f->r2 || !f->adot1 ||
+        !f->adot2 || !f->adot3 || !f->q1 || !f->q2 || !f->q3 || !f->partial || !f->rmse || !a->feature_grads || !a->features ||
+        !a->act1 || !a->act2 || !a->act3 || !a->dact1 || !a->dact2 || !a->dact3 || !a->dz1 || !a->dz2 || !a->dz3)
+        return ANI_ERR_NULL_POINTER;
+    if (a->activation < 0 || a->activation > 3) return ANI_ERR_BAD_SIZE;
+    for (int t = 0; t < kTypes; t++)
+        if (acs[t] > 0 && (!a->packed[t] || !a->w4[t] || !a->dw1[t] || !a->dw2[t] || !a->dw3[t] || !a->dw4[t] || !a->db1[t] ||
+                           !a->db2[t] || !a->db3[t]))
+            return ANI_ERR_NULL_POINTER;
+    if (!all_aligned16({f->feature_rates, f->r1, f->r2, f->adot1, f->adot2, f->adot3, f->q1, f->q2, f->q3}))
+        return ANI_ERR_MISALIGNED;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int n = (int)n_atoms;
+
+    // coordinate gradients of the energy: the first-order pass, which also leaves dE/dA_l
+    ani_pass_args first = *a;
+    first.phases = (a->phases & (ANI_PASS_PACK | ANI_PASS_FEATURIZE)) | ANI_PASS_FORWARD;
+    first.labels = nullptr;
+    if (int rc = ani_network_pass_f32(&first, stream)) return rc;
+    {
+        ani_mlp_backward_args b;
+        size_t row = 0;
+        for (int t = 0; t < kTypes; t++) {
+            b.grad_energy[t] = a->grad_energy_sorted + row;
+            b.w1[t] = a->w1[t]; b.w2[t] = a->w2[t]; b.w3[t] = a->w3[t]; b.w4[t] = a->w4[t];
+            b.dact1[t] = a->dact1 + row * kMlpH1; b.dact2[t] = a->dact2 + row * kMlpH2; b.dact3[t] = a->dact3 + row * kMlpH3;
+            b.dz1[t] = a->dz1 + row * kMlpH1; b.dz2[t] = a->dz2 + row * kMlpH2; b.dz3[t] = a->dz3 + row * kMlpH3;
+            b.grad_features[t] = a->feature_grads + row * kTotal;
+            b.packed[t] = a->packed[t];
+            row += (size_t)acs[t];
+        }
+        if (int rc = backward_call(&b, acs, a->split_precision, f->r1, f->r2, st)) return rc;
+    }
+    first.phases = ANI_PASS_COORD_GRAD;
+    if (int rc = ani_network_pass_f32(&first, stream)) return rc;
+    // the loss, its derivative with respect to those gradients, and the rates of the features along it
+    ANI_CUDA(launch_chain(force_residual_kernel, kForceLossBlocks, kForceLossThreads, 0, st, 1, a->x_grads, a->y_grads,
+                          a->z_grads, f->fx, f->fy, f->fz, n, f->partial));
+    ANI_CUDA(launch_chain(force_loss_kernel, (n + kForceLossThreads - 1) / kForceLossThreads, kForceLossThreads, 0, st, 1,
+                          a->x_grads, a->y_grads, a->z_grads, f->fx, f->fy, f->fz, n, f->partial, f->vx, f->vy, f->vz,
+                          f->rmse));
+    float* rates[kTypes];
+    MlpTangentParams p;
+    MlpWgradParams w1, w2;      // F^T Q and U^T P
+    size_t row = 0;
+    int tiles = 0;
+    for (int t = 0; t < kTypes; t++) {
+        auto at = [&](float* base, int width) { return base + row * (size_t)width; };
+        rates[t] = at(f->feature_rates, kTotal);
+        p.count[t] = w1.count[t] = w2.count[t] = acs[t];
+        p.tile_start[t] = tiles;
+        tiles += (acs[t] + kMlpTile - 1) / kMlpTile;
+        p.u[t] = w2.feat[t] = rates[t];
+        p.w4[t] = a->w4[t];
+        p.packed[t] = (const unsigned char*)a->packed[t];
+        p.act1[t] = w1.act1[t] = at(a->act1, kMlpH1);
+        p.act2[t] = w1.act2[t] = at(a->act2, kMlpH2);
+        p.act3[t] = at(a->act3, kMlpH3);
+        if (a->activation == kActCelu && f->z1 && f->z2 && f->z3) {
+            p.act1[t] = f->z1 + row * kMlpH1;
+            p.act2[t] = f->z2 + row * kMlpH2;
+            p.act3[t] = f->z3 + row * kMlpH3;
+        }
+        p.dact1[t] = at(a->dact1, kMlpH1); p.dact2[t] = at(a->dact2, kMlpH2); p.dact3[t] = at(a->dact3, kMlpH3);
+        p.r1[t] = at(f->r1, kMlpH1); p.r2[t] = at(f->r2, kMlpH2);
+        p.adot1[t] = at(f->adot1, kMlpH1); p.adot2[t] = at(f->adot2, kMlpH2); p.adot3[t] = at(f->adot3, kMlpH3);
+        p.q1[t] = at(f->q1, kMlpH1); p.q2[t] = at(f->q2, kMlpH2); p.q3[t] = at(f->q3, kMlpH3);
+        w1.feat[t] = at(a->features, kTotal);
+        w1.dz1[t] = p.q1[t]; w1.dz2[t] = p.q2[t]; w1.dz3[t] = p.q3[t];
+        w2.act1[t] = p.adot1[t]; w2.act2[t] = p.adot2[t];
+        w2.dz1[t] = at(a->dz1, kMlpH1); w2.dz2[t] = at(a->dz2, kMlpH2); w2.dz3[t] = at(a->dz3, kMlpH3);
+        w1.act3[t] = w2.act3[t] = p.adot3[t];
+        w1.dw1[t] = w2.dw1[t] = a->dw1[t]; w1.dw2[t] = w2.dw2[t] = a->dw2[t]; w1.dw3[t] = w2.dw3[t] = a->dw3[t];
+        w1.db1[t] = a->db1[t]; w1.db2[t] = a->db2[t]; w1.db3[t] = a->db3[t];
+        w2.db1[t] = w2.db2[t] = w2.db3[t] = nullptr;
+        w1.dw4[t] = a->dw4[t];
+        w2.dw4[t] = nullptr;
+        w1.db4[t] = w2.db4[t] = nullptr;
+        w1.grad_energy[t] = w2.grad_energy[t] = nullptr;
+        row += (size_t)acs[t];
+    }
+    p.tile_start[kTypes] = tiles;
+    if (int rc = ani_featurize_grad_inverse_f32(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
+                                                a->n_mols, a->scatter_idxs, f->vx, f->vy, f->vz, rates[0], rates[1], rates[2],
+                                                rates[3], acs, stream))
+        return rc;
+    if (f->z_ready) ANI_CUDA(cudaStreamWaitEvent(st, (cudaEvent_t)f->z_ready, 0));
+    const bool split = a->split_precision != 0;
+    int rc = ANI_OK;
+    switch (a->activation) {
+        case kActCelu: rc = mlp_tangent_act<kActCelu>(p, tiles, split, st); break;
+        case kActGaussian: rc = mlp_tangent_act<kActGaussian>(p, tiles, split, st); break;
+        case kActNormal: rc = mlp_tangent_act<kActNormal>(p, tiles, split, st); break;
+        default: rc = mlp_tangent_act<kActSoftplus>(p, tiles, split, st);
+    }
+    if (rc) return rc;
+    if (a->zero_ptr && a->zero_bytes) ANI_CUDA(cudaMemsetAsync(a->zero_ptr, 0, a->zero_bytes, st));
+    if (int rc2 = wgrad_call(w1, a->split_precision, st)) return rc2;
+    return wgrad_call(w2, a->split_precision, st);
 }
 
 }  // extern "C"

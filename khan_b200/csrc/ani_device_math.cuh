@@ -116,6 +116,45 @@ template <typename T> __device__ __forceinline__ void angular_factors_dev(T cosv
     }
 }
 
+// The factors of angular_factors_dev and their derivatives along a direction in which cos(theta), the mean
+// distance and the product of the cutoffs change at the rates dcos, drbar and dfc:
+//   dA[t] = 8 b^7 (cos(theta_t) - sin(theta_t) c / s) dcos (0 for a numerically collinear triplet, as in
+//   angular_vjp_dev),  dBF[q] = pref e_q (dfc - 2 eta d_q drbar fcprod).
+template <typename T>
+__device__ __forceinline__ void angular_tangent_dev(T cosv, T sin2, T rbar, T fcprod, T dcos, T drbar, T dfc, T* A, T* BF,
+                                                    T* dA, T* dBF)
+{
+    const T c = Num<T>::max_((T)-1, Num<T>::min_((T)1, cosv));
+    const T s2 = Num<T>::min_((T)1, sin2);
+    const T s = Num<T>::sqrt_(s2);
+    const bool bent = s2 > (T)1e-12;
+    const T cot = bent ? c * Num<T>::rsqrt_(s2) : (T)0;
+    const T dc8 = bent ? (T)8 * dcos : (T)0, ds8 = dc8 * cot;
+#pragma unroll
+    for (int t = 0; t < kNumThetas; t++) {
+        const T b = c * theta_cos<T>(t) + (s * theta_sin<T>(t) + (T)1);
+        const T b2 = b * b, b4 = b2 * b2, b7 = b4 * b2 * b;
+        A[t] = b7 * b;
+        dA[t] = b7 * (dc8 * theta_cos<T>(t) - ds8 * theta_sin<T>(t));
+    }
+    T d[kNumARs], e[kNumARs];
+    if constexpr (sizeof(T) == 8) {
+        gaussians_f64<AngularGrid>(rbar, d, e);
+    } else {
+#pragma unroll
+        for (int q = 0; q < kNumARs; q++) {
+            d[q] = rbar - angular_shift<T>(q);
+            e[q] = Num<T>::exp_neg((T)kA_eta, d[q] * d[q]);
+        }
+    }
+    const T f = (T)kA_pref * fcprod, g = (T)kA_pref * dfc, h = (T)-2 * (T)kA_eta * drbar * f;
+#pragma unroll
+    for (int q = 0; q < kNumARs; q++) {
+        BF[q] = e[q] * f;
+        dBF[q] = e[q] * (g + d[q] * h);
+    }
+}
+
 // radial_vjp and angular_vjp of ani_params.h, arranged for the device: the same arithmetic, but every
 // constant (shift, cos / sin of a theta shift) is an immediate operand of a scalar instruction, and
 // only products of two computed values run as packed pairs.  (A packed instruction takes its

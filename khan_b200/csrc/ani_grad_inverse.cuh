@@ -63,6 +63,106 @@ __device__ __forceinline__ T angular_jvp_term(T c, T sin2, T rj, T rk, T fj, T d
     return (T)kA_pref * (pc * dcos + pj * drj + pk * drk);
 }
 
+// The row of atom i of a molecule of n atoms; nb: this warp's list in shared memory.
+template <typename T>
+__device__ __noinline__ void jvp_atom_streaming(const T* __restrict__ xs, const T* __restrict__ ys,
+                                                const T* __restrict__ zs, const int* __restrict__ types,
+                                                const T* __restrict__ vx, const T* __restrict__ vy,
+                                                const T* __restrict__ vz, int base, int n, int i, JvpNeighbor<T>* nb,
+                                                T* row)
+{
+    const int lane = lane_id();
+    const int gi = base + i;
+    const T xi = xs[gi], yi = ys[gi], zi = zs[gi];
+    const T vxi = vx[gi], vyi = vy[gi], vzi = vz[gi];
+
+    // ---- neighbour list (everything within R_Rc), scan order ----
+    int n_nb = 0;
+    for (int j0 = 0; j0 < n; j0 += kWarp) {
+        const int j = j0 + lane;
+        const bool live = j < n;
+        const int gj = base + (live ? j : 0);
+        const T dx = xi - xs[gj], dy = yi - ys[gj], dz = zi - zs[gj];
+        T r, inv;
+        length_and_inverse(dx * dx + dy * dy + dz * dz, &r, &inv);
+        const bool in_rad = live && j != i && r < (T)kR_Rc;
+        const unsigned mR = __ballot_sync(kFull, in_rad);
+        if (in_rad) {
+            const int pos = n_nb + __popc(mR & lanemask_lt());
+            if (pos < kJvpMaxNeighbors) {
+                JvpNeighbor<T> e;
+                e.u = Vec4<T>{dx * inv, dy * inv, dz * inv, r};
+                const T wx = vxi - vx[gj], wy = vyi - vy[gj], wz = vzi - vz[gj];
+                e.w = Vec4<T>{wx, wy, wz, e.u.x * wx + e.u.y * wy + e.u.z * wz};
+                cutoff<T>(r, (T)kR_Rc, &e.fcR, &e.dfcR);
+                e.angular = r < (T)kA_Rc ? 1 : 0;
+                e.fc = (T)0;
+                e.dfc = (T)0;
+                if (e.angular) cutoff<T>(r, (T)kA_Rc, &e.fc, &e.dfc);
+                e.type = checked_type(types[gj]);
+                nb[pos] = e;
+            }
+        }
+        n_nb += __popc(mR);
+    }
+    __syncwarp();
+    if (n_nb > kJvpMaxNeighbors) {
+        // Not supported by this kernel: more than 64 atoms within 4.6 A of one atom.
+        if (lane == 0) report(ANI_ERR_TOO_MANY_ATOMS);
+        for (int q = lane; q < kTotal; q += kWarp) row[q] = (T)0;
+        return;
+    }
+
+    // ---- radial block: lane = (half, shift) ----
+    {
+        const int half = lane >> 4;
+        const T shift = (T)c_tab.R_Rs[lane & 15];
+        T acc[kTypes] = {(T)0, (T)0, (T)0, (T)0};
+        for (int p = half; p < n_nb; p += 2) {
+            const JvpNeighbor<T>& e = nb[p];
+            const T val = radial_slope<T>(e.u.w, e.fcR, e.dfcR, shift) * e.w.w;
+#pragma unroll
+            for (int g = 0; g < kTypes; g++) acc[g] += e.type == g ? val : (T)0;
+        }
+#pragma unroll
+        for (int g = 0; g < kTypes; g++) acc[g] += __shfl_xor_sync(kFull, acc[g], 16);
+        row[lane] = lane < 16 ? acc[0] : acc[1];
+        row[32 + lane] = lane < 16 ? acc[2] : acc[3];
+    }
+
+    // ---- angular block: lane = (theta, shift), warp-uniform loops over pairs ----
+    const T ct = (T)c_tab.cos_t[lane >> 2], st = (T)c_tab.sin_t[lane >> 2];
+    const T shift = (T)c_tab.A_Rs[lane & 3];
+    T acc[kPairBuckets];
+#pragma unroll
+    for (int b = 0; b < kPairBuckets; b++) acc[b] = (T)0;
+    for (int a = 0; a < n_nb; a++) {
+        const JvpNeighbor<T>& ea = nb[a];
+        if (!ea.angular) continue;
+        const T ira = (T)1 / ea.u.w;
+        for (int b = a + 1; b < n_nb; b++) {
+            const JvpNeighbor<T>& eb = nb[b];
+            if (!eb.angular) continue;
+            T c = ea.u.x * eb.u.x + ea.u.y * eb.u.y + ea.u.z * eb.u.z;
+            c = Num<T>::max_((T)-1, Num<T>::min_((T)1, c));
+            const T s2 = sin2_from_cross<T>(ea.u.x, ea.u.y, ea.u.z, eb.u.x, eb.u.y, eb.u.z);
+            // d cos = [(u_b . w_a) - c (u_a . w_a)] / r_a + [(u_a . w_b) - c (u_b . w_b)] / r_b
+            const T ub_wa = eb.u.x * ea.w.x + eb.u.y * ea.w.y + eb.u.z * ea.w.z;
+            const T ua_wb = ea.u.x * eb.w.x + ea.u.y * eb.w.y + ea.u.z * eb.w.z;
+            const T irb = (T)1 / eb.u.w;
+            const T dcos = (ub_wa - c * ea.w.w) * ira + (ua_wb - c * eb.w.w) * irb;
+            const T val = angular_jvp_term<T>(c, s2, ea.u.w, eb.u.w, ea.fc, ea.dfc, eb.fc,
+                                              eb.dfc, dcos, ea.w.w, eb.w.w, ct, st, shift);
+            const int bk = pair_bucket(ea.type, eb.type);
+#pragma unroll
+            for (int q = 0; q < kPairBuckets; q++) acc[q] += bk == q ? val : (T)0;
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < kPairBuckets; b++) row[kRadial + b * kTS + lane] = acc[b];
+    __syncwarp();
+}
+
 template <typename T, int NW>
 __global__ void __launch_bounds__(NW* kWarp)
     featurize_grad_inverse_kernel(const T* __restrict__ xs, const T* __restrict__ ys,
@@ -100,94 +200,7 @@ __global__ void __launch_bounds__(NW* kWarp)
                 continue;
             }
             T* row = (ti == 0 ? out_h : (ti == 1 ? out_c : (ti == 2 ? out_n : out_o))) + (size_t)srow * kTotal;
-            const T xi = xs[gi], yi = ys[gi], zi = zs[gi];
-            const T vxi = vx[gi], vyi = vy[gi], vzi = vz[gi];
-
-            // ---- neighbour list (everything within R_Rc), scan order ----
-            int n_nb = 0;
-            for (int j0 = 0; j0 < n; j0 += kWarp) {
-                const int j = j0 + lane;
-                const bool live = j < n;
-                const int gj = base + (live ? j : 0);
-                const T dx = xi - xs[gj], dy = yi - ys[gj], dz = zi - zs[gj];
-                T r, inv;
-                length_and_inverse(dx * dx + dy * dy + dz * dz, &r, &inv);
-                const bool in_rad = live && j != i && r < (T)kR_Rc;
-                const unsigned mR = __ballot_sync(kFull, in_rad);
-                if (in_rad) {
-                    const int pos = n_nb + __popc(mR & lanemask_lt());
-                    if (pos < kJvpMaxNeighbors) {
-                        JvpNeighbor<T> e;
-                        e.u = Vec4<T>{dx * inv, dy * inv, dz * inv, r};
-                        const T wx = vxi - vx[gj], wy = vyi - vy[gj], wz = vzi - vz[gj];
-                        e.w = Vec4<T>{wx, wy, wz, e.u.x * wx + e.u.y * wy + e.u.z * wz};
-                        cutoff<T>(r, (T)kR_Rc, &e.fcR, &e.dfcR);
-                        e.angular = r < (T)kA_Rc ? 1 : 0;
-                        e.fc = (T)0;
-                        e.dfc = (T)0;
-                        if (e.angular) cutoff<T>(r, (T)kA_Rc, &e.fc, &e.dfc);
-                        e.type = checked_type(types[gj]);
-                        ws.nb[pos] = e;
-                    }
-                }
-                n_nb += __popc(mR);
-            }
-            __syncwarp();
-            if (n_nb > kJvpMaxNeighbors) {
-                // Not supported by this kernel: more than 64 atoms within 4.6 A of one atom.
-                if (lane == 0) report(ANI_ERR_TOO_MANY_ATOMS);
-                for (int q = lane; q < kTotal; q += kWarp) row[q] = (T)0;
-                continue;
-            }
-
-            // ---- radial block: lane = (half, shift) ----
-            {
-                const int half = lane >> 4;
-                const T shift = (T)c_tab.R_Rs[lane & 15];
-                T acc[kTypes] = {(T)0, (T)0, (T)0, (T)0};
-                for (int p = half; p < n_nb; p += 2) {
-                    const JvpNeighbor<T>& e = ws.nb[p];
-                    const T val = radial_slope<T>(e.u.w, e.fcR, e.dfcR, shift) * e.w.w;
-#pragma unroll
-                    for (int g = 0; g < kTypes; g++) acc[g] += e.type == g ? val : (T)0;
-                }
-#pragma unroll
-                for (int g = 0; g < kTypes; g++) acc[g] += __shfl_xor_sync(kFull, acc[g], 16);
-                row[lane] = lane < 16 ? acc[0] : acc[1];
-                row[32 + lane] = lane < 16 ? acc[2] : acc[3];
-            }
-
-            // ---- angular block: lane = (theta, shift), warp-uniform loops over pairs ----
-            const T ct = (T)c_tab.cos_t[lane >> 2], st = (T)c_tab.sin_t[lane >> 2];
-            const T shift = (T)c_tab.A_Rs[lane & 3];
-            T acc[kPairBuckets];
-#pragma unroll
-            for (int b = 0; b < kPairBuckets; b++) acc[b] = (T)0;
-            for (int a = 0; a < n_nb; a++) {
-                const JvpNeighbor<T>& ea = ws.nb[a];
-                if (!ea.angular) continue;
-                const T ira = (T)1 / ea.u.w;
-                for (int b = a + 1; b < n_nb; b++) {
-                    const JvpNeighbor<T>& eb = ws.nb[b];
-                    if (!eb.angular) continue;
-                    T c = ea.u.x * eb.u.x + ea.u.y * eb.u.y + ea.u.z * eb.u.z;
-                    c = Num<T>::max_((T)-1, Num<T>::min_((T)1, c));
-                    const T s2 = sin2_from_cross<T>(ea.u.x, ea.u.y, ea.u.z, eb.u.x, eb.u.y, eb.u.z);
-                    // d cos = [(u_b . w_a) - c (u_a . w_a)] / r_a + [(u_a . w_b) - c (u_b . w_b)] / r_b
-                    const T ub_wa = eb.u.x * ea.w.x + eb.u.y * ea.w.y + eb.u.z * ea.w.z;
-                    const T ua_wb = ea.u.x * eb.w.x + ea.u.y * eb.w.y + ea.u.z * eb.w.z;
-                    const T irb = (T)1 / eb.u.w;
-                    const T dcos = (ub_wa - c * ea.w.w) * ira + (ua_wb - c * eb.w.w) * irb;
-                    const T val = angular_jvp_term<T>(c, s2, ea.u.w, eb.u.w, ea.fc, ea.dfc, eb.fc,
-                                                      eb.dfc, dcos, ea.w.w, eb.w.w, ct, st, shift);
-                    const int bk = pair_bucket(ea.type, eb.type);
-#pragma unroll
-                    for (int q = 0; q < kPairBuckets; q++) acc[q] += bk == q ? val : (T)0;
-                }
-            }
-#pragma unroll
-            for (int b = 0; b < kPairBuckets; b++) row[kRadial + b * kTS + lane] = acc[b];
-            __syncwarp();
+            jvp_atom_streaming<T>(xs, ys, zs, types, vx, vy, vz, base, n, i, ws.nb, row);
         }
     }
 }

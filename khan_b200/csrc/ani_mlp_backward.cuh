@@ -37,6 +37,8 @@ struct MlpBackwardParams {
     float* dz3[kTypes];          // [count][64]
     float* grad_feat[kTypes];    // optional [count][384]
     const unsigned char* packed[kTypes];   // optional: the weights pre-packed by mlp_pack_kernel
+    float* r1[kTypes];           // optional [count][128]: dL/dA1, dZ1 before the factor D1
+    float* r2[kTypes];           // optional [count][128]
 };
 
 template <bool SPLIT>
@@ -113,6 +115,7 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_backward_kernel(const M
         const float* step_w[2] = {p.w3[e], p.w2[e]};
         const float* step_d[2] = {p.dact2[e], p.dact1[e]};
         float* step_out[2] = {p.dz2[e], p.dz1[e]};
+        float* step_raw[2] = {p.r2[e], p.r1[e]};
         bool ok = true;
 #pragma unroll 1
         for (int s = 0; s < 2 && ok; s++) {
@@ -129,6 +132,8 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_backward_kernel(const M
             {
                 float v[32], d[32];
                 tmem_load32(lane_addr + c0, v);
+                if (step_raw[s])
+                    warp_tile_to_global<false>(scratch, v, step_raw[s] + tile_atom0 * 128 + c0, 128, tile_rows);
                 warp_tile_from_global(scratch, d, step_d[s] + tile_atom0 * 128 + c0, 128, tile_rows);
 #pragma unroll
                 for (int i = 0; i < 32; i++) {

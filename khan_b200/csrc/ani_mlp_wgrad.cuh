@@ -33,13 +33,13 @@ struct MlpWgradParams {
     float* dw1[kTypes];            // [384][128]
     float* dw2[kTypes];            // [128][128]
     float* dw3[kTypes];            // [128][64]
-    float* db1[kTypes];            // [128]
+    float* db1[kTypes];            // [128] or null, as db2, db3
     float* db2[kTypes];            // [128]
     float* db3[kTypes];            // [64]
     const float* act3[kTypes];     // [count][64]
-    const float* grad_energy[kTypes];   // [count]
-    float* dw4[kTypes];            // [64]
-    float* db4[kTypes];            // [1]
+    const float* grad_energy[kTypes];   // [count], or null: ones
+    float* dw4[kTypes];            // [64], or null: no output layer
+    float* db4[kTypes];            // [1] or null
 };
 
 template <bool SPLIT>
@@ -77,6 +77,8 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_wgrad_kernel(const MlpW
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
+    pdl_trigger();
     const unsigned tmem = sh.tmem_base;
     const int nchunks = (n_here + kPipeK - 1) / kPipeK;
     if (warp == kMlpThreads / 32) {
@@ -111,14 +113,14 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_wgrad_kernel(const MlpW
         } else if (!ok && tid == 0) {
             report(ANI_ERR_TIMEOUT);
         }
-        if (blk == 4) {
+        if (blk == 4 && p.dw4[e]) {
             // output layer, done by the CTA with the lightest product: dw4 = A3^T g and db4 = sum g
             // over this range; no tensor cores involved
             const int q = tid & 15, a_in = tid >> 4;      // 16 column quads x 32 atoms per pass
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
             float gsum = 0.0f;
             for (int k = a_in; k < n_here; k += kMlpThreads / 16) {
-                const float g = p.grad_energy[e][first + k];
+                const float g = p.grad_energy[e] ? p.grad_energy[e][first + k] : 1.0f;
                 const float4 v = *reinterpret_cast<const float4*>(p.act3[e] + (size_t)(first + k) * kMlpH3 + 4 * q);
                 acc.x += v.x * g; acc.y += v.y * g; acc.z += v.z * g; acc.w += v.w * g;
                 gsum += q == 0 ? g : 0.0f;
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_wgrad_kernel(const MlpW
             atomicAdd(p.dw4[e] + 4 * q + 1, acc.y);
             atomicAdd(p.dw4[e] + 4 * q + 2, acc.z);
             atomicAdd(p.dw4[e] + 4 * q + 3, acc.w);
-            if (q == 0) atomicAdd(p.db4[e], gsum);
+            if (q == 0 && p.db4[e]) atomicAdd(p.db4[e], gsum);
         }
     }
     tc_fence_before();

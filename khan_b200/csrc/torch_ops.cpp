@@ -10,6 +10,7 @@
 // refuses and calls again.  A negative status of the library is returned as an int.  The entry points are
 // handed over as addresses (bind), so that there is one copy of the library in the process.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/core/LegacyTypeDispatch.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -33,8 +34,13 @@ SortFn g_sort = nullptr;
 FeaturizeFn g_featurize[2] = {};   // f32, f64
 GradFn g_grad[2] = {};
 
-void bind(uintptr_t sort, uintptr_t featurize_f32, uintptr_t featurize_f64, uintptr_t grad_f32, uintptr_t grad_f64)
+using BiasCeluFn = int (*)(float*, float*, const float* const*, const int*, int, void*);
+BiasCeluFn g_bias_celu = nullptr;
+
+void bind(uintptr_t sort, uintptr_t featurize_f32, uintptr_t featurize_f64, uintptr_t grad_f32, uintptr_t grad_f64,
+          uintptr_t bias_celu)
 {
+    g_bias_celu = reinterpret_cast<BiasCeluFn>(bias_celu);
     g_sort = reinterpret_cast<SortFn>(sort);
     g_featurize[0] = reinterpret_cast<FeaturizeFn>(featurize_f32);
     g_featurize[1] = reinterpret_cast<FeaturizeFn>(featurize_f64);
@@ -177,6 +183,62 @@ py::object featurize_grad(const at::Tensor& x, const at::Tensor& y, const at::Te
     return py::make_tuple(out.as_strided({n}, {1}, 0), out.as_strided({n}, {1}, n), out.as_strided({n}, {1}, 2 * n));
 }
 
+// Pre-activations z[l] of the three hidden layers with celu, in plain float32 products: one library GEMM per
+// element and layer (the call that at::mm makes, without its 6 us of dispatch) and one kernel per layer for
+// bias and activation of all elements, on a stream of their own beside the caller's.
+class CeluPreactivations {
+  public:
+    // weights / biases [layer * 4 + element]; z, a: [>= n, width] buffers per layer, a of the first two
+    CeluPreactivations(std::vector<at::Tensor> weights, std::vector<at::Tensor> biases, std::vector<at::Tensor> z,
+                       std::vector<at::Tensor> a)
+        : weights_(std::move(weights)), biases_(std::move(biases)), z_(std::move(z)), a_(std::move(a)),
+          stream_(c10::cuda::getStreamFromPool(false, z_.at(0).device().index()))
+    {
+        TORCH_CHECK(weights_.size() == 12 && biases_.size() == 12 && z_.size() == 3 && a_.size() == 2);
+        for (const auto* list : {&weights_, &biases_, &z_, &a_})
+            for (const at::Tensor& t : *list) TORCH_CHECK(fits(t, c10::kFloat, z_[0].device()));
+    }
+    // features: [>= n, 384], element-sorted, written by work enqueued on the current stream so far
+    int run(const at::Tensor& features, py::handle counts)
+    {
+        int acs[4];
+        TORCH_CHECK(read_counts(counts.ptr(), acs) && fits(features, c10::kFloat, z_[0].device()));
+        const c10::cuda::CUDAGuard device(features.device());
+        started_.record(c10::cuda::getCurrentCUDAStream());
+        started_.block(stream_);
+        const c10::cuda::CUDAStreamGuard guard(stream_);
+        const int64_t inputs[3] = {kFeatures, 128, 128};
+        const float one = 1.0f, zero = 0.0f;
+        for (int l = 0; l < 3; l++) {
+            const float* in = l == 0 ? features.const_data_ptr<float>() : a_[l - 1].const_data_ptr<float>();
+            float* out = z_[l].mutable_data_ptr<float>();
+            const int64_t k = inputs[l], n = z_[l].size(1);
+            int64_t row = 0;
+            const float* bias[4];
+            for (int t = 0; t < 4; t++) {
+                bias[t] = biases_[l * 4 + t].const_data_ptr<float>();
+                if (acs[t] > 0)
+                    TORCH_CHECK(cublasSgemm(at::cuda::getCurrentCUDABlasHandle(), CUBLAS_OP_N, CUBLAS_OP_N, (int)n, acs[t],
+                                            (int)k, &one, weights_[l * 4 + t].const_data_ptr<float>(), (int)n, in + row * k,
+                                            (int)k, &zero, out + row * n, (int)n) == CUBLAS_STATUS_SUCCESS,
+                                "cublasSgemm");
+                row += acs[t];
+            }
+            if (const int rc = g_bias_celu(out, l < 2 ? a_[l].mutable_data_ptr<float>() : nullptr, bias, acs, (int)n,
+                                           stream_.stream()))
+                return rc;
+        }
+        done_.record(stream_);
+        return 0;
+    }
+    uintptr_t done() { return reinterpret_cast<uintptr_t>(done_.event()); }
+
+  private:
+    std::vector<at::Tensor> weights_, biases_, z_, a_;
+    c10::cuda::CUDAStream stream_;
+    at::cuda::CUDAEvent started_, done_;
+};
+
 }  // namespace
 
 PYBIND11_MODULE(_torch_ops, m)
@@ -186,4 +248,8 @@ PYBIND11_MODULE(_torch_ops, m)
     m.def("featurize", &featurize);
     m.def("featurize_into", &featurize_into);
     m.def("featurize_grad", &featurize_grad);
+    py::class_<CeluPreactivations>(m, "CeluPreactivations")
+        .def(py::init<std::vector<at::Tensor>, std::vector<at::Tensor>, std::vector<at::Tensor>, std::vector<at::Tensor>>())
+        .def("run", &CeluPreactivations::run)
+        .def("done", &CeluPreactivations::done);
 }

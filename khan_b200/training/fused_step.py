@@ -216,6 +216,61 @@ class FusedTrainStep:
     KERNELS = 11   # weight packing, sort, featurize, mlp fwd, molecule energy, mlp bwd, memset, wgrad, featurize_grad, sumsq, nadam
 
 
+class ForceFitStep(FusedTrainStep):
+    """The force-training step (``train_op_forces`` of the reference) on the C ABI only: weight gradients of
+    exp(force rmse) in one call (``ani_force_fit_pass_f32``), added into the flat buffer."""
+
+    def __init__(self, model, optimizer: FlatNadam, n_atoms: int, n_mols: int, device="cuda:0"):
+        super().__init__(model, optimizer, n_atoms, n_mols, device)
+        f32 = dict(dtype=torch.float32, device=self.device)
+        self.grad_energy_sorted.fill_(1.0)           # dE_molecule/dE_atom
+        self.v = torch.empty((3, n_atoms), **f32)
+        self.feature_rates = torch.empty((n_atoms, FEATURE_SIZE), **f32)
+        self.second = {name: torch.empty((n_atoms, width), **f32) for name, width in (
+            ("r1", 128), ("r2", 128), ("adot1", 128), ("adot2", 128), ("adot3", 64), ("q1", 128), ("q2", 128), ("q3", 64))}
+        self.partial = torch.empty(192, dtype=torch.float64, device=self.device)
+        self.rmse = torch.zeros(1, **f32)
+        self.celu = model.activation_fn is activations.celu
+        if self.celu:      # see bias_celu_kernel: the signs of the pre-activations come from plain float32 products
+            self.z = [torch.empty((n_atoms, w), **f32) for w in (128, 128, 64)]
+            layers = [[t.detach() for t in ts] for ts in zip(*[ann.Ws[:3] + ann.bs[:3] for ann in model.anns])]
+            self.preactivations = _lib.torch_ops().CeluPreactivations(
+                sum(layers[:3], []), sum(layers[3:], []), self.z, [torch.empty((n_atoms, 128), **f32) for _ in range(2)])
+
+        f = self._force_args = _lib.ForceFitArgs()      # a batch changes the pass and the targets only
+        f.vx, f.vy, f.vz = (self.v[k].data_ptr() for k in range(3))
+        f.feature_rates, f.partial, f.rmse = self.feature_rates.data_ptr(), self.partial.data_ptr(), self.rmse.data_ptr()
+        for name, t in self.second.items():
+            setattr(f, name, t.data_ptr())
+        if self.celu:
+            f.z1, f.z2, f.z3 = (z.data_ptr() for z in self.z)
+
+    def weight_gradients_of_forces(self, sb: StagedBatch, forces: torch.Tensor) -> None:
+        """``forces``: the batch's target forces ``[3, n_atoms]``.  Afterwards ``self.rmse`` holds the sum of
+        the rmses over x, y and z, the optimiser's flat buffer the weight gradients and ``sb.grads`` the
+        coordinate gradients of the energy."""
+        self._check(sb)
+        stream = self._stream()
+        if self.model.packed_weights() is None:
+            self.model.pack_weights(stream)          # allocates the packed copy (first use)
+        a = self._pass_args(sb)
+        g, cap, size = sb.grads.data_ptr(), sb.n_atoms_cap, sb.grads.element_size()
+        a.x_grads, a.y_grads, a.z_grads = g, g + cap * size, g + 2 * cap * size
+        a.feature_grads, a.labels = sb.upstream.data_ptr(), None
+        a.phases = _lib.PASS_PACK | _lib.PASS_FEATURIZE
+        if self.celu:
+            _lib.check(_lib.lib().ani_network_pass_f32(ctypes.byref(a), stream), "ani_network_pass_f32")
+            a.phases = 0
+            _lib.check(self.preactivations.run(sb.features, sb.acs_host), "CeluPreactivations")
+        f = self._force_args
+        f.pass_ = a
+        f.fx, f.fy, f.fz = (forces[k].data_ptr() for k in range(3))
+        if self.celu:
+            f.z_ready = self.preactivations.done()
+        _lib.check(_lib.lib().ani_force_fit_pass_f32(ctypes.byref(f), stream), "ani_force_fit_pass_f32")
+        self._args_key = None
+
+
 class StepPipeline:
     """Training steps over a pool of resident batches with the independent kernels side by side:
 

@@ -169,6 +169,7 @@ class TrainerMultiTower:
         self.max_norm_ops = _Op("max_norm_ops")
         self._device_l2s = _Op("_device_l2s")          # squared errors left on the device (no host wait)
         self._single, self._single_lock = None, threading.Lock()   # evaluator of energy_and_gradient
+        self._force_fit = None                          # (capacity, StagedBatch, ForceFitStep) of force training
         self._fused = None                              # (capacity, StagedBatch, FusedTrainStep) of the fused path
 
     # ------------------------------------------------------------------ bookkeeping
@@ -349,11 +350,17 @@ class TrainerMultiTower:
         fused = (self.num_towers == 1 and isinstance(self.optimizer, FlatNadam) and self.model.fused
                  and len(training) == 1 and training[0] != "train_op_forces" and set(names) <= fused_names
                  and packed.ys is not None and packed.num_mols() > 0)
+        force_fit = (self.num_towers == 1 and isinstance(self.optimizer, FlatNadam) and self.model.fused
+                     and training == ["train_op_forces"]
+                     and set(names) <= {"train_op_forces", "tower_force_rmses", "tower_bids"}
+                     and packed.grads is not None and packed.ys is not None and packed.num_mols() > 0)
         # the fused path works on two batches at a time (this one's networks, the next one's featurizer)
         it = BatchFeeder(packed, batch_size, shuffle, fuzz, devices=self.towers, depth=3 if fused else 2,
                          hold=2 if fused else self.num_towers)
         try:
-            if fused:
+            if force_fit:
+                yield from self._force_rounds(it, names, packed.capacity(batch_size), before_hooks)
+            elif fused:
                 yield from self._fused_rounds(it, names, training[0], packed.capacity(batch_size), before_hooks)
             else:
                 yield from self._feed_rounds(it, names, training, need_grad, need_coord, before_hooks)
@@ -436,6 +443,36 @@ class TrainerMultiTower:
                     elif n == "tower_bids":
                         row.append([np.array(fed.index)])
                 fed, k = nxt, k + 1
+            yield row
+
+    def _force_rounds(self, it, names, capacity, before_hooks):
+        """Force training on one device without autograd (``ForceFitStep``)."""
+        from ..staged import StagedBatch
+        from .fused_step import ForceFitStep
+        cap_atoms, cap_mols = max(capacity[0], 1), max(capacity[1], 1)
+        dev = self.towers[0]
+        if self._force_fit is None or self._force_fit[0][0] < cap_atoms or self._force_fit[0][1] < cap_mols:
+            self._force_fit = ((cap_atoms, cap_mols), StagedBatch(cap_atoms, cap_mols, device=dev),
+                               ForceFitStep(self.model, self.optimizer, cap_atoms, cap_mols, device=dev))
+        _, sb, step = self._force_fit
+        for fed in it:
+            if before_hooks is not None:
+                self._run_hooks(before_hooks)
+            with torch.cuda.device(dev), torch.no_grad():
+                fed.wait()
+                sb.adopt(fed)
+                step.weight_gradients_of_forces(sb, fed.grads)
+                average_gradients(self.parameters, self.optimizer.flat_grads)
+                self.optimizer.step()
+                self.global_step += 1
+                row = []
+                for n in names:
+                    if n == "tower_force_rmses":
+                        row.append([float(step.rmse)])
+                    elif n == "tower_bids":
+                        row.append([np.array(fed.index)])
+                    else:
+                        row.append(None)
             yield row
 
     def _feed_rounds(self, it, names, training, need_grad, need_coord, before_hooks):

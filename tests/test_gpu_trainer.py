@@ -425,3 +425,41 @@ def test_energy_server_answers_with_the_trainers_numbers():
         minus[atom, 1 + axis] -= 1e-5
         fd = (es.evaluate(tr, plus.tolist())["energy"] - es.evaluate(tr, minus.tolist())["energy"]) / 2e-5
         assert abs(fd - g[atom, axis]) < 1e-6 * max(1.0, abs(fd))
+
+
+@pytest.mark.parametrize("act", ["celu", "gaussian", "normal", "softplus"])
+@pytest.mark.parametrize("n_mols", [1, 37, 200])
+def test_force_training_step_matches_the_autograd_path(act, n_mols):
+    """ForceFitStep against the differentiable float64 path: weight gradients of exp(force rmse) and the rmse."""
+    import torch
+    from khan_b200 import RawDataset, TrainerMultiTower
+    from khan_b200.data import synthetic as syn
+    from khan_b200.model import activations
+    mols = syn.gdb_like_batch(n_mols, seed=n_mols).molecules()
+    rng = np.random.default_rng(1)
+    ds = RawDataset(mols, list(rng.normal(size=n_mols)), [rng.normal(0.0, 0.2, (len(m), 3)) for m in mols])
+
+    def step(precision, fused):
+        tr = TrainerMultiTower(None, [torch.device("cuda", 0)], precision=precision, layer_sizes=(128, 128, 64, 1),
+                               activation_fn=activations.get_fn_by_name(act), seed=5)
+        with torch.no_grad():      # float32 weights in both, biases that are not zero
+            gen = torch.Generator().manual_seed(9)
+            ref = TrainerMultiTower(None, [torch.device("cuda", 0)], precision="float32", layer_sizes=(128, 128, 64, 1),
+                                    activation_fn=activations.get_fn_by_name(act), seed=5)
+            for p, q in zip(tr.parameters, ref.parameters):
+                p.copy_(q + (0.1 * torch.randn(q.shape, generator=gen)).to(q.device) * (q.dim() == 1))
+        ops = [tr.train_op_forces, tr.tower_force_rmses] + ([] if fused else [tr.tower_preds])
+        (row,) = list(tr.feed_dataset(ds, False, ops, n_mols))
+        assert (tr._force_fit is not None) == fused
+        return [p.grad for p in tr.parameters], row[1][0]
+
+    got, got_rmse = step("float32", True)
+    want, want_rmse = step("float64", False)
+    assert abs(got_rmse - want_rmse) < 1e-5 * want_rmse
+    norm = max(float(w.abs().max()) for w in want if w is not None)
+    # the autograd path clips its gradients in place (norm 5); the flat optimiser does so inside the update
+    total = float(torch.sqrt(sum((g.double() ** 2).sum() for g in got)))
+    scale = min(1.0, 5.0 / total)
+    for g, w in zip(got, want):
+        w = torch.zeros_like(g, dtype=torch.float64) if w is None else w
+        assert float((g.double() * scale - w).abs().max()) < 1e-4 * norm
