@@ -407,7 +407,7 @@ int ani_charge_grad_f64(const double* xs, const double* ys, const double* zs, co
  * coordinates before the cast, the sum formed in double (the coordinate fuzz of
  * RawDataset.iterate, drawn by the caller so that the random stream stays numpy's).
  * Destination: dst_xyz / dst_grads [3][dst_stride] and dst_ys in float (dst_is_f64 = 0) or
- * double, dst_types[cap_atoms], dst_mol_ids[cap_atoms] (index of the molecule within the batch),
+ * double, dst_types[cap_atoms], dst_mol_ids[cap_atoms] (index of the molecule within the batch; optional),
  * dst_mol_offsets / dst_mol_counts[cap_mols].  n_atoms_out receives the atoms of the batch and
  * acs_out[4] the atoms per element.  ANI_ERR_BAD_SIZE if the batch does not fit cap_atoms /
  * cap_mols (nothing is written then), ANI_ERR_BAD_INDEX for a pick outside the dataset.
@@ -439,6 +439,7 @@ typedef struct ani_host_pack_args {
     int* acs_out;
     const int* src_mol_acs;   /* optional [n_mols_total][4]: atoms per element of every molecule of the dataset;
                                  when given, the per-batch element counts are sums of these rows */
+    long long noise_stride;   /* 0: noise is [atoms of the batch][3]; else [3][noise_stride] */
 } ani_host_pack_args;
 int ani_host_pack_batch(const ani_host_pack_args* args);
 
@@ -577,6 +578,13 @@ typedef struct ani_feeder_batch {
 typedef struct ani_feeder ani_feeder;
 int ani_feeder_create(int device, const ani_feeder_slot* slots, int n_slots, ani_feeder** out);
 int ani_feeder_begin(ani_feeder* f, const long long* order, long long n_order, int batch_size);
+/* The same with coordinate noise, uniform in [-fuzz, fuzz): drawn by the feeder's thread from the MT19937 stream
+ * of numpy's legacy generator, whose state is key[624] and pos (np.random.get_state()), so the batches are the
+ * ones numpy would have given.  ani_feeder_random_state returns the state after the batches prepared so far; call
+ * it after ani_feeder_end. */
+int ani_feeder_begin_fuzz(ani_feeder* f, const long long* order, long long n_order, int batch_size, const unsigned* key,
+                          int pos, double fuzz);
+int ani_feeder_random_state(ani_feeder* f, unsigned* key, int* pos);
 int ani_feeder_next(ani_feeder* f, ani_feeder_batch* out);
 int ani_feeder_wait(ani_feeder* f, int slot, void* stream);
 int ani_feeder_release(ani_feeder* f, int slot, void* stream);

@@ -17,7 +17,7 @@ LIB_PATH = os.environ.get("ANI_B200_LIB") or os.path.join(_HERE, "libani_b200.so
 CSRC = os.path.join(_HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(_HERE), "include")
 SOURCES = ["ani_b200.cu"]
-HEADERS = ["ani_params.h", "ani_common.cuh", "ani_device_math.cuh", "ani_feeder.h", "ani_peer.cuh", "ani_sort.cuh", "ani_featurize.cuh", "ani_featurize_mol.cuh", "ani_featurize_large.cuh", "ani_featurize_round_passes.inl", "ani_grad.cuh", "ani_grad_mol.cuh", "ani_grad_pair_pass.inl",
+HEADERS = ["ani_params.h", "ani_common.cuh", "ani_device_math.cuh", "ani_feeder.h", "ani_mt19937.h", "ani_peer.cuh", "ani_sort.cuh", "ani_featurize.cuh", "ani_featurize_mol.cuh", "ani_featurize_large.cuh", "ani_featurize_round_passes.inl", "ani_grad.cuh", "ani_grad_mol.cuh", "ani_grad_pair_pass.inl",
            "ani_grad_inverse.cuh", "ani_tangent_mol.cuh", "ani_mlp.cuh", "ani_mlp_pipe.cuh", "ani_mlp_forward.cuh", "ani_mlp_backward.cuh", "ani_mlp_wgrad.cuh", "ani_mlp_small.cuh", "ani_mlp_tangent.cuh", "ani_launch.cuh", "ani_charge.cuh", "ani_optim.cuh", "ani_energy.cuh", "ani_host_pack.h"]
 
 NVCC_FLAGS = [
@@ -59,7 +59,7 @@ class HostPackArgs(ctypes.Structure):
                 ("dst_is_f64", ctypes.c_int), ("dst_types", ctypes.c_void_p), ("dst_mol_ids", ctypes.c_void_p),
                 ("dst_mol_offsets", ctypes.c_void_p), ("dst_mol_counts", ctypes.c_void_p),
                 ("cap_atoms", ctypes.c_int), ("cap_mols", ctypes.c_int), ("n_atoms_out", ctypes.c_void_p),
-                ("acs_out", ctypes.c_void_p), ("src_mol_acs", ctypes.c_void_p)]
+                ("acs_out", ctypes.c_void_p), ("src_mol_acs", ctypes.c_void_p), ("noise_stride", ctypes.c_longlong)]
 
 
 class FeederSlot(ctypes.Structure):
@@ -157,6 +157,8 @@ SIGNATURES = {
     "ani_energy_pass_f64": (_i, [ctypes.POINTER(EnergyArgs64), _vp]),
     "ani_feeder_create": (_i, [_i, _vp, _i, ctypes.POINTER(_vp)]),
     "ani_feeder_begin": (_i, [_vp, _vp, ctypes.c_longlong, _i]),
+    "ani_feeder_begin_fuzz": (_i, [_vp, _vp, ctypes.c_longlong, _i, _vp, _i, ctypes.c_double]),
+    "ani_feeder_random_state": (_i, [_vp, _vp, ctypes.POINTER(_i)]),
     "ani_feeder_next": (_i, [_vp, ctypes.POINTER(FeederBatch)]),
     "ani_feeder_wait": (_i, [_vp, _i, _vp]),
     "ani_feeder_release": (_i, [_vp, _i, _vp]),

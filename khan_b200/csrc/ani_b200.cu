@@ -1032,7 +1032,18 @@ int ani_feeder_create(int device, const ani_feeder_slot* slots, int n_slots, ani
 
 int ani_feeder_begin(ani_feeder* f, const long long* order, long long n_order, int batch_size)
 {
-    return f ? f->impl.begin(order, n_order, batch_size) : ANI_ERR_NULL_POINTER;
+    return f ? f->impl.begin(order, n_order, batch_size, nullptr, 0, 0.0) : ANI_ERR_NULL_POINTER;
+}
+
+int ani_feeder_begin_fuzz(ani_feeder* f, const long long* order, long long n_order, int batch_size, const unsigned* key,
+                          int pos, double fuzz)
+{
+    return f && key ? f->impl.begin(order, n_order, batch_size, key, pos, fuzz) : ANI_ERR_NULL_POINTER;
+}
+
+int ani_feeder_random_state(ani_feeder* f, unsigned* key, int* pos)
+{
+    return f && key && pos ? f->impl.random_state(key, pos) : ANI_ERR_NULL_POINTER;
 }
 
 int ani_feeder_next(ani_feeder* f, ani_feeder_batch* out)

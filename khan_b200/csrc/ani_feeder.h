@@ -1,4 +1,4 @@
-// Submitter thread of the batch feeder in native code: packs the batches of one pass over a packed
+// Submitter threads of the batch feeder in native code: packs the batches of one pass over a packed
 // data set into a ring of pinned host arenas and uploads each with one asynchronous copy on its own
 // copy stream, ahead of the consumer.  The reference does this with a Python thread that runs
 // feed_dict into a TensorFlow FIFOQueue (khan/training/trainer_multi_tower.py:749-828); a Python
@@ -26,6 +26,7 @@
 
 #include "../../include/ani_b200.h"
 #include "ani_host_pack.h"
+#include "ani_mt19937.h"
 
 namespace ani {
 
@@ -80,23 +81,32 @@ public:
     }
 
     // Starts a pass: batch b is the molecules order[b * batch_size ... ) of the data set.
-    int begin(const long long* order, long long n_order, int batch_size)
+    // With `key` (the 624 words and the position of numpy's MT19937 state) every coordinate of a batch gets
+    // noise uniform in [-fuzz, fuzz), drawn x of all atoms, then y, then z.
+    int begin(const long long* order, long long n_order, int batch_size, const unsigned* key, int pos, double fuzz)
     {
         if (n_order < 0 || batch_size <= 0 || (n_order > 0 && !order)) return ANI_ERR_BAD_SIZE;
+        if (key && (pos < 0 || pos > Mt19937::kN)) return ANI_ERR_BAD_SIZE;
         end();
+        noisy_ = key != nullptr;
+        fuzz_ = fuzz;
+        if (noisy_) random_.set(key, pos);
         order_.assign(order, order + n_order);
         batch_size_ = batch_size;
         n_batches_ = (n_order + batch_size - 1) / batch_size;
         {
             std::lock_guard<std::mutex> lk(mu_);
             stop_ = false;
-            finished_ = false;
+            finished_ = n_batches_ == 0;
+            next_batch_ = noise_turn_ = publish_turn_ = 0;
             error_ = ANI_OK;
             free_.clear();
             ready_.clear();
             for (int s = 0; s < (int)slots_.size(); s++) free_.push_back(s);
         }
-        thread_ = std::thread([this] { run(); });
+        // Packing 1024 shuffled molecules takes a core 0.1 ms, their noise as much again, the GPU 0.15 ms: one thread
+        // could not keep up.  A second one is worth its start (30 us) from the third batch on.
+        for (int t = 0; t < (n_batches_ > 2 ? 2 : 1); t++) threads_.emplace_back([this] { run(); });
         return ANI_OK;
     }
 
@@ -152,7 +162,16 @@ public:
             stop_ = true;
         }
         cv_.notify_all();
-        if (thread_.joinable()) thread_.join();
+        for (std::thread& t : threads_) t.join();
+        threads_.clear();
+    }
+
+    // State of the random stream behind the batches prepared so far; only after end().
+    int random_state(unsigned* key, int* pos)
+    {
+        if (!threads_.empty()) return ANI_ERR_BAD_SIZE;
+        random_.get(key, pos);
+        return ANI_OK;
     }
 
     // Host wait for every copy this feeder has enqueued (before the arenas are reused elsewhere).
@@ -167,22 +186,34 @@ private:
     {
         {
             std::lock_guard<std::mutex> lk(mu_);
-            error_ = code;
+            if (!error_) error_ = code;
             finished_ = true;
         }
         cv_.notify_all();
     }
 
+    // True when the pass is being stopped, or has failed, while waiting for `ready`; `lk` holds mu_.
+    template <typename F> bool wait_or_stop(std::unique_lock<std::mutex>& lk, F ready)
+    {
+        cv_.wait(lk, [&] { return ready() || stop_ || error_; });
+        return stop_ || error_;
+    }
+
+    // One of the submitter's threads.  Batches are taken, given their noise and published in order; what lies
+    // between, the packing, overlaps.
     void run()
     {
         if (device_ >= 0 && cudaSetDevice(device_) != cudaSuccess) return fail(ANI_ERR_CUDA);
         const long long n_order = (long long)order_.size();
-        for (long long b = 0; b < n_batches_; b++) {
+        std::vector<double> noise;
+        for (;;) {
+            long long b;
             int s;
             {
                 std::unique_lock<std::mutex> lk(mu_);
-                cv_.wait(lk, [this] { return !free_.empty() || stop_; });
-                if (stop_) return;
+                if (wait_or_stop(lk, [this] { return !free_.empty() || next_batch_ >= n_batches_; })) return;
+                if (next_batch_ >= n_batches_) return;
+                b = next_batch_++;
                 s = free_.front();
                 free_.pop_front();
             }
@@ -195,12 +226,38 @@ private:
             ani_host_pack_args a = sl.args;
             a.picks = order_.data() + first;
             a.n_picks = (int)((n_order - first < batch_size_) ? n_order - first : batch_size_);
-            a.noise = nullptr;
             a.n_atoms_out = &sl.n_atoms;
             a.acs_out = sl.acs;
+            a.noise = nullptr;
+            if (noisy_) {
+                long long n = 0;
+                for (int m = 0; m < a.n_picks; m++) {
+                    const long long p = a.picks[m];
+                    if (p < 0 || p >= a.n_mols_total) return fail(ANI_ERR_BAD_INDEX);
+                    n += a.mol_ptr[p + 1] - a.mol_ptr[p];
+                }
+                if (n > a.cap_atoms) return fail(ANI_ERR_BAD_SIZE);
+                noise.resize((size_t)(3 * n));
+                {
+                    std::unique_lock<std::mutex> lk(mu_);
+                    if (wait_or_stop(lk, [&] { return noise_turn_ == b; })) return;
+                }
+                random_.uniform(noise.data(), 3 * n, -fuzz_, fuzz_ - -fuzz_);
+                {
+                    std::lock_guard<std::mutex> lk(mu_);
+                    noise_turn_ = b + 1;
+                }
+                cv_.notify_all();
+                a.noise = noise.data();
+                a.noise_stride = n;
+            }
             if (int rc = host_pack_batch(a)) return fail(rc);
             sl.n_mols = a.n_picks;
             sl.batch_index = b;
+            {
+                std::unique_lock<std::mutex> lk(mu_);
+                if (wait_or_stop(lk, [&] { return publish_turn_ == b; })) return;
+            }
             if (device_ >= 0) {
                 if (sl.has_consumed && cudaStreamWaitEvent(copy_stream_, sl.consumed, 0) != cudaSuccess)
                     return fail(ANI_ERR_CUDA);
@@ -214,14 +271,11 @@ private:
             {
                 std::lock_guard<std::mutex> lk(mu_);
                 ready_.push_back(s);
+                publish_turn_ = b + 1;
+                finished_ = publish_turn_ == n_batches_;
             }
             cv_.notify_all();
         }
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            finished_ = true;
-        }
-        cv_.notify_all();
     }
 
     int device_;
@@ -230,12 +284,16 @@ private:
     std::vector<long long> order_;
     int batch_size_ = 1;
     long long n_batches_ = 0;
-    std::thread thread_;
+    long long next_batch_ = 0, noise_turn_ = 0, publish_turn_ = 0;
+    std::vector<std::thread> threads_;
     std::mutex mu_;
     std::condition_variable cv_;
     std::deque<int> free_, ready_;
     bool stop_ = true, finished_ = true;
     int error_ = ANI_OK;
+    bool noisy_ = false;
+    double fuzz_ = 0.0;
+    Mt19937 random_;
 };
 
 }  // namespace ani

@@ -24,7 +24,10 @@ inline void pack_coordinates(const ani_host_pack_args& a)
         for (int c = 0; c < 3; c++) {
             const SRC* s = src + (long long)c * a.src_stride + s0;
             DST* d = dst + (long long)c * a.dst_stride + d0;
-            if (a.noise) {      // noise is [n_total][3] doubles; the sum is formed in double, as numpy does
+            if (a.noise && a.noise_stride) {      // [3][noise_stride]; the sum is formed in double, as numpy does
+                const double* nz = a.noise + (size_t)c * a.noise_stride + d0;
+                for (long long k = 0; k < cnt; k++) d[k] = (DST)((double)s[k] + nz[k]);
+            } else if (a.noise) {                 // [n_total][3]
                 const double* nz = a.noise + 3 * d0 + c;
                 for (long long k = 0; k < cnt; k++) d[k] = (DST)((double)s[k] + nz[3 * k]);
             } else if (sizeof(SRC) == sizeof(DST)) {
@@ -38,8 +41,7 @@ inline void pack_coordinates(const ani_host_pack_args& a)
 
 inline int host_pack_batch(const ani_host_pack_args& a)
 {
-    if (!a.picks || !a.mol_ptr || !a.src_xyz || !a.src_types || !a.dst_xyz || !a.dst_types || !a.dst_mol_ids ||
-        !a.dst_mol_offsets || !a.dst_mol_counts || !a.n_atoms_out || !a.acs_out)
+    if (!a.picks || !a.mol_ptr || !a.src_xyz || !a.src_types || !a.dst_xyz || !a.dst_types || !a.dst_mol_offsets || !a.dst_mol_counts || !a.n_atoms_out || !a.acs_out)
         return ANI_ERR_NULL_POINTER;
     if (a.n_picks < 0 || a.n_picks > a.cap_mols || a.n_mols_total < 0 || a.cap_atoms < 0) return ANI_ERR_BAD_SIZE;
     if ((a.src_ys && !a.dst_ys) || (a.src_grads && !a.dst_grads)) return ANI_ERR_NULL_POINTER;
@@ -64,13 +66,20 @@ inline int host_pack_batch(const ani_host_pack_args& a)
     const size_t esize = a.dst_is_f64 ? 8 : 4;
     // Consecutive picks (an unshuffled pass: predict, evaluation) are one contiguous range of every
     // array of the data set: whole-range copies instead of one small copy per molecule and array.
-    bool consecutive = a.n_picks > 0 && !a.noise && a.src_is_f64 == a.dst_is_f64;
+    bool consecutive = a.n_picks > 0 && !a.noise && (a.src_is_f64 || !a.dst_is_f64);
     for (int m = 1; consecutive && m < a.n_picks; m++) consecutive = a.picks[m] == a.picks[0] + m;
     if (consecutive) {
         const long long s0 = a.mol_ptr[a.picks[0]];
         for (int c = 0; c < 3; c++) {
-            std::memcpy(static_cast<char*>(a.dst_xyz) + (size_t)c * a.dst_stride * esize,
-                        static_cast<const char*>(a.src_xyz) + ((size_t)c * a.src_stride + s0) * esize, (size_t)n * esize);
+            if (a.src_is_f64 == a.dst_is_f64) {
+                std::memcpy(static_cast<char*>(a.dst_xyz) + (size_t)c * a.dst_stride * esize,
+                            static_cast<const char*>(a.src_xyz) + ((size_t)c * a.src_stride + s0) * esize,
+                            (size_t)n * esize);
+            } else {      // the loaders give doubles, the float32 networks take floats
+                const double* s = static_cast<const double*>(a.src_xyz) + (size_t)c * a.src_stride + s0;
+                float* d = static_cast<float*>(a.dst_xyz) + (size_t)c * a.dst_stride;
+                for (long long k = 0; k < n; k++) d[k] = (float)s[k];
+            }
             if (a.src_grads)
                 std::memcpy(static_cast<char*>(a.dst_grads) + (size_t)c * a.dst_stride * esize,
                             static_cast<const char*>(a.src_grads) + ((size_t)c * a.src_stride + s0) * esize,
@@ -81,7 +90,7 @@ inline int host_pack_batch(const ani_host_pack_args& a)
             std::memcpy(a.dst_ys, static_cast<const char*>(a.src_ys) + (size_t)a.picks[0] * esize, (size_t)a.n_picks * esize);
         for (int m = 0; m < a.n_picks; m++) {
             const long long d0 = a.dst_mol_offsets[m], cnt = a.dst_mol_counts[m];
-            std::fill(a.dst_mol_ids + d0, a.dst_mol_ids + d0 + cnt, (long long)m);
+            if (a.dst_mol_ids) std::fill(a.dst_mol_ids + d0, a.dst_mol_ids + d0 + cnt, (long long)m);
             if (a.src_mol_acs) {
                 const int* row = a.src_mol_acs + 4 * a.picks[m];
                 for (int t = 0; t < 4; t++) acs[t] += row[t];
@@ -106,7 +115,7 @@ inline int host_pack_batch(const ani_host_pack_args& a)
     for (int m = 0; m < a.n_picks; m++) {
         const long long s0 = a.mol_ptr[a.picks[m]], cnt = a.mol_ptr[a.picks[m] + 1] - s0, d0 = a.dst_mol_offsets[m];
         std::memcpy(a.dst_types + d0, a.src_types + s0, (size_t)cnt * sizeof(int));
-        std::fill(a.dst_mol_ids + d0, a.dst_mol_ids + d0 + cnt, (long long)m);
+        if (a.dst_mol_ids) std::fill(a.dst_mol_ids + d0, a.dst_mol_ids + d0 + cnt, (long long)m);
         if (a.src_mol_acs) {
             const int* row = a.src_mol_acs + 4 * a.picks[m];
             for (int t = 0; t < 4; t++) acs[t] += row[t];

@@ -193,9 +193,10 @@ class PackedDataset:
 
 def _layout(cap_atoms: int, cap_mols: int, itemsize: int):
     """Byte offsets of the sections of a slot; every section starts on a 256-byte boundary."""
-    sections = [("xyz", 3 * cap_atoms * itemsize), ("grads", 3 * cap_atoms * itemsize),
-                ("ys", cap_mols * itemsize), ("mol_ids", cap_atoms * 8), ("types", cap_atoms * 4),
-                ("mol_offsets", cap_mols * 4), ("mol_counts", cap_mols * 4)]
+    # what every batch has comes first, so that the upload can stop before what a pass does not use
+    sections = [("xyz", 3 * cap_atoms * itemsize), ("types", cap_atoms * 4), ("mol_offsets", cap_mols * 4),
+                ("mol_counts", cap_mols * 4), ("ys", cap_mols * itemsize), ("grads", 3 * cap_atoms * itemsize),
+                ("mol_ids", cap_atoms * 8)]
     table, off = {}, 0
     for name, size in sections:
         table[name] = (off, size)
@@ -232,6 +233,11 @@ class HostSlot:
         self.acs = np.zeros(4, np.int32)
 
 
+    def used_bytes(self, has_grads: bool, mol_ids: bool) -> int:
+        """Length of the part of the arena that a pass with these arrays uses."""
+        return self.nbytes if mol_ids else self.table["mol_ids" if has_grads else "grads"][0]
+
+
 def arena_views(host: "HostSlot", arena: torch.Tensor) -> dict:
     """Full-capacity typed views of the arrays laid out in ``arena`` (a device or host copy of the slot's
     arena).  Built once per slot: a batch only slices them."""
@@ -251,7 +257,8 @@ class FedBatch:
     """What the feeder hands to the consumer: tensors of one batch (device tensors when the
     feeder has a device, host tensors otherwise) plus the host-side sizes the C ABI needs."""
 
-    def __init__(self, index: int, device, host: HostSlot, arena: torch.Tensor, ready, views=None, waiter=None):
+    def __init__(self, index: int, device, host: HostSlot, arena: torch.Tensor, ready, views=None, waiter=None,
+                 mol_ids=True):
         self.index, self.device, self.ready = index, device, ready
         self._waiter = waiter    # native submitter: makes a stream wait for the slot's upload
         n, m = host.n_atoms, host.n_mols
@@ -265,7 +272,7 @@ class FedBatch:
         self.types = v["types"][:n]
         self.mol_offsets = v["mol_offsets"][:m]
         self.mol_counts = v["mol_counts"][:m]
-        self.mol_ids = v["mol_ids"][:n]
+        self.mol_ids = v["mol_ids"][:n] if mol_ids else None
         self.ys = v["ys"][:m] if host.has_ys else None
         self.grads = v["grads"][:, :n] if host.has_grads else None
 
@@ -335,10 +342,10 @@ def _drop_native(ring) -> None:
         nat["owner"].__del__()
 
 
-def _native_submitter(ring, packed: "PackedDataset", dev) -> dict:
+def _native_submitter(ring, packed: "PackedDataset", dev, mol_ids: bool) -> dict:
     """The native submitter bound to (ring, data set), made once and kept with the ring."""
     nat = ring[0].get("native")
-    if nat is not None and nat["packed"] is packed:
+    if nat is not None and nat["packed"] is packed and nat["mol_ids"] == mol_ids:
         return nat
     _drop_native(ring)
     for slot in ring:       # what a Python submitter left behind on these slots
@@ -354,12 +361,14 @@ def _native_submitter(ring, packed: "PackedDataset", dev) -> dict:
         packed.fill_pack_args(arr[k].pack, host)
         arr[k].host_arena = host.arena.data_ptr()
         arr[k].dev_arena = None if dev is None else slot["arena"].data_ptr()
-        arr[k].nbytes = host.nbytes
+        arr[k].nbytes = host.used_bytes(packed.grads is not None, mol_ids)
+        if not mol_ids:
+            arr[k].pack.dst_mol_ids = None
         host.pack_args = None
     index = -1 if dev is None else (torch.device(dev).index if torch.device(dev).index is not None
                                     else torch.cuda.current_device())
     owner = _NativeHandle(index, arr, n)
-    nat = {"owner": owner, "handle": owner.ptr, "packed": packed, "slots": arr, "batch": _lib.FeederBatch(),
+    nat = {"owner": owner, "handle": owner.ptr, "packed": packed, "mol_ids": mol_ids, "slots": arr, "batch": _lib.FeederBatch(),
            "order": None, "keep": (packed.xyz, packed.types, packed.ys, packed.grads, packed.ptr, packed.mol_acs())}
     ring[0]["native"] = nat
     return nat
@@ -377,7 +386,7 @@ class BatchFeeder:
     """
 
     def __init__(self, packed: PackedDataset, batch_size: int, shuffle: bool, fuzz=None, devices=None,
-                 depth: int = 2, hold=None):
+                 depth: int = 2, hold=None, mol_ids: bool = True):
         self.packed, self.batch_size, self.shuffle, self.fuzz = packed, batch_size, shuffle, fuzz
         self.devices = list(devices) if devices else [None]
         self.depth = max(1, depth)
@@ -398,11 +407,15 @@ class BatchFeeder:
         self._started = False
         self._finished = False
         self._held = []
-        # One device and no fuzz (whose draws come from numpy's global generator, batch by batch): the
-        # submitter is the library's native thread, and the interpreter lock stays with the consumer.
+        # One device: the submitter is the library's native thread, and the interpreter lock stays with the
+        # consumer.  It draws the fuzz itself from numpy's global stream (ani_mt19937.h) unless the global
+        # generator has been replaced by another kind.
         self._native = None
-        if fuzz is None and len(self.devices) == 1:
-            self._native = _native_submitter(self._slots[0], packed, self.devices[0])
+        self._random = None       # numpy's state when the pass began
+        self.mol_ids = True
+        if len(self.devices) == 1 and (fuzz is None or np.random.get_state(legacy=False)["bit_generator"] == "MT19937"):
+            self.mol_ids = mol_ids      # the per-atom molecule index, for consumers that read FedBatch.mol_ids
+            self._native = _native_submitter(self._slots[0], packed, self.devices[0], mol_ids)
         else:
             for ring in self._slots:
                 _drop_native(ring)
@@ -474,8 +487,15 @@ class BatchFeeder:
             if self.shuffle:
                 np.random.shuffle(perm)
             nat["order"] = perm     # read by the native thread until the pass ends
-            _lib.check(L.ani_feeder_begin(nat["handle"], perm.ctypes.data, len(perm), self.batch_size),
-                       "ani_feeder_begin")
+            if self.fuzz is None:
+                _lib.check(L.ani_feeder_begin(nat["handle"], perm.ctypes.data, len(perm), self.batch_size),
+                           "ani_feeder_begin")
+            else:
+                self._random = np.random.get_state()
+                key = np.ascontiguousarray(self._random[1], dtype=np.uint32)
+                _lib.check(L.ani_feeder_begin_fuzz(nat["handle"], perm.ctypes.data, len(perm), self.batch_size,
+                                                   key.ctypes.data, int(self._random[2]), float(self.fuzz)),
+                           "ani_feeder_begin_fuzz")
         while len(self._held) >= self.hold:
             self.release(self._held[0][2])
         fb = nat["batch"]
@@ -500,7 +520,7 @@ class BatchFeeder:
 
             def waiter(s=s):
                 _lib.check(L.ani_feeder_wait(handle, s, self._stream_ptr()), "ani_feeder_wait")
-        fed = FedBatch(int(fb.batch_index), dev, host, slot["arena"], None, slot["views"], waiter)
+        fed = FedBatch(int(fb.batch_index), dev, host, slot["arena"], None, slot["views"], waiter, self.mol_ids)
         self._held.append((0, s, fed))
         return fed
 
@@ -540,6 +560,21 @@ class BatchFeeder:
                 self._free[tower].put(s)
                 return
 
+    def _advance_numpy(self) -> None:
+        """Moves numpy's global stream past the draws of the native submitter -- unless somebody else has drawn
+        from it meanwhile: then it stays where that left it."""
+        if self._random is None:
+            return
+        kind, key, pos, has_gauss, cached = self._random
+        self._random = None
+        now = np.random.get_state()
+        if now[0] != kind or now[2] != pos or not np.array_equal(now[1], key):
+            return
+        new_key, new_pos = np.zeros(624, np.uint32), ctypes.c_int(0)
+        _lib.check(_lib.lib().ani_feeder_random_state(self._native["handle"], new_key.ctypes.data, ctypes.byref(new_pos)),
+                   "ani_feeder_random_state")
+        np.random.set_state((kind, new_key, new_pos.value, has_gauss, cached))
+
     def close(self) -> None:
         """Stops the submitter and hands the slot rings to the next feeder of the same shape.  Call it after
         the work on the last batches has been enqueued (the iterator does so when it is exhausted)."""
@@ -547,6 +582,7 @@ class BatchFeeder:
             if self._slots is None:
                 return
             _lib.lib().ani_feeder_end(self._native["handle"])
+            self._advance_numpy()
             for _, _, fed in list(self._held):
                 self.release(fed)
             self._native["order"] = None

@@ -356,7 +356,7 @@ class TrainerMultiTower:
                      and packed.grads is not None and packed.ys is not None and packed.num_mols() > 0)
         # the fused path works on two batches at a time (this one's networks, the next one's featurizer)
         it = BatchFeeder(packed, batch_size, shuffle, fuzz, devices=self.towers, depth=3 if fused else 2,
-                         hold=2 if fused else self.num_towers)
+                         hold=2 if fused else self.num_towers, mol_ids=not (fused or force_fit))
         try:
             if force_fit:
                 yield from self._force_rounds(it, names, packed.capacity(batch_size), before_hooks)
@@ -663,7 +663,7 @@ class TrainerMultiTower:
             twin = self._infer_twin = (StagedBatch(sb.n_atoms_cap, sb.n_mols_cap, self.precision, device=dev),
                                        torch.cuda.Stream(device=dev))
         sbs, side = (sb, twin[0]), twin[1]
-        it = BatchFeeder(packed, batch_size, False, None, devices=self.towers, depth=3, hold=2)
+        it = BatchFeeder(packed, batch_size, False, None, devices=self.towers, depth=3, hold=2, mol_ids=False)
         preds, l2s = [], []
 
         def start(fed, target):
@@ -703,7 +703,7 @@ class TrainerMultiTower:
         ring = getattr(self, "_grad_ring", None)
         if ring is None or ring[0].shape[0] < cap:
             ring = self._grad_ring = [torch.empty((cap, 3), dtype=self.precision).pin_memory() for _ in range(3)]
-        it = BatchFeeder(packed, batch_size, False, None, devices=self.towers, depth=2, hold=1)
+        it = BatchFeeder(packed, batch_size, False, None, devices=self.towers, depth=2, hold=1, mol_ids=False)
         pending = []      # (host buffer, event, n_atoms, batch index) of batches whose copy is in flight
         slices = packed.batch_slices(batch_size)
 
