@@ -25,6 +25,7 @@
 #include "ani_mlp_forward.cuh"
 #include "ani_mlp_backward.cuh"
 #include "ani_mlp_wgrad.cuh"
+#include "ani_mlp_chain.cuh"
 #include "ani_mlp_small.cuh"
 #include "ani_mlp_tangent.cuh"
 #include "ani_charge.cuh"
@@ -474,6 +475,38 @@ template <bool SPLIT> int mlp_backward_launch(const MlpBackwardParams& p, int n_
     return ANI_OK;
 }
 
+template <int ACT, bool SPLIT, int MODE> int mlp_chain_launch(const MlpChainParams& p, cudaStream_t st)
+{
+    auto kernel = mlp_chain_kernel<ACT, SPLIT, MODE>;
+    const size_t smem = sizeof(ChainShared);
+    static thread_local int configured_dev = -1;
+    int dev = 0;
+    ANI_CUDA(cudaGetDevice(&dev));
+    if (configured_dev != dev) {
+        if (int rc = set_smem(kernel, smem)) return rc;
+        configured_dev = dev;
+    }
+    ANI_CUDA(launch_chain(kernel, p.tile_start[kTypes], kChainThreads, smem, st, 1, p));
+    return ANI_OK;
+}
+template <int ACT, int MODE> int mlp_chain_split(const MlpChainParams& p, bool split, cudaStream_t st)
+{
+    return split ? mlp_chain_launch<ACT, true, MODE>(p, st) : mlp_chain_launch<ACT, false, MODE>(p, st);
+}
+template <int MODE> int mlp_chain_act(const MlpChainParams& p, int activation, bool split, cudaStream_t st)
+{
+    if constexpr (MODE == kChainBackward) {      // no activation in it
+        return mlp_chain_split<kActCelu, MODE>(p, split, st);
+    } else {
+        switch (activation) {
+            case kActCelu: return mlp_chain_split<kActCelu, MODE>(p, split, st);
+            case kActGaussian: return mlp_chain_split<kActGaussian, MODE>(p, split, st);
+            case kActNormal: return mlp_chain_split<kActNormal, MODE>(p, split, st);
+            default: return mlp_chain_split<kActSoftplus, MODE>(p, split, st);
+        }
+    }
+}
+
 template <bool SPLIT> int mlp_wgrad_launch(const MlpWgradParams& p, int n_ranges, cudaStream_t st)
 {
     auto kernel = mlp_wgrad_kernel<SPLIT>;
@@ -533,7 +566,7 @@ int energy_launch(const T* atom_energy_sorted, const int* gather, const int* mos
 template <typename T>
 int mlp_small_launch(const T* feat, const int* acs, const T* const* w1, const T* const* b1, const T* const* w2,
                      const T* const* b2, const T* const* w3, const T* const* b3, const T* const* w4, const T* const* b4,
-                     const T* grad_energy, T* energy, T* grad_feat, int activation, cudaStream_t st)
+                     const T* grad_energy, T* energy, T* grad_feat, int activation, bool early_weights, cudaStream_t st)
 {
     if (activation < 0 || activation > 3) return ANI_ERR_BAD_SIZE;
     MlpSmallParams<T> p;
@@ -542,6 +575,7 @@ int mlp_small_launch(const T* feat, const int* acs, const T* const* w1, const T*
     p.energy = energy;
     p.grad_feat = grad_feat;
     p.activation = activation;
+    p.early_weights = early_weights;
     int tiles = 0, row = 0;
     if (!feat || !energy) return ANI_ERR_NULL_POINTER;
     if (!all_aligned16({feat, grad_feat})) return ANI_ERR_MISALIGNED;
@@ -571,6 +605,14 @@ int mlp_small_launch(const T* feat, const int* acs, const T* const* w1, const T*
     }
     ANI_CUDA(launch_chain(kernel, tiles * kSmallCtas, kSmallThreads, smem, st, kSmallCtas, p));
     return ANI_OK;
+}
+
+// True when every element that has atoms comes with packed weights.
+bool all_packed(const void* const* packed, const int* acs)
+{
+    for (int t = 0; t < kTypes; t++)
+        if (acs[t] > 0 && !packed[t]) return false;
+    return true;
 }
 
 // Adds the weight gradients described by p (range fields are set here).
@@ -649,6 +691,23 @@ int backward_call(const ani_mlp_backward_args* a, const int* acs_host, int split
         if (reinterpret_cast<uintptr_t>(a->packed[t]) & 15) return ANI_ERR_MISALIGNED;
     }
     p.tile_start[kTypes] = tiles;
+    if (all_packed(a->packed, acs_host)) {
+        MlpChainParams c = {};
+        for (int t = 0; t <= kTypes; t++) c.tile_start[t] = p.tile_start[t];
+        for (int t = 0; t < kTypes; t++) {
+            c.count[t] = p.count[t];
+            c.packed[t] = p.packed[t];
+            c.w4[t] = p.w4[t];
+            c.grad_energy[t] = p.grad_energy[t];
+            c.dact1[t] = const_cast<float*>(p.dact1[t]);
+            c.dact2[t] = const_cast<float*>(p.dact2[t]);
+            c.dact3[t] = const_cast<float*>(p.dact3[t]);
+            c.dz1[t] = p.dz1[t]; c.dz2[t] = p.dz2[t]; c.dz3[t] = p.dz3[t];
+            c.r1[t] = p.r1[t]; c.r2[t] = p.r2[t];
+            c.grad_feat[t] = p.grad_feat[t];
+        }
+        return mlp_chain_act<kChainBackward>(c, kActCelu, split_precision != 0, st);
+    }
     return split_precision ? mlp_backward_launch<true>(p, tiles, st) : mlp_backward_launch<false>(p, tiles, st);
 }
 
@@ -858,6 +917,21 @@ int ani_mlp_forward_f32(const ani_mlp_args* a, const int* acs_host, int activati
     p.tile_start[kTypes] = tiles;
     cudaStream_t st = (cudaStream_t)stream;
     const bool split = split_precision != 0;
+    if (all_packed(a->packed, acs_host)) {
+        MlpChainParams c = {};
+        for (int t = 0; t <= kTypes; t++) c.tile_start[t] = p.tile_start[t];
+        for (int t = 0; t < kTypes; t++) {
+            c.count[t] = p.count[t];
+            c.packed[t] = p.packed[t];
+            c.feat[t] = p.feat[t];
+            c.b1[t] = p.b1[t]; c.b2[t] = p.b2[t]; c.b3[t] = p.b3[t]; c.b4[t] = p.b4[t];
+            c.w4[t] = p.w4[t];
+            c.energy[t] = p.energy[t];
+            c.act1[t] = p.act1[t]; c.act2[t] = p.act2[t]; c.act3[t] = p.act3[t];
+            c.dact1[t] = p.dact1[t]; c.dact2[t] = p.dact2[t]; c.dact3[t] = p.dact3[t];
+        }
+        return mlp_chain_act<kChainForward>(c, activation, split, st);
+    }
     switch (activation) {
         case kActCelu: return mlp_launch_act<kActCelu>(p, tiles, split, st);
         case kActGaussian: return mlp_launch_act<kActGaussian>(p, tiles, split, st);
@@ -1257,8 +1331,34 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
             if (int rc = mlp_small_launch<float>(a->features, acs, a->w1, a->b1, a->w2, a->b2, a->w3, a->b3, a->w4, a->b4,
                                                  a->grad_energy_sorted, a->energy_sorted,
                                                  backward ? a->feature_grads : nullptr, a->activation,
-                                                 (cudaStream_t)stream))
+                                                 (a->phases & ANI_PASS_FEATURIZE) != 0, (cudaStream_t)stream))
                 return rc;
+        backward_done = true;
+    } else if ((a->phases & ANI_PASS_FORWARD) && (a->phases & ANI_PASS_BACKWARD) && transient && a->feature_grads &&
+               !(a->phases & ANI_PASS_WEIGHT_GRAD) && !a->labels && n_atoms > 0 && all_packed(a->packed, acs)) {
+        // energies + forces: forward and backward of a tile in one kernel, nothing of the networks in global memory
+        if (a->activation < 0 || a->activation > 3) return ANI_ERR_BAD_SIZE;
+        if (!a->features || !a->energy_sorted) return ANI_ERR_NULL_POINTER;
+        if (!all_aligned16({a->features, a->feature_grads})) return ANI_ERR_MISALIGNED;
+        MlpChainParams c = {};
+        int tiles = 0;
+        for (int t = 0; t < kTypes; t++) {
+            c.tile_start[t] = tiles;
+            c.count[t] = acs[t];
+            tiles += (acs[t] + kMlpTile - 1) / kMlpTile;
+            if (acs[t] == 0) continue;
+            if (!a->b1[t] || !a->b2[t] || !a->b3[t] || !a->w4[t] || !a->b4[t]) return ANI_ERR_NULL_POINTER;
+            if (!all_aligned16({a->packed[t]})) return ANI_ERR_MISALIGNED;
+            c.packed[t] = (const unsigned char*)a->packed[t];
+            c.feat[t] = rows(a->features, t, kTotal);
+            c.b1[t] = a->b1[t]; c.b2[t] = a->b2[t]; c.b3[t] = a->b3[t]; c.b4[t] = a->b4[t];
+            c.w4[t] = a->w4[t];
+            c.energy[t] = rows(a->energy_sorted, t, 1);
+            c.grad_energy[t] = rows(a->grad_energy_sorted, t, 1);
+            c.grad_feat[t] = rows(a->feature_grads, t, kTotal);
+        }
+        c.tile_start[kTypes] = tiles;
+        if (int rc = mlp_chain_act<kChainForces>(c, a->activation, a->split_precision != 0, (cudaStream_t)stream)) return rc;
         backward_done = true;
     } else if (a->phases & ANI_PASS_FORWARD) {
         // what only the backward steps read is not written when they do not follow
@@ -1352,7 +1452,8 @@ int ani_energy_pass_f64(const ani_energy_args_f64* a, void* stream)
         if (backward && !a->feature_grads) return ANI_ERR_NULL_POINTER;
         if (int rc = mlp_small_launch<double>(a->features, acs, a->w1, a->b1, a->w2, a->b2, a->w3, a->b3, a->w4, a->b4,
                                               nullptr, a->energy_sorted, backward ? a->feature_grads : nullptr,
-                                              a->activation, (cudaStream_t)stream))
+                                              a->activation, (a->phases & ANI_PASS_FEATURIZE) != 0,
+                                              (cudaStream_t)stream))
             return rc;
     }
     if ((a->phases & ANI_PASS_ENERGY) && a->n_mols > 0) {

@@ -15,10 +15,9 @@
 //   * epilogues read the accumulator with tcgen05.ld (warp w: rows 32 (w % 4) .., columns
 //     32 (w / 4) ..) and move 32 x 32 tiles to and from global memory through a per-warp
 //     transposition scratch, so that every 16-byte access covers whole 128-byte row segments.
-// With SPLIT = true every operand is staged as a high part (the value with its low 13 mantissa
-// bits cleared, exact in tf32) and a low part (the remainder), and hi*hi + hi*lo + lo*hi are
-// accumulated: three MMAs per step give products that are accurate to about 2^-21 instead of
-// the 2^-10 of plain tf32.
+// With SPLIT = true every operand is staged as a high part (the value rounded to tf32) and a low
+// part (the remainder), and hi*hi + hi*lo + lo*hi are accumulated: three MMAs per step give
+// products that are accurate to about 2^-22 instead of the 2^-11 of plain tf32.
 #pragma once
 
 #include "ani_common.cuh"

@@ -39,30 +39,24 @@ __device__ __forceinline__ unsigned long long pipe_desc(unsigned byte_addr)
     return d;
 }
 
+// An operand value as its tf32 part(s): rounded to nearest, and with SPLIT what that leaves.
+__device__ __forceinline__ float tf32_round(float x)
+{
+    unsigned r;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+    return __uint_as_float(r);
+}
 template <bool SPLIT> __device__ __forceinline__ void pipe_store4(unsigned char* hi, unsigned char* lo, int off, float4 v)
 {
-    if (SPLIT) {
-        float4 h, l;
-        h.x = __uint_as_float(__float_as_uint(v.x) & 0xffffe000u);
-        h.y = __uint_as_float(__float_as_uint(v.y) & 0xffffe000u);
-        h.z = __uint_as_float(__float_as_uint(v.z) & 0xffffe000u);
-        h.w = __uint_as_float(__float_as_uint(v.w) & 0xffffe000u);
-        l.x = v.x - h.x; l.y = v.y - h.y; l.z = v.z - h.z; l.w = v.w - h.w;
-        *reinterpret_cast<float4*>(hi + off) = h;
-        *reinterpret_cast<float4*>(lo + off) = l;
-    } else {
-        *reinterpret_cast<float4*>(hi + off) = v;
-    }
+    const float4 h = make_float4(tf32_round(v.x), tf32_round(v.y), tf32_round(v.z), tf32_round(v.w));
+    *reinterpret_cast<float4*>(hi + off) = h;
+    if (SPLIT) *reinterpret_cast<float4*>(lo + off) = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
 }
 template <bool SPLIT> __device__ __forceinline__ void pipe_store1(unsigned char* hi, unsigned char* lo, int off, float v)
 {
-    if (SPLIT) {
-        const float h = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
-        *reinterpret_cast<float*>(hi + off) = h;
-        *reinterpret_cast<float*>(lo + off) = v - h;
-    } else {
-        *reinterpret_cast<float*>(hi + off) = v;
-    }
+    const float h = tf32_round(v);
+    *reinterpret_cast<float*>(hi + off) = h;
+    if (SPLIT) *reinterpret_cast<float*>(lo + off) = v - h;
 }
 
 // (row, group of 4 K values) of direct-staging slot j of this thread: 8 consecutive rows first

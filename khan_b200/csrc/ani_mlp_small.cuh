@@ -46,6 +46,7 @@ template <typename T> struct MlpSmallParams {
     T* energy;                   // [atoms]
     T* grad_feat;                // [atoms][384], or null: forward only
     int activation;
+    int early_weights;           // a featurizer kernel of the same call precedes: the weights may be read ahead of it
 };
 
 template <typename T> struct MlpSmallShared {
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) mlp_small_kernel(const MlpSm
     const size_t row0 = (size_t)p.row_start[e] + row_in;
     const bool backward = p.grad_feat != nullptr;
 
+    if (!p.early_weights) pdl_wait();
     cluster_arrive();      // (0) every CTA of the cluster runs before the first store into its memory
     // ---- weights first (they do not depend on the features), then the features ----
     small_load(sh.w1c, kSmallC, p.w1[e] + kSmallC * rank, kMlpH1, kMlpIn, kSmallC);
