@@ -27,7 +27,7 @@
 #include "ani_mlp_wgrad.cuh"
 #include "ani_mlp_chain.cuh"
 #include "ani_mlp_small.cuh"
-#include "ani_mlp_tangent.cuh"
+#include "ani_force_fit.cuh"
 #include "ani_charge.cuh"
 #include "ani_optim.cuh"
 #include "ani_energy.cuh"
@@ -639,25 +639,6 @@ int wgrad_call(MlpWgradParams& p, int split_precision, cudaStream_t st)
     return split_precision ? mlp_wgrad_launch<true>(p, ranges, st) : mlp_wgrad_launch<false>(p, ranges, st);
 }
 
-template <int ACT, bool SPLIT> int mlp_tangent_launch(const MlpTangentParams& p, int n_tiles, cudaStream_t st)
-{
-    auto kernel = mlp_tangent_kernel<ACT, SPLIT>;
-    const size_t smem = sizeof(MlpShared) + 1024;
-    static thread_local int configured_dev = -1;
-    int dev = 0;
-    ANI_CUDA(cudaGetDevice(&dev));
-    if (configured_dev != dev) {
-        if (int rc = set_smem(kernel, smem)) return rc;
-        configured_dev = dev;
-    }
-    ANI_CUDA(launch_chain(kernel, n_tiles, kMlpAllThreads, smem, st, 1, p));
-    return ANI_OK;
-}
-template <int ACT> int mlp_tangent_act(const MlpTangentParams& p, int n_tiles, bool split, cudaStream_t st)
-{
-    return split ? mlp_tangent_launch<ACT, true>(p, n_tiles, st) : mlp_tangent_launch<ACT, false>(p, n_tiles, st);
-}
-
 // ani_mlp_backward_f32, with dL/dA_l of the two inner layers in r1 and r2 (element-sorted rows) when given.
 int backward_call(const ani_mlp_backward_args* a, const int* acs_host, int split_precision, float* r1, float* r2,
                   cudaStream_t st)
@@ -684,7 +665,6 @@ int backward_call(const ani_mlp_backward_args* a, const int* acs_host, int split
         p.dact1[t] = a->dact1[t]; p.dact2[t] = a->dact2[t]; p.dact3[t] = a->dact3[t];
         p.dz1[t] = a->dz1[t]; p.dz2[t] = a->dz2[t]; p.dz3[t] = a->dz3[t];
         p.grad_feat[t] = a->grad_features[t];
-        p.packed[t] = (const unsigned char*)a->packed[t];
         p.r1[t] = r1 && acs_host[t] > 0 ? r1 + (size_t)row * kMlpH1 : nullptr;
         p.r2[t] = r2 && acs_host[t] > 0 ? r2 + (size_t)row * kMlpH2 : nullptr;
         row += acs_host[t];
@@ -696,7 +676,7 @@ int backward_call(const ani_mlp_backward_args* a, const int* acs_host, int split
         for (int t = 0; t <= kTypes; t++) c.tile_start[t] = p.tile_start[t];
         for (int t = 0; t < kTypes; t++) {
             c.count[t] = p.count[t];
-            c.packed[t] = p.packed[t];
+            c.packed[t] = (const unsigned char*)a->packed[t];
             c.w4[t] = p.w4[t];
             c.grad_energy[t] = p.grad_energy[t];
             c.dact1[t] = const_cast<float*>(p.dact1[t]);
@@ -911,7 +891,6 @@ int ani_mlp_forward_f32(const ani_mlp_args* a, const int* acs_host, int activati
         p.energy[t] = a->energy[t];
         p.act1[t] = a->act1[t]; p.act2[t] = a->act2[t]; p.act3[t] = a->act3[t];
         p.dact1[t] = a->dact1[t]; p.dact2[t] = a->dact2[t]; p.dact3[t] = a->dact3[t];
-        p.packed[t] = (const unsigned char*)a->packed[t];
         if (reinterpret_cast<uintptr_t>(a->packed[t]) & 15) return ANI_ERR_MISALIGNED;
     }
     p.tile_start[kTypes] = tiles;
@@ -922,7 +901,7 @@ int ani_mlp_forward_f32(const ani_mlp_args* a, const int* acs_host, int activati
         for (int t = 0; t <= kTypes; t++) c.tile_start[t] = p.tile_start[t];
         for (int t = 0; t < kTypes; t++) {
             c.count[t] = p.count[t];
-            c.packed[t] = p.packed[t];
+            c.packed[t] = (const unsigned char*)a->packed[t];
             c.feat[t] = p.feat[t];
             c.b1[t] = p.b1[t]; c.b2[t] = p.b2[t]; c.b3[t] = p.b3[t]; c.b4[t] = p.b4[t];
             c.w4[t] = p.w4[t];
@@ -1547,7 +1526,7 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
                           a->x_grads, a->y_grads, a->z_grads, f->fx, f->fy, f->fz, n, f->partial, f->vx, f->vy, f->vz,
                           f->rmse));
     float* rates[kTypes];
-    MlpTangentParams p;
+    MlpChainParams p = {};
     MlpWgradParams w1, w2;      // F^T Q and U^T P
     size_t row = 0;
     int tiles = 0;
@@ -1557,16 +1536,16 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
         p.count[t] = w1.count[t] = w2.count[t] = acs[t];
         p.tile_start[t] = tiles;
         tiles += (acs[t] + kMlpTile - 1) / kMlpTile;
-        p.u[t] = w2.feat[t] = rates[t];
+        p.feat[t] = w2.feat[t] = rates[t];
         p.w4[t] = a->w4[t];
         p.packed[t] = (const unsigned char*)a->packed[t];
-        p.act1[t] = w1.act1[t] = at(a->act1, kMlpH1);
-        p.act2[t] = w1.act2[t] = at(a->act2, kMlpH2);
+        w1.act1[t] = p.act1[t] = at(a->act1, kMlpH1);
+        w1.act2[t] = p.act2[t] = at(a->act2, kMlpH2);
         p.act3[t] = at(a->act3, kMlpH3);
         if (a->activation == kActCelu && f->z1 && f->z2 && f->z3) {
-            p.act1[t] = f->z1 + row * kMlpH1;
-            p.act2[t] = f->z2 + row * kMlpH2;
-            p.act3[t] = f->z3 + row * kMlpH3;
+            p.act1[t] = const_cast<float*>(f->z1) + row * kMlpH1;
+            p.act2[t] = const_cast<float*>(f->z2) + row * kMlpH2;
+            p.act3[t] = const_cast<float*>(f->z3) + row * kMlpH3;
         }
         p.dact1[t] = at(a->dact1, kMlpH1); p.dact2[t] = at(a->dact2, kMlpH2); p.dact3[t] = at(a->dact3, kMlpH3);
         p.r1[t] = at(f->r1, kMlpH1); p.r2[t] = at(f->r2, kMlpH2);
@@ -1592,15 +1571,7 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
                                                 rates[3], acs, stream))
         return rc;
     if (f->z_ready) ANI_CUDA(cudaStreamWaitEvent(st, (cudaEvent_t)f->z_ready, 0));
-    const bool split = a->split_precision != 0;
-    int rc = ANI_OK;
-    switch (a->activation) {
-        case kActCelu: rc = mlp_tangent_act<kActCelu>(p, tiles, split, st); break;
-        case kActGaussian: rc = mlp_tangent_act<kActGaussian>(p, tiles, split, st); break;
-        case kActNormal: rc = mlp_tangent_act<kActNormal>(p, tiles, split, st); break;
-        default: rc = mlp_tangent_act<kActSoftplus>(p, tiles, split, st);
-    }
-    if (rc) return rc;
+    if (int rc = mlp_chain_act<kChainTangent>(p, a->activation, a->split_precision != 0, st)) return rc;
     if (a->zero_ptr && a->zero_bytes) ANI_CUDA(cudaMemsetAsync(a->zero_ptr, 0, a->zero_bytes, st));
     if (int rc2 = wgrad_call(w1, a->split_precision, st)) return rc2;
     return wgrad_call(w2, a->split_precision, st);

@@ -56,7 +56,6 @@ struct MlpParams {
     float* dact1[kTypes];        // optional [count][128]: derivative of the activation at the same place
     float* dact2[kTypes];        // optional [count][128]
     float* dact3[kTypes];        // optional [count][64]
-    const unsigned char* packed[kTypes];   // optional: the weights pre-packed by mlp_pack_kernel
 };
 
 struct MlpShared {

@@ -1,21 +1,25 @@
 // Atomic networks 384-128-128-64-1 as ONE chain of products per tile of 128 atoms, on the tensor cores, with
-// packed weights: forward, forward + backward to the features, or backward alone.
+// packed weights: forward, forward + backward to the features, backward alone, or the second-order pass of
+// force training.
 //
 // Computes what ani_mlp_forward.cuh / ani_mlp_backward.cuh compute (AtomNN of the reference,
 // khan/model/nn.py:39-67,165-172, and its gradient, khan/training/trainer_multi_tower.py:350-419); those remain
-// for weights that are not packed.
+// for weights that are not packed.  The second-order pass is described in ani_force_fit.cuh.
 //
 // A tile is three products forward (K = 384, 128, 128) and five backward (K = 64, 128, 3 x 128), 38 chunks of 32
-// values of K, each 0.4 us of the tensor core (three tf32 products) and 32 KB of weights from L2 (0.3 us at
-// 64 B a clock).  The previous kernels took 1 us a chunk and 2-3 us between two products: two stages for both
-// operands, weights requested by a thread that also stages activations and runs epilogues, and every activation
-// through shared memory and back as the next A operand.  Here
+// values of K, each 0.4 us of the tensor core (three tf32 products).  The previous kernels took 1-2 us a chunk and
+// 2-3 us between two products: two stages for both operands, weights requested by a thread that also stages
+// activations and runs epilogues, and every activation through shared memory and back as the next A operand.  Here
 //   * one thread streams the weights through a ring of four stages, ahead over the whole chain, also across
 //     epilogues;
-//   * the activations never leave the tensor memory side: an epilogue reads the accumulator, splits the new
-//     activations into their tf32 parts and stores those to TMEM, where the next product takes its A operand
-//     (columns: accumulator 0-127, spare 128-255, A high 256-383, A low 384-511);
-//   * only the features go through shared memory (three stages, global loads two chunks ahead);
+//   * every A operand is in tensor memory: an epilogue reads the accumulator, splits the new activations into
+//     their tf32 parts and stores those to TMEM, where the next product takes them (columns: accumulator 0-127,
+//     spare 128-255, A high 256-383, A low 384-511).  The shared memory's 128 bytes a clock are what a chunk is
+//     short of: with both operands there, the products read 96 KB of it and staging wrote 64 KB, 1250 clocks
+//     against the tensor core's 830; now the weights are 80 KB of it;
+//   * the features of a chunk are copied to shared memory as they are (16 KB), four warps read them row by row and
+//     store their parts to TMEM; four groups of four warps take the chunks in turn (four stages of 64 columns in
+//     the place of the later A operands).
 //   * forward + backward in one kernel needs nothing of the activations in global memory: the derivatives of
 //     layer 1 wait in the spare columns, those of layer 2 where the feature stages were.
 // TODO_CHAIN
@@ -27,35 +31,39 @@
 
 namespace ani {
 
-constexpr int kChainA = 3, kChainB = 4;                 // stages of 32 KB (high and low part)
+constexpr int kChainA = 8, kChainB = 3;                 // feature chunks of 16 KB, weight stages of 32 KB (high, low)
 constexpr int kChainEpi = 512;                          // epilogue / staging threads (16 warps)
 constexpr int kChainThreads = kChainEpi + 64;           // + the MMA warp + the weight warp
+constexpr int kChainGroups = 4;                         // groups of 128 threads that take the feature chunks in turn
 constexpr unsigned kTmemAcc = 0, kTmemSpare = 128, kTmemHi = 256, kTmemLo = 384;
 
-enum ChainMode { kChainForward = 0, kChainForces = 1, kChainBackward = 2 };
+enum ChainMode { kChainForward = 0, kChainForces = 1, kChainBackward = 2, kChainTangent = 3 };
 
 struct MlpChainParams {
     int count[kTypes];
     int tile_start[kTypes + 1];
     const unsigned char* packed[kTypes];
-    const float* feat[kTypes];       // [count][384]                                   (forward)
+    const float* feat[kTypes];       // [count][384]          (forward; tangent: rates of the features)
     const float *b1[kTypes], *b2[kTypes], *b3[kTypes], *b4[kTypes];
     const float* w4[kTypes];         // [64]
     float* energy[kTypes];           // [count]
-    float *act1[kTypes], *act2[kTypes], *act3[kTypes];      // optional                 (forward)
-    float *dact1[kTypes], *dact2[kTypes], *dact3[kTypes];   // optional; read by the backward mode
+    float *act1[kTypes], *act2[kTypes], *act3[kTypes];      // optional (forward); read by the tangent mode (celu:
+                                                            // or pre-activations there, only the sign is used)
+    float *dact1[kTypes], *dact2[kTypes], *dact3[kTypes];   // optional; read by the backward and tangent modes
     const float* grad_energy[kTypes];   // [count], null: ones                          (forces, backward)
     float *dz1[kTypes], *dz2[kTypes], *dz3[kTypes];         //                          (backward)
-    float *r1[kTypes], *r2[kTypes];  // optional: dL/dA of the inner layers             (backward)
+    float *r1[kTypes], *r2[kTypes];  // optional: dL/dA of the inner layers (backward); read by the tangent mode
+    float *adot1[kTypes], *adot2[kTypes], *adot3[kTypes];   // rates of the activations (tangent)
+    float *q1[kTypes], *q2[kTypes], *q3[kTypes];            //                          (tangent)
     float* grad_feat[kTypes];        // [count][384]; optional in the backward mode
 };
 
 struct ChainShared {
-    alignas(1024) unsigned char a[kChainA][2 * kPipeOperandBytes];
+    alignas(1024) unsigned char a[kChainA][kPipeOperandBytes];
     alignas(1024) unsigned char b[kChainB][2 * kPipeOperandBytes];
     float bias[kMlpH1 + kMlpH2 + kMlpH3], w4[kMlpH3];
     float epart[kMlpTile];
-    alignas(8) unsigned long long a_full[kChainA], a_empty[kChainA], b_full[kChainB], b_empty[kChainB];
+    alignas(8) unsigned long long a_full[kChainGroups], a_empty[kChainGroups], b_full[kChainB], b_empty[kChainB];
     unsigned long long acc_full[2];      // accumulator (0) / spare (1) holds a finished product
     unsigned long long operand_ready;    // the epilogue has stored the next A operand
     unsigned long long acc_free;         // the epilogue has read the accumulator
@@ -105,6 +113,15 @@ struct ChainWait {
     }
 };
 
+// Second derivative of the activation from the activation a and its first derivative d.
+template <int ACT> __device__ __forceinline__ float mlp_activation_second(float a, float d)
+{
+    if (ACT == kActCelu) return a < 0.0f ? 10.0f * d : 0.0f;                       // exp(x / 0.1) / 0.1
+    if (ACT == kActGaussian) return a > 0.0f ? d * d / a - 2.0f * a : 0.0f;        // (4 x^2 - 2) a, d = -2 x a
+    if (ACT == kActNormal) return a > 0.0f ? d * d / a - a : 0.0f;                 // (x^2 - 1) a, d = -x a
+    return d * (1.0f - d);
+}
+
 template <int ACT, bool SPLIT, int MODE>
 __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpChainParams p)
 {
@@ -118,12 +135,12 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
     for (int t = 1; t < kTypes; t++) e += (int)blockIdx.x >= p.tile_start[t] ? 1 : 0;
     const int row0 = ((int)blockIdx.x - p.tile_start[e]) * kMlpTile;
     const int n_rows = min(kMlpTile, p.count[e] - row0);
-    const bool want_feat = kHasBackward && p.grad_feat[e] != nullptr;
+    const bool want_feat = kHasBackward && MODE != kChainTangent && p.grad_feat[e] != nullptr;
 
     if (warp == kChainEpi / 32) tmem_alloc(&sh.tmem_base, 512);
     if (tid == 0) {
-        for (int s = 0; s < kChainA; s++) {
-            mbar_init(&sh.a_full[s], kChainEpi);
+        for (int s = 0; s < kChainGroups; s++) {
+            mbar_init(&sh.a_full[s], kChainEpi / kChainGroups);
             mbar_init(&sh.a_empty[s], 1);
         }
         for (int s = 0; s < kChainB; s++) {
@@ -173,37 +190,26 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
         // ---- the products ----
         ChainWait wait;
         int bc = 0, ready = 0;
-        auto issue = [&](unsigned d, unsigned a_hi_smem, int k_chunk, int s, int N, bool first) {
+        auto issue = [&](unsigned d, unsigned a_hi, unsigned a_lo, int s, int N, bool first) {
             const unsigned idesc = instr_desc(kMlpTile, N);
             const unsigned b_hi = smem_u32(sh.b[s]), b_lo = b_hi + kPipeOperandBytes;
 #pragma unroll
             for (int ks = 0; ks < kPipeK / 8; ks++) {
-                const unsigned step = ks * 2 * kMlpLbo;
-                const bool acc = !(first && ks == 0);
-                if (a_hi_smem) {
-                    const unsigned a_lo = a_hi_smem + kPipeOperandBytes;
-                    mma_tf32(d, pipe_desc(a_hi_smem + step), pipe_desc(b_hi + step), idesc, acc);
-                    if (SPLIT) {
-                        mma_tf32(d, pipe_desc(a_hi_smem + step), pipe_desc(b_lo + step), idesc, true);
-                        mma_tf32(d, pipe_desc(a_lo + step), pipe_desc(b_hi + step), idesc, true);
-                    }
-                } else {
-                    const unsigned col = k_chunk * kPipeK + ks * 8;
-                    mma_tf32_ts(d, tmem + kTmemHi + col, pipe_desc(b_hi + step), idesc, acc);
-                    if (SPLIT) {
-                        mma_tf32_ts(d, tmem + kTmemHi + col, pipe_desc(b_lo + step), idesc, true);
-                        mma_tf32_ts(d, tmem + kTmemLo + col, pipe_desc(b_hi + step), idesc, true);
-                    }
+                const unsigned step = ks * 2 * kMlpLbo, col = ks * 8;
+                mma_tf32_ts(d, tmem + a_hi + col, pipe_desc(b_hi + step), idesc, !(first && ks == 0));
+                if (SPLIT) {
+                    mma_tf32_ts(d, tmem + a_hi + col, pipe_desc(b_lo + step), idesc, true);
+                    mma_tf32_ts(d, tmem + a_lo + col, pipe_desc(b_hi + step), idesc, true);
                 }
             }
         };
-        // one product with its A operand in tensor memory
+        // one product behind layer 1
         auto product = [&](unsigned d, int chunks, int N, unsigned long long* done) {
             for (int c = 0; c < chunks; c++, bc++) {
                 const int s = bc % kChainB;
                 if (wait(sh, &sh.b_full[s], (unsigned)(bc / kChainB) & 1u) && lane == 0) {
                     tc_fence_after();
-                    issue(tmem + d, 0u, c, s, N, c == 0);
+                    issue(tmem + d, kTmemHi + c * kPipeK, kTmemLo + c * kPipeK, s, N, c == 0);
                     mma_commit(&sh.b_empty[s]);
                     if (c == chunks - 1) mma_commit(done);
                 }
@@ -217,11 +223,11 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
         };
         if (kHasForward) {
             for (int c = 0; c < kMlpIn / kPipeK; c++, bc++) {
-                const int s = bc % kChainB, sa = c % kChainA;
-                wait(sh, &sh.a_full[sa], (unsigned)(c / kChainA) & 1u);
+                const int s = bc % kChainB, sa = c % kChainGroups;
+                wait(sh, &sh.a_full[sa], (unsigned)(c / kChainGroups) & 1u);
                 if (wait(sh, &sh.b_full[s], (unsigned)(bc / kChainB) & 1u) && lane == 0) {
                     tc_fence_after();
-                    issue(tmem + kTmemAcc, smem_u32(sh.a[sa]), 0, s, kMlpH1, c == 0);
+                    issue(tmem + kTmemAcc, kTmemHi + sa * 2 * kPipeK, kTmemHi + sa * 2 * kPipeK + kPipeK, s, kMlpH1, c == 0);
                     mma_commit(&sh.b_empty[s]);
                     mma_commit(&sh.a_empty[sa]);
                     if (c == kMlpIn / kPipeK - 1) mma_commit(&sh.acc_full[0]);
@@ -280,7 +286,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
             tc_fence_after();
         };
 
-        if (kHasForward) {
+        if (kHasForward && MODE != kChainTangent) {
             if (tid < kMlpH1) sh.bias[tid] = p.b1[e][tid];
             else if (tid < kMlpH1 + kMlpH2) sh.bias[tid] = p.b2[e][tid - kMlpH1];
             else if (tid < kMlpH1 + kMlpH2 + kMlpH3) sh.bias[tid] = p.b3[e][tid - kMlpH1 - kMlpH2];
@@ -289,36 +295,98 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
         producer_sync();
 
         if (kHasForward) {
-            // ---- layer 1: the features, loads two chunks ahead ----
+            // ---- layer 1: group g of 128 threads takes chunks g, g + 4, g + 8; thread = row (TMEM lane) ----
+            const int g = warp >> 2, me = tid & 127;
             const float* feat = p.feat[e] + (size_t)row0 * kMlpIn;
-            float4 reg[3][2];
-            auto load = [&](int c, float4* r) {
+            auto request = [&](int j) {      // 16-byte pieces, piece q of row r at place q ^ (r mod 8): no bank conflicts
+                unsigned char* dst = sh.a[g * 2 + (j & 1)];
+                const float* src = feat + (g + 4 * j) * kPipeK;
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    int rr, kg;
-                    pipe_slot(j, &rr, &kg);
-                    r[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (rr < n_rows) r[j] = *reinterpret_cast<const float4*>(feat + (size_t)rr * kMlpIn + c * kPipeK + kg * 4);
+                for (int i = 0; i < 8; i++) {
+                    const int rr = i * 16 + (me >> 3), q = me & 7;
+                    const unsigned bytes = rr < n_rows ? 16u : 0u;      // rows past the end become zeros
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                                     smem_u32(dst + rr * 128 + ((q ^ (rr & 7)) << 4))),
+                                 "l"(src + (size_t)(rr < n_rows ? rr : 0) * kMlpIn + q * 4), "r"(bytes)
+                                 : "memory");
                 }
+                asm volatile("cp.async.commit_group;" ::: "memory");
             };
-            load(0, reg[0]);
-            load(1, reg[1]);
+            request(0);
+            request(1);
 #pragma unroll
-            for (int c = 0; c < kMlpIn / kPipeK; c++) {
-                if (c + 2 < kMlpIn / kPipeK) load(c + 2, reg[(c + 2) % 3]);
-                const int s = c % kChainA;
-                if (c >= kChainA) wait(sh, &sh.a_empty[s], (unsigned)(c / kChainA - 1) & 1u);
+            for (int j = 0; j < 3; j++) {
+                if (j < 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                asm volatile("bar.sync %0, 128;" ::"r"(3 + g) : "memory");
+                float v[32];
+                const unsigned char* src = sh.a[g * 2 + (j & 1)] + me * 128;
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    int rr, kg;
-                    pipe_slot(j, &rr, &kg);
-                    const float4 v = reg[c % 3][j];
-                    const int off = pipe_offset(rr, kg * 4);
-                    pipe_store4<SPLIT>(sh.a[s], sh.a[s] + kPipeOperandBytes, off, v);
+                for (int q = 0; q < 8; q++) {
+                    const float4 x = *reinterpret_cast<const float4*>(src + ((q ^ (me & 7)) << 4));
+                    v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
                 }
-                fence_async_smem();
-                mbar_arrive(&sh.a_full[s]);
+                if (j == 0) {      // the buffer has been read: the group's last chunk
+                    asm volatile("bar.sync %0, 128;" ::"r"(3 + g) : "memory");
+                    request(2);
+                }
+                if (j > 0) {
+                    wait(sh, &sh.a_empty[g], (unsigned)(j - 1) & 1u);
+                    tc_fence_after();
+                }
+                float part[32];
+#pragma unroll
+                for (int i = 0; i < 32; i++) part[i] = tf32_round(v[i]);
+                tmem_store32(lanes + kTmemHi + g * 2 * kPipeK, part);
+                if (SPLIT) {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) part[i] = v[i] - part[i];
+                    tmem_store32(lanes + kTmemHi + g * 2 * kPipeK + kPipeK, part);
+                }
+                tmem_store_wait();
+                tc_fence_before();
+                mbar_arrive(&sh.a_full[g]);
             }
+            if (MODE == kChainTangent) {
+                // ---- A' = D T goes on, S T R stays (q); layer 3: its q is the first operand of the way back ----
+#pragma unroll 1
+                for (int l = 0; l < 3; l++) {
+                    const int N = l == 2 ? kMlpH3 : 128;
+                    if (c0 >= N) {
+                        accumulator();
+                        operand_done();
+                        continue;
+                    }
+                    const size_t g0 = atom0 * N + c0;
+                    float t[32], d[32], s[32];
+                    accumulator();
+                    warp_tile_from_global(scratch, s, (l == 0 ? p.act1[e] : (l == 1 ? p.act2[e] : p.act3[e])) + g0, N, tile_rows);
+                    warp_tile_from_global(scratch, d, (l == 0 ? p.dact1[e] : (l == 1 ? p.dact2[e] : p.dact3[e])) + g0, N,
+                                          tile_rows);
+#pragma unroll
+                    for (int i = 0; i < 32; i++) s[i] = mlp_activation_second<ACT>(s[i], d[i]);
+                    if (l < 2) {
+                        warp_tile_from_global(scratch, t, (l == 0 ? p.r1[e] : p.r2[e]) + g0, N, tile_rows);
+#pragma unroll
+                        for (int i = 0; i < 32; i++) s[i] *= t[i];
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; i++) s[i] *= sh.w4[c0 + i];
+                    }
+                    tmem_load32(lanes + kTmemAcc + c0, t);
+#pragma unroll
+                    for (int i = 0; i < 32; i++) {
+                        s[i] *= t[i];
+                        d[i] *= t[i];
+                    }
+                    if (l < 2) to_operand(d);
+                    else to_operand(s);
+                    operand_done();
+                    warp_tile_to_global<false>(scratch, d, (l == 0 ? p.adot1[e] : (l == 1 ? p.adot2[e] : p.adot3[e])) + g0, N,
+                                               tile_rows);
+                    warp_tile_to_global<false>(scratch, s, (l == 0 ? p.q1[e] : (l == 1 ? p.q2[e] : p.q3[e])) + g0, N, tile_rows);
+                }
+            } else {
             // ---- epilogues of layers 1 and 2 ----
 #pragma unroll 1
             for (int l = 0; l < 2; l++) {
@@ -386,6 +454,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                 }
             }
             if (MODE == kChainForces) operand_done();
+            }
         } else {
             // ---- dZ3 = g w4 D3 ----
             if (c0 < kMlpH3) {
@@ -407,7 +476,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
             for (int l = 1; l >= 0; l--) {
                 float v[32], d[32];
                 const float* dact = l == 1 ? p.dact2[e] : p.dact1[e];
-                if (MODE == kChainBackward)      // before the wait: the loads run under the product
+                if (MODE == kChainBackward || MODE == kChainTangent)      // before the wait: the loads run under the product
                     warp_tile_from_global(scratch, d, dact + atom0 * 128 + c0, 128, tile_rows);
                 accumulator();
                 tmem_load32(lanes + kTmemAcc + c0, v);
@@ -423,6 +492,18 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                 if (raw) warp_tile_to_global<false>(scratch, v, raw + atom0 * 128 + c0, 128, tile_rows);
 #pragma unroll
                 for (int i = 0; i < 32; i++) v[i] *= d[i];
+                if (MODE == kChainTangent) {      // + what this warp stored on the way forward
+                    float* q = (l == 1 ? p.q2[e] : p.q1[e]) + atom0 * 128 + c0;
+                    warp_tile_from_global(scratch, d, q, 128, tile_rows);
+#pragma unroll
+                    for (int i = 0; i < 32; i++) v[i] += d[i];
+                    if (l == 1) {
+                        to_operand(v);
+                        operand_done();
+                    }
+                    warp_tile_to_global<false>(scratch, v, q, 128, tile_rows);
+                    continue;
+                }
                 if (l == 1 || want_feat) {
                     to_operand(v);
                     operand_done();

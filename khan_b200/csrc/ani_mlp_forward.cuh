@@ -1,4 +1,5 @@
-// Per-element atomic network 384-128-128-64-1, forward pass, one kernel.
+// Per-element atomic network 384-128-128-64-1, forward pass, one kernel, for weights that are not packed (with
+// packed weights: ani_mlp_chain.cuh, which gives the same bits).
 //
 // What it computes is AtomNN of the reference (khan/model/nn.py:39-67): for the atoms of one
 // element, A1 = act(F W1 + b1), A2 = act(A1 W2 + b2), A3 = act(A2 W3 + b3), E = A3 w4 + b4, with
@@ -71,16 +72,8 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_forward_kernel(const Ml
             DirectGlobal<SPLIT> a_feat{p.feat[e] + (size_t)row0 * kMlpIn, (size_t)kMlpIn, kMlpTile, n_rows, 0};
             // B[n = out][k = in] = W[k][n]: the weights are read as stored ([in][out]) and transposed
             Transposed<SPLIT> b_w{layer_w[layer], (size_t)N, 0, N, 0, K, make_float4(0.f, 0.f, 0.f, 0.f)};
-            if (p.packed[e]) {      // pre-packed weights: one bulk copy per chunk instead of staging
-                const int first_chunk = layer == 0 ? kPackFwdL1 : (layer == 1 ? kPackFwdL2 : kPackFwdL3);
-                PackedB b_packed{p.packed[e] + (size_t)first_chunk * kPackedChunkBytes};
-                if (layer == 0) pipe_produce<SPLIT, false>(sh, K / kPipeK, ps, a_feat, a_sh, b_packed);
-                else pipe_produce<SPLIT, true>(sh, K / kPipeK, ps, a_feat, a_sh, b_packed);
-            } else if (layer == 0) {
-                pipe_produce<SPLIT, false>(sh, K / kPipeK, ps, a_feat, a_sh, b_w);
-            } else {
-                pipe_produce<SPLIT, true>(sh, K / kPipeK, ps, a_feat, a_sh, b_w);
-            }
+            if (layer == 0) pipe_produce<SPLIT, false>(sh, K / kPipeK, ps, a_feat, a_sh, b_w);
+            else pipe_produce<SPLIT, true>(sh, K / kPipeK, ps, a_feat, a_sh, b_w);
             ok = pipe_drain(sh, ps);
             if (!ok) break;
             // ---- epilogue: bias, activation and its derivative; the row goes back to shared

@@ -77,7 +77,6 @@ struct PipeRegs {
 // Rows [0, rows) of a row-major global matrix (row stride ld); rows >= rows_valid read as zero;
 // chunk c covers columns k0 + 32 c .. + 31.
 template <bool SPLIT> struct DirectGlobal {
-    static constexpr bool kBulk = false;
     const float* base;
     size_t ld;
     int rows, rows_valid, k0;
@@ -134,7 +133,6 @@ __device__ __forceinline__ int transposed_quad(int rows)
 // rotate which of their four values they store -- times 4 different k.
 // colsum accumulates this thread's column sums (four columns) over everything it staged.
 template <bool SPLIT> struct Transposed {
-    static constexpr bool kBulk = false;
     const float* base;
     size_t ld;
     int col0, rows;
@@ -178,19 +176,9 @@ template <bool SPLIT> struct Transposed {
     }
 };
 
-// A B operand that was packed beforehand (mlp_pack_kernel): chunk c of the product is 32 KiB at
-// base + c * 32 KiB, already split into high and low parts and laid out exactly as a stage wants
-// it, so one thread moves it with ONE bulk asynchronous copy (TMA) that reports to the stage's
-// "full" barrier; the other 511 producers spend nothing on B.
+// Packed layout of one element's weights: chunk indices of every product; a chunk is [128 rows of N][32 of K] in
+// the operand's core-matrix layout, high parts and behind them low parts.
 constexpr unsigned kPackedChunkBytes = 2 * kPipeOperandBytes;
-struct PackedB {
-    static constexpr bool kBulk = true;
-    const unsigned char* base;
-    __device__ __forceinline__ void load(int, PipeRegs&) const {}
-    __device__ __forceinline__ void store(const PipeRegs&, unsigned char*, unsigned char*) const {}
-};
-
-// Packed layout of one element's weights: chunk indices of every product.
 constexpr int kPackFwdL1 = 0, kPackFwdL2 = 12, kPackFwdL3 = 16;          // forward: W1 (12 chunks), W2 (4), W3 (4)
 constexpr int kPackBwdS0 = 20, kPackBwdS1 = 22, kPackBwdF = 26;          // backward: W3 (2), W2 (4), W1 blocks (3 x 4)
 constexpr int kPackChunks = 38;
@@ -231,15 +219,7 @@ __device__ __forceinline__ void pipe_produce(MlpShared& sh, int nchunks, PipeSta
         const int s = (int)(ps.chunks & 1u);
         unsigned char* stage = sh.a_hi + s * kPipeStageBytes;
         pipe_wait_stage(sh, ps, s);
-        if (BSrc::kBulk) {
-            if (threadIdx.x == 0) {      // registered before this thread's own arrival below
-                mbar_expect_tx(&sh.full_bar[s], kPackedChunkBytes);
-                bulk_copy_to_shared(stage + 2 * kPipeOperandBytes, b_src.base + (size_t)c * kPackedChunkBytes,
-                                    kPackedChunkBytes, &sh.full_bar[s]);
-            }
-        } else {
-            b_src.store(rb, stage + 2 * kPipeOperandBytes, stage + 3 * kPipeOperandBytes);
-        }
+        b_src.store(rb, stage + 2 * kPipeOperandBytes, stage + 3 * kPipeOperandBytes);
         if (ASHARED) a_sh.store_chunk(c, stage, stage + kPipeOperandBytes);
         else a_src.store(ra, stage, stage + kPipeOperandBytes);
         if (c + 1 < nchunks) {           // the next chunk's loads fly while this one is consumed
@@ -253,12 +233,11 @@ __device__ __forceinline__ void pipe_produce(MlpShared& sh, int nchunks, PipeSta
     }
 }
 
-// Packs the weights of the four elements into the stage layout (both products that read them:
-// forward B[n = out][k = in] = W[k][n], backward B[n = in][k = out] = W[n][k]), high and low tf32
-// parts; one CTA per (chunk, element), once per weight update.  2.4 MB read, 4.9 MB written: bound by
-// latency, so a thread moves four values of K at a time with 16-byte stores (a core matrix per 8 lanes);
-// reads are rows of 128 consecutive values (forward) or 64-byte pieces of rows (backward).  One value at a
-// time along K, with 512 bytes between the lanes of a read, took 8.7 us.
+// Packs the weights of the four elements into the operand layout of both products that read them (forward
+// B[n = out][k = in] = W[k][n], backward B[n = in][k = out] = W[n][k]), tf32 parts; one CTA per (chunk, element),
+// once per weight update.  2.4 MB read, 4.9 MB written: bound by latency, so a thread moves four values of K at a
+// time with 16-byte stores (a core matrix per 8 lanes); reads are rows of 128 consecutive values (forward) or 64-byte
+// pieces of rows (backward).
 struct MlpPackParams {
     const float* w1[kTypes];   // [384][128]
     const float* w2[kTypes];   // [128][128]
