@@ -105,10 +105,18 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_forward_kernel(const Ml
             if (tid < kMlpH3) sh.vec[tid] = p.w4[e][tid];
             producer_sync();
             if (tid < n_rows) {
-                float acc = p.b4[e][0];
-#pragma unroll 8
-                for (int i = 0; i < kMlpH3; i++) acc += sh.act[tid * kMlpActStride + i] * sh.vec[i];
-                p.energy[e][row0 + tid] = acc;
+                // four shares of 16 columns (8 q .. and 32 + 8 q ..), added in order, as in mlp_chain_kernel
+                float share[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    share[q] = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        const int c = 32 * (i >> 3) + 8 * q + (i & 7);
+                        share[q] += sh.act[tid * kMlpActStride + c] * sh.vec[c];
+                    }
+                }
+                p.energy[e][row0 + tid] = p.b4[e][0] + share[0] + share[1] + share[2] + share[3];
             }
         } else if (tid == 0) {
             report(ANI_ERR_TIMEOUT);
