@@ -412,6 +412,9 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                 for (int i = 0; i < 8; i++) part[i] = v[i] - part[i];
                 tmem_store8(lanes + kTmemLo + s * 32 + sub * 8, part);
             }
+        };
+        // blocks are handed over one behind the stores, so that these run under the next block's arithmetic
+        auto hand_over = [&](int s) {
             tmem_store_wait();
             tc_fence_before();
             mbar_arrive(&sh.operand_ready[s]);
@@ -437,13 +440,18 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
             request(0);
             request(1);
         }
-        if (kHasForward && MODE != kChainTangent) {
-            if (tid < kMlpH1) sh.bias[tid] = p.b1[e][tid];
-            else if (tid < kMlpH1 + kMlpH2) sh.bias[tid] = p.b2[e][tid - kMlpH1];
-            else if (tid < kMlpH1 + kMlpH2 + kMlpH3) sh.bias[tid] = p.b3[e][tid - kMlpH1 - kMlpH2];
-        }
-        if (tid >= kChainEpi - kMlpH3) sh.w4[tid - (kChainEpi - kMlpH3)] = p.w4[e][tid - (kChainEpi - kMlpH3)];
-        if (!kHasForward) producer_sync();      // else: read behind the barriers of layer 1
+        // biases and output weights, one value per thread: requested here, stored behind layer 1
+        float vec = 0.0f;
+        constexpr int kBiases = kMlpH1 + kMlpH2 + kMlpH3;
+        if (kHasForward && MODE != kChainTangent && tid < kBiases)
+            vec = tid < kMlpH1 ? p.b1[e][tid] : (tid < kMlpH1 + kMlpH2 ? p.b2[e][tid - kMlpH1] : p.b3[e][tid - kMlpH1 - kMlpH2]);
+        if (tid >= kBiases && tid < kBiases + kMlpH3) vec = p.w4[e][tid - kBiases];
+        auto store_vec = [&]() {
+            if (tid < kBiases) sh.bias[tid] = vec;
+            else if (tid < kBiases + kMlpH3) sh.w4[tid - kBiases] = vec;
+            producer_sync();
+        };
+        if (!kHasForward) store_vec();
 
         if (kHasForward) {
             // ---- layer 1: group g of 128 threads takes chunks g, g + 4, g + 8; thread = row (TMEM lane) ----
@@ -480,7 +488,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                 tc_fence_before();
                 mbar_arrive(&sh.a_full[g]);
             }
-            producer_sync();      // bias and output weights are in shared memory, the feature chunks have been read
+            store_vec();      // (behind it the feature chunks have been read, too)
             if (MODE == kChainTangent) {
                 // ---- A' = D T goes on, S T R stays (q); layer 3: its q is the first operand of the way back ----
 #pragma unroll 1
@@ -505,8 +513,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                                 s[i] *= t[i];
                                 d[i] *= t[i];
                             }
+                            if (b > 0) hand_over(b - 1);
                             operand(d + 8 * b, b);
                         }
+                        hand_over(3);
                         tile.store<4>(d, adot, 128, n_rows);
                         tile.store<4>(s, q, 128, n_rows);
                     } else {
@@ -520,8 +530,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                                 s[i] = mlp_activation_second<ACT>(s[i], d[i]) * sh.w4[32 * b + 8 * sub + (i & 7)] * t[i];
                                 d[i] *= t[i];
                             }
+                            if (b > 0) hand_over(b - 1);
                             operand(s + 8 * b, b);
                         }
+                        hand_over(1);
                         tile.store<2>(d, adot, kMlpH3, n_rows);
                         tile.store<2>(s, q, kMlpH3, n_rows);
                     }
@@ -542,6 +554,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                             v[i] = mlp_activation<ACT>(x);
                             d[i] = mlp_activation_grad<ACT>(x, v[i]);
                         }
+                        if (b > 0) hand_over(b - 1);
                         operand(v + 8 * b, b);
                         if (MODE == kChainForces) {
 #pragma unroll
@@ -549,6 +562,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                                 hold[(32 * b + 8 * sub + (i & 7)) * kMlpTile + row] = d[i];
                         }
                     }
+                    hand_over(3);
                     if (MODE == kChainForward) {
                         float* act = l == 0 ? p.act1[e] : p.act2[e];
                         float* dact = l == 0 ? p.dact1[e] : p.dact2[e];
@@ -573,8 +587,12 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                         share += v[i] * w;
                         if (MODE == kChainForces) v[i] = ge * w * d[i];      // dZ3
                     }
-                    if (MODE == kChainForces) operand(v + 8 * b, b);
+                    if (MODE == kChainForces) {
+                        if (b > 0) hand_over(b - 1);
+                        operand(v + 8 * b, b);
+                    }
                 }
+                if (MODE == kChainForces) hand_over(1);
                 // the biases of layers 1 and 2 have been used by every warp: their place takes two of the four shares
                 float* shares = sub < 2 ? sh.bias + sub * kMlpTile : sh.more_shares + (sub - 2) * kMlpTile;
                 shares[row] = share;
@@ -596,8 +614,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
             for (int b = 0; b < 2; b++) {
 #pragma unroll
                 for (int i = 8 * b; i < 8 * b + 8; i++) v[i] *= ge * sh.w4[32 * b + 8 * sub + (i & 7)];
+                if (b > 0) hand_over(b - 1);
                 operand(v + 8 * b, b);
             }
+            hand_over(1);
             tile.store<2>(v, p.dz3[e] + atom0 * kMlpH3, kMlpH3, n_rows);
         }
         if (kHasBackward) {
@@ -618,8 +638,12 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                     for (int b = 0; b < 4; b++) {
 #pragma unroll
                         for (int i = 8 * b; i < 8 * b + 8; i++) v[i] += d[i];
-                        if (l == 1) operand(v + 8 * b, b);
+                        if (l == 1) {
+                            if (b > 0) hand_over(b - 1);
+                            operand(v + 8 * b, b);
+                        }
                     }
+                    if (l == 1) hand_over(3);
                     tile.store<4>(v, q, 128, n_rows);
                     continue;
                 }
@@ -631,8 +655,12 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
 #pragma unroll
                     for (int i = 8 * b; i < 8 * b + 8; i++)
                         v[i] *= MODE == kChainForces ? hold[(32 * b + 8 * sub + (i & 7)) * kMlpTile + row] : d[i];
-                    if (l == 1 || want_feat) operand(v + 8 * b, b);
+                    if (l == 1 || want_feat) {
+                        if (b > 0) hand_over(b - 1);
+                        operand(v + 8 * b, b);
+                    }
                 }
+                if (l == 1 || want_feat) hand_over(3);
                 if (MODE == kChainBackward)
                     tile.store<4>(v, (l == 1 ? p.dz2[e] : p.dz1[e]) + g0, 128, n_rows);
             }
