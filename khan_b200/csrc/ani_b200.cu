@@ -507,10 +507,10 @@ template <int MODE> int mlp_chain_act(const MlpChainParams& p, int activation, b
     }
 }
 
-template <bool SPLIT> int mlp_wgrad_launch(const MlpWgradParams& p, int n_ranges, cudaStream_t st)
+template <bool SPLIT> int mlp_wgrad_launch(const MlpWgradSets& p, int n_ranges, int n_sets, cudaStream_t st)
 {
     auto kernel = mlp_wgrad_kernel<SPLIT>;
-    const size_t smem = sizeof(MlpShared) + 1024;
+    const size_t smem = sizeof(WgradShared);
     static thread_local int configured_dev = -1;
     int dev = 0;
     ANI_CUDA(cudaGetDevice(&dev));
@@ -518,7 +518,7 @@ template <bool SPLIT> int mlp_wgrad_launch(const MlpWgradParams& p, int n_ranges
         if (int rc = set_smem(kernel, smem)) return rc;
         configured_dev = dev;
     }
-    ANI_CUDA(launch_chain(kernel, dim3(n_ranges, kWgradBlocks), kMlpAllThreads, smem, st, 1, p));
+    ANI_CUDA(launch_chain(kernel, dim3(n_ranges, kWgradBlocks, n_sets), kMlpAllThreads, smem, st, 1, p));
     return ANI_OK;
 }
 
@@ -615,28 +615,29 @@ bool all_packed(const void* const* packed, const int* acs)
     return true;
 }
 
-// Adds the weight gradients described by p (range fields are set here).
-int wgrad_call(MlpWgradParams& p, int split_precision, cudaStream_t st)
+// Adds the weight gradients of the first n_sets sets of p (counts and ranges are set here).
+int wgrad_call(MlpWgradSets& p, const int* acs, int n_sets, int split_precision, cudaStream_t st)
 {
-    // atoms per CTA: the smallest multiple of 64 for which the grid fits the SMs once (the
-    // kernels run one CTA per SM, so a second partial wave would double the time)
+    // atoms per CTA: the smallest multiple of 32 for which the grid fits the SMs once (the kernel runs one CTA per
+    // SM, so a second partial wave would double the time), but no fewer than a chunk for each of its four groups
     int dev = 0, sms = 0;
     ANI_CUDA(cudaGetDevice(&dev));
     ANI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    int range = 256;
-    for (;; range += 64) {
+    int range = kChainGroups * kPipeK;
+    for (;; range += kPipeK) {
         long long ctas = 0;
-        for (int t = 0; t < kTypes; t++) ctas += (p.count[t] + range - 1) / range;
-        if (ctas * kWgradBlocks <= sms || range >= (1 << 20)) break;
+        for (int t = 0; t < kTypes; t++) ctas += (acs[t] + range - 1) / range;
+        if (ctas * kWgradBlocks * n_sets <= sms || range >= (1 << 20)) break;
     }
     p.range = range;
     int ranges = 0;
     for (int t = 0; t < kTypes; t++) {
+        p.count[t] = acs[t];
         p.range_start[t] = ranges;
-        ranges += (p.count[t] + range - 1) / range;
+        ranges += (acs[t] + range - 1) / range;
     }
     p.range_start[kTypes] = ranges;
-    return split_precision ? mlp_wgrad_launch<true>(p, ranges, st) : mlp_wgrad_launch<false>(p, ranges, st);
+    return split_precision ? mlp_wgrad_launch<true>(p, ranges, n_sets, st) : mlp_wgrad_launch<false>(p, ranges, n_sets, st);
 }
 
 // ani_mlp_backward_f32, with dL/dA_l of the two inner layers in r1 and r2 (element-sorted rows) when given.
@@ -942,9 +943,9 @@ int ani_mlp_weight_grad_f32(const ani_mlp_weight_grad_args* a, const int* acs_ho
     if (!a) return ANI_ERR_NULL_POINTER;
     if (int rc = check_acs(acs_host, &n_atoms)) return rc;
     if (n_atoms == 0) return ANI_OK;
-    MlpWgradParams p;
+    MlpWgradSets sets = {};
+    MlpWgradParams& p = sets.set[0];
     for (int t = 0; t < kTypes; t++) {
-        p.count[t] = acs_host[t];
         if (acs_host[t] > 0 && (!a->features[t] || !a->act1[t] || !a->act2[t] || !a->dz1[t] || !a->dz2[t] ||
                                 !a->dz3[t] || !a->dw1[t] || !a->dw2[t] || !a->dw3[t] || !a->db1[t] ||
                                 !a->db2[t] || !a->db3[t] || !a->act3[t] || !a->grad_energy[t] ||
@@ -963,7 +964,7 @@ int ani_mlp_weight_grad_f32(const ani_mlp_weight_grad_args* a, const int* acs_ho
         p.act3[t] = a->act3[t]; p.grad_energy[t] = a->grad_energy[t];
         p.dw4[t] = a->dw4[t]; p.db4[t] = a->db4[t];
     }
-    return wgrad_call(p, split_precision, (cudaStream_t)stream);
+    return wgrad_call(sets, acs_host, 1, split_precision, (cudaStream_t)stream);
 }
 
 int ani_molecule_energy_f32(const float* atom_energy_sorted, const int* gather_idxs, const int* mol_offsets,
@@ -1528,13 +1529,14 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
                           f->rmse));
     float* rates[kTypes];
     MlpChainParams p = {};
-    MlpWgradParams w1, w2;      // F^T Q and U^T P
+    MlpWgradSets sets = {};
+    MlpWgradParams &w1 = sets.set[0], &w2 = sets.set[1];      // F^T Q and U^T P
     size_t row = 0;
     int tiles = 0;
     for (int t = 0; t < kTypes; t++) {
         auto at = [&](float* base, int width) { return base + row * (size_t)width; };
         rates[t] = at(f->feature_rates, kTotal);
-        p.count[t] = w1.count[t] = w2.count[t] = acs[t];
+        p.count[t] = acs[t];
         p.tile_start[t] = tiles;
         tiles += (acs[t] + kMlpTile - 1) / kMlpTile;
         p.feat[t] = w2.feat[t] = rates[t];
@@ -1574,8 +1576,7 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
     if (f->z_ready) ANI_CUDA(cudaStreamWaitEvent(st, (cudaEvent_t)f->z_ready, 0));
     if (int rc = mlp_chain_act<kChainTangent>(p, a->activation, a->split_precision != 0, st)) return rc;
     if (a->zero_ptr && a->zero_bytes) ANI_CUDA(cudaMemsetAsync(a->zero_ptr, 0, a->zero_bytes, st));
-    if (int rc2 = wgrad_call(w1, a->split_precision, st)) return rc2;
-    return wgrad_call(w2, a->split_precision, st);
+    return wgrad_call(sets, acs, 2, a->split_precision, st);
 }
 
 }  // extern "C"

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_forward_kernel(const Ml
             if (tid < N) sh.vec[tid] = layer_b[layer][tid];   // read in the epilogue, after the drain barrier
             DirectGlobal<SPLIT> a_feat{p.feat[e] + (size_t)row0 * kMlpIn, (size_t)kMlpIn, kMlpTile, n_rows, 0};
             // B[n = out][k = in] = W[k][n]: the weights are read as stored ([in][out]) and transposed
-            Transposed<SPLIT> b_w{layer_w[layer], (size_t)N, 0, N, 0, K, make_float4(0.f, 0.f, 0.f, 0.f)};
+            Transposed<SPLIT> b_w{layer_w[layer], (size_t)N, 0, N, 0, K};
             if (layer == 0) pipe_produce<SPLIT, false>(sh, K / kPipeK, ps, a_feat, a_sh, b_w);
             else pipe_produce<SPLIT, true>(sh, K / kPipeK, ps, a_feat, a_sh, b_w);
             ok = pipe_drain(sh, ps);

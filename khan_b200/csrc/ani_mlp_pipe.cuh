@@ -1,4 +1,4 @@
-// Two-stage operand pipeline shared by the three atomic-network kernels.
+// Two-stage operand pipeline of the atomic-network kernels for weights that are not packed, and the weight packing.
 //
 // A product  acc[128 x N] (+)= A[128 x K] * B[N x K]^T  is cut into chunks of 32 values of K.  The
 // 128 KiB operand area of MlpShared holds two stages (each: A hi, A lo, B hi, B lo, 16 KiB
@@ -130,14 +130,12 @@ __device__ __forceinline__ int transposed_quad(int rows)
 // four 128-byte row segments; stores are conflict-free because the bank of an operand element
 // is 4 (row mod 8) + (k mod 4) and each store instruction writes 8 different (row mod 8) -- lanes
 // rotate which of their four values they store -- times 4 different k.
-// colsum accumulates this thread's column sums (four columns) over everything it staged.
 template <bool SPLIT> struct Transposed {
     const float* base;
     size_t ld;
     int col0, rows;
     long long r0;
     int n_valid;
-    float4 colsum;
     __device__ __forceinline__ int passes() const { return (rows >> 5) * (kPipeK / 4) / (kMlpThreads / 32); }   // 2 or 1
     __device__ __forceinline__ int k_of(int b) const
     {
@@ -164,7 +162,6 @@ template <bool SPLIT> struct Transposed {
             if (b >= passes()) break;
             const int k = k_of(b);
             const float4 v = r.v[b];
-            colsum.x += v.x; colsum.y += v.y; colsum.z += v.z; colsum.w += v.w;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const int jj = (j + rot) & 3;
