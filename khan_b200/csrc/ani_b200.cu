@@ -537,8 +537,7 @@ int pack_params(const float* const* w1, const float* const* w2, const float* con
 }
 int pack_launch(const MlpPackParams& p, cudaStream_t st)
 {
-    mlp_pack_kernel<<<dim3(kPackChunks, kTypes), kMlpThreads, 0, st>>>(p);
-    ANI_CUDA(cudaGetLastError());
+    ANI_CUDA(launch_chain(mlp_pack_kernel, dim3(kPackChunks, kTypes), kMlpThreads, 0, st, 1, p));
     return ANI_OK;
 }
 
@@ -992,11 +991,10 @@ int ani_nadam_step_f32(float* params, const float* grads, float* m, float* v, fl
     const long long want = (n + 4 * kOptimThreads - 1) / (4 * kOptimThreads);
     const int grid = (int)(want < (long long)sms * 4 ? want : (long long)sms * 4);
     cudaStream_t st = (cudaStream_t)stream;
-    grad_sumsq_kernel<<<grid, kOptimThreads, 0, st>>>(grads, n, (OptimState*)state);
-    ANI_CUDA(cudaGetLastError());
-    nadam_update_kernel<<<grid, kOptimThreads, 0, st>>>(params, grads, m, v, ema, n, (const OptimHyper*)hyper,
-                                                        (OptimState*)state);
-    ANI_CUDA(cudaGetLastError());
+    if (want > 0x7fffffffLL) return ANI_ERR_BAD_SIZE;
+    ANI_CUDA(launch_chain(grad_sumsq_kernel, grid, kOptimThreads, 0, st, 1, grads, n, (OptimState*)state));
+    ANI_CUDA(launch_chain(nadam_update_kernel, (int)want, kOptimThreads, 0, st, 1, params, grads, m, v, ema, n,
+                          (const OptimHyper*)hyper, (OptimState*)state));
     return ANI_OK;
 }
 
@@ -1008,9 +1006,8 @@ int ani_clip_rows_f32(float* params, const int* row_offsets, const int* row_leng
     if (!params || !row_offsets || !row_lengths) return ANI_ERR_NULL_POINTER;
     const int per_block = kOptimThreads / kWarp;
     const int grid = (n_rows + per_block - 1) / per_block;
-    clip_rows_kernel<<<grid, kOptimThreads, 0, (cudaStream_t)stream>>>(params, row_offsets, row_lengths, n_rows,
-                                                                       max_norm);
-    ANI_CUDA(cudaGetLastError());
+    ANI_CUDA(launch_chain(clip_rows_kernel, grid, kOptimThreads, 0, (cudaStream_t)stream, 1, params, row_offsets, row_lengths,
+                          n_rows, max_norm));
     return ANI_OK;
 }
 
@@ -1020,8 +1017,8 @@ int ani_scale_by_loss_f32(float* grads, long long n, const float* l2s, int n_mol
     if (n < 0 || n_mols <= 0 || (kind != 1 && kind != 2)) return ANI_ERR_BAD_SIZE;
     if (!l2s || (n > 0 && !grads)) return ANI_ERR_NULL_POINTER;
     const long long blocks = std::max<long long>(1, std::min<long long>((n + kOptimThreads - 1) / kOptimThreads, 296));
-    loss_scale_kernel<<<(int)blocks, kOptimThreads, 0, (cudaStream_t)stream>>>(grads, n, l2s, n_mols, kind, rmse_out);
-    ANI_CUDA(cudaGetLastError());
+    ANI_CUDA(launch_chain(loss_scale_kernel, (int)blocks, kOptimThreads, 0, (cudaStream_t)stream, 1, grads, n, l2s, n_mols,
+                          kind, rmse_out));
     return ANI_OK;
 }
 

@@ -275,7 +275,11 @@ __device__ __forceinline__ void pack_chunk(const MlpPackParams& p, int chunk, in
         pipe_store4<true>(hi, lo, pipe_offset(n, k), v);
     }
 }
-__global__ void __launch_bounds__(kMlpThreads) mlp_pack_kernel(const MlpPackParams p) { pack_chunk(p, blockIdx.x, blockIdx.y); }
+__global__ void __launch_bounds__(kMlpThreads) mlp_pack_kernel(const MlpPackParams p)
+{
+    pdl_wait();      // no trigger: the kernel writes weights
+    pack_chunk(p, blockIdx.x, blockIdx.y);
+}
 
 // MMA-warp side of the same product: waits (bounded) for each filled stage, issues its MMAs and
 // commits them to the stage's barrier.  `fresh` = overwrite the accumulator with the first chunk.

@@ -11,6 +11,7 @@
 #pragma once
 
 #include "ani_common.cuh"
+#include "ani_launch.cuh"
 
 namespace ani {
 
@@ -31,6 +32,8 @@ __global__ void __launch_bounds__(kOptimThreads)
     grad_sumsq_kernel(const float* __restrict__ g, long long n, OptimState* __restrict__ st)
 {
     __shared__ float warp_sums[kOptimThreads / kWarp];
+    pdl_wait();
+    pdl_trigger();
     float acc = 0.0f;
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long n4 = n >> 2;
@@ -53,6 +56,26 @@ __global__ void __launch_bounds__(kOptimThreads)
     }
 }
 
+struct NadamFactors {
+    float scale, lr_t, one_minus_decay;
+};
+// One weight: returns the new value, updates the moments and the average.
+__device__ __forceinline__ float nadam_one(const OptimHyper& h, const NadamFactors& f, float w, float g, float* m, float* v,
+                                           float* ema)
+{
+    const float gi = g * f.scale;
+    const float mi = h.beta1 * *m + (1.0f - h.beta1) * gi;
+    const float vi = h.beta2 * *v + (1.0f - h.beta2) * gi * gi;
+    const float wi = w - f.lr_t * (h.beta1 * mi + (1.0f - h.beta1) * gi) / (sqrtf(vi) + h.eps);
+    *m = mi;
+    *v = vi;
+    *ema -= f.one_minus_decay * (*ema - wi);
+    return wi;
+}
+
+// 296 k weights are 9.5 MB of traffic, 2 us; what counts is the chain of latencies, so a thread has four
+// consecutive weights, all its loads are issued at once and ahead of the wait for the sum of squares (the launch
+// directly before, which writes none of what they read).  With four strided weights one after the other: 10 us.
 __global__ void __launch_bounds__(kOptimThreads)
     nadam_update_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
                         float* __restrict__ v, float* __restrict__ ema, long long n,
@@ -60,21 +83,40 @@ __global__ void __launch_bounds__(kOptimThreads)
 {
     const OptimHyper h = *hyper;
     const int step = st->step;
+    const long long i4 = (long long)blockIdx.x * kOptimThreads + threadIdx.x;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |
+                           reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(ema)) & 15) == 0;
+    const bool whole = aligned && 4 * i4 + 4 <= n;
+    float4 gq, mq, vq, wq, eq = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (whole) {
+        gq = reinterpret_cast<const float4*>(g)[i4];
+        mq = reinterpret_cast<const float4*>(m)[i4];
+        vq = reinterpret_cast<const float4*>(v)[i4];
+        wq = reinterpret_cast<const float4*>(w)[i4];
+        if (ema) eq = reinterpret_cast<const float4*>(ema)[i4];
+    }
     const float t = (float)(step + 1);
+    NadamFactors f;
+    f.lr_t = h.lr * sqrtf(1.0f - powf(h.beta2, t)) / (1.0f - powf(h.beta1, t));
+    f.one_minus_decay = 1.0f - fminf(h.ema_decay, (1.0f + t) / (10.0f + t));
+    pdl_wait();      // no early trigger: the kernel writes weights
     const float norm = sqrtf(st->norm2[step & 1]);
-    const float scale = h.clip_norm > 0.0f ? h.clip_norm / fmaxf(norm, h.clip_norm) : 1.0f;
-    const float lr_t = h.lr * sqrtf(1.0f - powf(h.beta2, t)) / (1.0f - powf(h.beta1, t));
-    const float decay = fminf(h.ema_decay, (1.0f + t) / (10.0f + t));
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const float gi = g[i] * scale;
-        const float mi = h.beta1 * m[i] + (1.0f - h.beta1) * gi;
-        const float vi = h.beta2 * v[i] + (1.0f - h.beta2) * gi * gi;
-        const float wi = w[i] - lr_t * (h.beta1 * mi + (1.0f - h.beta1) * gi) / (sqrtf(vi) + h.eps);
-        m[i] = mi;
-        v[i] = vi;
-        w[i] = wi;
-        if (ema) ema[i] -= (1.0f - decay) * (ema[i] - wi);
+    f.scale = h.clip_norm > 0.0f ? h.clip_norm / fmaxf(norm, h.clip_norm) : 1.0f;
+    if (whole) {
+        wq.x = nadam_one(h, f, wq.x, gq.x, &mq.x, &vq.x, &eq.x);
+        wq.y = nadam_one(h, f, wq.y, gq.y, &mq.y, &vq.y, &eq.y);
+        wq.z = nadam_one(h, f, wq.z, gq.z, &mq.z, &vq.z, &eq.z);
+        wq.w = nadam_one(h, f, wq.w, gq.w, &mq.w, &vq.w, &eq.w);
+        reinterpret_cast<float4*>(w)[i4] = wq;
+        reinterpret_cast<float4*>(m)[i4] = mq;
+        reinterpret_cast<float4*>(v)[i4] = vq;
+        if (ema) reinterpret_cast<float4*>(ema)[i4] = eq;
+    } else {
+        for (long long i = 4 * i4; i < n && i < 4 * i4 + 4; i++) {
+            float e = ema ? ema[i] : 0.0f;
+            w[i] = nadam_one(h, f, w[i], g[i], m + i, v + i, &e);
+            if (ema) ema[i] = e;
+        }
     }
     // the last block to finish advances the step and clears the slot the next step will use
     __syncthreads();
@@ -97,6 +139,7 @@ __global__ void __launch_bounds__(kOptimThreads)
     clip_rows_kernel(float* __restrict__ w, const int* __restrict__ row_offsets, const int* __restrict__ row_lengths,
                      int n_rows, float max_norm)
 {
+    pdl_wait();      // no trigger: the kernel writes weights
     const int lane = lane_id();
     const int warps = gridDim.x * (kOptimThreads / kWarp);
     for (int r = blockIdx.x * (kOptimThreads / kWarp) + warp_id(); r < n_rows; r += warps) {
@@ -125,6 +168,8 @@ __global__ void __launch_bounds__(kOptimThreads)
 {
     __shared__ float warp_sums[kOptimThreads / kWarp];
     __shared__ float factor_sh;
+    pdl_wait();
+    pdl_trigger();
     float acc = 0.0f;
     for (int i = threadIdx.x; i < n_mols; i += kOptimThreads) acc += l2s[i];
 #pragma unroll
