@@ -32,7 +32,8 @@ constexpr int kMlpAllThreads = kMlpThreads + 32;   // plus one warp that only is
 constexpr int kMlpLbo = 128;              // bytes between core matrices adjacent in K
 constexpr int kMlpOperandBytes = 32 * 1024;   // four of these make the 128 KiB operand area
 constexpr int kMlpActStride = 129;        // floats per row of the activation buffer (bank-conflict free)
-constexpr int kMlpTmemCols = 128;
+constexpr int kMlpTmemCols = 256;          // accumulator, and behind it that of the two small products
+constexpr int kMlpSmallCols = 128;
 constexpr unsigned kMlpSpinLimit = 1u << 24;
 
 enum MlpActivation { kActCelu = 0, kActGaussian = 1, kActNormal = 2, kActSoftplus = 3 };
@@ -178,6 +179,18 @@ __device__ __forceinline__ void tmem_load32(unsigned taddr, float* v)
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// The same of a product in split precision: the accumulators of its large and of its small parts.
+template <bool SPLIT> __device__ __forceinline__ void tmem_result32(unsigned taddr, float* v)
+{
+    tmem_load32(taddr, v);
+    if (SPLIT) {
+        float small[32];
+        tmem_load32(taddr + kMlpSmallCols, small);
+#pragma unroll
+        for (int i = 0; i < 32; i++) v[i] += small[i];
+    }
 }
 
 template <int ACT> __device__ __forceinline__ float mlp_activation(float x)

@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_backward_kernel(const M
             if (!ok) break;
             {
                 float v[32], d[32];
-                tmem_load32(lane_addr + c0, v);
+                tmem_result32<SPLIT>(lane_addr + c0, v);
                 if (step_raw[s])
                     warp_tile_to_global<false>(scratch, v, step_raw[s] + tile_atom0 * 128 + c0, 128, tile_rows);
                 warp_tile_from_global(scratch, d, step_d[s] + tile_atom0 * 128 + c0, 128, tile_rows);
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_backward_kernel(const M
                 ok = pipe_drain(sh, ps);
                 if (!ok) break;
                 float v[32];
-                tmem_load32(lane_addr + c0, v);
+                tmem_result32<SPLIT>(lane_addr + c0, v);
                 warp_tile_to_global<false>(scratch, v, p.grad_feat[e] + tile_atom0 * kMlpIn + n0 + c0, kMlpIn, tile_rows);
                 tc_fence_before();
                 producer_sync();   // the accumulator and the scratch are overwritten by the next product

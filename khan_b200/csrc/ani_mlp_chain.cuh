@@ -11,11 +11,11 @@
 // that.  The previous kernels took 1-2 us a chunk and 2-3 us between two products.  Here
 //   * one thread streams the weights through a ring of stages, ahead over the whole chain, also across epilogues;
 //   * every A operand is in tensor memory: an epilogue reads the accumulator, splits the new activations into
-//     their tf32 parts and stores those to TMEM, where the next product takes them (columns: accumulators 0-127 and
-//     128-255 in turn, A high 256-383, A low 384-511).  With both operands in shared memory a chunk needs 160 KB of
+//     their tf32 parts and stores those to TMEM, where the next product takes them (columns: accumulators 0-127 for
+//     hi hi and 128-255 for hi lo + lo hi, A high 256-383, A low 384-511).  With both operands in shared memory a chunk needs 160 KB of
 //     its bandwidth, 1250 clocks against the tensor core's 830; now the weights are 80 KB of it;
-//   * an epilogue of all 16 warps hands over 32 columns at a time, and the next product, which accumulates in the
-//     other columns, starts with the first of them: its 3300 clocks run beside the epilogue's 3000 to 5000;
+//   * an epilogue of all 16 warps reads the accumulators and then hands over 32 columns at a time, and the next
+//     product starts with the first of them: its 3300 clocks run beside the epilogue's 3000 to 5000;
 //   * the features of a chunk are copied to shared memory as they are (16 KB), four warps read them row by row and
 //     store their parts to TMEM; four groups of four warps take the chunks in turn (four stages of 64 columns in
 //     the place of the later A operands);
@@ -24,7 +24,9 @@
 //     elsewhere (300 a barrier) is lost there;
 //   * forward + backward in one kernel needs nothing of the activations in global memory: their derivatives wait
 //     where the feature chunks were.
-// Split precision: x = hi + lo with hi rounded to nearest, hi hi + hi lo + lo hi accumulated.  Every wait is
+// Split precision: x = hi + lo with hi rounded to nearest, hi hi + hi lo + lo hi accumulated; the two small products
+// apart, because the tensor core cuts its sums off at the accumulator's last place and three times the additions
+// there were most of the error (energies against float64: 5e-6 -> 1.2e-6, plain float32 products give 0.7e-6).  Every wait is
 // bounded; after a timeout the kernel reports, waits for its own copies, frees its tensor memory and returns.
 #pragma once
 
@@ -36,7 +38,7 @@ constexpr int kChainA = 8, kChainB = 3;                 // feature chunks of 16 
 constexpr int kChainEpi = 512;                          // epilogue / staging threads (16 warps)
 constexpr int kChainThreads = kChainEpi + 64;           // + the MMA warp + the weight warp
 constexpr int kChainGroups = 4;                         // groups of 128 threads that take the feature chunks in turn
-constexpr unsigned kTmemAcc = 0, kTmemHi = 256, kTmemLo = 384;      // two accumulators of 128 columns
+constexpr unsigned kTmemAcc = 0, kTmemSmall = 128, kTmemHi = 256, kTmemLo = 384;
 
 enum ChainMode { kChainForward = 0, kChainForces = 1, kChainBackward = 2, kChainTangent = 3 };
 
@@ -67,9 +69,9 @@ struct ChainShared {
     float bias[kMlpH1 + kMlpH2 + kMlpH3], w4[kMlpH3];
     float more_shares[2 * kMlpTile];
     alignas(8) unsigned long long a_full[kChainGroups], a_empty[kChainGroups], b_full[kChainB], b_empty[kChainB];
-    unsigned long long acc_full[2];      // the accumulator holds a finished product
+    unsigned long long acc_full;         // the accumulators hold a finished product
     unsigned long long operand_ready[4]; // the epilogue has stored columns 32 c .. of the next A operand
-    unsigned long long acc_free;         // the epilogue has read the first block of the feature gradient
+    unsigned long long acc_free;         // the epilogue has read a block of the feature gradient
     unsigned tmem_base;
     int failed;
 };
@@ -248,8 +250,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
             mbar_init(&sh.b_full[s], 1);
             mbar_init(&sh.b_empty[s], 1);
         }
-        mbar_init(&sh.acc_full[0], 1);
-        mbar_init(&sh.acc_full[1], 1);
+        mbar_init(&sh.acc_full, 1);
         for (int c = 0; c < 4; c++) mbar_init(&sh.operand_ready[c], kChainEpi);
         mbar_init(&sh.acc_free, kChainEpi);
         sh.failed = 0;
@@ -295,10 +296,9 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
             ChainWait wait;
             int b_stage = 0;
             unsigned b_parity = 0, ready_parity = 0;      // bit c: parity of operand_ready[c]
-            int done_products = 0;
             unsigned b_seen = 0, a_seen = 0;              // the next chunk's barriers, looked at while issuing this one
             // The products of a chunk; `next_a` / `next_parity`: barrier of the next chunk's A operand (or null).
-            auto issue = [&](unsigned d, unsigned a_hi, unsigned a_lo, int N, bool first, unsigned long long* next_a,
+            auto issue = [&](unsigned a_hi, unsigned a_lo, int N, bool first, unsigned long long* next_a,
                              unsigned next_parity) {
                 const unsigned idesc = instr_desc(kMlpTile, N);
                 const unsigned b_hi = smem_u32(sh.b[b_stage]), b_lo = b_hi + kPipeOperandBytes;
@@ -310,10 +310,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
 #pragma unroll
                 for (int ks = 0; ks < kPipeK / 8; ks++) {
                     const unsigned step = ks * 2 * kMlpLbo, col = ks * 8;
-                    mma_tf32_ts(d, tmem + a_hi + col, pipe_desc(b_hi + step), idesc, !(first && ks == 0));
+                    mma_tf32_ts(tmem + kTmemAcc, tmem + a_hi + col, pipe_desc(b_hi + step), idesc, !(first && ks == 0));
                     if (SPLIT) {
-                        mma_tf32_ts(d, tmem + a_hi + col, pipe_desc(b_lo + step), idesc, true);
-                        mma_tf32_ts(d, tmem + a_lo + col, pipe_desc(b_hi + step), idesc, true);
+                        mma_tf32_ts(tmem + kTmemSmall, tmem + a_hi + col, pipe_desc(b_lo + step), idesc, !(first && ks == 0));
+                        mma_tf32_ts(tmem + kTmemSmall, tmem + a_lo + col, pipe_desc(b_hi + step), idesc, true);
                     }
                     if (ks == 1) {
                         b_seen = mbar_test(&sh.b_full[b_stage], b_parity);
@@ -327,7 +327,6 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
             };
             // one product behind layer 1; fresh: its A operand comes from the epilogue, else it is the last one's
             auto product = [&](int chunks, int N, bool fresh) {
-                const int acc = done_products & 1;
                 for (int c = 0; c < chunks; c++) {
                     if (fresh) {
                         if (!a_seen) wait(sh, &sh.operand_ready[c], (ready_parity >> c) & 1u);
@@ -337,11 +336,10 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                     if (!wait.ok) return;
                     tc_fence_after();
                     const bool more = fresh && c + 1 < chunks;
-                    issue(tmem + kTmemAcc + acc * 128, kTmemHi + c * kPipeK, kTmemLo + c * kPipeK, N, c == 0,
+                    issue(kTmemHi + c * kPipeK, kTmemLo + c * kPipeK, N, c == 0,
                           more ? &sh.operand_ready[c + 1] : nullptr, more ? (ready_parity >> (c + 1)) & 1u : 0u);
                 }
-                mma_commit(&sh.acc_full[acc]);
-                done_products++;
+                mma_commit(&sh.acc_full);
                 a_seen = 0;
             };
             if (kHasForward) {
@@ -352,12 +350,11 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                     if (!wait.ok) break;
                     tc_fence_after();
                     const bool more = c + 1 < kMlpIn / kPipeK;
-                    issue(tmem + kTmemAcc, kTmemHi + g * 2 * kPipeK, kTmemHi + g * 2 * kPipeK + kPipeK, kMlpH1, c == 0,
+                    issue(kTmemHi + g * 2 * kPipeK, kTmemHi + g * 2 * kPipeK + kPipeK, kMlpH1, c == 0,
                           more ? &sh.a_full[(c + 1) % kChainGroups] : nullptr, (unsigned)((c + 1) / kChainGroups) & 1u);
                     mma_commit(&sh.a_empty[g]);
                 }
-                if (wait.ok) mma_commit(&sh.acc_full[0]);
-                done_products = 1;
+                if (wait.ok) mma_commit(&sh.acc_full);
                 a_seen = 0;
                 product(kMlpH1 / kPipeK, kMlpH2, true);
                 product(kMlpH2 / kPipeK, kMlpH3, true);
@@ -367,8 +364,9 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                 product(kMlpH2 / kPipeK, kMlpH1, true);
                 if (want_feat) {
                     product(kMlpH1 / kPipeK, 128, true);
-                    product(kMlpH1 / kPipeK, 128, false);
                     wait(sh, &sh.acc_free, 0u);
+                    product(kMlpH1 / kPipeK, 128, false);
+                    wait(sh, &sh.acc_free, 1u);
                     product(kMlpH1 / kPipeK, 128, false);
                 }
             }
@@ -386,20 +384,22 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
         float* hold2 = hold1 + kMlpH1 * kMlpTile;
         int done_products = 0;
 
-        // the accumulator of the next product, 8 values of each of the first `segs` blocks of 32 columns
+        // the result of the next product, 8 values of each of the first `segs` blocks of 32 columns
         auto accumulator = [&](float* v, int segs) {
-            const int acc = done_products & 1;
-            wait(sh, &sh.acc_full[acc], (unsigned)(done_products >> 1) & 1u);
+            wait(sh, &sh.acc_full, (unsigned)done_products & 1u);
             done_products++;
             tc_fence_after();
-            unsigned r[32];
+            unsigned r[32], q[32];
 #pragma unroll
             for (int s = 0; s < 4; s++)
-                if (s < segs) tmem_load8(lanes + kTmemAcc + acc * 128 + s * 32 + sub * 8, r + 8 * s);
+                if (s < segs) {
+                    tmem_load8(lanes + kTmemAcc + s * 32 + sub * 8, r + 8 * s);
+                    if (SPLIT) tmem_load8(lanes + kTmemSmall + s * 32 + sub * 8, q + 8 * s);
+                }
             tmem_load_wait();
 #pragma unroll
             for (int i = 0; i < 32; i++)
-                if (i < 8 * segs) v[i] = __uint_as_float(r[i]);
+                if (i < 8 * segs) v[i] = SPLIT ? __uint_as_float(r[i]) + __uint_as_float(q[i]) : __uint_as_float(r[i]);
         };
         // 8 values of block s of the next A operand
         auto operand = [&](const float* v, int s) {
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                 for (int blk = 0; blk < 3; blk++) {
                     float v[32];
                     accumulator(v, 4);
-                    if (blk == 0) {
+                    if (blk < 2) {
                         tc_fence_before();
                         mbar_arrive(&sh.acc_free);
                     }

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_forward_kernel(const Ml
             const int c0 = ecg * 32;
             if (c0 < N) {
                 float v[32], d[32];
-                tmem_load32(tmem + ((unsigned)((warp & 3) * 32) << 16) + c0, v);
+                tmem_result32<SPLIT>(tmem + ((unsigned)((warp & 3) * 32) << 16) + c0, v);
 #pragma unroll
                 for (int i = 0; i < 32; i++) {
                     const float x = v[i] + sh.vec[c0 + i];

@@ -311,9 +311,9 @@ __device__ __forceinline__ void pipe_issue(MlpShared& sh, unsigned tmem, int N, 
                 const unsigned step = ks * 2 * kMlpLbo;
                 const bool first = fresh && c == 0 && ks == 0;
                 mma_tf32(tmem, pipe_desc(a_hi + step), pipe_desc(b_hi + step), idesc, !first);
-                if (SPLIT) {
-                    mma_tf32(tmem, pipe_desc(a_hi + step), pipe_desc(b_lo + step), idesc, true);
-                    mma_tf32(tmem, pipe_desc(a_lo + step), pipe_desc(b_hi + step), idesc, true);
+                if (SPLIT) {      // apart, as in mlp_chain_kernel
+                    mma_tf32(tmem + kMlpSmallCols, pipe_desc(a_hi + step), pipe_desc(b_lo + step), idesc, !first);
+                    mma_tf32(tmem + kMlpSmallCols, pipe_desc(a_lo + step), pipe_desc(b_hi + step), idesc, true);
                 }
             }
             mma_commit(&sh.stage_bar[s]);

@@ -128,10 +128,10 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_wgrad_kernel(const MlpW
 #pragma unroll
                 for (int ks = 0; ks < kPipeK / 8; ks++) {
                     const unsigned step = ks * 2 * kMlpLbo, col = ks * 8;
-                    mma_tf32_ts(tmem, a_hi + col, pipe_desc(b_hi + step), idesc, !(c == 0 && ks == 0));
+                    mma_tf32_ts(tmem + kTmemAcc, a_hi + col, pipe_desc(b_hi + step), idesc, !(c == 0 && ks == 0));
                     if (SPLIT) {
-                        mma_tf32_ts(tmem, a_hi + col, pipe_desc(b_lo + step), idesc, true);
-                        mma_tf32_ts(tmem, a_lo + col, pipe_desc(b_hi + step), idesc, true);
+                        mma_tf32_ts(tmem + kTmemSmall, a_hi + col, pipe_desc(b_lo + step), idesc, !(c == 0 && ks == 0));
+                        mma_tf32_ts(tmem + kTmemSmall, a_lo + col, pipe_desc(b_hi + step), idesc, true);
                     }
                     if (ks == 1 && c + 1 < nchunks)
                         seen = mbar_test(&sh.full[(c + 1) % kChainGroups], (unsigned)((c + 1) / kChainGroups) & 1u);
@@ -200,7 +200,13 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_wgrad_kernel(const MlpW
             float* bias_out = blk == 0 ? p.db1[e] : (blk == 3 ? p.db2[e] : (blk == 4 ? p.db3[e] : nullptr));
             if (c0 < N) {
                 float v[32];
-                tmem_load32(lanes + c0, v);
+                tmem_load32(lanes + kTmemAcc + c0, v);
+                if (SPLIT) {
+                    float small[32];
+                    tmem_load32(lanes + kTmemSmall + c0, small);
+#pragma unroll
+                    for (int i = 0; i < 32; i++) v[i] += small[i];
+                }
                 float* scratch = reinterpret_cast<float*>(sh.b[0]) + warp * (32 * kMlpScratchStride);
                 warp_tile_to_global<true>(scratch, v, out + (size_t)tile_row0 * N + c0, N, 32);
             }
