@@ -590,6 +590,54 @@ int ani_feeder_wait(ani_feeder* f, int slot, void* stream);
 int ani_feeder_release(ani_feeder* f, int slot, void* stream);
 int ani_feeder_end(ani_feeder* f);
 int ani_feeder_destroy(ani_feeder* f);
+/* Other source arrays (another data set) for the same arenas; between passes only. */
+int ani_feeder_set_slots(ani_feeder* f, const ani_feeder_slot* slots, int n_slots);
+
+/* The work on one batch of a feeder's pass as one call: step() takes the next batch from the feeder, enqueues its work
+ * and gives its slot back:
+ *   ANI_DRIVER_ENERGIES   molecule energies, into `energies` (of all molecules in order) or, when that is NULL,
+ *                         into place b % ANI_DRIVER_RING of ring_host for batch b
+ *   ANI_DRIVER_GRADIENTS  energies + coordinate gradients; the latter as rows [n_atoms][3] into that place
+ *   ANI_DRIVER_TRAIN      optional row clip, loss and its weight gradients, loss scaling, optional update
+ * Training runs on `stream`, with the features of the next batch on streams[0]; the other two run batch b on
+ * streams[b & 1], behind what `stream` held at the first step.  ani_driver_join makes `stream` wait for all of it.
+ * ring_host is pinned memory that the kernels write; ani_driver_wait(d, place) blocks until the results last
+ * enqueued for a place are there, and the caller has read a place before the step that fills it again.
+ * pass / pass64: the argument block of each of the two sets of buffers used in turn (pass64: double precision,
+ * not for training); what describes the batch is filled in here.  slots: the device arrays behind each slot of
+ * the feeder.  step() returns 1 (*batch is the one enqueued), 0 (pass over) or a negative status. */
+#define ANI_DRIVER_RING 3
+enum { ANI_DRIVER_ENERGIES = 0, ANI_DRIVER_GRADIENTS = 1, ANI_DRIVER_TRAIN = 2 };
+typedef struct ani_driver_slot {
+    const void *xs, *ys, *zs;
+    const int *atomic_numbers, *mol_offsets, *mol_counts;
+    const float* labels;             /* training only */
+} ani_driver_slot;
+typedef struct ani_driver_args {
+    int mode, n_slots;
+    const ani_driver_slot* slots;
+    const ani_pass_args* pass[2];
+    const ani_energy_args_f64* pass64[2];
+    void* streams[2];                /* training: the first only */
+    void* energies;                  /* [all molecules] or NULL */
+    void* ring_host[ANI_DRIVER_RING];
+    float *params, *grads, *m, *v, *ema;       /* training: ani_nadam_step_f32 (update != 0) */
+    long long n_params;
+    const float* hyper;
+    int* state;
+    int update;
+    int loss_kind;                   /* 0: leave the gradients of the mse; else ani_scale_by_loss_f32 */
+    float* rmse;
+    int clip_n_rows;                 /* > 0: ani_clip_rows_f32 before the batch */
+    const int *clip_row_offsets, *clip_row_lengths;
+    float clip_max_norm;
+} ani_driver_args;
+typedef struct ani_driver ani_driver;
+int ani_driver_create(const ani_driver_args* args, ani_driver** out);
+int ani_driver_step(ani_driver* d, ani_feeder* f, void* stream, ani_feeder_batch* batch);
+int ani_driver_wait(ani_driver* d, int place);
+int ani_driver_join(ani_driver* d, void* stream);
+int ani_driver_destroy(ani_driver* d);
 
 /*
  * Mean of a float buffer over the GPUs of one node through peer memory, one kernel launch per rank

@@ -17,7 +17,7 @@ LIB_PATH = os.environ.get("ANI_B200_LIB") or os.path.join(_HERE, "libani_b200.so
 CSRC = os.path.join(_HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(_HERE), "include")
 SOURCES = ["ani_b200.cu"]
-HEADERS = ["ani_params.h", "ani_common.cuh", "ani_device_math.cuh", "ani_feeder.h", "ani_mt19937.h", "ani_peer.cuh", "ani_sort.cuh", "ani_featurize.cuh", "ani_featurize_mol.cuh", "ani_featurize_large.cuh", "ani_featurize_round_passes.inl", "ani_grad.cuh", "ani_grad_mol.cuh", "ani_grad_pair_pass.inl",
+HEADERS = ["ani_params.h", "ani_common.cuh", "ani_device_math.cuh", "ani_feeder.h", "ani_driver.h", "ani_mt19937.h", "ani_peer.cuh", "ani_sort.cuh", "ani_featurize.cuh", "ani_featurize_mol.cuh", "ani_featurize_large.cuh", "ani_featurize_round_passes.inl", "ani_grad.cuh", "ani_grad_mol.cuh", "ani_grad_pair_pass.inl",
            "ani_grad_inverse.cuh", "ani_tangent_mol.cuh", "ani_mlp.cuh", "ani_mlp_pipe.cuh", "ani_mlp_forward.cuh", "ani_mlp_backward.cuh", "ani_mlp_wgrad.cuh", "ani_mlp_small.cuh", "ani_mlp_chain.cuh", "ani_force_fit.cuh", "ani_launch.cuh", "ani_charge.cuh", "ani_optim.cuh", "ani_energy.cuh", "ani_host_pack.h"]
 
 NVCC_FLAGS = [
@@ -109,6 +109,27 @@ class EnergyArgs64(ctypes.Structure):
                 + [(n, ctypes.c_void_p * 4) for n in ("w1", "b1", "w2", "b2", "w3", "b3", "w4", "b4")])
 
 
+class DriverSlot(ctypes.Structure):
+    """``ani_driver_slot`` of include/ani_b200.h."""
+    _fields_ = [(n, ctypes.c_void_p) for n in ("xs", "ys", "zs", "atomic_numbers", "mol_offsets", "mol_counts", "labels")]
+
+
+DRIVER_ENERGIES, DRIVER_GRADIENTS, DRIVER_TRAIN, DRIVER_RING = 0, 1, 2, 3
+
+
+class DriverArgs(ctypes.Structure):
+    """``ani_driver_args`` of include/ani_b200.h."""
+    _fields_ = ([("mode", ctypes.c_int), ("n_slots", ctypes.c_int), ("slots", ctypes.POINTER(DriverSlot)),
+                 ("pass_", ctypes.POINTER(PassArgs) * 2), ("pass64", ctypes.POINTER(EnergyArgs64) * 2),
+                 ("streams", ctypes.c_void_p * 2), ("energies", ctypes.c_void_p),
+                 ("ring_host", ctypes.c_void_p * DRIVER_RING)]
+                + [(n, ctypes.c_void_p) for n in ("params", "grads", "m", "v", "ema")]
+                + [("n_params", ctypes.c_longlong), ("hyper", ctypes.c_void_p), ("state", ctypes.c_void_p),
+                   ("update", ctypes.c_int), ("loss_kind", ctypes.c_int), ("rmse", ctypes.c_void_p),
+                   ("clip_n_rows", ctypes.c_int), ("clip_row_offsets", ctypes.c_void_p),
+                   ("clip_row_lengths", ctypes.c_void_p), ("clip_max_norm", ctypes.c_float)])
+
+
 PASS_PACK, PASS_FEATURIZE, PASS_FORWARD, PASS_ENERGY, PASS_BACKWARD, PASS_WEIGHT_GRAD, PASS_COORD_GRAD, PASS_TRANSIENT = (
     1, 2, 4, 8, 16, 32, 64, 128)
 
@@ -164,6 +185,12 @@ SIGNATURES = {
     "ani_feeder_release": (_i, [_vp, _i, _vp]),
     "ani_feeder_end": (_i, [_vp]),
     "ani_feeder_destroy": (_i, [_vp]),
+    "ani_feeder_set_slots": (_i, [_vp, _vp, _i]),
+    "ani_driver_create": (_i, [ctypes.POINTER(DriverArgs), ctypes.POINTER(_vp)]),
+    "ani_driver_step": (_i, [_vp, _vp, _vp, ctypes.POINTER(FeederBatch)]),
+    "ani_driver_wait": (_i, [_vp, _i]),
+    "ani_driver_join": (_i, [_vp, _vp]),
+    "ani_driver_destroy": (_i, [_vp]),
     "ani_peer_create": (_i, [_i, _i, ctypes.c_longlong, ctypes.POINTER(_vp)]),
     "ani_peer_handle": (_i, [_vp, _vp]),
     "ani_peer_connect": (_i, [_vp, _i, _vp]),

@@ -33,6 +33,7 @@
 #include "ani_energy.cuh"
 #include "ani_sort.cuh"
 #include "ani_host_pack.h"
+#include "ani_driver.h"
 #include "ani_feeder.h"
 #include "ani_peer.cuh"
 
@@ -1126,6 +1127,59 @@ int ani_feeder_destroy(ani_feeder* f)
     const int rc = f->impl.drain();
     delete f;
     return rc;
+}
+
+int ani_feeder_set_slots(ani_feeder* f, const ani_feeder_slot* slots, int n_slots)
+{
+    if (!f || !slots) return ANI_ERR_NULL_POINTER;
+    for (int s = 0; s < n_slots; s++)
+        if (!slots[s].host_arena) return ANI_ERR_NULL_POINTER;
+    return f->impl.set_slots(slots, n_slots);
+}
+
+struct ani_driver {
+    ani::Driver impl;
+    explicit ani_driver(const ani_driver_args& a) : impl(a) {}
+};
+
+int ani_driver_create(const ani_driver_args* a, ani_driver** out)
+{
+    if (!a || !out || !a->slots || !a->streams[0]) return ANI_ERR_NULL_POINTER;
+    if (a->n_slots <= 0 || a->mode < ANI_DRIVER_ENERGIES || a->mode > ANI_DRIVER_TRAIN) return ANI_ERR_BAD_SIZE;
+    const bool train = a->mode == ANI_DRIVER_TRAIN;
+    if (!train && !a->streams[1]) return ANI_ERR_NULL_POINTER;
+    for (int k = 0; k < 2; k++)
+        if (!a->pass[k] && (train || !a->pass64[k])) return ANI_ERR_NULL_POINTER;
+    if (train && (!a->params || !a->grads || (a->loss_kind && !a->rmse))) return ANI_ERR_NULL_POINTER;
+    if (a->mode == ANI_DRIVER_GRADIENTS || (a->mode == ANI_DRIVER_ENERGIES && !a->energies))
+        for (void* p : a->ring_host)
+            if (!p) return ANI_ERR_NULL_POINTER;
+    ani_driver* d = new (std::nothrow) ani_driver(*a);
+    if (!d) return ANI_ERR_CUDA;
+    if (int rc = d->impl.init()) {
+        delete d;
+        return rc;
+    }
+    *out = d;
+    return ANI_OK;
+}
+
+int ani_driver_step(ani_driver* d, ani_feeder* f, void* stream, ani_feeder_batch* batch)
+{
+    return d && f && batch ? d->impl.step(f->impl, static_cast<cudaStream_t>(stream), batch) : ANI_ERR_NULL_POINTER;
+}
+
+int ani_driver_wait(ani_driver* d, int place) { return d ? d->impl.wait(place) : ANI_ERR_NULL_POINTER; }
+
+int ani_driver_join(ani_driver* d, void* stream)
+{
+    return d ? d->impl.join(static_cast<cudaStream_t>(stream)) : ANI_ERR_NULL_POINTER;
+}
+
+int ani_driver_destroy(ani_driver* d)
+{
+    delete d;
+    return ANI_OK;
 }
 
 struct ani_peer {

@@ -45,12 +45,20 @@ class Feeder {
 public:
     Feeder(int device, const ani_feeder_slot* slots, int n_slots) : device_(device), slots_(n_slots)
     {
+        set_slots(slots, n_slots);
+    }
+
+    // Between passes.  A handle is kept over data sets because a new one costs 0.3 ms (stream and events).
+    int set_slots(const ani_feeder_slot* slots, int n_slots)
+    {
+        if (n_slots != (int)slots_.size() || !threads_.empty()) return ANI_ERR_BAD_SIZE;
         for (int s = 0; s < n_slots; s++) {
             slots_[s].args = slots[s].pack;
             slots_[s].host_arena = slots[s].host_arena;
             slots_[s].dev_arena = slots[s].dev_arena;
             slots_[s].nbytes = slots[s].nbytes;
         }
+        return ANI_OK;
     }
 
     int init()
@@ -111,11 +119,14 @@ public:
     }
 
     // Blocks until the next batch has been packed and its copy enqueued.  1: *out is a batch;
-    // 0: the pass is over; negative: the submitter failed with that code.
-    int next(ani_feeder_batch* out)
+    // 0: the pass is over; negative: the submitter failed with that code.  With block = false kNotYet instead of waiting.
+    static constexpr int kNotYet = 2;
+    int next(ani_feeder_batch* out, bool block = true)
     {
         std::unique_lock<std::mutex> lk(mu_);
-        cv_.wait(lk, [this] { return !ready_.empty() || finished_ || stop_; });
+        const auto there = [this] { return !ready_.empty() || finished_ || stop_; };
+        if (!block && !there()) return kNotYet;
+        cv_.wait(lk, there);
         if (ready_.empty()) return error_ ? error_ : 0;
         const int s = ready_.front();
         ready_.pop_front();

@@ -40,6 +40,7 @@ class PackedDataset:
         self.ptr = np.zeros(n_mols + 1, np.int64)
         np.cumsum(self.counts, out=self.ptr[1:])
         self._mol_acs = None
+        self._capacity, self._sources = {}, None
         cat = np.concatenate(all_Xs, axis=0) if n_mols else np.zeros((0, 4))
         self.types = np.ascontiguousarray(cat[:, 0].astype(np.int32))
         # coordinates stay in the precision they were given in; the cast to `dtype` happens per
@@ -82,9 +83,11 @@ class PackedDataset:
 
     def capacity(self, batch_size: int):
         """(atoms, molecules) that any batch of ``batch_size`` molecules fits in."""
-        k = min(batch_size, self.num_mols())
-        top = np.sort(self.counts)[-k:] if k else np.zeros(0, np.int64)
-        return int(top.sum()), k
+        if batch_size not in self._capacity:
+            k = min(batch_size, self.num_mols())
+            top = np.sort(self.counts)[-k:] if k else np.zeros(0, np.int64)
+            self._capacity[batch_size] = (int(top.sum()), k)
+        return self._capacity[batch_size]
 
     def batch_slices(self, batch_size: int):
         """For an UNSHUFFLED pass: per batch, the row range of every molecule within the batch, as ready-made
@@ -117,18 +120,22 @@ class PackedDataset:
 
     def fill_pack_args(self, a, slot: "HostSlot") -> None:
         """The fields of an ``ani_host_pack_args`` that depend only on (data set, slot)."""
-        a.n_mols_total, a.mol_ptr = self.num_mols(), self.ptr.ctypes.data
-        a.src_xyz, a.src_stride = self.xyz.ctypes.data, self.xyz.shape[1]
-        a.src_is_f64 = int(self.xyz.dtype == np.float64)
-        a.src_types = self.types.ctypes.data
-        a.src_ys = None if self.ys is None else self.ys.ctypes.data
-        a.src_grads = None if self.grads is None else self.grads.ctypes.data
-        a.src_mol_acs = self.mol_acs().ctypes.data
+        self.fill_sources(a)
         a.dst_xyz, a.dst_grads, a.dst_ys = slot.xyz.ctypes.data, slot.grads.ctypes.data, slot.ys.ctypes.data
         a.dst_stride, a.dst_is_f64 = slot.cap_atoms, int(slot.np_dtype == np.float64)
         a.dst_types, a.dst_mol_ids = slot.types.ctypes.data, slot.mol_ids.ctypes.data
         a.dst_mol_offsets, a.dst_mol_counts = slot.mol_offsets.ctypes.data, slot.mol_counts.ctypes.data
         a.cap_atoms, a.cap_mols = slot.cap_atoms, slot.cap_mols
+
+    def fill_sources(self, a) -> None:
+        """The fields that depend only on the data set."""
+        arrays = (self.ptr, self.xyz, self.types, self.ys, self.grads)
+        if self._sources is None or any(x is not y for x, y in zip(self._sources[0], arrays)):
+            self._sources = (arrays, tuple(None if x is None else x.ctypes.data for x in arrays), self.mol_acs().ctypes.data)
+        a.mol_ptr, a.src_xyz, a.src_types, a.src_ys, a.src_grads = self._sources[1]
+        a.src_mol_acs = self._sources[2]
+        a.n_mols_total = self.num_mols()
+        a.src_stride, a.src_is_f64 = self.xyz.shape[1], int(self.xyz.dtype == np.float64)
 
     def gather(self, picks: np.ndarray, slot: "HostSlot", fuzz=None) -> None:
         """Writes the batch made of molecules ``picks`` (in that order) into ``slot``: one call of
@@ -225,6 +232,7 @@ class HostSlot:
         self.grads = view("grads", self.np_dtype, (3, cap_atoms))
         self.ys = view("ys", self.np_dtype, (cap_mols,))
         self.mol_ids = view("mol_ids", np.int64, (cap_atoms,))
+        self.mol_ids_ptr = self.mol_ids.ctypes.data
         self.types = view("types", np.int32, (cap_atoms,))
         self.mol_offsets = view("mol_offsets", np.int32, (cap_mols,))
         self.mol_counts = view("mol_counts", np.int32, (cap_mols,))
@@ -343,35 +351,97 @@ def _drop_native(ring) -> None:
 
 
 def _native_submitter(ring, packed: "PackedDataset", dev, mol_ids: bool) -> dict:
-    """The native submitter bound to (ring, data set), made once and kept with the ring."""
+    """The native submitter of a ring, made once and kept with it; bound here to the data set of the next pass."""
     nat = ring[0].get("native")
     if nat is not None and nat["packed"] is packed and nat["mol_ids"] == mol_ids:
         return nat
-    _drop_native(ring)
-    for slot in ring:       # what a Python submitter left behind on these slots
-        for key in ("consumed", "uploaded"):
-            if slot[key] is not None:
-                slot[key].synchronize()
-                slot[key] = None
     n = len(ring)
-    arr = (_lib.FeederSlot * n)()
+    arr = (_lib.FeederSlot * n)() if nat is None else nat["slots"]
     for k, slot in enumerate(ring):
         host = slot["host"]
         packed.check_shapes(host)
-        packed.fill_pack_args(arr[k].pack, host)
-        arr[k].host_arena = host.arena.data_ptr()
-        arr[k].dev_arena = None if dev is None else slot["arena"].data_ptr()
+        if nat is None:
+            for key in ("consumed", "uploaded"):      # what a Python submitter left behind on this slot
+                if slot[key] is not None:
+                    slot[key].synchronize()
+                    slot[key] = None
+            packed.fill_pack_args(arr[k].pack, host)
+            arr[k].host_arena = host.arena.data_ptr()
+            arr[k].dev_arena = None if dev is None else slot["arena"].data_ptr()
+        else:
+            packed.fill_sources(arr[k].pack)
         arr[k].nbytes = host.used_bytes(packed.grads is not None, mol_ids)
-        if not mol_ids:
-            arr[k].pack.dst_mol_ids = None
+        arr[k].pack.dst_mol_ids = host.mol_ids_ptr if mol_ids else None
         host.pack_args = None
-    index = -1 if dev is None else (torch.device(dev).index if torch.device(dev).index is not None
-                                    else torch.cuda.current_device())
-    owner = _NativeHandle(index, arr, n)
-    nat = {"owner": owner, "handle": owner.ptr, "packed": packed, "mol_ids": mol_ids, "slots": arr, "batch": _lib.FeederBatch(),
-           "order": None, "keep": (packed.xyz, packed.types, packed.ys, packed.grads, packed.ptr, packed.mol_acs())}
+    if nat is None:
+        index = -1 if dev is None else (torch.device(dev).index if torch.device(dev).index is not None
+                                        else torch.cuda.current_device())
+        owner = _NativeHandle(index, arr, n)
+        nat = {"owner": owner, "handle": owner.ptr, "slots": arr, "batch": _lib.FeederBatch(), "order": None}
+        nat["driver_slots"] = None if dev is None else _driver_slots(ring)
+    else:
+        _lib.check(_lib.lib().ani_feeder_set_slots(nat["handle"], ctypes.addressof(arr), n), "ani_feeder_set_slots")
+    nat.update(packed=packed, mol_ids=mol_ids,
+               keep=(packed.xyz, packed.types, packed.ys, packed.grads, packed.ptr, packed.mol_acs()))
     ring[0]["native"] = nat
     return nat
+
+
+def _driver_slots(ring):
+    """The device arrays of every slot, as a ``BatchDriver`` takes them."""
+    arr = (_lib.DriverSlot * len(ring))()
+    for d, slot in zip(arr, ring):
+        v, host = slot["views"], slot["host"]
+        d.xs, d.ys, d.zs = (v["xyz"][k].data_ptr() for k in range(3))
+        d.atomic_numbers, d.mol_offsets, d.mol_counts = (v[k].data_ptr() for k in ("types", "mol_offsets", "mol_counts"))
+        d.labels = v["ys"].data_ptr()
+    return arr
+
+
+class BatchDriver:
+    """One pass of a feeder with the work on every batch in native code (``ani_driver_step``): energies, gradients
+    or training updates.  ``blocks``: the argument blocks of the two sets of buffers used in turn; ``streams``: one for
+    training, two otherwise; ``fields``: what else ``ani_driver_args`` needs."""
+
+    def __init__(self, feeder: "BatchFeeder", mode: int, blocks, streams, ring=(), keep=(), **fields):
+        self.feeder, self.batch = feeder, _lib.FeederBatch()
+        self._keep = (blocks, streams, ring, keep)
+        a = self._args = _lib.DriverArgs()
+        slots = feeder.native["driver_slots"]
+        a.mode, a.slots, a.n_slots = mode, slots, len(slots)
+        for k, stream in enumerate(streams):
+            a.streams[k] = stream.cuda_stream
+        for k, block in enumerate(blocks):
+            (a.pass64 if isinstance(block, _lib.EnergyArgs64) else a.pass_)[k] = ctypes.pointer(block)
+        for k, buf in enumerate(ring):
+            a.ring_host[k] = buf.data_ptr()
+        for name, value in fields.items():
+            setattr(a, name, value)
+        self._ptr = ctypes.c_void_p()
+        _lib.check(_lib.lib().ani_driver_create(ctypes.byref(a), ctypes.byref(self._ptr)), "ani_driver_create")
+        feeder.begin()
+
+    def step(self) -> bool:
+        """Enqueues the work on the next batch on the current stream; False when the pass is over.  Afterwards
+        ``self.batch`` describes the batch."""
+        rc = _lib.lib().ani_driver_step(self._ptr, self.feeder.native["handle"], self.feeder._stream_ptr(),
+                                        ctypes.byref(self.batch))
+        if rc < 0:
+            _lib.check(rc, "ani_driver_step")
+        return rc == 1
+
+    def join(self) -> None:
+        """Makes the current stream wait for everything enqueued so far."""
+        _lib.check(_lib.lib().ani_driver_join(self._ptr, self.feeder._stream_ptr()), "ani_driver_join")
+
+    def wait(self, place: int) -> None:
+        """Blocks until the results last enqueued for ``place`` of the ring are in host memory."""
+        _lib.check(_lib.lib().ani_driver_wait(self._ptr, place), "ani_driver_wait")
+
+    def __del__(self):
+        if getattr(self, "_ptr", None):
+            _lib.lib().ani_driver_destroy(self._ptr)
+            self._ptr = ctypes.c_void_p()
 
 
 class BatchFeeder:
@@ -395,7 +465,6 @@ class BatchFeeder:
         cap_atoms, cap_mols = max(cap_atoms, 1), max(cap_mols, 1)
         self._shape = (cap_atoms, cap_mols, packed.dtype)
         self._slots = [_take_ring(dev, cap_atoms, cap_mols, packed.dtype, self.depth) for dev in self.devices]
-        self._copy_streams = [torch.cuda.Stream(device=d) if d is not None else None for d in self.devices]
         self._ready = queue.Queue(maxsize=self.depth * len(self.devices))
         self._free = [queue.Queue() for _ in self.devices]
         for t, ring in enumerate(self._slots):
@@ -417,8 +486,14 @@ class BatchFeeder:
             self.mol_ids = mol_ids      # the per-atom molecule index, for consumers that read FedBatch.mol_ids
             self._native = _native_submitter(self._slots[0], packed, self.devices[0], mol_ids)
         else:
+            self._copy_streams = [torch.cuda.Stream(device=d) if d is not None else None for d in self.devices]
             for ring in self._slots:
                 _drop_native(ring)
+
+    @property
+    def native(self):
+        """The native submitter of this pass, or None."""
+        return self._native
 
     # ---- submitter thread ---------------------------------------------------------------
     def _take_free(self, tower: int):
@@ -479,7 +554,8 @@ class BatchFeeder:
         dev = self.devices[0]
         return None if dev is None else ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
 
-    def _next_native(self) -> FedBatch:
+    def begin(self) -> None:
+        """Starts the native submitter (the first batch asked for does so otherwise)."""
         nat, p, L = self._native, self.packed, _lib.lib()
         if not self._started:
             self._started = True
@@ -496,6 +572,10 @@ class BatchFeeder:
                 _lib.check(L.ani_feeder_begin_fuzz(nat["handle"], perm.ctypes.data, len(perm), self.batch_size,
                                                    key.ctypes.data, int(self._random[2]), float(self.fuzz)),
                            "ani_feeder_begin_fuzz")
+
+    def _next_native(self) -> FedBatch:
+        nat, p, L = self._native, self.packed, _lib.lib()
+        self.begin()
         while len(self._held) >= self.hold:
             self.release(self._held[0][2])
         fb = nat["batch"]

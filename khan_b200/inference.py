@@ -78,6 +78,13 @@ class EnergyForces:
         a.x_grads, a.y_grads, a.z_grads = g, g + cap * esz, g + 2 * cap * esz
         return a
 
+    def pass_block(self, sb: StagedBatch):
+        """Argument block of passes over ``sb`` for a ``BatchDriver``, which fills in what describes the batch."""
+        if not self.f64 and self.model.packed_weights() is None:
+            self.model.pack_weights()                # allocates the packed copy (first use)
+        a = self._pass_args(sb)
+        return type(a).from_buffer_copy(a)
+
     def _call(self, sb: StagedBatch, phases: int, stream, where: str) -> None:
         if sb.n_atoms > self.n_atoms_cap or sb.n_mols > self.n_mols_cap or sb.dtype != self.dtype:
             raise ValueError("batch does not fit this evaluator")
@@ -117,6 +124,28 @@ class EnergyForces:
                    | ((_lib.PASS_BACKWARD | _lib.PASS_COORD_GRAD) if forces else 0), stream, "EnergyForces.run")
 
     KERNELS_PER_PASS = 7   # weight packing (unless pack=False), sort, featurize, mlp forward, molecule sums, mlp backward, featurize_grad
+
+
+class PassTools:
+    """What a pass over a data set (``predict``, ``coordinate_gradients``) keeps for the next one: two sets of device
+    buffers, a stream for each, and pinned buffers for the results."""
+
+    def __init__(self, model, cap_atoms: int, cap_mols: int, device):
+        self.staged = [StagedBatch(cap_atoms, cap_mols, model.precision, device=device) for _ in range(2)]
+        self.evaluators = [EnergyForces(model, cap_atoms, cap_mols, device=device) for _ in range(2)]
+        self.streams = [torch.cuda.Stream(device=device) for _ in range(2)]
+        self.ring = []
+
+    def fits(self, cap_atoms: int, cap_mols: int) -> bool:
+        return self.staged[0].n_atoms_cap >= cap_atoms and self.staged[0].n_mols_cap >= cap_mols
+
+    def blocks(self):
+        return [ev.pass_block(sb) for ev, sb in zip(self.evaluators, self.staged)]
+
+    def host_ring(self, size: int):
+        if size and (not self.ring or self.ring[0].numel() < size):
+            self.ring = [torch.empty(size, dtype=self.staged[0].dtype).pin_memory() for _ in range(_lib.DRIVER_RING)]
+        return self.ring if size else []
 
 
 class SingleGeometry:

@@ -183,6 +183,12 @@ class FusedTrainStep:
         a.features = sb.features.data_ptr()
         return a
 
+    def pass_blocks(self, staged):
+        """Argument blocks of passes over ``staged`` for a ``BatchDriver``, which fills in what describes the batch."""
+        if self.model.packed_weights() is None:
+            self.model.pack_weights(self._stream())  # allocates the packed copy (first use)
+        return [_lib.PassArgs.from_buffer_copy(self._pass_args(sb)) for sb in staged]
+
     def forward_backward(self, sb: StagedBatch, labels: torch.Tensor, feature_grad: bool = True,
                          featurized: bool = False) -> None:
         """Everything up to the weight gradients, in order on the current stream: weight packing, sort,

@@ -78,6 +78,15 @@ class FlatNadam:
         """Max-norm constraint on the rows of the matrices ``self.params[k]``, k in ``indices``
         (``tf.clip_by_norm(w, max_norm, axes=1)``): one launch over a row table that is built on the
         first call."""
+        f = self.clip_fields(indices, max_norm)
+        stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        with torch.cuda.device(self.device):
+            _lib.check(_lib.lib().ani_clip_rows_f32(self.flat_params.data_ptr(), f["clip_row_offsets"],
+                                                    f["clip_row_lengths"], f["clip_n_rows"], f["clip_max_norm"], stream),
+                       "ani_clip_rows_f32")
+
+    def clip_fields(self, indices, max_norm: float) -> dict:
+        """The row table of :meth:`clip_rows` as fields of ``ani_driver_args``."""
         key = tuple(indices)
         if getattr(self, "_row_key", None) != key:
             offs, lens = [], []
@@ -89,11 +98,20 @@ class FlatNadam:
             self._row_offsets = torch.tensor(offs, dtype=torch.int32, device=self.device)
             self._row_lengths = torch.tensor(lens, dtype=torch.int32, device=self.device)
             self._row_key = key
+        return dict(clip_row_offsets=self._row_offsets.data_ptr(), clip_row_lengths=self._row_lengths.data_ptr(),
+                    clip_n_rows=int(self._row_offsets.numel()), clip_max_norm=float(max_norm))
+
+    def driver_fields(self, update: bool) -> dict:
+        """The buffers of :meth:`step` as fields of ``ani_driver_args``."""
+        return dict(params=self.flat_params.data_ptr(), grads=self.flat_grads.data_ptr(), m=self.m.data_ptr(),
+                    v=self.v.data_ptr(), ema=self.ema.data_ptr(), n_params=self.n, hyper=self.hyper.data_ptr(),
+                    state=self.state.data_ptr(), update=int(update))
+
+    def scale_by_loss(self, l2s: torch.Tensor, kind: int, rmse: torch.Tensor) -> None:
+        """Gradients of the mse -> of the rmse (kind 1) or exp(rmse) (kind 2); ``rmse`` receives the rmse."""
         stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
-        with torch.cuda.device(self.device):
-            _lib.check(_lib.lib().ani_clip_rows_f32(self.flat_params.data_ptr(), self._row_offsets.data_ptr(),
-                                                    self._row_lengths.data_ptr(), int(self._row_offsets.numel()),
-                                                    float(max_norm), stream), "ani_clip_rows_f32")
+        _lib.check(_lib.lib().ani_scale_by_loss_f32(self.flat_grads.data_ptr(), self.n, l2s.data_ptr(), l2s.numel(), kind,
+                                                    rmse.data_ptr(), stream), "ani_scale_by_loss_f32")
 
     def steps_done(self) -> int:
         """The device-side step counter (synchronises)."""

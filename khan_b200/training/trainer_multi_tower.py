@@ -26,7 +26,7 @@ import torch
 
 from .. import _lib, ani_mod
 from ..data.dataset import RawDataset
-from ..data.feeder import BatchFeeder, PackedDataset
+from ..data.feeder import BatchDriver, BatchFeeder, PackedDataset
 from ..model import activations
 from ..model.nn import MoleculeNN
 from ..utils.helpers import ed_harder_rmse
@@ -48,6 +48,11 @@ def flatten_results(res, pos=0):
     return np.concatenate(flattened).reshape((-1,))
 
 
+def single_rank() -> bool:
+    import torch.distributed as dist
+    return not (dist.is_available() and dist.is_initialized()) or dist.get_world_size() == 1
+
+
 def average_gradients(parameters, flat_grads=None, peer=None):
     """Mean of the weight gradients over all ranks: ONE all-reduce of a flat bucket (296,452
     values for four 384-128-128-64-1 networks), the data-parallel replacement of the reference's
@@ -56,9 +61,9 @@ def average_gradients(parameters, flat_grads=None, peer=None):
     slices of (``FlatNadam.flat_grads``); it is reduced in place with no packing.  ``peer``: a
     ``PeerAllReduce`` -- the mean is then one kernel of this library over peer memory instead of the
     library collective (and may be captured in a CUDA graph)."""
-    import torch.distributed as dist
-    if not (dist.is_available() and dist.is_initialized()) or dist.get_world_size() == 1:
+    if single_rank():
         return
+    import torch.distributed as dist
     if peer is not None and flat_grads is not None:
         peer.mean_(flat_grads)
         return
@@ -386,63 +391,65 @@ class TrainerMultiTower:
         _, sbs, step, side = self._fused
         if getattr(self, "_rmse_buf", None) is None:
             self._rmse_buf = torch.zeros((), dtype=torch.float32, device=dev)
-        # Two batches in flight: sort + featurize of the NEXT batch run on a side stream beside the network
-        # kernels of this one (they need nothing but the coordinates; the network kernels leave a quarter of
-        # the SMs free), as in StepPipeline.  The sequence of weights is that of the serial order.
-        feeder = iter(it)
+        loss_kind = {"train_op": 2, "train_op_rmse": 1}.get(kind, 0)
+        hooks = [] if before_hooks is None else list(before_hooks if isinstance(before_hooks, (list, tuple)) else [before_hooks])
+        optimizer = self.optimizer
+        if it.native is not None:
+            # The step of a batch is one native call (BatchDriver); with several ranks it ends before the update, which
+            # waits for the other ranks' gradients.  Two batches are in flight, as in StepPipeline, and the sequence of
+            # weights is that of the serial order.
+            alone = single_rank()
+            fields = optimizer.driver_fields(update=alone)
+            fields.update(loss_kind=loss_kind, rmse=self._rmse_buf.data_ptr())
+            if len(hooks) == 1 and isinstance(hooks[0], _Op) and hooks[0].name == "max_norm_ops":
+                fields.update(optimizer.clip_fields(self._weight_matrix_indices(), 3.0))
+                hooks = []
+            with torch.cuda.device(dev):
+                driver = BatchDriver(it, _lib.DRIVER_TRAIN, step.pass_blocks(sbs), [side], keep=(sbs, step), **fields)
 
-        def start(fed, sb):
-            """Sort + featurize of a fed batch on the side stream, behind everything enqueued on the main one
-            (the previous use of ``sb`` among it)."""
-            side.wait_stream(torch.cuda.current_stream(dev))
-            with torch.cuda.stream(side):
+            def advance():
+                if not driver.step():
+                    return None
+                if not alone:
+                    average_gradients(self.parameters, optimizer.flat_grads)
+                    optimizer.step()
+                return driver.batch.n_mols, driver.batch.batch_index
+        else:
+            def advance():
+                fed = next(it, None)
+                if fed is None:
+                    return None
                 fed.wait()
-                sb.adopt(fed)
-                step.featurize_pass(sb)
+                sbs[0].adopt(fed)
+                step.forward_backward(sbs[0], fed.ys, feature_grad=False)
+                if loss_kind:
+                    optimizer.scale_by_loss(step.l2s[:fed.n_mols], loss_kind, self._rmse_buf)
+                average_gradients(self.parameters, optimizer.flat_grads)
+                optimizer.step()
+                return fed.n_mols, fed.index
 
-        with torch.cuda.device(dev):
-            fed = next(feeder, None)
-            if fed is not None:
-                start(fed, sbs[0])
-        k = 0
-        while fed is not None:
-            if before_hooks is not None:
-                self._run_hooks(before_hooks)
+        for _ in range(it.packed.num_batches(it.batch_size)):
+            if hooks:
+                self._run_hooks(hooks)
             with torch.cuda.device(dev), torch.no_grad():
-                sb = sbs[k & 1]
-                main = torch.cuda.current_stream(dev)
-                main.wait_stream(side)                      # this batch's features are there
-                nxt = next(feeder, None)
-                if nxt is not None:
-                    start(nxt, sbs[(k + 1) & 1])
-                step.forward_backward(sb, fed.ys, feature_grad=False, featurized=True)
-                l2 = step.l2s[:fed.n_mols]
-                rmse = None
-                if kind in ("train_op", "train_op_rmse"):
-                    # one launch: rmse on the device, the weight gradients scaled by d loss / d mse
-                    rmse = self._rmse_buf
-                    g = self.optimizer.flat_grads
-                    _lib.check(_lib.lib().ani_scale_by_loss_f32(
-                        g.data_ptr(), g.numel(), l2.data_ptr(), fed.n_mols, 2 if kind == "train_op" else 1,
-                        rmse.data_ptr(), ctypes.c_void_p(main.cuda_stream)), "ani_scale_by_loss_f32")
-                elif "tower_exp_loss" in names:
-                    rmse = l2.mean().sqrt().clamp_min(1e-30)
-                average_gradients(self.parameters, self.optimizer.flat_grads)
-                self.optimizer.step()
+                done = advance()
+                if done is None:
+                    return
+                n_mols, index = done
                 self.global_step += 1
                 row = []
                 for n in names:
                     if n.startswith("train_op"):
                         row.append(None)
                     elif n in ("unordered_l2s", "tower_l2s"):
-                        row.append([l2.cpu().numpy()])
+                        row.append([step.l2s[:n_mols].cpu().numpy()])
                     elif n == "_device_l2s":
-                        row.append([l2.clone()])
+                        row.append([step.l2s[:n_mols].clone()])
                     elif n == "tower_exp_loss":
+                        rmse = self._rmse_buf if loss_kind else step.l2s[:n_mols].mean().sqrt().clamp_min(1e-30)
                         row.append([float(torch.exp(rmse.double()))])
                     elif n == "tower_bids":
-                        row.append([np.array(fed.index)])
-                fed, k = nxt, k + 1
+                        row.append([np.array(index)])
             yield row
 
     def _force_rounds(self, it, names, capacity, before_hooks):
@@ -542,10 +549,7 @@ class TrainerMultiTower:
             if isinstance(h, _Op) and h.name == "max_norm_ops":
                 # tf.clip_by_norm(w, 3.0, axes=1) over all weight matrices, trainer_multi_tower.py:432-436
                 if isinstance(self.optimizer, FlatNadam):
-                    if not hasattr(self, "_weight_indices"):
-                        weights = {id(w) for w in self._weight_matrices()}
-                        self._weight_indices = [k for k, p in enumerate(self.parameters) if id(p) in weights]
-                    self.optimizer.clip_rows(self._weight_indices, 3.0)
+                    self.optimizer.clip_rows(self._weight_matrix_indices(), 3.0)
                     continue
                 with torch.no_grad():
                     for w in self._weight_matrices():
@@ -553,6 +557,12 @@ class TrainerMultiTower:
                         w.mul_(torch.clamp(3.0 / norms, max=1.0))
             elif callable(h):
                 h()
+
+    def _weight_matrix_indices(self):
+        if not hasattr(self, "_weight_indices"):
+            weights = {id(w) for w in self._weight_matrices()}
+            self._weight_indices = [k for k, p in enumerate(self.parameters) if id(p) in weights]
+        return self._weight_indices
 
     def _apply_gradients(self, losses):
         """Average of the tower gradients (and of all ranks when torch.distributed is up),
@@ -579,9 +589,15 @@ class TrainerMultiTower:
         """Energies (and squared errors, when the data set has targets) of every batch, left on
         the devices: nothing here waits for the GPU, so the host runs ahead of it by as many
         batches as the feeder allows, and the caller synchronises once."""
-        np_dt = np.float32 if self.precision == torch.float32 else np.float64
+        np_dt = self._np_dtype()
         if self._evaluator_usable(dataset):
-            return self._evaluator_predictions(dataset, batch_size)
+            packed = PackedDataset.from_raw(dataset, np_dt)
+            with torch.cuda.device(self.towers[0]):
+                out = torch.empty(packed.num_mols(), dtype=self.precision, device=self.towers[0])
+                for _, tools in self._driven(packed, batch_size, _lib.DRIVER_ENERGIES, energies=out.data_ptr()):
+                    pass
+                self._infer = tools
+                return [out], [] if packed.ys is None else [(out - torch.from_numpy(packed.ys).to(out.device)) ** 2]
         it = BatchFeeder(PackedDataset.from_raw(dataset, np_dt), batch_size, False, None,
                          devices=self.towers, depth=2, hold=self.num_towers)
         preds, l2s = [], []
@@ -598,6 +614,8 @@ class TrainerMultiTower:
 
     def predict(self, dataset, batch_size=2048):
         """Predicted energies in dataset order (``trainer_multi_tower.py:655-678``)."""
+        if self._evaluator_usable(dataset):
+            return self._evaluator_energies(dataset, batch_size)
         preds, _ = self._device_predictions(dataset, batch_size)
         if not preds:
             return []
@@ -639,97 +657,66 @@ class TrainerMultiTower:
     def _np_dtype(self):
         return np.float32 if self.precision == torch.float32 else np.float64
 
-    def _evaluator(self, packed, batch_size):
-        from ..inference import EnergyForces
-        from ..staged import StagedBatch
+    def _driven(self, packed, batch_size, mode, host_width=0, **fields):
+        """Runs the evaluator over ``packed``, two batches in flight, yielding (driver, tools) behind each batch.
+        ``host_width``: values per atom (gradients) or molecule (energies) of the results left in host memory.  The
+        caller gives the tools back (``self._infer``) once it has read its results."""
         cap_atoms, cap_mols = (max(v, 1) for v in packed.capacity(batch_size))
+        host_size = host_width * (cap_mols if mode == _lib.DRIVER_ENERGIES else cap_atoms)
         dev = self.towers[0]
-        cached = getattr(self, "_infer", None)
-        if cached is None or cached[0][0] < cap_atoms or cached[0][1] < cap_mols:
-            self._infer = cached = ((cap_atoms, cap_mols), StagedBatch(cap_atoms, cap_mols, self.precision, device=dev),
-                                    EnergyForces(self.model, cap_atoms, cap_mols, device=dev))
-        return cached[1], cached[2]
-
-    def _evaluator_predictions(self, dataset, batch_size):
-        """``_device_predictions`` through the evaluator: sort, featurize, networks forward and the
-        molecule sums as four C-ABI calls per batch, the weights packed once."""
-        packed = PackedDataset.from_raw(dataset, self._np_dtype())
-        sb, ev = self._evaluator(packed, batch_size)
-        dev = self.towers[0]
-        # two batches at a time: sort + featurize of the next one on a side stream beside the networks of this one
-        twin = getattr(self, "_infer_twin", None)
-        if twin is None or twin[0].n_atoms_cap < sb.n_atoms_cap or twin[0].n_mols_cap < sb.n_mols_cap:
-            from ..staged import StagedBatch
-            twin = self._infer_twin = (StagedBatch(sb.n_atoms_cap, sb.n_mols_cap, self.precision, device=dev),
-                                       torch.cuda.Stream(device=dev))
-        sbs, side = (sb, twin[0]), twin[1]
+        # taken away while the pass runs, so that a pass begun in the middle of another one has its own
+        tools = self.__dict__.pop("_infer", None)
+        if tools is None or not tools.fits(cap_atoms, cap_mols):
+            from ..inference import PassTools
+            tools = PassTools(self.model, cap_atoms, cap_mols, dev)
         it = BatchFeeder(packed, batch_size, False, None, devices=self.towers, depth=3, hold=2, mol_ids=False)
-        preds, l2s = [], []
-
-        def start(fed, target):
-            side.wait_stream(torch.cuda.current_stream(dev))      # the previous use of `target` is among it
-            with torch.cuda.stream(side):
-                fed.wait()
-                target.adopt(fed)
-                ev.featurize(target)
-
+        driver = None
         try:
-            with torch.cuda.device(dev), torch.no_grad():
-                feeder = iter(it)
-                fed, k = next(feeder, None), 0
-                if fed is not None:
-                    start(fed, sbs[0])
-                while fed is not None:
-                    torch.cuda.current_stream(dev).wait_stream(side)
-                    nxt = next(feeder, None)
-                    if nxt is not None:
-                        start(nxt, sbs[(k + 1) & 1])
-                    ev.run(sbs[k & 1], pack=(k == 0), forces=False, featurized=True)
-                    preds.append(ev.mol_energy[:fed.n_mols].clone())
-                    if fed.ys is not None:
-                        l2s.append((preds[-1] - fed.ys) ** 2)
-                    fed, k = nxt, k + 1
+            with torch.cuda.device(dev):
+                driver = BatchDriver(it, mode, tools.blocks(), tools.streams, tools.host_ring(host_size), keep=tools, **fields)
+            while True:
+                with torch.cuda.device(dev):
+                    more = driver.step()
+                if not more:
+                    break
+                yield driver, tools
         finally:
+            if driver is not None:
+                with torch.cuda.device(dev):
+                    driver.join()
             it.close()
-        return preds, l2s
+
+    def _behind(self, driven, finished):
+        """``finished(host buffer, n_atoms, n_mols, index)`` of every batch once its results are in host memory, up to
+        two batches behind the GPU: the host works on a batch while the GPU works on the next ones."""
+        pending, driver, tools = [], None, None
+        for k, (driver, tools) in enumerate(driven):
+            b, place = driver.batch, k % _lib.DRIVER_RING
+            pending.append((place, tools.ring[place].numpy(), b.n_atoms, b.n_mols, int(b.batch_index)))
+            if len(pending) == _lib.DRIVER_RING:       # the place of batch k + 1 must be free again
+                driver.wait(pending[0][0])
+                yield finished(*pending.pop(0)[1:])
+        for entry in pending:
+            driver.wait(entry[0])
+            yield finished(*entry[1:])
+        self._infer = tools
+
+    def _evaluator_energies(self, dataset, batch_size):
+        packed = PackedDataset.from_raw(dataset, self._np_dtype())
+        out = []
+        for part in self._behind(self._driven(packed, batch_size, _lib.DRIVER_ENERGIES, 1),
+                                 lambda buf, n_atoms, n_mols, index: buf[:n_mols].tolist()):
+            out += part
+        return out
 
     def _evaluator_gradients(self, dataset, batch_size):
-        """Gradients of all molecules through the evaluator, one list per batch.  The result of a batch is copied to a pinned
-        host buffer behind its kernels, and the host cuts the PREVIOUS batch into per-molecule arrays while
-        the GPU works on this one (cutting 32,768 molecules takes as long as computing them)."""
+        """Gradients of all molecules through the evaluator, one list per batch (cutting a batch into per-molecule
+        arrays takes as long as computing it)."""
         packed = PackedDataset.from_raw(dataset, self._np_dtype())
-        sb, ev = self._evaluator(packed, batch_size)
-        cap = sb.n_atoms_cap
-        ring = getattr(self, "_grad_ring", None)
-        if ring is None or ring[0].shape[0] < cap:
-            ring = self._grad_ring = [torch.empty((cap, 3), dtype=self.precision).pin_memory() for _ in range(3)]
-        it = BatchFeeder(packed, batch_size, False, None, devices=self.towers, depth=2, hold=1, mol_ids=False)
-        pending = []      # (host buffer, event, n_atoms, batch index) of batches whose copy is in flight
         slices = packed.batch_slices(batch_size)
-
-        def finished(entry):
-            buf, evt, n, k = entry
-            evt.synchronize()
-            return list(map(buf[:n].numpy().copy().__getitem__, slices[k]))
-
-        try:
-            with torch.cuda.device(self.towers[0]), torch.no_grad():
-                for k, fed in enumerate(it):
-                    fed.wait()
-                    sb.adopt(fed)
-                    ev.run(sb, pack=(k == 0))
-                    n = fed.n_atoms
-                    buf = ring[k % len(ring)]
-                    buf[:n].copy_(sb.grads[:, :n].t(), non_blocking=True)      # (n_atoms, 3), strided read on the device
-                    evt = torch.cuda.Event()
-                    evt.record()
-                    pending.append((buf, evt, n, fed.index))
-                    if len(pending) == len(ring):       # the buffer of batch k + 1 must be free again
-                        yield finished(pending.pop(0))
-        finally:
-            it.close()
-        for entry in pending:
-            yield finished(entry)
+        return self._behind(self._driven(packed, batch_size, _lib.DRIVER_GRADIENTS, 3),
+                            lambda buf, n_atoms, n_mols, index:
+                            list(map(buf[:3 * n_atoms].reshape(n_atoms, 3).copy().__getitem__, slices[index])))
 
     def energy_and_gradient(self, X):
         """Energy and ``(n, 3)`` gradient of ONE geometry ``[[type, x, y, z], ...]``: what ``predict`` and
