@@ -199,10 +199,7 @@ template <typename K> int set_smem(K kernel, size_t bytes)
 // 256 molecules of 64-256 atoms: 26 % fewer instructions and 104 instead of 139 us alone, but 99
 // instead of 90 us per launch with four batches in flight, so it is not used.)
 constexpr int kMolMeanLimit = 24;
-#ifndef ANI_MOL_GRAD_WARPS
-#define ANI_MOL_GRAD_WARPS 4
-#endif
-constexpr int kMolGradWarps = ANI_MOL_GRAD_WARPS;   // warps of a CTA (= molecule) of the small-molecule gradient kernel
+constexpr int kSms = 148;
 bool small_molecules(long long n_atoms, int n_mols) { return n_mols > 0 && n_atoms <= (long long)n_mols * kMolMeanLimit; }
 
 // True when every non-null pointer of the list is 16-byte aligned.
@@ -242,13 +239,21 @@ int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, cons
 
     int dev = 0;
     ANI_CUDA(cudaGetDevice(&dev));
-    // small molecules with outputs that take 16-byte stores: one warp (= one CTA) per round of four
+    // small molecules with outputs that take 16-byte stores: one warp (= one CTA) per round of one to four
     // central atoms
     if (small_molecules(n_atoms, n_mols) && all_aligned16({oh, oc, on, oo}) &&
-        (long long)n_mols * kMolRounds <= 0x7fffffffLL) {
-        ANI_CUDA(launch_chain(featurize_mol_kernel<T>, n_mols * kMolRounds, kWarp, 0, (cudaStream_t)stream, 1, xs, ys, zs,
+        (long long)n_mols * kMolMaxAtoms <= 0x7fffffffLL) {
+        // As few central atoms per warp as still find all warps resident at once (28 per SM in float, 20 in double): with
+        // four, the scans and triplets of one warp are a chain of 12 us (float; double 22 us), however small the batch.
+        // Few atoms per warp cost more instructions (load, sort and table per round), so not beyond that.  Microseconds
+        // with 4 / 2 / 1 atoms in float, 64 molecules 13.6 / 10.3 / 8.3, 256: 16.5 / 13.3 / 13.2, 512: 19.8 / 17.4 / 20.5,
+        // 1024: 24.9 / 26.5 / 39.0; in double, 64: 25 / 18 / 15, 512: 39 / 41 / 47.
+        const int resident = kSms * (sizeof(T) == 4 ? 28 : 20);
+        const int per_round = (int)std::min<long long>((n_atoms + resident - 1) / resident, kMolCentrals);
+        const int rounds = (kMolMaxAtoms + per_round - 1) / per_round;
+        ANI_CUDA(launch_chain(featurize_mol_kernel<T>, n_mols * rounds, kWarp, 0, (cudaStream_t)stream, 1, xs, ys, zs,
                               types, mos, macs, n_mols, (int)n_atoms, sis, oh, oc, on, oo, acs_host[0], acs_host[1],
-                              acs_host[2], acs_host[3]));
+                              acs_host[2], acs_host[3], per_round));
         return ANI_OK;
     }
 
@@ -303,23 +308,35 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
     // One CTA per molecule when the molecules are small and the upstream rows can be fetched with
     // 16-byte copies: writes every output itself, so no zero fill.
     if (n_mols > 0 && small_molecules(n_atoms, n_mols) && all_aligned16({gh, gc, gn, go}) &&
-        (long long)n_mols * kMolGradClasses <= 0x7fffffffLL) {
+        (long long)n_mols * 3 <= 0x7fffffffLL) {
         if (!xs || !ys || !zs || !types || !mos || !macs || !sis) return ANI_ERR_NULL_POINTER;
         for (int t = 0; t < kTypes; t++)
             if (acs_host[t] > 0 && !gin[t]) return ANI_ERR_NULL_POINTER;
-        auto mol_kernel = featurize_grad_mol_kernel<T, kMolGradWarps>;
-        const size_t mol_smem = mol_grad_smem_bytes<T, kMolGradWarps>();
-        static thread_local int mol_configured_dev = -1;
-        int dev = 0;
-        ANI_CUDA(cudaGetDevice(&dev));
-        if (mol_configured_dev != dev) {
-            if (int rc = set_smem(mol_kernel, mol_smem)) return rc;
-            mol_configured_dev = dev;
-        }
-        ANI_CUDA(launch_chain(mol_kernel, n_mols * kMolGradClasses, kMolGradWarps * kWarp, mol_smem, st, 1, xs, ys, zs, types,
-                              mos, macs, n_mols, (int)n_atoms, sis, gh, gc, gn, go, gx, gy, gz, acs_host[0], acs_host[1],
-                              acs_host[2], acs_host[3]));
-        return ANI_OK;
+        auto launch = [&](auto warps) -> int {
+            constexpr int NW = decltype(warps)::value;
+            constexpr size_t smem = mol_grad_smem_bytes<T, NW>();
+            static thread_local int configured_dev = -1;     // one per NW
+            int dev = 0;
+            ANI_CUDA(cudaGetDevice(&dev));
+            if (configured_dev != dev) {
+                if (int rc = set_smem(featurize_grad_mol_kernel<T, NW>, smem)) return rc;
+                configured_dev = dev;
+            }
+            // More molecules than are resident at once: by size class, largest first (classes relative to the mean, of
+            // which the data sets' largest molecules are twice).  Alone, 1024 molecules of up to 8 heavy atoms: float
+            // 35.6 -> 32.2 us, double 101 -> 78; 2048: 52.8 -> 47.3, 155 -> 139; without effect at 8192.
+            const bool classes = (long long)n_mols * NW > (long long)kSms * (sizeof(T) == 4 ? 20 : 12);
+            const int mean8 = (int)(8 * n_atoms / n_mols);
+            ANI_CUDA(launch_chain(featurize_grad_mol_kernel<T, NW>, classes ? 3 * n_mols : n_mols, NW * kWarp, smem, st, 1, xs,
+                                  ys, zs, types, mos, macs, n_mols, (int)n_atoms, sis, gh, gc, gn, go, gx, gy, gz,
+                                  acs_host[0], acs_host[1], acs_host[2], acs_host[3], mean8 * 7 / 64, mean8 * 12 / 64));
+            return ANI_OK;
+        };
+        // Eight warps a molecule shorten its chain of scans and pair passes (64 molecules 14.8 -> 10.6 us, 512: 27.4 ->
+        // 20.4, double 38 -> 25 and 68 -> 58), four keep more of the lanes and the SM busy once there are several
+        // molecules per SM (1024: 32.2 against 34.5, 8192: 159 against 222; double 78 against 107).
+        if (n_mols <= kSms * (sizeof(T) == 4 ? 6 : 4)) return launch(std::integral_constant<int, 8>{});
+        return launch(std::integral_constant<int, 4>{});
     }
     {
         const int threads = 256;

@@ -1,9 +1,9 @@
 // Forward kernel for batches of small molecules (at most 32 atoms each, the size range of the
 // data sets khan trains on: its loaders drop larger molecules, data_utils.py:54,281-283).
 //
-// The central atoms of a molecule, in element order, are dealt to ROUNDS of at most four atoms
-// (round r of R takes atoms r, r + R, ...), and a CTA is ONE WARP doing one round: a molecule has 8 CTAs (8 rounds, 32 atoms), a
-// CTA whose round lies behind the end of the molecule leaves after one load.  No warp needs
+// The central atoms of a molecule, in element order, are dealt to ROUNDS of at most `per_round` <= 4 atoms
+// (round r of R takes atoms r, r + R, ...), and a CTA is ONE WARP doing one round: a molecule has as many CTAs as 32
+// atoms have rounds, and a CTA whose round lies behind the end of the molecule leaves after one load.  No warp needs
 // anything from another, every round gives its registers and shared memory back as soon as it
 // is done, and the rounds of a large molecule spread over the SMs.  A warp keeps the whole
 // molecule in registers, lane = atom:
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
                          const int* __restrict__ types, const int* __restrict__ mol_offsets,
                          const int* __restrict__ mol_counts, int n_mols, int n_atoms,
                          const int* __restrict__ scatter, T* out_h, T* out_c, T* out_n, T* out_o,
-                         int acs0, int acs1, int acs2, int acs3)
+                         int acs0, int acs1, int acs2, int acs3, int per_round)
 {
     __shared__ MolFwdWarpShared<T> ws;
     using Granule = Vec4<float>;                      // 16 bytes of zeros, whatever T is
@@ -187,14 +187,15 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
 
     // Round-major order of the grid: all first rounds (every molecule has one), then all second rounds, ...
     // so the work that exists starts first and is spread evenly over the SMs, and the CTAs of rounds that
-    // most molecules do not have come last.
+    // most molecules do not have come last.  (The other way round, big molecules first: 8 to 13 % slower, the CTAs
+    // without work then hold up the start.)
     const int round = blockIdx.x / n_mols, m = blockIdx.x - round * n_mols;
     MolRange mol;
     if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) return;
     const int n = mol.n, base = mol.base;
 
     if (n > kMolMaxAtoms) {   // a large molecule in a batch of small ones: its CTAs take one atom at a time
-        for (int i = round; i < n; i += kMolRounds) {
+        for (int i = round; i < n; i += gridDim.x / n_mols) {
             const int gi = base + i;
             const int ti = checked_type(types[gi]);
             const int srow = scatter[gi];
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     // Round r of a molecule with R rounds takes the central atoms r, r + R, r + 2 R, r + 3 R: every round
     // gets the same mix of light and heavy atoms (atoms are in element order, and the cost of a central
     // atom grows with the square of its neighbour count), so the rounds of a molecule cost about the same.
-    const int n_rounds = (n + kMolCentrals - 1) / kMolCentrals;
+    const int n_rounds = (n + per_round - 1) / per_round;
     if (round >= n_rounds) return;
     const int G = (n - round + n_rounds - 1) / n_rounds;
 

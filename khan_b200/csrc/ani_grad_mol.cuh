@@ -34,10 +34,6 @@
 
 namespace ani {
 
-#ifndef ANI_MOL_GRAD_CLASSES
-#define ANI_MOL_GRAD_CLASSES 1
-#endif
-constexpr int kMolGradClasses = ANI_MOL_GRAD_CLASSES;   // size classes of molecules (1 or 3), in the order in which their CTAs start
 constexpr int kMolGradPitch = kMolMaxAtoms + 1;   // odd: rows and columns of the force table are both conflict-free
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
@@ -129,7 +125,7 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
                               const int* __restrict__ mol_counts, int n_mols, int n_atoms,
                               const int* __restrict__ scatter, const T* __restrict__ gh,
                               const T* __restrict__ gc, const T* __restrict__ gn, const T* __restrict__ go,
-                              T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3)
+                              T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3, int mid_size, int big_size)
 {
     constexpr int GR = MolGradCfg<T>::kRowBufs;   // central atoms per round
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -143,169 +139,165 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
         return part[(plane * kMolMaxAtoms + c) * kMolGradPitch + j];
     };
 
-    // The grid has kMolGradClasses CTAs per molecule, class-major.  With 3 classes: first one CTA for
-    // every molecule, of which only those of the largest molecules work (the others leave after one
-    // load), then the same for the middle sizes, then for the small ones; CTAs start in index order, so
-    // the expensive molecules start first and the cheap ones fill the SMs behind them.  Measured on
-    // 1024-molecule batches: a kernel running alone ends 10 % sooner (shorter tail), but with several
-    // batches in flight the extra CTAs cost 5 % of the throughput, so the default is one class.
-    for (int item = blockIdx.x; item < n_mols * kMolGradClasses; item += gridDim.x) {
-        const int cls = item / n_mols, m = item - cls * n_mols;
-        MolRange mol;
-        if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) continue;
-        const int n = mol.n, base = mol.base;
-        if (kMolGradClasses > 1 && cls != (n > 20 ? 0 : (n > 12 ? 1 : 2))) continue;
+    // With three CTAs per molecule in the grid, class-major: first one CTA for every molecule, of which only those of
+    // molecules above big_size work (the others leave after one load), then the same for those above mid_size, then for
+    // the rest; CTAs start in index order, so the expensive molecules start first and the cheap ones fill the SMs
+    // behind them.
+    const bool classes = (int)gridDim.x > n_mols;
+    const int cls = blockIdx.x / n_mols, m = blockIdx.x - cls * n_mols;
+    MolRange mol;
+    if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) return;
+    const int n = mol.n, base = mol.base;
+    if (classes && cls != (n > big_size ? 0 : (n > mid_size ? 1 : 2))) return;
 
-        if (n > kMolMaxAtoms) {   // a large molecule in a batch of small ones
-            for (int j = threadIdx.x; j < n; j += NW * kWarp) {
-                gx[base + j] = (T)0;
-                gy[base + j] = (T)0;
-                gz[base + j] = (T)0;
-            }
-            __syncthreads();
-            for (int i = warp; i < n; i += NW) {
-                const int gi = base + i;
-                const int ti = checked_type(types[gi]);
-                const int srow = scatter[gi];
-                const int cap = ti == 0 ? acs0 : (ti == 1 ? acs1 : (ti == 2 ? acs2 : acs3));
-                if (srow < 0 || srow >= cap) {
-                    if (lane == 0) report(ANI_ERR_BAD_INDEX);
-                    continue;
-                }
-                const T* grow = (ti == 0 ? gh : (ti == 1 ? gc : (ti == 2 ? gn : go))) + (size_t)srow * kTotal;
-                T* g = ws.g[0];
-                g[lane] = grow[lane];
-                g[32 + lane] = grow[32 + lane];
-                for (int bk = 0; bk < kPairBuckets; bk++)
-                    g[kRadial + bk * kGradBucketStride + lane] = grow[kRadial + bk * kTS + lane];
-                __syncwarp();
-                grad_atom_streaming_radial<T>(xs, ys, zs, types, base, n, i, g, gx, gy, gz);
-                grad_atom_streaming<T>(xs, ys, zs, types, base, n, i, g, gx, gy, gz);
-                __syncwarp();
-            }
-            continue;
-        }
-
-        // every warp needs the sort for the last step, also one without a round of its own
-        MolLanes<T> ml;
-        load_sorted_molecule<T>(xs, ys, zs, types, scatter, base, n, &ws.sort, &ml);
-
-        // Warp w takes the central atoms w, w + NW, w + 2 NW, ... (element order) and walks them in rounds
-        // of GR: every warp gets the same number of atoms (no idle warps) AND the same mix of light and heavy
-        // ones -- the cost of a central atom grows with the square of its neighbour count, and consecutive
-        // atoms are of one element.  Which warp starts with atom 0 rotates with the molecule: a warp's
-        // scheduler is fixed by its index, and the last warps have one atom less.
-        const int w0 = (warp + m) % NW;
-        const int K = w0 < n ? (n - w0 + NW - 1) / NW : 0;   // central atoms of this warp
-        for (int k_first = 0; k_first < K; k_first += GR) {
-            const int G = min(GR, K - k_first);
-            // ---- upstream rows of the round: one commit group per row slot ----
-#pragma unroll
-            for (int g = 0; g < GR; g++) {
-                const int c = min(w0 + (k_first + g) * NW, n - 1);
-                const int ti = __shfl_sync(kFull, ml.type, c), sr = ws.sort.srow[c];
-                const int cap = ti == 0 ? acs0 : (ti == 1 ? acs1 : (ti == 2 ? acs2 : acs3));
-                if (g < G && sr >= 0 && sr < cap) {
-                    const T* grow = (ti == 0 ? gh : (ti == 1 ? gc : (ti == 2 ? gn : go))) + (size_t)sr * kTotal;
-                    T* dst = ws.g[g];
-                    constexpr int V = 16 / (int)sizeof(T);   // values per 16-byte copy
-#pragma unroll
-                    for (int s = 0; s < kTotal / V / kWarp; s++) {
-                        const int v = (lane + s * kWarp) * V;
-                        const int d = v < kRadial
-                                          ? v
-                                          : kRadial + ((v - kRadial) >> 5) * kGradBucketStride + ((v - kRadial) & 31);
-                        cp_async16(dst + d, grow + v);
-                    }
-                }
-                cp_async_commit();
-            }
-
-            int g = 0;
-            while (g < G) {
-                // ---- A: scan central atoms into the neighbour list until it is full ----
-                int used = 0, max_half = 0, taken = 0;
-                while (g < G) {
-                    const int c = w0 + (k_first + g) * NW;
-                    const T xi = __shfl_sync(kFull, ml.x, c), yi = __shfl_sync(kFull, ml.y, c),
-                            zi = __shfl_sync(kFull, ml.z, c);
-                    const int ti = __shfl_sync(kFull, ml.type, c), sr = ws.sort.srow[c];
-                    const int cap = ti == 0 ? acs0 : (ti == 1 ? acs1 : (ti == 2 ? acs2 : acs3));
-                    const bool ok = sr >= 0 && sr < cap;
-                    const T dx = xi - ml.x, dy = yi - ml.y, dz = zi - ml.z;
-                    T r, inv;
-                    length_and_inverse(dx * dx + dy * dy + dz * dz, &r, &inv);
-                    const bool in_rad = ok && lane < n && lane != c && r < (T)kR_Rc;
-                    const bool in_ang = in_rad && r < (T)kA_Rc;
-                    const unsigned mA = __ballot_sync(kFull, in_ang);
-                    const int nA = __popc(mA);
-                    if (taken > 0 && used + nA > kWarp) break;   // this central atom opens the next pass
-
-                    // row slot g has landed when at most GR - 1 - g younger groups are pending
-                    if (g == 0) cp_async_wait<GR - 1>();
-                    else if (g == 1) cp_async_wait<(GR > 2 ? GR - 2 : 0)>();
-                    else if (g == 2) cp_async_wait<(GR > 3 ? GR - 3 : 0)>();
-                    else cp_async_wait<0>();
-                    __syncwarp();
-                    if (!ok && lane == 0) report(ANI_ERR_BAD_INDEX);
-                    const T* grow = ws.g[g];
-                    const T ux = dx * inv, uy = dy * inv, uz = dz * inv;
-                    T fx = (T)0, fy = (T)0, fz = (T)0;
-                    if (in_rad) {
-                        T fc, dfc;
-                        cutoff<T>(r, (T)kR_Rc, &fc, &dfc);
-                        T w[kNumRs];
-#pragma unroll
-                        for (int q = 0; q < kNumRs; q += 4) load4(grow + ml.type * kNumRs + q, w + q);
-                        const T d = radial_vjp_dev<T>(r, fc, dfc, w);
-                        fx = d * ux; fy = d * uy; fz = d * uz;
-                    }
-                    if (lane < n) {   // force on atom j from the radial terms of central atom c (0 out of range)
-                        part_at(0, c, lane) = -fx;
-                        part_at(1, c, lane) = -fy;
-                        part_at(2, c, lane) = -fz;
-                    }
-                    if (in_ang) {
-                        MolGradNeighbor<T> e;
-                        e.u = Vec4<T>{ux, uy, uz, r};
-                        e.inv_r = inv;
-                        cutoff<T>(r, (T)kA_Rc, &e.fc, &e.dfc);
-                        e.info = ml.type | (lane << 2) | (used << 7) | (nA << 12) | (g << 18) | (c << 20);
-                        ws.nb[used + __popc(mA & lanemask_lt())] = e;
-                    }
-                    used += nA;
-                    taken++;
-                    max_half = max(max_half, nA >> 1);
-                    g++;
-                }
-                __syncwarp();
-
-                // ---- B: neighbour pairs of every central atom in the list, circulant order ----
-                if (max_half > 0) {
-#include "ani_grad_pair_pass.inl"
-                    if (lane < used) {
-                        const int cen = (ea.info >> 20) & 31, at = (ea.info >> 2) & 31;
-                        part_at(0, cen, at) += fax;
-                        part_at(1, cen, at) += fay;
-                        part_at(2, cen, at) += faz;
-                    }
-                }
-                __syncwarp();
-            }
-            cp_async_wait<0>();   // row slots of a short round are empty groups; nothing may stay pending
+    if (n > kMolMaxAtoms) {   // a large molecule in a batch of small ones
+        for (int j = threadIdx.x; j < n; j += NW * kWarp) {
+            gx[base + j] = (T)0;
+            gy[base + j] = (T)0;
+            gz[base + j] = (T)0;
         }
         __syncthreads();
-        // gradient of atom j = what the central atoms handed to j (column j) - what j handed out (row j)
-        for (int plane = warp; plane < 3; plane += NW) {
-            if (lane < n) {
-                T col = (T)0, rw = (T)0;
-                for (int c = 0; c < n; c++) col += part_at(plane, c, lane);
-                for (int j = 0; j < n; j++) rw += part_at(plane, lane, j);
-                T* dst = plane == 0 ? gx : (plane == 1 ? gy : gz);
-                dst[base + ws.sort.src[lane]] = col - rw;
+        for (int i = warp; i < n; i += NW) {
+            const int gi = base + i;
+            const int ti = checked_type(types[gi]);
+            const int srow = scatter[gi];
+            const int cap = ti == 0 ? acs0 : (ti == 1 ? acs1 : (ti == 2 ? acs2 : acs3));
+            if (srow < 0 || srow >= cap) {
+                if (lane == 0) report(ANI_ERR_BAD_INDEX);
+                continue;
             }
+            const T* grow = (ti == 0 ? gh : (ti == 1 ? gc : (ti == 2 ? gn : go))) + (size_t)srow * kTotal;
+            T* g = ws.g[0];
+            g[lane] = grow[lane];
+            g[32 + lane] = grow[32 + lane];
+            for (int bk = 0; bk < kPairBuckets; bk++)
+                g[kRadial + bk * kGradBucketStride + lane] = grow[kRadial + bk * kTS + lane];
+            __syncwarp();
+            grad_atom_streaming_radial<T>(xs, ys, zs, types, base, n, i, g, gx, gy, gz);
+            grad_atom_streaming<T>(xs, ys, zs, types, base, n, i, g, gx, gy, gz);
+            __syncwarp();
         }
-        __syncthreads();   // the table is reused by the next molecule of this CTA
+        return;
+    }
+
+    // every warp needs the sort for the last step, also one without a round of its own
+    MolLanes<T> ml;
+    load_sorted_molecule<T>(xs, ys, zs, types, scatter, base, n, &ws.sort, &ml);
+
+    // Warp w takes the central atoms w, w + NW, w + 2 NW, ... (element order) and walks them in rounds
+    // of GR: every warp gets the same number of atoms (no idle warps) AND the same mix of light and heavy
+    // ones -- the cost of a central atom grows with the square of its neighbour count, and consecutive
+    // atoms are of one element.  Which warp starts with atom 0 rotates with the molecule: a warp's
+    // scheduler is fixed by its index, and the last warps have one atom less.
+    const int w0 = (warp + m) % NW;
+    const int K = w0 < n ? (n - w0 + NW - 1) / NW : 0;   // central atoms of this warp
+    for (int k_first = 0; k_first < K; k_first += GR) {
+        const int G = min(GR, K - k_first);
+        // ---- upstream rows of the round: one commit group per row slot ----
+#pragma unroll
+        for (int g = 0; g < GR; g++) {
+            const int c = min(w0 + (k_first + g) * NW, n - 1);
+            const int ti = __shfl_sync(kFull, ml.type, c), sr = ws.sort.srow[c];
+            const int cap = ti == 0 ? acs0 : (ti == 1 ? acs1 : (ti == 2 ? acs2 : acs3));
+            if (g < G && sr >= 0 && sr < cap) {
+                const T* grow = (ti == 0 ? gh : (ti == 1 ? gc : (ti == 2 ? gn : go))) + (size_t)sr * kTotal;
+                T* dst = ws.g[g];
+                constexpr int V = 16 / (int)sizeof(T);   // values per 16-byte copy
+#pragma unroll
+                for (int s = 0; s < kTotal / V / kWarp; s++) {
+                    const int v = (lane + s * kWarp) * V;
+                    const int d = v < kRadial
+                                      ? v
+                                      : kRadial + ((v - kRadial) >> 5) * kGradBucketStride + ((v - kRadial) & 31);
+                    cp_async16(dst + d, grow + v);
+                }
+            }
+            cp_async_commit();
+        }
+
+        int g = 0;
+        while (g < G) {
+            // ---- A: scan central atoms into the neighbour list until it is full ----
+            int used = 0, max_half = 0, taken = 0;
+            while (g < G) {
+                const int c = w0 + (k_first + g) * NW;
+                const T xi = __shfl_sync(kFull, ml.x, c), yi = __shfl_sync(kFull, ml.y, c),
+                        zi = __shfl_sync(kFull, ml.z, c);
+                const int ti = __shfl_sync(kFull, ml.type, c), sr = ws.sort.srow[c];
+                const int cap = ti == 0 ? acs0 : (ti == 1 ? acs1 : (ti == 2 ? acs2 : acs3));
+                const bool ok = sr >= 0 && sr < cap;
+                const T dx = xi - ml.x, dy = yi - ml.y, dz = zi - ml.z;
+                T r, inv;
+                length_and_inverse(dx * dx + dy * dy + dz * dz, &r, &inv);
+                const bool in_rad = ok && lane < n && lane != c && r < (T)kR_Rc;
+                const bool in_ang = in_rad && r < (T)kA_Rc;
+                const unsigned mA = __ballot_sync(kFull, in_ang);
+                const int nA = __popc(mA);
+                if (taken > 0 && used + nA > kWarp) break;   // this central atom opens the next pass
+
+                // row slot g has landed when at most GR - 1 - g younger groups are pending
+                if (g == 0) cp_async_wait<GR - 1>();
+                else if (g == 1) cp_async_wait<(GR > 2 ? GR - 2 : 0)>();
+                else if (g == 2) cp_async_wait<(GR > 3 ? GR - 3 : 0)>();
+                else cp_async_wait<0>();
+                __syncwarp();
+                if (!ok && lane == 0) report(ANI_ERR_BAD_INDEX);
+                const T* grow = ws.g[g];
+                const T ux = dx * inv, uy = dy * inv, uz = dz * inv;
+                T fx = (T)0, fy = (T)0, fz = (T)0;
+                if (in_rad) {
+                    T fc, dfc;
+                    cutoff<T>(r, (T)kR_Rc, &fc, &dfc);
+                    T w[kNumRs];
+#pragma unroll
+                    for (int q = 0; q < kNumRs; q += 4) load4(grow + ml.type * kNumRs + q, w + q);
+                    const T d = radial_vjp_dev<T>(r, fc, dfc, w);
+                    fx = d * ux; fy = d * uy; fz = d * uz;
+                }
+                if (lane < n) {   // force on atom j from the radial terms of central atom c (0 out of range)
+                    part_at(0, c, lane) = -fx;
+                    part_at(1, c, lane) = -fy;
+                    part_at(2, c, lane) = -fz;
+                }
+                if (in_ang) {
+                    MolGradNeighbor<T> e;
+                    e.u = Vec4<T>{ux, uy, uz, r};
+                    e.inv_r = inv;
+                    cutoff<T>(r, (T)kA_Rc, &e.fc, &e.dfc);
+                    e.info = ml.type | (lane << 2) | (used << 7) | (nA << 12) | (g << 18) | (c << 20);
+                    ws.nb[used + __popc(mA & lanemask_lt())] = e;
+                }
+                used += nA;
+                taken++;
+                max_half = max(max_half, nA >> 1);
+                g++;
+            }
+            __syncwarp();
+
+            // ---- B: neighbour pairs of every central atom in the list, circulant order ----
+            if (max_half > 0) {
+#include "ani_grad_pair_pass.inl"
+                if (lane < used) {
+                    const int cen = (ea.info >> 20) & 31, at = (ea.info >> 2) & 31;
+                    part_at(0, cen, at) += fax;
+                    part_at(1, cen, at) += fay;
+                    part_at(2, cen, at) += faz;
+                }
+            }
+            __syncwarp();
+        }
+        cp_async_wait<0>();   // row slots of a short round are empty groups; nothing may stay pending
+    }
+    __syncthreads();
+    // gradient of atom j = what the central atoms handed to j (column j) - what j handed out (row j)
+    for (int plane = warp; plane < 3; plane += NW) {
+        if (lane < n) {
+            T col = (T)0, rw = (T)0;
+            for (int c = 0; c < n; c++) col += part_at(plane, c, lane);
+            for (int j = 0; j < n; j++) rw += part_at(plane, lane, j);
+            T* dst = plane == 0 ? gx : (plane == 1 ? gy : gz);
+            dst[base + ws.sort.src[lane]] = col - rw;
+        }
     }
 }
 

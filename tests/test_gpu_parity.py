@@ -299,6 +299,21 @@ def test_gradient_vs_oracle(gpu, oracle_mod, case, dt):
         assert normwise(out[k], ref[k]) < FTOL[dt], (case, k)
 
 
+@pytest.mark.parametrize("n_mols", [140, 310, 600, 1100])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_small_molecules_at_every_split(gpu, oracle_mod, n_mols, dt):
+    """Central atoms per warp (features), warps per molecule and size classes (gradient) depend on the batch size."""
+    b = _concat(syn.gdb_like_batch(n_mols, 21), CASES["large_among_small"](), CASES["dense_small"]())
+    si, gi, ac = oracle_mod.ani_sort(b.atomic_numbers)
+    up = syn.upstream_grads(b, ac, dtype=dt)
+    args = [v.astype(np.float64) for v in b.coords(dt)] + [b.atomic_numbers, b.mol_offsets, b.mol_atom_counts, si, ac]
+    for out, ref in zip(gpu.gpu_featurize(b, dt), oracle_mod.featurize(*args, impl="port", threads=8)):
+        assert normwise(out, ref) < FTOL[dt]
+    ref = oracle_mod.featurize_grad(*args, *[u.astype(np.float64) for u in up], impl="port", threads=8)
+    for k, out in enumerate(gpu.gpu_featurize_grad(b, dt, up)):
+        assert normwise(out, ref[k]) < FTOL[dt]
+
+
 def test_float32_gradient_vs_the_float32_reference_where_it_is_finite(gpu, oracle_mod, ref_impl):
     """The reference's own float32 gradient divides by sin(theta) and by 1 + cos(theta_t - theta) without a
     guard (gpu_featurizer/kernel_cpu.cpp:335-353) and is non-finite for part of realistic inputs, so the
