@@ -20,6 +20,7 @@
 #include "ani_featurize_large.cuh"
 #include "ani_grad.cuh"
 #include "ani_grad_mol.cuh"
+#include "ani_grad_large.cuh"
 #include "ani_grad_inverse.cuh"
 #include "ani_tangent_mol.cuh"
 #include "ani_mlp_forward.cuh"
@@ -190,14 +191,11 @@ template <typename K> int set_smem(K kernel, size_t bytes)
     return ANI_OK;
 }
 
-// Batches whose MEAN molecule size is at most this take the one-CTA-per-molecule kernels (their
-// fast path covers molecules of up to kMolMaxAtoms atoms; a larger molecule in such a batch is
-// still handled, slowly).  Batches of larger molecules take featurize_large_kernel (rounds of four
-// central atoms per warp, the molecule scanned from global memory) for the forward pass and the
-// one-warp-per-atom kernel for the gradient; the one-warp-per-atom forward kernel remains for outputs
-// that are not 16-byte aligned.  (A gradient kernel built like the large forward one was measured on
-// 256 molecules of 64-256 atoms: 26 % fewer instructions and 104 instead of 139 us alone, but 99
-// instead of 90 us per launch with four batches in flight, so it is not used.)
+// Batches whose MEAN molecule size is at most this take the kernels for small molecules (their fast path covers
+// molecules of up to kMolMaxAtoms atoms; a larger molecule in such a batch is still handled, slowly).  Batches of
+// larger molecules take featurize_large_kernel and featurize_grad_large_kernel (a few central atoms per warp, the
+// molecule scanned from global memory); the one-warp-per-atom forward kernel remains for outputs that are not 16-byte
+// aligned.
 constexpr int kMolMeanLimit = 24;
 constexpr int kSms = 148;
 bool small_molecules(long long n_atoms, int n_mols) { return n_mols > 0 && n_atoms <= (long long)n_mols * kMolMeanLimit; }
@@ -257,17 +255,17 @@ int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, cons
         return ANI_OK;
     }
 
-    // larger molecules: the same rounds of four central atoms, the molecule scanned from global memory;
+    // larger molecules: the same rounds of one to four central atoms, the molecule scanned from global memory;
     // a CTA takes every rounds_in_grid-th round of its molecule
     if (n_mols > 0 && all_aligned16({oh, oc, on, oo})) {
-        const long long mean_rounds = (n_atoms / n_mols + kMolCentrals) / kMolCentrals;
-        const int rounds_in_grid = (int)std::min<long long>(std::max<long long>(mean_rounds, kMolRounds), 64);
-        if ((long long)n_mols * rounds_in_grid <= 0x7fffffffLL) {
-            ANI_CUDA(launch_chain(featurize_large_kernel<T>, n_mols * rounds_in_grid, kWarp, 0, (cudaStream_t)stream, 1,
-                                  xs, ys, zs, types, mos, macs, n_mols, (int)n_atoms, rounds_in_grid, sis, oh, oc, on, oo,
-                                  acs_host[0], acs_host[1], acs_host[2], acs_host[3]));
-            return ANI_OK;
-        }
+        const int resident = kSms * (sizeof(T) == 4 ? 22 : 14);
+        const int per_round = (int)std::min<long long>((n_atoms + resident - 1) / resident, kMolCentrals);
+        const long long mean_rounds = (n_atoms / n_mols + per_round) / per_round;
+        const long long rounds = std::min(std::min<long long>(mean_rounds, 256), 0x7fffffffLL / n_mols);
+        ANI_CUDA(launch_chain(featurize_large_kernel<T>, (int)(n_mols * rounds), kWarp, 0, (cudaStream_t)stream, 1, xs, ys, zs,
+                              types, mos, macs, n_mols, (int)n_atoms, per_round, sis, oh, oc, on, oo, acs_host[0],
+                              acs_host[1], acs_host[2], acs_host[3]));
+        return ANI_OK;
     }
 
     auto kernel = featurize_kernel<T, kNW, CAPT, CAPR>;
@@ -349,8 +347,9 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
     for (int t = 0; t < kTypes; t++)
         if (acs_host[t] > 0 && !gin[t]) return ANI_ERR_NULL_POINTER;
 
-    auto kernel = featurize_grad_kernel<T, kNW>;
-    const size_t smem = kNW * sizeof(GradWarpShared<T>);
+    // one to three central atoms per warp, as in the features: few while all warps are resident anyway
+    const auto kernel = featurize_grad_large_kernel<T>;
+    const size_t smem = sizeof(LargeGradWarpShared<T>);
     static thread_local int configured_dev = -1;
     int dev = 0;
     ANI_CUDA(cudaGetDevice(&dev));
@@ -358,16 +357,13 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
         if (int rc = set_smem(kernel, smem)) return rc;
         configured_dev = dev;
     }
-    static thread_local int cached_grid_dev = -1, cached_resident = 0;
-    if (cached_grid_dev != dev) {
-        if (int rc = featurizer_grid(kernel, smem, 1 << 24, &cached_resident)) return rc;
-        cached_grid_dev = dev;
-    }
-    const int slot_shift = pick_slot_shift(n_atoms, n_mols);
-    const long long needed = (long long)n_mols * ((1 << (slot_shift & 31)) / kNW);
-    const int grid = (int)(needed < cached_resident ? needed : cached_resident);
-    ANI_CUDA(launch_chain(kernel, grid, kNW * kWarp, smem, st, 1, xs, ys, zs, types, mos, macs, n_mols, (int)n_atoms,
-                          slot_shift, sis, gh, gc, gn, go, gx, gy, gz, acs_host[0], acs_host[1], acs_host[2], acs_host[3]));
+    const int resident = kSms * (sizeof(T) == 4 ? 20 : 12);
+    const int per_round = (int)std::min<long long>((n_atoms + resident - 1) / resident, kLargeGradCentrals);
+    const long long mean_rounds = (n_atoms / n_mols + per_round) / per_round;
+    const long long rounds = std::min(std::min<long long>(mean_rounds, 256), 0x7fffffffLL / n_mols);
+    ANI_CUDA(launch_chain(kernel, (int)(n_mols * rounds), kWarp, smem, st, 1, xs, ys, zs, types, mos, macs, n_mols,
+                          (int)n_atoms, per_round, all_aligned16({gh, gc, gn, go}), sis, gh, gc, gn, go, gx, gy, gz,
+                          acs_host[0], acs_host[1], acs_host[2], acs_host[3]));
     return ANI_OK;
 }
 

@@ -7,10 +7,11 @@
 // shift)) are the very same code, ani_featurize_round_passes.inl -- but the molecule does not fit the lanes,
 // so the scan differs:
 //   A. the molecule is read from global memory 32 candidates at a time, once per round; every lane
-//      tests its candidate against the (up to) four central atoms, whose coordinates all lanes hold.
-//      Radial neighbours go to the central atom's radial list in arrival order with their element,
+//      tests its candidate against the (up to) four central atoms, whose coordinates all lanes hold, by squared
+//      distance.  Radial neighbours go to the central atom's radial list in arrival order with their element,
 //      angular neighbours to its angular list (32 at most);
-//   S. each angular list is put into element order by one ballot sort (lane = entry), which is what
+//   L. lengths and cutoffs of the radial lists, lane = entry (in the scan 3 of 32 lanes had work for them);
+//   S. each angular list gets its lengths and cutoffs and is put into element order by one ballot sort (lane = entry), which is what
 //      pass T needs; the per-element counts fall out of the same ballots;
 //   R. radial features of the whole round, lane = (central atom, pair of shifts): every lane walks
 //      the radial list of its central atom and adds to the sum of the neighbour's element.
@@ -18,6 +19,9 @@
 // than 32 angular neighbours goes through the streaming routine of ani_featurize.cuh.  A CTA takes the rounds r, r + R0, r + 2 R0, ... of its molecule
 // (R0 rounds per molecule in the grid, chosen by the host from the mean molecule size), so molecules
 // of any size are covered.  Nothing is accumulated with atomics; rows need no zero fill by the caller.
+//
+// 256 molecules of 64 to 256 atoms: 95 us (float, as before), double 341 -> 256 (lengths and cutoffs off the scan);
+// 8 molecules 41 -> 21 us with one central atom per warp instead of four.
 //
 // Computes what featurize_cpu of the reference computes (gpu_featurizer/kernel_cpu.cpp:406-537).
 #pragma once
@@ -33,17 +37,18 @@ constexpr int kLargeCapR = 64;   // radial neighbours kept per central atom
 constexpr int kLargeCapA = 32;   // angular neighbours kept per central atom (one ballot sort covers 32 entries)
 
 template <typename T> struct LargeFwdWarpShared {
-    MolAngularShared<T, kMolCentrals * kLargeCapA, kLargeCapA, kLargeCapR> ang;   // its radial lists are in arrival order
+    MolAngularShared<T, kMolCentrals * kLargeCapA, kLargeCapA> ang;
+    Vec2<T> rad[kMolCentrals][kLargeCapR];           // squared distance; from step L on (r, f_C(r, R_Rc))
     unsigned char rad_t[kMolCentrals][kLargeCapR];   // element of that neighbour
     unsigned char ang_t[kMolCentrals * kLargeCapA];    // element of each angular neighbour before the sort
     int cnt_r[kMolCentrals];
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
+__global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 22 : 1)
     featurize_large_kernel(const T* __restrict__ xs, const T* __restrict__ ys, const T* __restrict__ zs,
                            const int* __restrict__ types, const int* __restrict__ mol_offsets,
-                           const int* __restrict__ mol_counts, int n_mols, int n_atoms, int rounds_in_grid,
+                           const int* __restrict__ mol_counts, int n_mols, int n_atoms, int per_round,
                            const int* __restrict__ scatter, T* out_h, T* out_c, T* out_n, T* out_o,
                            int acs0, int acs1, int acs2, int acs3)
 {
@@ -59,7 +64,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
     MolRange mol;
     if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) return;
     const int n = mol.n, base = mol.base;
-    const int n_rounds = (n + kMolCentrals - 1) / kMolCentrals;
+    const int n_rounds = (n + per_round - 1) / per_round, rounds_in_grid = gridDim.x / n_mols;
 
     for (int round = round0; round < n_rounds; round += rounds_in_grid) {
         // round r takes the central atoms r, r + R, r + 2 R, r + 3 R (R = rounds of the molecule)
@@ -130,17 +135,16 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
             for (int g = 0; g < kMolCentrals; g++) {
                 if ((skip >> g) & 1u) continue;   // warp-uniform
                 const T dx = xi[g] - px, dy = yi[g] - py, dz = zi[g] - pz;
-                T r, inv;
-                length_and_inverse(dx * dx + dy * dy + dz * dz, &r, &inv);
-                const bool in_rad = live && j != ci[g] && r < (T)kR_Rc;
-                const bool in_ang = in_rad && r < (T)kA_Rc;
+                const T d2 = dx * dx + dy * dy + dz * dz;
+                const bool in_rad = live && j != ci[g] && d2 < (T)(kR_Rc * kR_Rc);
+                const bool in_ang = in_rad && d2 < (T)(kA_Rc * kA_Rc);
                 const unsigned mR = __ballot_sync(kFull, in_rad);
                 if (mR == 0) continue;
                 const unsigned mA = __ballot_sync(kFull, in_ang);
                 if (in_rad) {
                     const int pos = cR[g] + __popc(mR & lanemask_lt());
                     if (pos < kLargeCapR) {
-                        ws.ang.rad[g][pos] = Vec2<T>{r, cutoff_value<T>(r, (T)kR_Rc)};
+                        ws.rad[g][pos].x = d2;
                         ws.rad_t[g][pos] = (unsigned char)tj;
                     }
                 }
@@ -148,8 +152,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
                     const int pos = cA[g] + __popc(mA & lanemask_lt());
                     if (pos < kLargeCapA) {
                         const int p = g * kLargeCapA + pos;
-                        ws.ang.ang_u[p] = Vec4<T>{dx * inv, dy * inv, dz * inv, r};
-                        ws.ang.ang_fc[p] = cutoff_value<T>(r, (T)kA_Rc);
+                        ws.ang.ang_u[p] = Vec4<T>{dx, dy, dz, d2};
                         ws.ang_t[p] = (unsigned char)tj;
                     }
                 }
@@ -174,6 +177,16 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
             if (lane == 0 && !((skip >> g) & 1u)) ws.cnt_r[g] = cR[g];
         __syncwarp();
 
+        // ---- L: lengths and cutoffs, lane = list entry ----
+#pragma unroll
+        for (int g = 0; g < kMolCentrals; g++)
+            for (int p = lane; p < ws.cnt_r[g]; p += kWarp) {
+                T r, inv;
+                length_and_inverse(ws.rad[g][p].x, &r, &inv);
+                ws.rad[g][p] = Vec2<T>{r, cutoff_value<T>(r, (T)kR_Rc)};
+            }
+        __syncwarp();
+
         // ---- R: radial features of the round, lane = (central atom, pair of shifts) ----
         {
             const int g = lane >> 3, sp = lane & 7;
@@ -183,7 +196,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
 #pragma unroll
             for (int t = 0; t < kTypes; t++) acc[t] = Pair<T>{(T)0, (T)0};
             for (int p = 0; p < cnt; p++) {
-                const Vec2<T> e = ws.ang.rad[g][p];
+                const Vec2<T> e = ws.rad[g][p];
                 const int t = ws.rad_t[g][p];
                 const Pair<T> d{e.x - sh0, e.x - sh1};
                 const Pair<T> d2 = pmul(d, d);
@@ -222,8 +235,9 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
             }
             const bool have = lane < cA[g];
             const int p = g * kLargeCapA + (have ? lane : 0);
-            const Vec4<T> u = ws.ang.ang_u[p];
-            const T fc = ws.ang.ang_fc[p];
+            const Vec4<T> v = ws.ang.ang_u[p];
+            T r, inv;
+            length_and_inverse(v.w, &r, &inv);
             const int t = have ? ws.ang_t[p] : kTypes;
             const unsigned m0 = __ballot_sync(kFull, t == 0), m1 = __ballot_sync(kFull, t == 1),
                            m2 = __ballot_sync(kFull, t == 2), m3 = __ballot_sync(kFull, t == 3);
@@ -233,8 +247,8 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 1)
             __syncwarp();   // every entry has been read
             if (have) {
                 const int q = g * kLargeCapA + start + __popc(mine & lanemask_lt());
-                ws.ang.ang_u[q] = u;
-                ws.ang.ang_fc[q] = fc;
+                ws.ang.ang_u[q] = Vec4<T>{v.x * inv, v.y * inv, v.z * inv, r};
+                ws.ang.ang_fc[q] = cutoff_value<T>(r, (T)kA_Rc);
             }
             if (lane == 0)
                 *reinterpret_cast<int4*>(&ws.ang.cnt_a[g * kTypes]) = make_int4(c0, c1, c2, __popc(m3));

@@ -84,10 +84,9 @@ struct MolSortShared {
 // What the angular passes (T, B, C) of a round work on: the angular neighbour lists of the round's
 // central atoms (element order inside each list), the group table, the factor chunks and the rows.
 // POOL = entries of the lists together, MAXA = longest list (list indices are packed into 8 bits).
-template <typename T, int POOL, int MAXA, int CAPR> struct MolAngularShared {
+template <typename T, int POOL, int MAXA> struct MolAngularShared {
     Vec4<T> ang_u[POOL];                  // (x_i - x_j) / r_ij and r_ij, element order, per central atom
     T ang_fc[POOL];                       // f_C(r_ij, A_Rc)
-    Vec2<T> rad[kMolCentrals][CAPR];      // (r_ij, f_C(r_ij, R_Rc)) per central atom: the radial pass reads it, not T / B / C
     alignas(16) T A[kNumThetas][kMolChunkStride];
     alignas(16) T BF[kNumARs][kMolChunkStride];
     MolGroupInfo tab[kMolCentrals * kMolGroupStride];
@@ -98,7 +97,8 @@ template <typename T, int POOL, int MAXA, int CAPR> struct MolAngularShared {
 };
 
 template <typename T> struct MolFwdWarpShared {
-    MolAngularShared<T, kMolPool, kMolMaxAtoms - 1, kMolMaxAtoms> ang;   // its radial table: every atom j of the molecule, f_C = 0 out of range
+    MolAngularShared<T, kMolPool, kMolMaxAtoms - 1> ang;
+    Vec2<T> rad[kMolCentrals][kMolMaxAtoms];   // (r_ij, f_C(r_ij, R_Rc)) of every atom j of the molecule, f_C = 0 out of range
     MolSortShared sort;
 };
 
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
             for (int i = 0; i < (kGranules + kWarp - 1) / kWarp; i++)
                 if (i * kWarp + lane < kGranules) zero[i * kWarp + lane] = Granule{0.f, 0.f, 0.f, 0.f};
         }
-        ws.ang.rad[g][lane] = Vec2<T>{r, in_rad ? cutoff_value<T>(r, (T)kR_Rc) : (T)0};
+        ws.rad[g][lane] = Vec2<T>{r, in_rad ? cutoff_value<T>(r, (T)kR_Rc) : (T)0};
         if (in_ang) {
             const int p = used + __popc(mA & lanemask_lt());
             ws.ang.ang_u[p] = Vec4<T>{dx * inv, dy * inv, dz * inv, r};
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     // ---- R: radial features of the whole round, lane = (central atom, pair of shifts) ----
     {
         const int g = lane >> 3, sp = lane & 7;
-        const Vec2<T>* list = ws.ang.rad[g];
+        const Vec2<T>* list = ws.rad[g];
         const T sh0 = (T)c_tab.R_Rs[2 * sp], sh1 = (T)c_tab.R_Rs[2 * sp + 1];
         const uint4 tmq = *reinterpret_cast<const uint4*>(ws.sort.tmask);
         const int run_end[kTypes] = {__popc(tmq.x), __popc(tmq.x | tmq.y), __popc(tmq.x | tmq.y | tmq.z), n};

@@ -17,7 +17,7 @@
 
 namespace ani {
 
-template <typename T> struct TangentRound : MolAngularShared<T, kMolPool, kMolMaxAtoms - 1, 1> {
+template <typename T> struct TangentRound : MolAngularShared<T, kMolPool, kMolMaxAtoms - 1> {
     Vec4<T> du[kMolPool];                          // d (unit vector) and d r along v
     T fc_dot[kMolPool];                            // d f_C(r, A_Rc)
     alignas(16) T dA[kNumThetas][kMolChunkStride];

@@ -314,6 +314,21 @@ def test_small_molecules_at_every_split(gpu, oracle_mod, n_mols, dt):
         assert normwise(out, ref[k]) < FTOL[dt]
 
 
+@pytest.mark.parametrize("n_mols", [1, 30, 75])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_large_molecules_at_every_split(gpu, oracle_mod, n_mols, dt):
+    """One to four central atoms per warp, with neighbourhoods beyond the pool and the lists among them."""
+    b = _concat(syn.config4(seed=n_mols, n_mols=n_mols), _dense_blobs(1, 40, 2.3, 11), _dense_blobs(1, 110, 2.4, 12))
+    si, gi, ac = oracle_mod.ani_sort(b.atomic_numbers)
+    up = syn.upstream_grads(b, ac, dtype=dt)
+    args = [v.astype(np.float64) for v in b.coords(dt)] + [b.atomic_numbers, b.mol_offsets, b.mol_atom_counts, si, ac]
+    for out, ref in zip(gpu.gpu_featurize(b, dt), oracle_mod.featurize(*args, impl="port", threads=8)):
+        assert normwise(out, ref) < FTOL[dt]
+    ref = oracle_mod.featurize_grad(*args, *[u.astype(np.float64) for u in up], impl="port", threads=8)
+    for k, out in enumerate(gpu.gpu_featurize_grad(b, dt, up)):
+        assert normwise(out, ref[k]) < FTOL[dt]
+
+
 def test_float32_gradient_vs_the_float32_reference_where_it_is_finite(gpu, oracle_mod, ref_impl):
     """The reference's own float32 gradient divides by sin(theta) and by 1 + cos(theta_t - theta) without a
     guard (gpu_featurizer/kernel_cpu.cpp:335-353) and is non-finite for part of realistic inputs, so the
