@@ -306,7 +306,7 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
     // One CTA per molecule when the molecules are small and the upstream rows can be fetched with
     // 16-byte copies: writes every output itself, so no zero fill.
     if (n_mols > 0 && small_molecules(n_atoms, n_mols) && all_aligned16({gh, gc, gn, go}) &&
-        (long long)n_mols * 3 <= 0x7fffffffLL) {
+        (long long)n_mols * 2 <= 0x7fffffffLL) {
         if (!xs || !ys || !zs || !types || !mos || !macs || !sis) return ANI_ERR_NULL_POINTER;
         for (int t = 0; t < kTypes; t++)
             if (acs_host[t] > 0 && !gin[t]) return ANI_ERR_NULL_POINTER;
@@ -320,14 +320,15 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
                 if (int rc = set_smem(featurize_grad_mol_kernel<T, NW>, smem)) return rc;
                 configured_dev = dev;
             }
-            // More molecules than are resident at once: by size class, largest first (classes relative to the mean, of
-            // which the data sets' largest molecules are twice).  Alone, 1024 molecules of up to 8 heavy atoms: float
-            // 35.6 -> 32.2 us, double 101 -> 78; 2048: 52.8 -> 47.3, 155 -> 139; without effect at 8192.
+            // More molecules than are resident at once: those well above the mean start first.  Alone, 1024 molecules
+            // of up to 8 heavy atoms: float 35.2 -> 33.1 us, double 98 -> 79; 2048: 52.3 -> 46.4, 151 -> 137; 4096: 94
+            // -> 82.  (In three classes 31.8 at 1024 and the same from there on, but with eight streams in flight the
+            // CTAs without work then cost 6 % of the throughput, in two classes 3 %.)
             const bool classes = (long long)n_mols * NW > (long long)kSms * (sizeof(T) == 4 ? 20 : 12);
-            const int mean8 = (int)(8 * n_atoms / n_mols);
-            ANI_CUDA(launch_chain(featurize_grad_mol_kernel<T, NW>, classes ? 3 * n_mols : n_mols, NW * kWarp, smem, st, 1, xs,
+            const int big_size = (int)(n_atoms * 19 / (16LL * n_mols));
+            ANI_CUDA(launch_chain(featurize_grad_mol_kernel<T, NW>, classes ? 2 * n_mols : n_mols, NW * kWarp, smem, st, 1, xs,
                                   ys, zs, types, mos, macs, n_mols, (int)n_atoms, sis, gh, gc, gn, go, gx, gy, gz,
-                                  acs_host[0], acs_host[1], acs_host[2], acs_host[3], mean8 * 7 / 64, mean8 * 12 / 64));
+                                  acs_host[0], acs_host[1], acs_host[2], acs_host[3], big_size));
             return ANI_OK;
         };
         // Eight warps a molecule shorten its chain of scans and pair passes (64 molecules 14.8 -> 10.6 us, 512: 27.4 ->

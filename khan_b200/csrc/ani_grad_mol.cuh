@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
                               const int* __restrict__ mol_counts, int n_mols, int n_atoms,
                               const int* __restrict__ scatter, const T* __restrict__ gh,
                               const T* __restrict__ gc, const T* __restrict__ gn, const T* __restrict__ go,
-                              T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3, int mid_size, int big_size)
+                              T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3, int big_size)
 {
     constexpr int GR = MolGradCfg<T>::kRowBufs;   // central atoms per round
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -139,16 +139,15 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
         return part[(plane * kMolMaxAtoms + c) * kMolGradPitch + j];
     };
 
-    // With three CTAs per molecule in the grid, class-major: first one CTA for every molecule, of which only those of
-    // molecules above big_size work (the others leave after one load), then the same for those above mid_size, then for
-    // the rest; CTAs start in index order, so the expensive molecules start first and the cheap ones fill the SMs
-    // behind them.
+    // With two CTAs per molecule in the grid, class-major: first one CTA for every molecule, of which only those of
+    // molecules above big_size work (the others leave after one load), then the same for the rest; CTAs start in index
+    // order, so the expensive molecules start first and the cheap ones fill the SMs behind them.
     const bool classes = (int)gridDim.x > n_mols;
     const int cls = blockIdx.x / n_mols, m = blockIdx.x - cls * n_mols;
     MolRange mol;
     if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) return;
     const int n = mol.n, base = mol.base;
-    if (classes && cls != (n > big_size ? 0 : (n > mid_size ? 1 : 2))) return;
+    if (classes && cls != (n > big_size ? 0 : 1)) return;
 
     if (n > kMolMaxAtoms) {   // a large molecule in a batch of small ones
         for (int j = threadIdx.x; j < n; j += NW * kWarp) {
