@@ -140,14 +140,15 @@ class FusedTrainStep:
         _lib.check(lib.ani_mlp_backward_f32(ctypes.byref(bwd), sb._acs_ptr, int(self.split), stream),
                    "ani_mlp_backward_f32")
 
-    def weight_gradients(self, sb: StagedBatch) -> None:
-        """Zeroes the flat gradient buffer and adds the weight gradients of this batch to it."""
+    def weight_gradients(self, sb: StagedBatch, zeroed: bool = False) -> None:
+        """Zeroes the flat gradient buffer (unless ``zeroed``) and adds the weight gradients of this batch to it."""
         stream = self._stream()
         if self._args_key is not None and self._args_key[0] == id(sb) and self._args_key[1:5] == tuple(int(c) for c in sb.acs_host):
             wg = self._args[2]          # the blocks networks() built for this batch
         else:
             wg = self._network_args(sb, True)[2]
-        self.optimizer.flat_grads.zero_()
+        if not zeroed:
+            self.optimizer.flat_grads.zero_()
         _lib.check(_lib.lib().ani_mlp_weight_grad_f32(ctypes.byref(wg), sb._acs_ptr, int(self.split), stream),
                    "ani_mlp_weight_grad_f32")
 
@@ -321,6 +322,8 @@ class StepPipeline:
         cur = torch.cuda.current_stream(step.device)
         self.feature_stream.wait_stream(cur)
         with torch.cuda.stream(self.feature_stream):
+            # cleared here, beside the networks: between them and the weight gradients it was 4 us of 146
+            step.optimizer.flat_grads.zero_()
             step.featurize(self.staged[(b + 1) % self.nb])
         step.networks(self.staged[b], self.labels[b])
         # the featurizer joins here: letting it run on into the gradient kernels was measured slower
@@ -328,7 +331,7 @@ class StepPipeline:
         self.gradient_stream.wait_stream(cur)
         with torch.cuda.stream(self.gradient_stream):
             step.coordinate_gradient(self.staged[b])
-        step.weight_gradients(self.staged[b])
+        step.weight_gradients(self.staged[b], zeroed=True)
         if update:       # single GPU, or the mean over the ranks as a kernel of this library
             if self.peer is not None:
                 self.peer.mean_(step.optimizer.flat_grads)
