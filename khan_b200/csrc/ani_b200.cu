@@ -290,11 +290,17 @@ int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, cons
     return ANI_OK;
 }
 
+// The coordinate gradients of such a batch are computed a molecule per CTA (and molecule energies with them).
+bool grad_per_molecule(long long n_atoms, int n_mols, std::initializer_list<const void*> rows)
+{
+    return n_mols > 0 && small_molecules(n_atoms, n_mols) && all_aligned16(rows) && (long long)n_mols * 2 <= 0x7fffffffLL;
+}
+
 template <typename T>
 int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types, const int* mos,
                         const int* macs, int n_mols, const int* sis, const T* gh, const T* gc,
                         const T* gn, const T* go, T* gx, T* gy, T* gz, const int* acs_host,
-                        void* stream)
+                        void* stream, const MolEnergySums<T>& sums = MolEnergySums<T>{})
 {
     long long n_atoms = 0;
     if (int rc = check_acs(acs_host, &n_atoms)) return rc;
@@ -305,8 +311,7 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
     const T* gin[kTypes] = {gh, gc, gn, go};
     // One CTA per molecule when the molecules are small and the upstream rows can be fetched with
     // 16-byte copies: writes every output itself, so no zero fill.
-    if (n_mols > 0 && small_molecules(n_atoms, n_mols) && all_aligned16({gh, gc, gn, go}) &&
-        (long long)n_mols * 2 <= 0x7fffffffLL) {
+    if (grad_per_molecule(n_atoms, n_mols, {gh, gc, gn, go})) {
         if (!xs || !ys || !zs || !types || !mos || !macs || !sis) return ANI_ERR_NULL_POINTER;
         for (int t = 0; t < kTypes; t++)
             if (acs_host[t] > 0 && !gin[t]) return ANI_ERR_NULL_POINTER;
@@ -328,7 +333,7 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
             const int big_size = (int)(n_atoms * 19 / (16LL * n_mols));
             ANI_CUDA(launch_chain(featurize_grad_mol_kernel<T, NW>, classes ? 2 * n_mols : n_mols, NW * kWarp, smem, st, 1, xs,
                                   ys, zs, types, mos, macs, n_mols, (int)n_atoms, sis, gh, gc, gn, go, gx, gy, gz,
-                                  acs_host[0], acs_host[1], acs_host[2], acs_host[3], big_size));
+                                  acs_host[0], acs_host[1], acs_host[2], acs_host[3], big_size, sums));
             return ANI_OK;
         };
         // Eight warps a molecule shorten its chain of scans and pair passes (64 molecules 14.8 -> 10.6 us, 512: 27.4 ->
@@ -1428,7 +1433,10 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
         }
         if (int rc = ani_mlp_forward_f32(&f, acs, a->activation, a->split_precision, stream)) return rc;
     }
-    if (a->phases & ANI_PASS_ENERGY) {
+    const bool sums_with_grads = (a->phases & ANI_PASS_ENERGY) && (a->phases & ANI_PASS_COORD_GRAD) && !a->labels &&
+                                 grad_per_molecule(n_atoms, a->n_mols, {a->feature_grads}) && n_atoms > 0;
+    if (sums_with_grads && (!a->energy_sorted || !a->gather_idxs || !a->mol_energy)) return ANI_ERR_NULL_POINTER;
+    if ((a->phases & ANI_PASS_ENERGY) && !sums_with_grads) {
         if (int rc = ani_molecule_energy_f32(a->energy_sorted, a->gather_idxs, a->mol_offsets, a->mol_atom_counts,
                                              a->n_mols, a->n_atoms, a->labels, a->grad_scale, a->mol_energy,
                                              a->labels ? a->l2s : nullptr,
@@ -1463,11 +1471,13 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
         if (int rc = ani_mlp_weight_grad_f32(&w, acs, a->split_precision, stream)) return rc;
     }
     if (a->phases & ANI_PASS_COORD_GRAD) {
-        if (int rc = ani_featurize_grad_f32(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
-                                            a->n_mols, a->scatter_idxs, rows(a->feature_grads, 0, kTotal),
-                                            rows(a->feature_grads, 1, kTotal), rows(a->feature_grads, 2, kTotal),
-                                            rows(a->feature_grads, 3, kTotal), a->x_grads, a->y_grads, a->z_grads,
-                                            acs, stream))
+        MolEnergySums<float> sums = {};
+        if (sums_with_grads) sums = {a->energy_sorted, a->gather_idxs, a->mol_energy};
+        if (int rc = featurize_grad_impl<float>(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
+                                                a->n_mols, a->scatter_idxs, rows(a->feature_grads, 0, kTotal),
+                                                rows(a->feature_grads, 1, kTotal), rows(a->feature_grads, 2, kTotal),
+                                                rows(a->feature_grads, 3, kTotal), a->x_grads, a->y_grads, a->z_grads,
+                                                acs, stream, sums))
             return rc;
     }
     return ANI_OK;
@@ -1504,7 +1514,10 @@ int ani_energy_pass_f64(const ani_energy_args_f64* a, void* stream)
                                               (cudaStream_t)stream))
             return rc;
     }
-    if ((a->phases & ANI_PASS_ENERGY) && a->n_mols > 0) {
+    const bool sums_with_grads = (a->phases & ANI_PASS_ENERGY) && (a->phases & ANI_PASS_COORD_GRAD) && n_atoms > 0 &&
+                                 grad_per_molecule(n_atoms, a->n_mols, {a->feature_grads});
+    if (sums_with_grads && (!a->energy_sorted || !a->gather_idxs || !a->mol_energy)) return ANI_ERR_NULL_POINTER;
+    if ((a->phases & ANI_PASS_ENERGY) && a->n_mols > 0 && !sums_with_grads) {
         if (!a->mol_offsets || !a->mol_atom_counts || !a->mol_energy) return ANI_ERR_NULL_POINTER;
         if (n_atoms > 0 && (!a->energy_sorted || !a->gather_idxs)) return ANI_ERR_NULL_POINTER;
         if (int rc = energy_launch<double>(a->energy_sorted, a->gather_idxs, a->mol_offsets, a->mol_atom_counts, a->n_mols,
@@ -1512,9 +1525,11 @@ int ani_energy_pass_f64(const ani_energy_args_f64* a, void* stream)
             return rc;
     }
     if (a->phases & ANI_PASS_COORD_GRAD) {
-        if (int rc = ani_featurize_grad_f64(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
-                                            a->n_mols, a->scatter_idxs, grad_rows[0], grad_rows[1], grad_rows[2],
-                                            grad_rows[3], a->x_grads, a->y_grads, a->z_grads, acs, stream))
+        MolEnergySums<double> sums = {};
+        if (sums_with_grads) sums = {a->energy_sorted, a->gather_idxs, a->mol_energy};
+        if (int rc = featurize_grad_impl<double>(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
+                                                 a->n_mols, a->scatter_idxs, grad_rows[0], grad_rows[1], grad_rows[2],
+                                                 grad_rows[3], a->x_grads, a->y_grads, a->z_grads, acs, stream, sums))
             return rc;
     }
     return ANI_OK;

@@ -118,6 +118,14 @@ __device__ __noinline__ void grad_atom_streaming_radial(const T* __restrict__ xs
     }
 }
 
+// Molecule energies on the side: a pass that wants energies and forces has one launch less (2 to 3 us), and the warp
+// that takes none of the three output planes at the end has nothing else to do.  mol_energy == nullptr: none.
+template <typename T> struct MolEnergySums {
+    const T* atom_energy_sorted;
+    const int* gather;
+    T* mol_energy;
+};
+
 template <typename T, int NW>
 __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
     featurize_grad_mol_kernel(const T* __restrict__ xs, const T* __restrict__ ys, const T* __restrict__ zs,
@@ -125,7 +133,7 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
                               const int* __restrict__ mol_counts, int n_mols, int n_atoms,
                               const int* __restrict__ scatter, const T* __restrict__ gh,
                               const T* __restrict__ gc, const T* __restrict__ gn, const T* __restrict__ go,
-                              T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3, int big_size)
+                              T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3, int big_size, const MolEnergySums<T> sums)
 {
     constexpr int GR = MolGradCfg<T>::kRowBufs;   // central atoms per round
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -145,11 +153,33 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
     const bool classes = (int)gridDim.x > n_mols;
     const int cls = blockIdx.x / n_mols, m = blockIdx.x - cls * n_mols;
     MolRange mol;
-    if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) return;
+    if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) {
+        if (sums.mol_energy && cls == 0 && threadIdx.x == 0) sums.mol_energy[m] = (T)0;
+        return;
+    }
     const int n = mol.n, base = mol.base;
     if (classes && cls != (n > big_size ? 0 : 1)) return;
 
+    T energy = (T)0;
+    auto load_energy = [&] {
+        if (!sums.mol_energy || warp != NW - 1) return;
+        for (int i = lane; i < n; i += kWarp) {
+            const int g = sums.gather[base + i];
+            if (g >= 0 && g < n_atoms) energy += sums.atom_energy_sorted[g];
+            else report(ANI_ERR_BAD_INDEX);
+        }
+    };
+    auto write_energy = [&] {
+        if (!sums.mol_energy || warp != NW - 1) return;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) energy += __shfl_xor_sync(kFull, energy, o);
+        if (lane == 0) sums.mol_energy[m] = energy;
+    };
+    // requested early; in double, where the registers are all in use, only at the end
+    if (sizeof(T) == 4 || n > kMolMaxAtoms) load_energy();
+
     if (n > kMolMaxAtoms) {   // a large molecule in a batch of small ones
+        write_energy();
         for (int j = threadIdx.x; j < n; j += NW * kWarp) {
             gx[base + j] = (T)0;
             gy[base + j] = (T)0;
@@ -288,6 +318,8 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
         cp_async_wait<0>();   // row slots of a short round are empty groups; nothing may stay pending
     }
     __syncthreads();
+    if (sizeof(T) == 8) load_energy();
+    write_energy();
     // gradient of atom j = what the central atoms handed to j (column j) - what j handed out (row j)
     for (int plane = warp; plane < 3; plane += NW) {
         if (lane < n) {

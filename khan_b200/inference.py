@@ -123,7 +123,7 @@ class EnergyForces:
                    | _lib.PASS_ENERGY | _lib.PASS_TRANSIENT
                    | ((_lib.PASS_BACKWARD | _lib.PASS_COORD_GRAD) if forces else 0), stream, "EnergyForces.run")
 
-    KERNELS_PER_PASS = 6   # weight packing (unless pack=False), sort, featurize, networks, molecule sums, featurize_grad
+    KERNELS_PER_PASS = 5   # small molecules: weight packing (unless pack=False), sort, featurize, networks, featurize_grad + molecule sums
 
 
 class PassTools:
