@@ -540,6 +540,19 @@ typedef struct ani_energy_args_f64 {
 } ani_energy_args_f64;
 int ani_energy_pass_f64(const ani_energy_args_f64* args, void* stream);
 
+/* One request: copy in, a pass (pass64 when given, else pass), copy out, wait for the results. */
+typedef struct ani_request_args {
+    const void* in_host;             /* pinned */
+    void* in_dev;
+    size_t in_bytes;
+    const void* out_dev;
+    void* out_host;                  /* pinned */
+    size_t out_bytes;
+    const ani_pass_args* pass;
+    const ani_energy_args_f64* pass64;
+} ani_request_args;
+int ani_request(const ani_request_args* args, void* stream);
+
 /*
  * The submitter thread of the batch feeder in native code (the reference: a Python thread that
  * pushes feed_dicts into a TensorFlow FIFOQueue, khan/training/trainer_multi_tower.py:749-828,

@@ -109,6 +109,13 @@ class EnergyArgs64(ctypes.Structure):
                 + [(n, ctypes.c_void_p * 4) for n in ("w1", "b1", "w2", "b2", "w3", "b3", "w4", "b4")])
 
 
+class RequestArgs(ctypes.Structure):
+    """``ani_request_args`` of include/ani_b200.h."""
+    _fields_ = [("in_host", ctypes.c_void_p), ("in_dev", ctypes.c_void_p), ("in_bytes", ctypes.c_size_t),
+                ("out_dev", ctypes.c_void_p), ("out_host", ctypes.c_void_p), ("out_bytes", ctypes.c_size_t),
+                ("pass_", ctypes.POINTER(PassArgs)), ("pass64", ctypes.POINTER(EnergyArgs64))]
+
+
 class DriverSlot(ctypes.Structure):
     """``ani_driver_slot`` of include/ani_b200.h."""
     _fields_ = [(n, ctypes.c_void_p) for n in ("xs", "ys", "zs", "atomic_numbers", "mol_offsets", "mol_counts", "labels")]
@@ -176,6 +183,7 @@ SIGNATURES = {
     "ani_force_fit_pass_f32": (_i, [ctypes.POINTER(ForceFitArgs), _vp]),
     "ani_bias_celu_f32": (_i, [_vp, _vp, _vp, c_int_p, _i, _vp]),
     "ani_energy_pass_f64": (_i, [ctypes.POINTER(EnergyArgs64), _vp]),
+    "ani_request": (_i, [ctypes.POINTER(RequestArgs), _vp]),
     "ani_feeder_create": (_i, [_i, _vp, _i, ctypes.POINTER(_vp)]),
     "ani_feeder_begin": (_i, [_vp, _vp, ctypes.c_longlong, _i]),
     "ani_feeder_begin_fuzz": (_i, [_vp, _vp, ctypes.c_longlong, _i, _vp, _i, ctypes.c_double]),

@@ -1535,6 +1535,17 @@ int ani_energy_pass_f64(const ani_energy_args_f64* a, void* stream)
     return ANI_OK;
 }
 
+int ani_request(const ani_request_args* a, void* stream)
+{
+    if (!a || !a->in_host || !a->in_dev || !a->out_dev || !a->out_host || (!a->pass && !a->pass64)) return ANI_ERR_NULL_POINTER;
+    const cudaStream_t st = (cudaStream_t)stream;
+    ANI_CUDA(cudaMemcpyAsync(a->in_dev, a->in_host, a->in_bytes, cudaMemcpyHostToDevice, st));
+    if (int rc = a->pass64 ? ani_energy_pass_f64(a->pass64, stream) : ani_network_pass_f32(a->pass, stream)) return rc;
+    ANI_CUDA(cudaMemcpyAsync(a->out_host, a->out_dev, a->out_bytes, cudaMemcpyDeviceToHost, st));
+    ANI_CUDA(cudaStreamSynchronize(st));
+    return ANI_OK;
+}
+
 int ani_bias_celu_f32(float* z, float* a, const float* const* bias, const int* acs_host, int width, void* stream)
 {
     long long n_atoms = 0;

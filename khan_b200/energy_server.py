@@ -45,9 +45,9 @@ def evaluate(evaluator, X) -> dict:
     else:
         rd = RawDataset([arr], [0.0])
         energy, gradient = evaluator.predict(rd)[0], list(evaluator.coordinate_gradients(rd))[0]
-    energy = float(energy) + float(sum(SELF_ENERGY[t] for t in types))
+    energy = float(energy) + float(sum(map(SELF_ENERGY.__getitem__, types.tolist())))
     gradient = np.asarray(gradient, dtype=np.float64).reshape(-1)
-    return {"energy": energy, "gradient": [float(g) * BOHR for g in gradient]}
+    return {"energy": energy, "gradient": (gradient * BOHR).tolist()}
 
 
 def handle_request(evaluator, text: str) -> str:

@@ -179,17 +179,37 @@ class SingleGeometry:
         b.grads = self.dev_out[:3 * capacity].view(3, capacity)
         self.evaluator.mol_energy = self.dev_out[3 * capacity:]
 
+        self._request = r = _lib.RequestArgs()
+        r.in_host, r.in_dev, r.in_bytes = self.host_in.data_ptr(), self.dev_in.data_ptr(), nbytes
+        r.out_host, r.out_dev = self.host_out.data_ptr(), self.dev_out.data_ptr()
+        r.out_bytes = self.dev_out.numel() * size
+        self._weights = self._block = None
+
+    def _prepare(self):
+        """The argument block of the pass, again when the weights have moved."""
+        weights = self.evaluator.model.anns[0].Ws[0].data_ptr()
+        if self._weights != weights:
+            block = self._block = self.evaluator.pass_block(self.batch)
+            block.n_mols = 1
+            block.phases = (_lib.PASS_FEATURIZE | _lib.PASS_FORWARD | _lib.PASS_ENERGY | _lib.PASS_BACKWARD
+                            | _lib.PASS_COORD_GRAD)
+            if self.evaluator.f64:
+                self._request.pass64 = ctypes.pointer(block)
+            else:
+                block.phases |= _lib.PASS_PACK | _lib.PASS_TRANSIENT
+                self._request.pass_ = ctypes.pointer(block)
+            self._weights = weights
+        return self._block
+
     def evaluate(self, arr):
         """``arr``: float64 ``(n, 4)`` array, n up to the capacity.  Returns (energy, (n, 3) gradient)."""
-        n, b = len(arr), self.batch
+        n = len(arr)
         self._xyz[:, :n] = arr[:, 1:].T
         self._types[:n] = arr[:, 0]
         self._table[1] = n
-        b.set_shape(n, 1, np.bincount(self._types[:n], minlength=4))
-        with torch.cuda.device(b.device):
-            stream = torch.cuda.current_stream()
-            self.dev_in.copy_(self.host_in, non_blocking=True)
-            self.evaluator.run(b, stream=stream.cuda_stream)
-            self.host_out.copy_(self.dev_out, non_blocking=True)
-            stream.synchronize()
+        self.batch.set_shape(n, 1, np.bincount(self._types[:n], minlength=4))
+        with torch.cuda.device(self.batch.device):
+            self._prepare().n_atoms = n
+            _lib.check(_lib.lib().ani_request(ctypes.byref(self._request), torch.cuda.current_stream().cuda_stream),
+                       "ani_request")
         return float(self._out[-1]), self._out[:-1].reshape(3, self.capacity)[:, :n].T.copy()

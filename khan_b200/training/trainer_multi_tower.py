@@ -648,11 +648,13 @@ class TrainerMultiTower:
                 # one (n_atoms, 3) array per batch, cut once into per-molecule pieces
                 yield _split_rows(np.stack(grads[k], axis=1), mos[k])
 
-    def _evaluator_usable(self, dataset) -> bool:
+    def _has_evaluator(self) -> bool:
         """One CUDA tower with the networks that have kernels: batches can go through the
         allocation-free evaluator (``khan_b200.inference.EnergyForces``)."""
-        return (self.num_towers == 1 and self.model.has_kernels and self.towers[0].type == "cuda"
-                and dataset.num_mols() > 0)
+        return self.num_towers == 1 and self.model.has_kernels and self.towers[0].type == "cuda"
+
+    def _evaluator_usable(self, dataset) -> bool:
+        return self._has_evaluator() and dataset.num_mols() > 0
 
     def _np_dtype(self):
         return np.float32 if self.precision == torch.float32 else np.float64
@@ -723,8 +725,8 @@ class TrainerMultiTower:
         ``coordinate_gradients`` give for a data set of that molecule, from one evaluation.  With the networks
         that have kernels it is one copy in, one C-ABI call and one copy out."""
         arr = np.asarray(X, dtype=np.float64)
-        rd = RawDataset([arr], [0.0])
-        if not self._evaluator_usable(rd) or not len(arr):
+        if not self._has_evaluator() or not len(arr):
+            rd = RawDataset([arr], [0.0])
             return float(self.predict(rd)[0]), np.asarray(next(iter(self.coordinate_gradients(rd))))
         with self._single_lock:
             if self._single is None or self._single.capacity < len(arr):
