@@ -715,10 +715,13 @@ class TrainerMultiTower:
         """Gradients of all molecules through the evaluator, one list per batch (cutting a batch into per-molecule
         arrays takes as long as computing it)."""
         packed = PackedDataset.from_raw(dataset, self._np_dtype())
-        slices = packed.batch_slices(batch_size)
-        return self._behind(self._driven(packed, batch_size, _lib.DRIVER_GRADIENTS, 3),
-                            lambda buf, n_atoms, n_mols, index:
-                            list(map(buf[:3 * n_atoms].reshape(n_atoms, 3).copy().__getitem__, slices[index])))
+        split, ptr = _lib.torch_ops().split_rows, packed.ptr
+
+        def finished(buf, n_atoms, n_mols, index):
+            first = index * batch_size
+            return split(buf[:3 * n_atoms].reshape(n_atoms, 3).copy(), ptr[first:first + n_mols + 1])
+
+        return self._behind(self._driven(packed, batch_size, _lib.DRIVER_GRADIENTS, 3), finished)
 
     def energy_and_gradient(self, X):
         """Energy and ``(n, 3)`` gradient of ONE geometry ``[[type, x, y, z], ...]``: what ``predict`` and
