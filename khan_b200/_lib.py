@@ -254,7 +254,7 @@ def build_ops(force: bool = False) -> str:
     with _lock:
         if not force and os.path.exists(OPS_PATH) and os.path.getmtime(OPS_PATH) >= os.path.getmtime(OPS_SOURCE):
             return OPS_PATH
-        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_torch_ops", OPS_SOURCE, "-o", OPS_PATH]
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-pthread", "-shared", "-DTORCH_EXTENSION_NAME=_torch_ops", OPS_SOURCE, "-o", OPS_PATH]
         import numpy
         cmd += ["-I" + d for d in cpp_extension.include_paths("cuda") + [sysconfig.get_paths()["include"], numpy.get_include()]]
         cmd += ["-L" + d for d in cpp_extension.library_paths("cuda")]
