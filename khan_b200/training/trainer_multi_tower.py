@@ -691,16 +691,21 @@ class TrainerMultiTower:
     def _behind(self, driven, finished):
         """``finished(host buffer, n_atoms, n_mols, index)`` of every batch once its results are in host memory, up to
         two batches behind the GPU: the host works on a batch while the GPU works on the next ones."""
-        pending, driver, tools = [], None, None
-        for k, (driver, tools) in enumerate(driven):
-            b, place = driver.batch, k % _lib.DRIVER_RING
-            pending.append((place, tools.ring[place].numpy(), b.n_atoms, b.n_mols, int(b.batch_index)))
-            if len(pending) == _lib.DRIVER_RING:       # the place of batch k + 1 must be free again
+        pending, tools = [], None
+        try:
+            for k, (driver, tools) in enumerate(driven):
+                b, place = driver.batch, k % _lib.DRIVER_RING
+                pending.append((place, tools.ring[place].numpy(), b.n_atoms, b.n_mols, int(b.batch_index)))
+                if len(pending) == _lib.DRIVER_RING:       # the place of batch k + 1 must be free again
+                    driver.wait(pending[0][0])
+                    yield finished(*pending.pop(0)[1:])
+            while pending:
                 driver.wait(pending[0][0])
                 yield finished(*pending.pop(0)[1:])
-        for entry in pending:
-            driver.wait(entry[0])
-            yield finished(*entry[1:])
+        finally:
+            if pending:        # given up in the middle: nothing may write the host buffers any more when they go
+                for stream in tools.streams:
+                    stream.synchronize()
         self._infer = tools
 
     def _evaluator_energies(self, dataset, batch_size):

@@ -463,3 +463,20 @@ def test_force_training_step_matches_the_autograd_path(act, n_mols):
     for g, w in zip(got, want):
         w = torch.zeros_like(g, dtype=torch.float64) if w is None else w
         assert float((g.double() * scale - w).abs().max()) < 1e-4 * norm
+
+
+def test_passes_over_a_data_set_may_interleave_and_be_given_up():
+    """Two passes at once, one of them abandoned after its first molecules, give what undisturbed passes give."""
+    import torch
+    from khan_b200 import RawDataset, TrainerMultiTower
+    ds = RawDataset(syn.gdb_like_batch(150, seed=5).molecules())
+    tr = TrainerMultiTower(None, [torch.device("cuda", 0)], layer_sizes=(128, 128, 64, 1), seed=3)
+    want_e, want_g = tr.predict(ds, batch_size=16), list(tr.coordinate_gradients(ds, batch_size=16))
+    first, second = tr.coordinate_gradients(ds, batch_size=16), tr.coordinate_gradients(ds, batch_size=16)
+    for k in range(20):
+        assert np.array_equal(next(first), want_g[k])
+    assert tr.predict(ds, batch_size=16) == want_e
+    del first
+    got = list(second)
+    assert len(got) == 150 and all(np.array_equal(a, b) for a, b in zip(got, want_g))
+    assert tr.predict(ds, batch_size=64) == pytest.approx(want_e, rel=1e-5, abs=1e-5)
