@@ -513,6 +513,7 @@ typedef struct ani_force_fit_args {
     const float *z1, *z2, *z3;       /* pre-activations in plain float32 ([n_atoms][128], [128], [64], element-sorted), or
                                         NULL: whose sign decides about celu's second derivative (other activations: unused) */
     void* z_ready;                   /* cudaEvent_t after which they may be read, or NULL */
+    int part;                        /* 0: everything; 1: up to the feature rates, which need no z; 2: from there on */
 } ani_force_fit_args;
 int ani_force_fit_pass_f32(const ani_force_fit_args* args, void* stream);
 /* Between two dense layers: z[rows][width] += the bias of the row's element (rows element-sorted, acs_host of

@@ -95,7 +95,8 @@ class ForceFitArgs(ctypes.Structure):
     """``ani_force_fit_args`` of include/ani_b200.h."""
     _fields_ = ([("pass_", PassArgs)]
                 + [(n, ctypes.c_void_p) for n in ("fx", "fy", "fz", "vx", "vy", "vz", "feature_rates", "r1", "r2", "adot1",
-                                                  "adot2", "adot3", "q1", "q2", "q3", "partial", "rmse", "z1", "z2", "z3", "z_ready")])
+                                                  "adot2", "adot3", "q1", "q2", "q3", "partial", "rmse", "z1", "z2", "z3", "z_ready")]
+                + [("part", ctypes.c_int)])
 
 
 class EnergyArgs64(ctypes.Structure):

@@ -1583,7 +1583,7 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
         !f->adot2 || !f->adot3 || !f->q1 || !f->q2 || !f->q3 || !f->partial || !f->rmse || !a->feature_grads || !a->features ||
         !a->act1 || !a->act2 || !a->act3 || !a->dact1 || !a->dact2 || !a->dact3 || !a->dz1 || !a->dz2 || !a->dz3)
         return ANI_ERR_NULL_POINTER;
-    if (a->activation < 0 || a->activation > 3) return ANI_ERR_BAD_SIZE;
+    if (a->activation < 0 || a->activation > 3 || f->part < 0 || f->part > 2) return ANI_ERR_BAD_SIZE;
     for (int t = 0; t < kTypes; t++)
         if (acs[t] > 0 && (!a->packed[t] || !a->w4[t] || !a->dw1[t] || !a->dw2[t] || !a->dw3[t] || !a->dw4[t] || !a->db1[t] ||
                            !a->db2[t] || !a->db3[t]))
@@ -1594,32 +1594,34 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
     const int n = (int)n_atoms;
 
     // coordinate gradients of the energy: the first-order pass, which also leaves dE/dA_l
-    ani_pass_args first = *a;
-    first.phases = (a->phases & (ANI_PASS_PACK | ANI_PASS_FEATURIZE)) | ANI_PASS_FORWARD;
-    first.labels = nullptr;
-    if (int rc = ani_network_pass_f32(&first, stream)) return rc;
-    {
-        ani_mlp_backward_args b;
-        size_t row = 0;
-        for (int t = 0; t < kTypes; t++) {
-            b.grad_energy[t] = a->grad_energy_sorted + row;
-            b.w1[t] = a->w1[t]; b.w2[t] = a->w2[t]; b.w3[t] = a->w3[t]; b.w4[t] = a->w4[t];
-            b.dact1[t] = a->dact1 + row * kMlpH1; b.dact2[t] = a->dact2 + row * kMlpH2; b.dact3[t] = a->dact3 + row * kMlpH3;
-            b.dz1[t] = a->dz1 + row * kMlpH1; b.dz2[t] = a->dz2 + row * kMlpH2; b.dz3[t] = a->dz3 + row * kMlpH3;
-            b.grad_features[t] = a->feature_grads + row * kTotal;
-            b.packed[t] = a->packed[t];
-            row += (size_t)acs[t];
+    if (f->part != 2) {
+        ani_pass_args first = *a;
+        first.phases = (a->phases & (ANI_PASS_PACK | ANI_PASS_FEATURIZE)) | ANI_PASS_FORWARD;
+        first.labels = nullptr;
+        if (int rc = ani_network_pass_f32(&first, stream)) return rc;
+        {
+            ani_mlp_backward_args b;
+            size_t row = 0;
+            for (int t = 0; t < kTypes; t++) {
+                b.grad_energy[t] = a->grad_energy_sorted + row;
+                b.w1[t] = a->w1[t]; b.w2[t] = a->w2[t]; b.w3[t] = a->w3[t]; b.w4[t] = a->w4[t];
+                b.dact1[t] = a->dact1 + row * kMlpH1; b.dact2[t] = a->dact2 + row * kMlpH2; b.dact3[t] = a->dact3 + row * kMlpH3;
+                b.dz1[t] = a->dz1 + row * kMlpH1; b.dz2[t] = a->dz2 + row * kMlpH2; b.dz3[t] = a->dz3 + row * kMlpH3;
+                b.grad_features[t] = a->feature_grads + row * kTotal;
+                b.packed[t] = a->packed[t];
+                row += (size_t)acs[t];
+            }
+            if (int rc = backward_call(&b, acs, a->split_precision, f->r1, f->r2, st)) return rc;
         }
-        if (int rc = backward_call(&b, acs, a->split_precision, f->r1, f->r2, st)) return rc;
+        first.phases = ANI_PASS_COORD_GRAD;
+        if (int rc = ani_network_pass_f32(&first, stream)) return rc;
+        // the loss, its derivative with respect to those gradients, and the rates of the features along it
+        ANI_CUDA(launch_chain(force_residual_kernel, kForceLossBlocks, kForceLossThreads, 0, st, 1, a->x_grads, a->y_grads,
+                              a->z_grads, f->fx, f->fy, f->fz, n, f->partial));
+        ANI_CUDA(launch_chain(force_loss_kernel, (n + kForceLossThreads - 1) / kForceLossThreads, kForceLossThreads, 0, st, 1,
+                              a->x_grads, a->y_grads, a->z_grads, f->fx, f->fy, f->fz, n, f->partial, f->vx, f->vy, f->vz,
+                              f->rmse));
     }
-    first.phases = ANI_PASS_COORD_GRAD;
-    if (int rc = ani_network_pass_f32(&first, stream)) return rc;
-    // the loss, its derivative with respect to those gradients, and the rates of the features along it
-    ANI_CUDA(launch_chain(force_residual_kernel, kForceLossBlocks, kForceLossThreads, 0, st, 1, a->x_grads, a->y_grads,
-                          a->z_grads, f->fx, f->fy, f->fz, n, f->partial));
-    ANI_CUDA(launch_chain(force_loss_kernel, (n + kForceLossThreads - 1) / kForceLossThreads, kForceLossThreads, 0, st, 1,
-                          a->x_grads, a->y_grads, a->z_grads, f->fx, f->fy, f->fz, n, f->partial, f->vx, f->vy, f->vz,
-                          f->rmse));
     float* rates[kTypes];
     MlpChainParams p = {};
     MlpWgradSets sets = {};
@@ -1662,10 +1664,12 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
         row += (size_t)acs[t];
     }
     p.tile_start[kTypes] = tiles;
-    if (int rc = ani_featurize_grad_inverse_f32(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
-                                                a->n_mols, a->scatter_idxs, f->vx, f->vy, f->vz, rates[0], rates[1], rates[2],
-                                                rates[3], acs, stream))
-        return rc;
+    if (f->part != 2)
+        if (int rc = ani_featurize_grad_inverse_f32(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
+                                                    a->n_mols, a->scatter_idxs, f->vx, f->vy, f->vz, rates[0], rates[1],
+                                                    rates[2], rates[3], acs, stream))
+            return rc;
+    if (f->part == 1) return ANI_OK;
     if (f->z_ready) ANI_CUDA(cudaStreamWaitEvent(st, (cudaEvent_t)f->z_ready, 0));
     if (int rc = mlp_chain_act<kChainTangent>(p, a->activation, a->split_precision != 0, st)) return rc;
     if (a->zero_ptr && a->zero_bytes) ANI_CUDA(cudaMemsetAsync(a->zero_ptr, 0, a->zero_bytes, st));

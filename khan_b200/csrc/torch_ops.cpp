@@ -220,12 +220,17 @@ class CeluPreactivations {
         cv_.notify_all();
         for (std::thread& t : helpers_) t.join();
     }
-    // features: [>= n, 384], element-sorted, written by work enqueued on the current stream so far
+    // The features (and the last reader of z) are among the work enqueued on the current stream so far.
+    void begin()
+    {
+        const c10::cuda::CUDAGuard device(z_[0].device());
+        started_.record(c10::cuda::getCurrentCUDAStream());
+    }
+    // features: [>= n, 384], element-sorted, as of begin()
     int run(const at::Tensor& features, py::handle counts)
     {
         TORCH_CHECK(read_counts(counts.ptr(), acs_) && fits(features, c10::kFloat, z_[0].device()));
         const c10::cuda::CUDAGuard device(features.device());
-        started_.record(c10::cuda::getCurrentCUDAStream());
         features_ = features.const_data_ptr<float>();
         {
             std::lock_guard<std::mutex> lk(mu_);
@@ -358,6 +363,7 @@ PYBIND11_MODULE(_torch_ops, m)
     m.def("featurize_grad", &featurize_grad);
     py::class_<CeluPreactivations>(m, "CeluPreactivations")
         .def(py::init<std::vector<at::Tensor>, std::vector<at::Tensor>, std::vector<at::Tensor>, std::vector<at::Tensor>>())
+        .def("begin", &CeluPreactivations::begin)
         .def("run", &CeluPreactivations::run)
         .def("done", &CeluPreactivations::done);
 }

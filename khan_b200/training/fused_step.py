@@ -265,16 +265,21 @@ class ForceFitStep(FusedTrainStep):
         a.x_grads, a.y_grads, a.z_grads = g, g + cap * size, g + 2 * cap * size
         a.feature_grads, a.labels = sb.upstream.data_ptr(), None
         a.phases = _lib.PASS_PACK | _lib.PASS_FEATURIZE
+        f, call = self._force_args, _lib.lib().ani_force_fit_pass_f32
+        f.fx, f.fy, f.fz = (forces[k].data_ptr() for k in range(3))
+        f.part = 0
         if self.celu:
             _lib.check(_lib.lib().ani_network_pass_f32(ctypes.byref(a), stream), "ani_network_pass_f32")
             a.phases = 0
-            _lib.check(self.preactivations.run(sb.features, sb.acs_host), "CeluPreactivations")
-        f = self._force_args
+            self.preactivations.begin()
         f.pass_ = a
-        f.fx, f.fy, f.fz = (forces[k].data_ptr() for k in range(3))
         if self.celu:
-            f.z_ready = self.preactivations.done()
-        _lib.check(_lib.lib().ani_force_fit_pass_f32(ctypes.byref(f), stream), "ani_force_fit_pass_f32")
+            # the GPU has the first-order pass to work on while the host issues the library products
+            f.part = 1
+            _lib.check(call(ctypes.byref(f), stream), "ani_force_fit_pass_f32")
+            _lib.check(self.preactivations.run(sb.features, sb.acs_host), "CeluPreactivations")
+            f.z_ready, f.part = self.preactivations.done(), 2
+        _lib.check(call(ctypes.byref(f), stream), "ani_force_fit_pass_f32")
         self._args_key = None
 
 
