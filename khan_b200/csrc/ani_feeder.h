@@ -124,7 +124,7 @@ public:
     int next(ani_feeder_batch* out, bool block = true)
     {
         std::unique_lock<std::mutex> lk(mu_);
-        const auto there = [this] { return !ready_.empty() || finished_ || stop_; };
+        const auto there = [this] { return !ready_.empty() || finished_ || stop_ || error_; };
         if (!block && !there()) return kNotYet;
         cv_.wait(lk, there);
         if (ready_.empty()) return error_ ? error_ : 0;
@@ -193,12 +193,25 @@ public:
     }
 
 private:
+    // The failure of batch b takes its place in the order of the batches: the consumer gets every batch before it, then
+    // the code, whichever thread was faster.  The other thread can wait for nothing that this one still owes (the noise
+    // and the publication of a batch depend on earlier batches only), so the turn comes.
+    void fail(int code, long long b)
+    {
+        {
+            std::unique_lock<std::mutex> lk(mu_);
+            cv_.wait(lk, [&] { return publish_turn_ == b || stop_ || error_; });
+            if (!error_) error_ = code;
+        }
+        cv_.notify_all();
+    }
+
+    // A thread that cannot work at all.
     void fail(int code)
     {
         {
             std::lock_guard<std::mutex> lk(mu_);
             if (!error_) error_ = code;
-            finished_ = true;
         }
         cv_.notify_all();
     }
@@ -230,7 +243,7 @@ private:
             }
             FeederSlot& sl = slots_[s];
             if (sl.has_uploaded) {   // the pinned arena is still the source of this slot's previous copy
-                if (cudaEventSynchronize(sl.uploaded) != cudaSuccess) return fail(ANI_ERR_CUDA);
+                if (cudaEventSynchronize(sl.uploaded) != cudaSuccess) return fail(ANI_ERR_CUDA, b);
                 sl.has_uploaded = false;
             }
             const long long first = b * batch_size_;
@@ -244,10 +257,10 @@ private:
                 long long n = 0;
                 for (int m = 0; m < a.n_picks; m++) {
                     const long long p = a.picks[m];
-                    if (p < 0 || p >= a.n_mols_total) return fail(ANI_ERR_BAD_INDEX);
+                    if (p < 0 || p >= a.n_mols_total) return fail(ANI_ERR_BAD_INDEX, b);
                     n += a.mol_ptr[p + 1] - a.mol_ptr[p];
                 }
-                if (n > a.cap_atoms) return fail(ANI_ERR_BAD_SIZE);
+                if (n > a.cap_atoms) return fail(ANI_ERR_BAD_SIZE, b);
                 noise.resize((size_t)(3 * n));
                 {
                     std::unique_lock<std::mutex> lk(mu_);
@@ -262,7 +275,7 @@ private:
                 a.noise = noise.data();
                 a.noise_stride = n;
             }
-            if (int rc = host_pack_batch(a)) return fail(rc);
+            if (int rc = host_pack_batch(a)) return fail(rc, b);
             sl.n_mols = a.n_picks;
             sl.batch_index = b;
             {
@@ -271,19 +284,19 @@ private:
             }
             if (device_ >= 0) {
                 if (sl.has_consumed && cudaStreamWaitEvent(copy_stream_, sl.consumed, 0) != cudaSuccess)
-                    return fail(ANI_ERR_CUDA);
+                    return fail(ANI_ERR_CUDA, b);
                 sl.has_consumed = false;
                 if (cudaMemcpyAsync(sl.dev_arena, sl.host_arena, sl.nbytes, cudaMemcpyHostToDevice, copy_stream_) !=
                         cudaSuccess ||
                     cudaEventRecord(sl.uploaded, copy_stream_) != cudaSuccess)
-                    return fail(ANI_ERR_CUDA);
+                    return fail(ANI_ERR_CUDA, b);
                 sl.has_uploaded = true;
             }
             {
                 std::lock_guard<std::mutex> lk(mu_);
                 ready_.push_back(s);
                 publish_turn_ = b + 1;
-                finished_ = publish_turn_ == n_batches_;
+                if (publish_turn_ == n_batches_) finished_ = true;
             }
             cv_.notify_all();
         }

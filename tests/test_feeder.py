@@ -4,7 +4,7 @@ in order, shuffled and with fuzz -- while running ahead of the consumer on a thr
 import numpy as np
 import pytest
 
-from khan_b200 import RawDataset
+from khan_b200 import RawDataset, _lib
 from khan_b200.data import synthetic as syn
 from khan_b200.data.feeder import BatchFeeder, PackedDataset
 
@@ -204,3 +204,31 @@ def test_packed_copy_follows_replaced_lists_and_invalidate():
     assert PackedDataset.from_raw(raw) is second
     PackedDataset.invalidate(raw)
     assert float(PackedDataset.from_raw(raw).ys[0]) == 7.0
+
+
+@pytest.mark.parametrize("fuzz", [None, 0.05])
+def test_a_batch_that_fails_behind_others_raises_in_its_place(fuzz):
+    """Two threads prepare the batches of a pass; when one of them meets a molecule with a negative size, the consumer
+    gets every batch before that one and then the error, in every pass.  (The error used to be lost when the other
+    thread published an earlier batch at the same moment, and the consumer waited for good.)"""
+    import threading
+    mols = syn.config1(n_mols=400).molecules()
+    packed = PackedDataset(mols, np.zeros(len(mols)))
+    packed.capacity(40)                                   # before the table is damaged
+    packed.ptr[206] = packed.ptr[205] - 1                 # molecule 205, in batch 5 of 10
+    outcomes = []
+
+    def passes():
+        for _ in range(2000 if fuzz is None else 300):
+            got = []
+            with pytest.raises(_lib.AniError):
+                for fed in BatchFeeder(packed, 40, False, fuzz, depth=3, hold=1):
+                    got.append(fed.index)
+            outcomes.append(got)
+        outcomes.append("done")
+
+    worker = threading.Thread(target=passes, daemon=True)
+    worker.start()
+    worker.join(60)
+    assert outcomes and outcomes[-1] == "done", f"a pass neither ended nor raised after {len(outcomes)} passes"
+    assert all(got == [0, 1, 2, 3, 4] for got in outcomes[:-1])
