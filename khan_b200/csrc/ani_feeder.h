@@ -18,7 +18,9 @@
 #include <condition_variable>
 #include <cstdint>
 #include <deque>
+#include <exception>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -99,7 +101,12 @@ public:
         noisy_ = key != nullptr;
         fuzz_ = fuzz;
         if (noisy_) random_.set(key, pos);
-        order_.assign(order, order + n_order);
+        try {
+            order_.assign(order, order + n_order);
+            threads_.reserve(2);
+        } catch (const std::exception&) {
+            return ANI_ERR_BAD_SIZE;
+        }
         batch_size_ = batch_size;
         n_batches_ = (n_order + batch_size - 1) / batch_size;
         {
@@ -114,7 +121,11 @@ public:
         }
         // Packing 1024 shuffled molecules takes a core 0.1 ms, their noise as much again, the GPU 0.15 ms: one thread
         // could not keep up.  A second one is worth its start (30 us) from the third batch on.
-        for (int t = 0; t < (n_batches_ > 2 ? 2 : 1); t++) threads_.emplace_back([this] { run(); });
+        try {
+            for (int t = 0; t < (n_batches_ > 2 ? 2 : 1); t++) threads_.emplace_back([this] { run(); });
+        } catch (const std::system_error&) {     // no thread to be had; one is enough
+            if (threads_.empty()) return ANI_ERR_BAD_SIZE;
+        }
         return ANI_OK;
     }
 
@@ -223,15 +234,24 @@ private:
         return stop_ || error_;
     }
 
-    // One of the submitter's threads.  Batches are taken, given their noise and published in order; what lies
-    // between, the packing, overlaps.
+    // One of the submitter's threads.  No exception leaves it: that would end the process.
     void run()
     {
         if (device_ >= 0 && cudaSetDevice(device_) != cudaSuccess) return fail(ANI_ERR_CUDA);
+        long long b = -1;
+        try {
+            work(b);
+        } catch (const std::exception&) {      // no memory for the noise of batch b
+            b < 0 ? fail(ANI_ERR_BAD_SIZE) : fail(ANI_ERR_BAD_SIZE, b);
+        }
+    }
+
+    // Batches are taken, given their noise and published in order; what lies between, the packing, overlaps.
+    void work(long long& b)
+    {
         const long long n_order = (long long)order_.size();
         std::vector<double> noise;
         for (;;) {
-            long long b;
             int s;
             {
                 std::unique_lock<std::mutex> lk(mu_);
@@ -258,9 +278,11 @@ private:
                 for (int m = 0; m < a.n_picks; m++) {
                     const long long p = a.picks[m];
                     if (p < 0 || p >= a.n_mols_total) return fail(ANI_ERR_BAD_INDEX, b);
-                    n += a.mol_ptr[p + 1] - a.mol_ptr[p];
+                    const long long count = a.mol_ptr[p + 1] - a.mol_ptr[p];
+                    if (count < 0) return fail(ANI_ERR_BAD_INDEX, b);
+                    n += count;
+                    if (n > a.cap_atoms) return fail(ANI_ERR_BAD_SIZE, b);
                 }
-                if (n > a.cap_atoms) return fail(ANI_ERR_BAD_SIZE, b);
                 noise.resize((size_t)(3 * n));
                 {
                     std::unique_lock<std::mutex> lk(mu_);

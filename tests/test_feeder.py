@@ -232,3 +232,30 @@ def test_a_batch_that_fails_behind_others_raises_in_its_place(fuzz):
     worker.join(60)
     assert outcomes and outcomes[-1] == "done", f"a pass neither ended nor raised after {len(outcomes)} passes"
     assert all(got == [0, 1, 2, 3, 4] for got in outcomes[:-1])
+
+
+def test_a_negative_molecule_size_in_a_perturbed_pass_is_an_error():
+    """The noise of a batch is sized from the molecule table before the packer checks it; a table that gives a batch a
+    negative number of atoms has to end as an error of the pass.  (It used to end the process: the exception left the
+    thread that prepared the batch.)  In a process of its own."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+    program = (
+        "import numpy as np\n"
+        "from khan_b200 import _lib\n"
+        "from khan_b200.data import synthetic as syn\n"
+        "from khan_b200.data.feeder import BatchFeeder, PackedDataset\n"
+        "mols = syn.config1(n_mols=120).molecules()\n"
+        "packed = PackedDataset(mols, np.zeros(len(mols)))\n"
+        "packed.capacity(40)\n"
+        "packed.ptr[80] = -100000\n"                 # batch 1 of 3 has a negative number of atoms in all
+        "got = []\n"
+        "try:\n"
+        "    for fed in BatchFeeder(packed, 40, False, 0.05, depth=3, hold=1):\n"
+        "        got.append(fed.index)\n"
+        "except _lib.AniError:\n"
+        "    print('raised behind', got)\n")
+    done = subprocess.run([sys.executable, "-c", program], cwd=ROOT, capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0 and "raised behind [0]" in done.stdout, done.stderr[-500:]
