@@ -183,7 +183,6 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     constexpr int kPerGranule = 16 / (int)sizeof(T);  // values in a granule
     const int lane = lane_id();
     pdl_wait();
-    pdl_trigger();
 
     // Round-major order of the grid: all first rounds (every molecule has one), then all second rounds, ...
     // so the work that exists starts first and is spread evenly over the SMs, and the CTAs of rounds that
@@ -274,6 +273,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
         used += __popc(mA);
     }
     __syncwarp();
+    pdl_trigger();
 
 #include "ani_featurize_round_passes.inl"
     } while (g < G);

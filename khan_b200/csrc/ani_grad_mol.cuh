@@ -140,7 +140,6 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
     using WarpShared = MolGradWarpShared<T>;
     const int lane = lane_id(), warp = warp_id();
     pdl_wait();
-    pdl_trigger();
     WarpShared& ws = reinterpret_cast<WarpShared*>(smem_raw)[warp];
     T* part = reinterpret_cast<T*>(smem_raw + NW * sizeof(WarpShared));
     auto part_at = [part](int plane, int c, int j) -> T& {
@@ -317,6 +316,7 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
         }
         cp_async_wait<0>();   // row slots of a short round are empty groups; nothing may stay pending
     }
+    pdl_trigger();
     __syncthreads();
     if (sizeof(T) == 8) load_energy();
     write_energy();

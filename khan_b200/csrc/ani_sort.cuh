@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(kSortThreads)
 {
     __shared__ int red[kSortWarps][kTypes];
     pdl_wait();
-    pdl_trigger();
     sort_tile(types, n_atoms, blockIdx.x, scatter, gather, counts, red);
+    pdl_trigger();
 }
 
 // The same with the weight packing of a pass in the CTAs behind the tiles: the two have nothing to do with
