@@ -245,13 +245,14 @@ int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, cons
         // four, the scans and triplets of one warp are a chain of 12 us (float; double 22 us), however small the batch.
         // Few atoms per warp cost more instructions (load, sort and table per round), so not beyond that.  Microseconds
         // with 4 / 2 / 1 atoms in float, 64 molecules 13.6 / 10.3 / 8.3, 256: 16.5 / 13.3 / 13.2, 512: 19.8 / 17.4 / 20.5,
-        // 1024: 24.9 / 26.5 / 39.0; in double, 64: 25 / 18 / 15, 512: 39 / 41 / 47.
+        // 1024: 24.9 / 26.5 / 39.0; in double, 64: 25 / 18 / 15, 512: 39 / 41 / 47.  (32 float warps are resident, but with
+        // that line 1024 molecules take three atoms per warp: 27.3 instead of 25.2, and 1.5 more a batch with eight streams.)
         const int resident = kSms * (sizeof(T) == 4 ? 28 : 20);
         const int per_round = (int)std::min<long long>((n_atoms + resident - 1) / resident, kMolCentrals);
         const int rounds = (kMolMaxAtoms + per_round - 1) / per_round;
         ANI_CUDA(launch_chain(featurize_mol_kernel<T>, n_mols * rounds, kWarp, 0, (cudaStream_t)stream, 1, xs, ys, zs,
                               types, mos, macs, n_mols, (int)n_atoms, sis, oh, oc, on, oo, acs_host[0], acs_host[1],
-                              acs_host[2], acs_host[3], per_round));
+                              acs_host[2], acs_host[3], per_round, 65536 / per_round + 1));
         return ANI_OK;
     }
 

@@ -38,6 +38,11 @@
 // lone warp then worked on it for 30 us (float) to 140 us (double) after everything else had ended: the
 // three operators on 1024 molecules took 104 / 317 us with one, 70 / 178 us without.)
 //
+// What bounds it: instruction issue, with as many one-warp CTAs per SM as shared memory allows.  That is allotted in
+// steps of 1 KB (other kernels of the library align theirs to that): 6 KB + 1 KB reserved let 32 in, 7 + 1 let in 28.
+// A group table without gaps brought it from the one to the other: 1024 molecules 26.4 -> 25.5 us alone, 14.6 -> 14.2
+// a batch with eight in flight (a division less per warp among it).
+//
 // Computes what featurize_cpu of the reference computes (gpu_featurizer/kernel_cpu.cpp:406-537).
 #pragma once
 
@@ -51,7 +56,7 @@ namespace ani {
 constexpr int kMolMaxAtoms = 32;       // molecules up to this size take the fast path
 constexpr int kMolCentrals = 4;        // central atoms per round
 constexpr int kMolPool = 96;           // angular neighbours of the central atoms worked on together
-constexpr int kMolGroupStride = 16;    // group id = central slot * 16 + element-pair bucket
+constexpr int kMolGroups = kMolCentrals * kPairBuckets;   // group id = element-pair bucket * 4 + central slot
 constexpr int kMolNoGroup = 0xff;      // id of the quads behind the last group
 constexpr int kMolSlotsPerLane = 1;    // slots a lane evaluates per pass B (2 was measured: no gain)
 constexpr int kMolChunk = kMolSlotsPerLane * kWarp;   // slots per pass B / C
@@ -89,7 +94,7 @@ template <typename T, int POOL, int MAXA> struct MolAngularShared {
     T ang_fc[POOL];                       // f_C(r_ij, A_Rc)
     alignas(16) T A[kNumThetas][kMolChunkStride];
     alignas(16) T BF[kNumARs][kMolChunkStride];
-    MolGroupInfo tab[kMolCentrals * kMolGroupStride];
+    MolGroupInfo tab[kMolGroups];
     T* row[kMolCentrals];                     // feature row of each central atom of the round
     alignas(16) int cnt_a[kMolCentrals * kTypes];   // angular neighbours per element, per central atom
     int list_base[kMolCentrals];              // first entry of each central atom's list
@@ -176,7 +181,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
                          const int* __restrict__ types, const int* __restrict__ mol_offsets,
                          const int* __restrict__ mol_counts, int n_mols, int n_atoms,
                          const int* __restrict__ scatter, T* out_h, T* out_c, T* out_n, T* out_o,
-                         int acs0, int acs1, int acs2, int acs3, int per_round)
+                         int acs0, int acs1, int acs2, int acs3, int per_round, int per_round_recip)
 {
     __shared__ MolFwdWarpShared<T> ws;
     using Granule = Vec4<float>;                      // 16 bytes of zeros, whatever T is
@@ -212,7 +217,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     // Round r of a molecule with R rounds takes the central atoms r, r + R, r + 2 R, r + 3 R: every round
     // gets the same mix of light and heavy atoms (atoms are in element order, and the cost of a central
     // atom grows with the square of its neighbour count), so the rounds of a molecule cost about the same.
-    const int n_rounds = (n + per_round - 1) / per_round;
+    const int n_rounds = ((n + per_round - 1) * per_round_recip) >> 16;   // / per_round; n is at most 32 here
     if (round >= n_rounds) return;
     const int G = (n - round + n_rounds - 1) / n_rounds;
 
