@@ -75,7 +75,6 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 22 : 1)
             ws.ang.ang_fc[0] = (T)0;
         }
         if (lane < kMolCentrals * kTypes) ws.ang.cnt_a[lane] = 0;
-        if (lane < kMolCentrals) ws.ang.list_base[lane] = lane * kLargeCapA;
 
         // ---- the central atoms: coordinates to all lanes, rows, zero fill of the angular blocks ----
         T xi[kMolCentrals], yi[kMolCentrals], zi[kMolCentrals];

@@ -12,9 +12,8 @@
 //      is compacted in lane order comes out sorted by element for free;
 //   A. per central atom of the round (coordinates by shuffle): one distance per lane; (r, f_C)
 //      of every atom of the molecule goes to a table (f_C = 0 beyond R_Rc), and the neighbours
-//      within A_Rc, compacted by a ballot, to the list (unit vector, r, f_C) of this central atom.  The
-//      lists of the round share 96 entries: an atom whose list does not fit any more waits until T, B
-//      and C have worked off the ones before it (31 neighbours of one atom always fit);
+//      within A_Rc, compacted by a ballot, to the list (unit vector, r, f_C) of this central atom, which
+//      holds all 31 that there can be;
 //   R. the radial features of all central atoms of the round at once: lane = (central atom,
 //      pair of radial shifts) walks the table of its central atom.  The table is in element
 //      order for every central atom alike, so the loops over the four element runs are uniform
@@ -33,14 +32,16 @@
 // not depend on the launch shape.
 //
 // A molecule with more than 32 atoms met by this kernel (the host picks it from the MEAN
-// molecule size) goes through the streaming routine of ani_featurize.cuh.  (With 24 fixed entries per
-// central atom a denser atom streamed too.  One in a few batches of 1024 molecules has such an atom, and a
-// lone warp then worked on it for 30 us (float) to 140 us (double) after everything else had ended: the
-// three operators on 1024 molecules took 104 / 317 us with one, 70 / 178 us without.)
+// molecule size) goes through the streaming routine of ani_featurize.cuh.  No atom of a smaller one does: with lists of
+// 24 a denser atom streamed too, one in a few batches of 1024 molecules has such an atom, and a lone warp then worked
+// on it for 30 us (float) to 140 us (double) after everything else had ended.  Four lists that shared 96 entries, an
+// atom that did not fit opening another pass, cost every round the loop and its registers (25.2 us against 24.3
+// alone, 14.2 against 13.5 a batch with eight in flight, 1024 molecules); lists of 24 and the denser atoms after the
+// round 1 to 4 us in the batches that have one.  Four full lists fit where the radial table lies over the factors.
 //
 // What bounds it: instruction issue, with as many one-warp CTAs per SM as shared memory allows.  That is allotted in
 // steps of 1 KB (other kernels of the library align theirs to that): 6 KB + 1 KB reserved let 32 in, 7 + 1 let in 28.
-// A group table without gaps brought it from the one to the other: 1024 molecules 26.4 -> 25.5 us alone, 14.6 -> 14.2
+// A group table without gaps brought it from the one to the other: 1024 molecules 26.0 -> 25.2 us alone, 14.45 -> 14.2
 // a batch with eight in flight (a division less per warp among it).
 //
 // Computes what featurize_cpu of the reference computes (gpu_featurizer/kernel_cpu.cpp:406-537).
@@ -55,7 +56,7 @@ namespace ani {
 
 constexpr int kMolMaxAtoms = 32;       // molecules up to this size take the fast path
 constexpr int kMolCentrals = 4;        // central atoms per round
-constexpr int kMolPool = 96;           // angular neighbours of the central atoms worked on together
+constexpr int kMolCapA = kMolMaxAtoms - 1;   // angular neighbours of a central atom
 constexpr int kMolGroups = kMolCentrals * kPairBuckets;   // group id = element-pair bucket * 4 + central slot
 constexpr int kMolNoGroup = 0xff;      // id of the quads behind the last group
 constexpr int kMolSlotsPerLane = 1;    // slots a lane evaluates per pass B (2 was measured: no gain)
@@ -88,7 +89,8 @@ struct MolSortShared {
 
 // What the angular passes (T, B, C) of a round work on: the angular neighbour lists of the round's
 // central atoms (element order inside each list), the group table, the factor chunks and the rows.
-// POOL = entries of the lists together, MAXA = longest list (list indices are packed into 8 bits).
+// POOL = entries of the lists together, MAXA = longest list and distance of the lists (list indices are packed into 8
+// bits); a structure derived from this one may place the lists otherwise, with a first() of its own.
 template <typename T, int POOL, int MAXA> struct MolAngularShared {
     Vec4<T> ang_u[POOL];                  // (x_i - x_j) / r_ij and r_ij, element order, per central atom
     T ang_fc[POOL];                       // f_C(r_ij, A_Rc)
@@ -97,14 +99,17 @@ template <typename T, int POOL, int MAXA> struct MolAngularShared {
     MolGroupInfo tab[kMolGroups];
     T* row[kMolCentrals];                     // feature row of each central atom of the round
     alignas(16) int cnt_a[kMolCentrals * kTypes];   // angular neighbours per element, per central atom
-    int list_base[kMolCentrals];              // first entry of each central atom's list
     alignas(8) unsigned char quad_gid[mol_quad_bytes(MAXA, POOL)];
+    __device__ __forceinline__ int first(int g) const { return g * MAXA; }   // first entry of a central atom's list
 };
 
 template <typename T> struct MolFwdWarpShared {
-    MolAngularShared<T, kMolPool, kMolMaxAtoms - 1> ang;
-    Vec2<T> rad[kMolCentrals][kMolMaxAtoms];   // (r_ij, f_C(r_ij, R_Rc)) of every atom j of the molecule, f_C = 0 out of range
+    MolAngularShared<T, kMolCentrals * kMolCapA, kMolCapA> ang;
     MolSortShared sort;
+    // (r_ij, f_C(r_ij, R_Rc)) of every atom j of the molecule, f_C = 0 out of range.  It lies where pass B puts its
+    // factors: R has read it before.
+    __device__ __forceinline__ Vec2<T>* rad(int g) { return reinterpret_cast<Vec2<T>*>(&ang.A[0][0]) + g * kMolMaxAtoms; }
+    static_assert(sizeof(Vec2<T>) * kMolCentrals * kMolMaxAtoms <= sizeof(ang.A), "the radial table fits the factors");
 };
 
 __device__ __forceinline__ unsigned low_lanes(int c) { return c >= 32 ? 0xffffffffu : ((1u << c) - 1u); }
@@ -229,15 +234,12 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
         ws.ang.ang_u[0] = Vec4<T>{(T)1, (T)0, (T)0, (T)1};
         ws.ang.ang_fc[0] = (T)0;
     }
-    unsigned skip = 0;   // central atoms that are refused
-    int g = 0;
-    do {
     if (lane < kMolCentrals * kTypes) ws.ang.cnt_a[lane] = 0;
     __syncwarp();
 
-    // ---- A: scan, one central atom after another, as many as the lists have room for ----
-    int used = 0;
-    for (; g < G; g++) {
+    // ---- A: scan, one central atom after another ----
+    unsigned skip = 0;   // central atoms that are refused
+    for (int g = 0; g < G; g++) {
         const int c = round + g * n_rounds;
         const T xi = __shfl_sync(kFull, ml.x, c), yi = __shfl_sync(kFull, ml.y, c), zi = __shfl_sync(kFull, ml.z, c);
         const int ti = __shfl_sync(kFull, ml.type, c);
@@ -257,7 +259,6 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
         const bool in_rad = lane < n && lane != c && r < (T)kR_Rc;
         const bool in_ang = in_rad && r < (T)kA_Rc;
         const unsigned mA = __ballot_sync(kFull, in_ang);
-        if (used + __popc(mA) > kMolPool) break;   // this central atom opens the next pass
         // the angular blocks start as zeros (16-byte stores: 2.5 per lane); pass C writes the blocks of
         // the element pairs that occur, after a __syncwarp, so the order of the two is fixed
         {
@@ -267,26 +268,20 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
             for (int i = 0; i < (kGranules + kWarp - 1) / kWarp; i++)
                 if (i * kWarp + lane < kGranules) zero[i * kWarp + lane] = Granule{0.f, 0.f, 0.f, 0.f};
         }
-        ws.rad[g][lane] = Vec2<T>{r, in_rad ? cutoff_value<T>(r, (T)kR_Rc) : (T)0};
+        ws.rad(g)[lane] = Vec2<T>{r, in_rad ? cutoff_value<T>(r, (T)kR_Rc) : (T)0};
         if (in_ang) {
-            const int p = used + __popc(mA & lanemask_lt());
+            const int p = ws.ang.first(g) + __popc(mA & lanemask_lt());
             ws.ang.ang_u[p] = Vec4<T>{dx * inv, dy * inv, dz * inv, r};
             ws.ang.ang_fc[p] = cutoff_value<T>(r, (T)kA_Rc);
         }
         if (lane < kTypes) ws.ang.cnt_a[g * kTypes + lane] = __popc(mA & ws.sort.tmask[lane]);
-        if (lane == 0) ws.ang.list_base[g] = used;
-        used += __popc(mA);
     }
     __syncwarp();
-    pdl_trigger();
-
-#include "ani_featurize_round_passes.inl"
-    } while (g < G);
 
     // ---- R: radial features of the whole round, lane = (central atom, pair of shifts) ----
     {
         const int g = lane >> 3, sp = lane & 7;
-        const Vec2<T>* list = ws.rad[g];
+        const Vec2<T>* list = ws.rad(g);
         const T sh0 = (T)c_tab.R_Rs[2 * sp], sh1 = (T)c_tab.R_Rs[2 * sp + 1];
         const uint4 tmq = *reinterpret_cast<const uint4*>(ws.sort.tmask);
         const int run_end[kTypes] = {__popc(tmq.x), __popc(tmq.x | tmq.y), __popc(tmq.x | tmq.y | tmq.z), n};
@@ -310,6 +305,10 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
                 *reinterpret_cast<Vec2<T>*>(row + t * kNumRs + 2 * sp) = Vec2<T>{acc[t].x, acc[t].y};
         }
     }
+    pdl_trigger();
+    __syncwarp();
+
+#include "ani_featurize_round_passes.inl"
 }
 
 }  // namespace ani

@@ -35,7 +35,7 @@
             MolGroupInfo e;
             e.off = off;
             e.cnt = cnt;
-            const int first = ws.ang.list_base[g];
+            const int first = ws.ang.first(g);
             e.packed = (first + pick4(stv, ta)) | ((first + pick4(stv, tb)) << 8) | (nb << 16) |
                        ((ta == tb ? 1 : 0) << 24);
             e.recip = (unsigned)(65536.0f * __frcp_rn((float)nb)) + 1u;   // in [2^16 / nb, 2^16 / nb + 1.01)

@@ -17,12 +17,18 @@
 
 namespace ani {
 
-template <typename T> struct TangentRound : MolAngularShared<T, kMolPool, kMolMaxAtoms - 1> {
-    Vec4<T> du[kMolPool];                          // d (unit vector) and d r along v
-    T fc_dot[kMolPool];                            // d f_C(r, A_Rc)
+// The lists of a round share 96 entries: an atom whose list does not fit any more waits until T, B and C have worked off
+// the ones before it (31 neighbours of one atom always fit).
+constexpr int kTangentPool = 96;
+
+template <typename T> struct TangentRound : MolAngularShared<T, kTangentPool, kMolMaxAtoms - 1> {
+    int list_base[kMolCentrals];                   // first entry of each central atom's list
+    Vec4<T> du[kTangentPool];                      // d (unit vector) and d r along v
+    T fc_dot[kTangentPool];                        // d f_C(r, A_Rc)
     alignas(16) T dA[kNumThetas][kMolChunkStride];
     alignas(16) T dBF[kNumARs][kMolChunkStride];
     Vec4<T> slope[kMolCentrals][kMolMaxAtoms];     // r, -2 eta f_C dr, df_C dr of every atom of the molecule (R_Rc)
+    __device__ __forceinline__ int first(int g) const { return list_base[g]; }
 };
 
 template <typename T> struct TangentWarpShared {
@@ -115,7 +121,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 16 : 10)
             const bool in_rad = lane < n && lane != c && r < (T)kR_Rc;
             const bool in_ang = in_rad && r < (T)kA_Rc;
             const unsigned mA = __ballot_sync(kFull, in_ang);
-            if (used + __popc(mA) > kMolPool) break;
+            if (used + __popc(mA) > kTangentPool) break;
             {
                 Granule* zero = reinterpret_cast<Granule*>(row + kRadial);
                 constexpr int kGranules = kAngular / kPerGranule;

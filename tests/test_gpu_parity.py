@@ -314,6 +314,18 @@ def test_small_molecules_at_every_split(gpu, oracle_mod, n_mols, dt):
         assert normwise(out, ref[k]) < FTOL[dt]
 
 
+@pytest.mark.parametrize("n_mols,n", [(3, 24), (3, 25), (3, 26), (3, 32), (500, 26)])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_atoms_at_the_end_of_the_angular_list(gpu, oracle_mod, n_mols, n, dt):
+    """Molecules whose atoms all lie within A_Rc of one another: 23, 24, 25 and 31 neighbours for lists of 24, one to
+    four such atoms in a round (500 molecules: four)."""
+    b = _concat(_dense_blobs(n_mols, n, 1.54, n), syn.gdb_like_batch(20, 8, heavy_min=1, heavy_max=2))
+    si, gi, ac = oracle_mod.ani_sort(b.atomic_numbers)
+    args = [v.astype(np.float64) for v in b.coords(dt)] + [b.atomic_numbers, b.mol_offsets, b.mol_atom_counts, si, ac]
+    for out, ref in zip(gpu.gpu_featurize(b, dt), oracle_mod.featurize(*args, impl="port", threads=8)):
+        assert normwise(out, ref) < FTOL[dt]
+
+
 @pytest.mark.parametrize("n_mols", [1, 30, 75])
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 def test_large_molecules_at_every_split(gpu, oracle_mod, n_mols, dt):
