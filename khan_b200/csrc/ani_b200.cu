@@ -294,7 +294,7 @@ int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, cons
 // The coordinate gradients of such a batch are computed a molecule per CTA (and molecule energies with them).
 bool grad_per_molecule(long long n_atoms, int n_mols, std::initializer_list<const void*> rows)
 {
-    return n_mols > 0 && small_molecules(n_atoms, n_mols) && all_aligned16(rows) && (long long)n_mols * 2 <= 0x7fffffffLL;
+    return n_mols > 0 && small_molecules(n_atoms, n_mols) && all_aligned16(rows) && n_mols <= 0x7fffffff - kWarp;
 }
 
 template <typename T>
@@ -326,15 +326,13 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
                 if (int rc = set_smem(featurize_grad_mol_kernel<T, NW>, smem)) return rc;
                 configured_dev = dev;
             }
-            // More molecules than are resident at once: those well above the mean start first.  Alone, 1024 molecules
-            // of up to 8 heavy atoms: float 35.2 -> 33.1 us, double 98 -> 79; 2048: 52.3 -> 46.4, 151 -> 137; 4096: 94
-            // -> 82.  (In three classes 31.8 at 1024 and the same from there on, but with eight streams in flight the
-            // CTAs without work then cost 6 % of the throughput, in two classes 3 %.)
-            const bool classes = (long long)n_mols * NW > (long long)kSms * (sizeof(T) == 4 ? 20 : 12);
-            const int big_size = (int)(n_atoms * 19 / (16LL * n_mols));
-            ANI_CUDA(launch_chain(featurize_grad_mol_kernel<T, NW>, classes ? 2 * n_mols : n_mols, NW * kWarp, smem, st, 1, xs,
-                                  ys, zs, types, mos, macs, n_mols, (int)n_atoms, sis, gh, gc, gn, go, gx, gy, gz,
-                                  acs_host[0], acs_host[1], acs_host[2], acs_host[3], big_size, sums));
+            // More molecules than are resident at once: the larger ones start first (figures at kMolGradOrder).
+            const bool in_order = (long long)n_mols * NW > (long long)kSms * (sizeof(T) == 4 ? 20 : 12);
+            constexpr int kOrder = kMolGradOrder<T, NW>;
+            const dim3 grid = in_order ? dim3((n_mols + kOrder - 1) / kOrder, kOrder) : dim3(n_mols);
+            ANI_CUDA(launch_chain(featurize_grad_mol_kernel<T, NW>, grid, NW * kWarp, smem, st, 1, xs, ys, zs, types, mos,
+                                  macs, n_mols, (int)n_atoms, sis, gh, gc, gn, go, gx, gy, gz, acs_host[0], acs_host[1],
+                                  acs_host[2], acs_host[3], sums));
             return ANI_OK;
         };
         // Eight warps a molecule shorten its chain of scans and pair passes (64 molecules 14.8 -> 10.6 us, 512: 27.4 ->

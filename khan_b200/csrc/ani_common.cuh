@@ -112,13 +112,10 @@ struct MolRange {
     int n;     // atoms
 };
 
-// Reads and checks molecule m.  Returns false (after recording the problem) when the molecule
+// Checks the n atoms from `base` on.  Returns false (after recording the problem) when the molecule
 // must be skipped.
-__device__ __forceinline__ bool load_molecule(const int* __restrict__ mol_offsets,
-                                              const int* __restrict__ mol_counts, int m,
-                                              int n_atoms, MolRange* out)
+__device__ __forceinline__ bool check_molecule(int n, int base, int n_atoms, MolRange* out)
 {
-    const int n = mol_counts[m], base = mol_offsets[m];
     out->base = base;
     out->n = n;
     if (n <= 0) return false;
@@ -127,6 +124,14 @@ __device__ __forceinline__ bool load_molecule(const int* __restrict__ mol_offset
         return false;
     }
     return true;
+}
+
+// Reads and checks molecule m.
+__device__ __forceinline__ bool load_molecule(const int* __restrict__ mol_offsets,
+                                              const int* __restrict__ mol_counts, int m,
+                                              int n_atoms, MolRange* out)
+{
+    return check_molecule(mol_counts[m], mol_offsets[m], n_atoms, out);
 }
 
 __device__ __forceinline__ int checked_type(int t)

@@ -126,6 +126,13 @@ template <typename T> struct MolEnergySums {
     T* mol_energy;
 };
 
+// Molecules whose CTAs are put into order of size.  Microseconds alone with 4 / 8 / 16 / 32, and in two classes with two
+// CTAs per molecule as it was: eight warps, float, 600 molecules 22.6 / 21.0 / 20.2 / 20.6, 22.3; four warps, float, 1024:
+// 34.9 / 34.2 / 32.8 / 33.7, 35.6, 2048: 49.3 / 47.8 / 45.6 / 44.1, 48.8; double, 1024: 88 / 83 / 81 / 81, 86, 2048: 143 /
+// 139 / 131 / 126, 138.  But the order costs instructions, and with eight streams in flight, where it gains nothing, 1024
+// molecules in float take 18.3 / 18.5 / 18.9, in two classes 19.2 and without any order 18.2 (37.7 alone).
+template <typename T, int NW> constexpr int kMolGradOrder = sizeof(T) == 4 && NW == 4 ? 4 : 16;
+
 template <typename T, int NW>
 __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
     featurize_grad_mol_kernel(const T* __restrict__ xs, const T* __restrict__ ys, const T* __restrict__ zs,
@@ -133,7 +140,8 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
                               const int* __restrict__ mol_counts, int n_mols, int n_atoms,
                               const int* __restrict__ scatter, const T* __restrict__ gh,
                               const T* __restrict__ gc, const T* __restrict__ gn, const T* __restrict__ go,
-                              T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3, int big_size, const MolEnergySums<T> sums)
+                              T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3,
+                              const MolEnergySums<T> sums)
 {
     constexpr int GR = MolGradCfg<T>::kRowBufs;   // central atoms per round
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -146,18 +154,34 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
         return part[(plane * kMolMaxAtoms + c) * kMolGradPitch + j];
     };
 
-    // With two CTAs per molecule in the grid, class-major: first one CTA for every molecule, of which only those of
-    // molecules above big_size work (the others leave after one load), then the same for the rest; CTAs start in index
-    // order, so the expensive molecules start first and the cheap ones fill the SMs behind them.
-    const bool classes = (int)gridDim.x > n_mols;
-    const int cls = blockIdx.x / n_mols, m = blockIdx.x - cls * n_mols;
+    // In a grid of (X, Y) CTAs the molecules i, i + X, i + 2 X ... share the CTAs (i, 0), (i, 1), (i, 2) ... in order of
+    // their sizes: CTAs start in index order, so the expensive molecules start first and the cheap ones fill the SMs
+    // behind them.  Every CTA finds its molecule from the Y sizes; only those behind the end of the batch have none.
+    int m = blockIdx.x;
     MolRange mol;
-    if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) {
-        if (sums.mol_energy && cls == 0 && threadIdx.x == 0) sums.mol_energy[m] = (T)0;
+    bool usable;
+    if (gridDim.y == 1) {
+        usable = load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol);
+    } else {
+        constexpr int kLast = kMolGradOrder<T, NW> - 1;
+        const int mine = blockIdx.x + (lane & kLast) * gridDim.x;
+        const int size = mine < n_mols ? mol_counts[mine] : -1, first = mine < n_mols ? mol_offsets[mine] : 0;
+        int rank = 0;
+#pragma unroll
+        for (int d = 1; d <= kLast; d++) {
+            const int other = __shfl_xor_sync(kFull, size, d), other_lane = (lane ^ d) & kLast;
+            rank += other > size || (other == size && other_lane < (lane & kLast)) ? 1 : 0;
+        }
+        const int src = __ffs(__ballot_sync(kFull, rank == (int)blockIdx.y)) - 1;
+        m = blockIdx.x + (src & kLast) * gridDim.x;
+        if (m >= n_mols) return;
+        usable = check_molecule(__shfl_sync(kFull, size, src), __shfl_sync(kFull, first, src), n_atoms, &mol);
+    }
+    if (!usable) {
+        if (sums.mol_energy && threadIdx.x == 0) sums.mol_energy[m] = (T)0;
         return;
     }
     const int n = mol.n, base = mol.base;
-    if (classes && cls != (n > big_size ? 0 : 1)) return;
 
     T energy = (T)0;
     auto load_energy = [&] {

@@ -260,7 +260,9 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
     tc_fence_after();
     if (!(p.early_weights && warp == kChainEpi / 32 + 1)) {      // the weight warp may run ahead
         pdl_wait();
-        pdl_trigger();
+        // Energies + forces: the CTAs of the gradient kernel behind would gather on the SMs that have no tile, the largest
+        // molecules first (1024 molecules, a third of the SMs without one: 116 us a pass, 107.5 without the trigger).
+        if (MODE != kChainForces) pdl_trigger();
     }
     const unsigned tmem = sh.tmem_base;
     // chunks of packed weights in the order of the chain

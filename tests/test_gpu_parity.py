@@ -314,6 +314,39 @@ def test_small_molecules_at_every_split(gpu, oracle_mod, n_mols, dt):
         assert normwise(out, ref[k]) < FTOL[dt]
 
 
+@pytest.mark.parametrize("n_mols", [371, 384, 385, 1000, 1003])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_gradient_in_order_of_size(gpu, oracle_mod, n_mols, dt):
+    """From 371 molecules (float) on the CTAs of every 16 (4 in large float batches) take them in order of size:
+    remainders, equal sizes, molecules without atoms, and the molecule energies that ride along."""
+    import torch
+    from khan_b200.inference import EnergyForces
+    from khan_b200.model.nn import MoleculeNN
+    from khan_b200.staged import StagedBatch
+    b = syn.gdb_like_batch(n_mols - 3, 5)
+    at = [0, (n_mols - 3) // 2, n_mols - 3]             # empty molecules: first, in the middle, last
+    offsets = np.insert(b.mol_offsets, at, [0, b.mol_offsets[at[1]], b.n_atoms]).astype(np.int32)
+    b = syn.Batch(b.xs, b.ys, b.zs, b.atomic_numbers, offsets, np.insert(b.mol_atom_counts, at, 0).astype(np.int32))
+    si, gi, ac = oracle_mod.ani_sort(b.atomic_numbers)
+    up = syn.upstream_grads(b, ac, dtype=dt)
+    args = [v.astype(np.float64) for v in b.coords(dt)] + [b.atomic_numbers, b.mol_offsets, b.mol_atom_counts, si, ac]
+    ref = oracle_mod.featurize_grad(*args, *[u.astype(np.float64) for u in up], impl="port", threads=8)
+    for k, out in enumerate(gpu.gpu_featurize_grad(b, dt, up)):
+        assert normwise(out, ref[k]) < FTOL[dt]
+
+    real = torch.float32 if dt == np.float32 else torch.float64
+    sb = StagedBatch(b.n_atoms, n_mols, real, device="cuda:0")
+    sb.set_shape(b.n_atoms, n_mols, ac)
+    for to, v in zip((sb.x, sb.y, sb.z, sb.types, sb.mol_offsets, sb.mol_counts), gpu.batch_tensors(b, dt)):
+        to.copy_(v)
+    ev = EnergyForces(MoleculeNN(device="cuda:0", seed=3, precision=real), b.n_atoms, n_mols, device="cuda:0")
+    ev.mol_energy.fill_(float("nan"))
+    ev.run(sb)
+    atoms = ev.energy_sorted[:b.n_atoms].double()[sb.gather[:b.n_atoms].long()].cpu().numpy()
+    want = np.array([atoms[o:o + n].sum() for o, n in zip(b.mol_offsets, b.mol_atom_counts)])
+    assert normwise(ev.mol_energy[:n_mols].double().cpu().numpy(), want) < FTOL[dt]
+
+
 @pytest.mark.parametrize("n_mols,n", [(3, 24), (3, 25), (3, 26), (3, 32), (500, 26)])
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 def test_atoms_at_the_end_of_the_angular_list(gpu, oracle_mod, n_mols, n, dt):
