@@ -614,9 +614,12 @@ int ani_feeder_set_slots(ani_feeder* f, const ani_feeder_slot* slots, int n_slot
  *   ANI_DRIVER_GRADIENTS  energies + coordinate gradients; the latter as rows [n_atoms][3] into that place
  *   ANI_DRIVER_TRAIN      optional row clip, loss and its weight gradients, loss scaling, optional update
  * Training runs on `stream`, with the features of the next batch on streams[0]; the other two run batch b on
- * streams[b & 1], behind what `stream` held at the first step.  ani_driver_join makes `stream` wait for all of it.
+ * streams[b & 1], energies behind what `stream` held at the first step (the weights must not change during the pass),
+ * gradients each batch behind what `stream` held at its own step, with the weights as they were then (copied to
+ * weights[b % ANI_DRIVER_RING]): work enqueued between two steps may change them.  ani_driver_join makes `stream` wait
+ * for all of it.
  * ring_host is pinned memory that the kernels write; ani_driver_wait(d, place) blocks until the results last
- * enqueued for a place are there, and the caller has read a place before the step that fills it again.
+ * enqueued for a place are there, and the caller has waited for a place before the step that fills it again.
  * pass / pass64: the argument block of each of the two sets of buffers used in turn (pass64: double precision,
  * not for training); what describes the batch is filled in here.  slots: the device arrays behind each slot of
  * the feeder.  step() returns 1 (*batch is the one enqueued), 0 (pass over) or a negative status. */
@@ -635,6 +638,7 @@ typedef struct ani_driver_args {
     void* streams[2];                /* training: the first only */
     void* energies;                  /* [all molecules] or NULL */
     void* ring_host[ANI_DRIVER_RING];
+    void* weights[ANI_DRIVER_RING];  /* gradients only: ani_driver_weights_bytes() each, 256-byte aligned */
     float *params, *grads, *m, *v, *ema;       /* training: ani_nadam_step_f32 (update != 0) */
     long long n_params;
     const float* hyper;
@@ -647,6 +651,7 @@ typedef struct ani_driver_args {
     float clip_max_norm;
 } ani_driver_args;
 typedef struct ani_driver ani_driver;
+size_t ani_driver_weights_bytes(int double_precision);
 int ani_driver_create(const ani_driver_args* args, ani_driver** out);
 int ani_driver_step(ani_driver* d, ani_feeder* f, void* stream, ani_feeder_batch* batch);
 int ani_driver_wait(ani_driver* d, int place);

@@ -130,7 +130,7 @@ class DriverArgs(ctypes.Structure):
     _fields_ = ([("mode", ctypes.c_int), ("n_slots", ctypes.c_int), ("slots", ctypes.POINTER(DriverSlot)),
                  ("pass_", ctypes.POINTER(PassArgs) * 2), ("pass64", ctypes.POINTER(EnergyArgs64) * 2),
                  ("streams", ctypes.c_void_p * 2), ("energies", ctypes.c_void_p),
-                 ("ring_host", ctypes.c_void_p * DRIVER_RING)]
+                 ("ring_host", ctypes.c_void_p * DRIVER_RING), ("weights", ctypes.c_void_p * DRIVER_RING)]
                 + [(n, ctypes.c_void_p) for n in ("params", "grads", "m", "v", "ema")]
                 + [("n_params", ctypes.c_longlong), ("hyper", ctypes.c_void_p), ("state", ctypes.c_void_p),
                    ("update", ctypes.c_int), ("loss_kind", ctypes.c_int), ("rmse", ctypes.c_void_p),
@@ -195,6 +195,7 @@ SIGNATURES = {
     "ani_feeder_end": (_i, [_vp]),
     "ani_feeder_destroy": (_i, [_vp]),
     "ani_feeder_set_slots": (_i, [_vp, _vp, _i]),
+    "ani_driver_weights_bytes": (ctypes.c_size_t, [_i]),
     "ani_driver_create": (_i, [ctypes.POINTER(DriverArgs), ctypes.POINTER(_vp)]),
     "ani_driver_step": (_i, [_vp, _vp, _vp, ctypes.POINTER(FeederBatch)]),
     "ani_driver_wait": (_i, [_vp, _i]),

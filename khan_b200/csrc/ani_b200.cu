@@ -1162,6 +1162,8 @@ struct ani_driver {
     explicit ani_driver(const ani_driver_args& a) : impl(a) {}
 };
 
+size_t ani_driver_weights_bytes(int double_precision) { return ani::weights_bytes(double_precision != 0); }
+
 int ani_driver_create(const ani_driver_args* a, ani_driver** out)
 {
     if (!a || !out || !a->slots || !a->streams[0]) return ANI_ERR_NULL_POINTER;
@@ -1174,6 +1176,11 @@ int ani_driver_create(const ani_driver_args* a, ani_driver** out)
     if (a->mode == ANI_DRIVER_GRADIENTS || (a->mode == ANI_DRIVER_ENERGIES && !a->energies))
         for (void* p : a->ring_host)
             if (!p) return ANI_ERR_NULL_POINTER;
+    if (a->mode == ANI_DRIVER_GRADIENTS)
+        for (void* p : a->weights) {
+            if (!p) return ANI_ERR_NULL_POINTER;
+            if (reinterpret_cast<uintptr_t>(p) & 255) return ANI_ERR_MISALIGNED;
+        }
     ani_driver* d = new (std::nothrow) ani_driver(*a);
     if (!d) return ANI_ERR_CUDA;
     if (int rc = d->impl.init()) {

@@ -8,8 +8,13 @@
 // host time, nearly all of it launches.
 //
 // Two batches are in flight, each in a set of buffers of its own:
-//   * energies, gradients: batch b on stream b & 1.  The networks take whole waves of 128-atom tiles (220 tiles on 148
+//   * energies: batch b on stream b & 1.  The networks take whole waves of 128-atom tiles (220 tiles on 148
 //     SMs for 2048 molecules), and the other batch's kernels fill what the last wave leaves idle.
+//   * gradients: the same, but their consumer takes the results batch by batch and may enqueue anything in between, a
+//     training step among it.  So every batch has a copy of the weights of its own, made on the caller's stream at the
+//     batch's step: one small kernel, beside the batches in flight.  (With the weights themselves the caller's stream
+//     would have to wait for every batch and the next networks for that stream: 8 batches of 1024 molecules took 2500 us
+//     that way, 2360 with copies, 2290 without either: 9 us a batch, which the host takes for the launch and the events.)
 //   * training: sort + featurize of the next batch on a side stream beside this one's networks; each update waits for
 //     everything of its own batch.
 #pragma once
@@ -37,6 +42,45 @@ __global__ void __launch_bounds__(256) interleave3_kernel(const T* __restrict__ 
     if (i >= 3 * n) return;
     const int atom = i / 3, axis = i - 3 * atom;
     out[i] = (axis == 0 ? x : (axis == 1 ? y : z))[atom];
+}
+
+// The arrays of the four networks, one after another.
+constexpr int kWeightArrays = 8 * kTypes;       // w1, b1, ... w4, b4 of every element
+constexpr int weight_array_length(int k)
+{
+    return k == 0 ? kMlpIn * kMlpH1 : (k == 2 ? kMlpH1 * kMlpH2 : (k == 4 ? kMlpH2 * kMlpH3 : (k == 1 || k == 3 ? kMlpH1 :
+           (k == 7 ? 1 : kMlpH3))));
+}
+constexpr int weight_array_start(int i)         // in values; every array starts on 16 bytes
+{
+    int at = 0;
+    for (int j = 0; j < i; j++) at += (weight_array_length(j % 8) + 3) / 4 * 4;
+    return at;
+}
+template <typename T> struct WeightCopyParams {
+    const T* from[kWeightArrays];
+    int length[kWeightArrays];       // 0 where there is none
+    T* to[kWeightArrays];
+};
+// kCopyCtas CTAs for each array, and in float behind them one for each packed chunk.
+constexpr int kCopyCtas = 6;
+template <typename T>
+__global__ void __launch_bounds__(kMlpThreads) copy_weights_kernel(const WeightCopyParams<T> p, const MlpPackParams pack)
+{
+    if ((int)blockIdx.x >= kCopyCtas * kWeightArrays) {
+        const int c = (int)blockIdx.x - kCopyCtas * kWeightArrays;
+        pack_chunk(pack, c % kPackChunks, c / kPackChunks);
+        return;
+    }
+    const int i = blockIdx.x / kCopyCtas;
+    const T* from = p.from[i];
+    T* to = p.to[i];
+    for (int k = (blockIdx.x % kCopyCtas) * kMlpThreads + threadIdx.x; k < p.length[i]; k += kCopyCtas * kMlpThreads) to[k] = from[k];
+}
+constexpr size_t weights_bytes(bool f64)        // of a copy; in float with the packed form behind it
+{
+    const size_t values = (size_t)weight_array_start(kWeightArrays) * (f64 ? 8 : 4);
+    return (values + 255) / 256 * 256 + (f64 ? 0 : (size_t)kTypes * kPackChunks * kPackedChunkBytes);
 }
 
 class Driver {
@@ -109,12 +153,14 @@ class Driver {
             ani_energy_args_f64 p = *a_.pass64[which];
             describe(p, b);
             p.phases = phases & ~(ANI_PASS_PACK | ANI_PASS_TRANSIENT);
+            own_weights(p);
             if (void* out = energies(sizeof(double))) p.mol_energy = static_cast<double*>(out);
             return ani_energy_pass_f64(&p, stream);
         }
         ani_pass_args p = *a_.pass[which];
         describe(p, b);
         p.phases = phases;
+        own_weights(p);
         if (void* out = energies(sizeof(float))) p.mol_energy = static_cast<float*>(out);
         if (a_.mode == ANI_DRIVER_TRAIN) {
             p.labels = static_cast<const float*>(slots_[b.slot].labels);
@@ -128,22 +174,14 @@ class Driver {
         const int which = (int)(index_ & 1), r = (int)(index_ % kRing);
         cudaStream_t stream = streams_[which];
         int rc = ANI_OK;
-        if (index_ == 0) {     // the weights do not change during the pass: packed once
-            if (!a_.pass64[0]) {
-                ani_pass_args p = *a_.pass[0];
-                const int none[4] = {0, 0, 0, 0};
-                p.n_atoms = p.n_mols = 0;
-                p.acs_host = none;
-                p.phases = ANI_PASS_PACK;
-                if ((rc = ani_network_pass_f32(&p, main))) return rc;
-            }
-            if (cudaEventRecord(main_done_, main) != cudaSuccess) return ANI_ERR_CUDA;
-        }
+        const bool forces = a_.mode == ANI_DRIVER_GRADIENTS;
+        // energies: nobody else has a turn during the pass, so the weights are packed once
+        if (index_ == 0 && !forces && (rc = weights(main))) return rc;
         const int more = feeder.next(out);
         if (more <= 0) return more;
-        if (index_ < 2 && cudaStreamWaitEvent(stream, main_done_, 0) != cudaSuccess) return ANI_ERR_CUDA;
+        if (forces && (rc = weights(main))) return rc;
+        if ((forces || index_ < 2) && cudaStreamWaitEvent(stream, main_done_, 0) != cudaSuccess) return ANI_ERR_CUDA;
         if ((rc = feeder.wait(out->slot, stream))) return rc;
-        const bool forces = a_.mode == ANI_DRIVER_GRADIENTS;
         if ((rc = pass(which, *out, ANI_PASS_FEATURIZE | ANI_PASS_FORWARD | ANI_PASS_ENERGY | ANI_PASS_TRANSIENT |
                                         (forces ? ANI_PASS_BACKWARD | ANI_PASS_COORD_GRAD : 0), stream)))
             return rc;
@@ -154,6 +192,24 @@ class Driver {
                                  : rows_to_host(*a_.pass[which], out->n_atoms, static_cast<float*>(a_.ring_host[r]), stream);
         if (e == cudaSuccess) e = cudaEventRecord(ring_done_[r], stream);
         return e == cudaSuccess ? 1 : ANI_ERR_CUDA;
+    }
+    // The weights as the work on `main` so far leaves them, in the batch's copy if it has one, packed; what comes after
+    // main_done_ may read them.
+    int weights(cudaStream_t main)
+    {
+        if (a_.mode == ANI_DRIVER_GRADIENTS) {
+            // the batch that had this copy before has ended: the caller has read its results
+            const cudaError_t e = a_.pass64[0] ? copy_weights<double>(*a_.pass64[0], main) : copy_weights<float>(*a_.pass[0], main);
+            if (e != cudaSuccess) return ANI_ERR_CUDA;
+        } else if (!a_.pass64[0]) {
+            ani_pass_args p = *a_.pass[0];
+            const int none[4] = {0, 0, 0, 0};
+            p.n_atoms = p.n_mols = 0;
+            p.acs_host = none;
+            p.phases = ANI_PASS_PACK;
+            if (int rc = ani_network_pass_f32(&p, main)) return rc;
+        }
+        return cudaEventRecord(main_done_, main) == cudaSuccess ? ANI_OK : ANI_ERR_CUDA;
     }
     int train_step(Feeder& feeder, cudaStream_t main, ani_feeder_batch* out)
     {
@@ -210,6 +266,46 @@ class Driver {
                 return rc;
         if (!a_.update) return ANI_OK;
         return ani_nadam_step_f32(a_.params, a_.grads, a_.m, a_.v, a_.ema, a_.n_params, a_.hyper, a_.state, main);
+    }
+    template <typename T, typename P> cudaError_t copy_weights(const P& p, cudaStream_t stream)
+    {
+        WeightCopyParams<T> c = {};
+        const T* const* arrays[8] = {p.w1, p.b1, p.w2, p.b2, p.w3, p.b3, p.w4, p.b4};
+        for (int i = 0; i < kWeightArrays; i++) {
+            c.from[i] = arrays[i % 8][i / 8];
+            c.length[i] = c.from[i] ? weight_array_length(i % 8) : 0;
+            c.to[i] = static_cast<T*>(a_.weights[index_ % kRing]) + weight_array_start(i);
+        }
+        MlpPackParams pack = {};
+        if constexpr (sizeof(T) == 4) {
+            P own = p;
+            own_weights(own);
+            for (int t = 0; t < kTypes; t++) {
+                pack.w1[t] = p.w1[t]; pack.w2[t] = p.w2[t]; pack.w3[t] = p.w3[t];
+                pack.packed[t] = p.w1[t] && p.w2[t] && p.w3[t] ? static_cast<unsigned char*>(own.packed[t]) : nullptr;
+            }
+        }
+        const int grid = kCopyCtas * kWeightArrays + (sizeof(T) == 4 ? kPackChunks * kTypes : 0);
+        copy_weights_kernel<T><<<grid, kMlpThreads, 0, stream>>>(c, pack);
+        return cudaGetLastError();
+    }
+    // Points the pass at the batch's copy of the weights, if it has one.
+    template <typename P> void own_weights(P& p)
+    {
+        if (a_.mode != ANI_DRIVER_GRADIENTS) return;
+        using Real = std::remove_const_t<std::remove_pointer_t<decltype(p.xs)>>;
+        char* copy = static_cast<char*>(a_.weights[index_ % kRing]);
+        const Real* values = reinterpret_cast<const Real*>(copy);
+        const Real** arrays[8] = {p.w1, p.b1, p.w2, p.b2, p.w3, p.b3, p.w4, p.b4};
+        for (int t = 0; t < kTypes; t++)
+            for (int k = 0; k < 8; k++)
+                if (arrays[k][t]) arrays[k][t] = values + weight_array_start(8 * t + k);
+        if constexpr (sizeof(Real) == 4) {
+            constexpr size_t kPacked = (size_t)kPackChunks * kPackedChunkBytes;
+            char* packed = copy + weights_bytes(false) - kTypes * kPacked;
+            for (int t = 0; t < kTypes; t++)
+                if (p.packed[t]) p.packed[t] = packed + t * kPacked;
+        }
     }
     template <typename P, typename T> cudaError_t rows_to_host(const P& p, int n, T* to, cudaStream_t stream)
     {

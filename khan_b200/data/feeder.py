@@ -389,11 +389,12 @@ def _driver_slots(ring):
 class BatchDriver:
     """One pass of a feeder with the work on every batch in native code (``ani_driver_step``): energies, gradients
     or training updates.  ``blocks``: the argument blocks of the two sets of buffers used in turn; ``streams``: one for
-    training, two otherwise; ``fields``: what else ``ani_driver_args`` needs."""
+    training, two otherwise; ``ring``: pinned buffers for results, ``weights``: device buffers for the copies that a
+    pass for gradients makes of the weights; ``fields``: what else ``ani_driver_args`` needs."""
 
-    def __init__(self, feeder: "BatchFeeder", mode: int, blocks, streams, ring=(), keep=(), **fields):
+    def __init__(self, feeder: "BatchFeeder", mode: int, blocks, streams, ring=(), weights=(), keep=(), **fields):
         self.feeder, self.batch = feeder, _lib.FeederBatch()
-        self._keep = (blocks, streams, ring, keep)
+        self._keep = (blocks, streams, ring, weights, keep)
         a = self._args = _lib.DriverArgs()
         slots = feeder.native["driver_slots"]
         a.mode, a.slots, a.n_slots = mode, slots, len(slots)
@@ -403,11 +404,18 @@ class BatchDriver:
             (a.pass64 if isinstance(block, _lib.EnergyArgs64) else a.pass_)[k] = ctypes.pointer(block)
         for k, buf in enumerate(ring):
             a.ring_host[k] = buf.data_ptr()
+        for k, buf in enumerate(weights):
+            a.weights[k] = buf.data_ptr()
         for name, value in fields.items():
             setattr(a, name, value)
         self._ptr = ctypes.c_void_p()
         _lib.check(_lib.lib().ani_driver_create(ctypes.byref(a), ctypes.byref(self._ptr)), "ani_driver_create")
         feeder.begin()
+
+    def refresh(self, blocks) -> None:
+        """Other argument blocks for the batches from the next one on (the weights have moved)."""
+        for mine, block in zip(self._keep[0], blocks):
+            ctypes.memmove(ctypes.addressof(mine), ctypes.addressof(block), ctypes.sizeof(mine))
 
     def step(self) -> bool:
         """Enqueues the work on the next batch on the current stream; False when the pass is over.  Afterwards

@@ -59,12 +59,15 @@ class EnergyForces:
                 a.packed[t] = packed[t].data_ptr()
         return a
 
+    def weights_place(self):
+        """Changes when the model's weights have moved."""
+        packed = None if self.f64 else self.model.packed_weights()
+        return self.model.anns[0].Ws[0].data_ptr(), None if packed is None else packed.data_ptr()
+
     def _pass_args(self, sb: StagedBatch):
         """The argument block of the pass: everything that does not change from batch to batch is filled once
         (and again when the model's weights have moved), the batch's own fields per call."""
-        first = self.model.anns[0].Ws[0]
-        packed = None if self.f64 else self.model.packed_weights()
-        key = (first.data_ptr(), None if packed is None else packed.data_ptr())
+        packed, key = None if self.f64 else self.model.packed_weights(), self.weights_place()
         if getattr(self, "_pa_key", None) != key:
             self._pa, self._pa_key = self._fixed_args(packed), key
         a = self._pa
@@ -134,7 +137,7 @@ class PassTools:
         self.staged = [StagedBatch(cap_atoms, cap_mols, model.precision, device=device) for _ in range(2)]
         self.evaluators = [EnergyForces(model, cap_atoms, cap_mols, device=device) for _ in range(2)]
         self.streams = [torch.cuda.Stream(device=device) for _ in range(2)]
-        self.ring = []
+        self.ring, self.weights = [], []
 
     def fits(self, cap_atoms: int, cap_mols: int) -> bool:
         return self.staged[0].n_atoms_cap >= cap_atoms and self.staged[0].n_mols_cap >= cap_mols
@@ -146,6 +149,13 @@ class PassTools:
         if size and (not self.ring or self.ring[0].numel() < size):
             self.ring = [torch.empty(size, dtype=self.staged[0].dtype).pin_memory() for _ in range(_lib.DRIVER_RING)]
         return self.ring if size else []
+
+    def weight_copies(self):
+        if not self.weights:
+            size = _lib.lib().ani_driver_weights_bytes(int(self.evaluators[0].f64))
+            self.weights = [torch.empty(size, dtype=torch.uint8, device=self.evaluators[0].device)
+                            for _ in range(_lib.DRIVER_RING)]
+        return self.weights
 
 
 class SingleGeometry:

@@ -633,7 +633,10 @@ class TrainerMultiTower:
         """Per-molecule ``(n, 3)`` gradients of the predicted energy
         (``trainer_multi_tower.py:580-614``).  On one tower with the networks that have kernels the
         batches go through the allocation-free evaluator (``khan_b200.inference.EnergyForces``: C-ABI
-        calls only, no host wait per batch); ``use_evaluator=False`` forces the autograd path."""
+        calls only, no host wait per batch); ``use_evaluator=False`` forces the autograd path.
+
+        The iterator runs up to two batches ahead of its consumer.  It is in order with the stream that is current
+        when it is advanced: weights changed between two items are those of all batches enqueued afterwards."""
         # an iterator, as in the reference; the per-batch lists are chained in C, so a molecule costs no
         # Python frame of its own (two nested generators had cost more than cutting the arrays)
         if use_evaluator and self._evaluator_usable(dataset):
@@ -675,9 +678,14 @@ class TrainerMultiTower:
         driver = None
         try:
             with torch.cuda.device(dev):
-                driver = BatchDriver(it, mode, tools.blocks(), tools.streams, tools.host_ring(host_size), keep=tools, **fields)
+                driver = BatchDriver(it, mode, tools.blocks(), tools.streams, tools.host_ring(host_size),
+                                     tools.weight_copies() if mode == _lib.DRIVER_GRADIENTS else (), keep=tools, **fields)
+            place = tools.evaluators[0].weights_place()
             while True:
                 with torch.cuda.device(dev):
+                    if place != tools.evaluators[0].weights_place():
+                        driver.refresh(tools.blocks())
+                        place = tools.evaluators[0].weights_place()
                     more = driver.step()
                 if not more:
                     break

@@ -480,3 +480,38 @@ def test_passes_over_a_data_set_may_interleave_and_be_given_up():
     got = list(second)
     assert len(got) == 150 and all(np.array_equal(a, b) for a, b in zip(got, want_g))
     assert tr.predict(ds, batch_size=64) == pytest.approx(want_e, rel=1e-5, abs=1e-5)
+
+
+@pytest.mark.parametrize("change", ["copy", "train", "move"])
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+def test_weights_may_change_between_two_molecules_of_a_pass(precision, change):
+    """coordinate_gradients is an iterator: what its consumer enqueues between two items is ordered with its batches.
+    The batches enqueued by then (as many as the ring has places) have the old weights, all later ones the new."""
+    import torch
+    from khan_b200 import RawDataset, TrainerMultiTower, _lib
+    size = 1024 if precision == "float32" else 256
+    ds = RawDataset(syn.gdb_like_batch(7 * size + 5, seed=5).molecules())
+    small = syn.gdb_like_batch(64, seed=6).molecules()
+    train = RawDataset(small, list(np.linspace(-1.0, 1.0, len(small))))
+    tr = TrainerMultiTower(None, [torch.device("cuda", 0)], precision=getattr(torch, precision),
+                           layer_sizes=(128, 128, 64, 1), seed=3)
+    tr.set_learning_rate(1e-4)
+    for _ in range(3):
+        old = list(tr.coordinate_gradients(ds, batch_size=size))
+        passing = tr.coordinate_gradients(ds, batch_size=size)
+        got = [next(passing)]
+        if change == "copy":
+            with torch.no_grad():
+                for w in tr.parameters:
+                    w.mul_(1.25)
+        elif change == "move":
+            for w in tr.parameters:
+                w.data = w.data * 1.25
+        else:
+            list(tr.feed_dataset(train, True, [tr.train_op], 64))
+        got += passing
+        new = list(tr.coordinate_gradients(ds, batch_size=size))
+        cut = _lib.DRIVER_RING * size
+        assert not np.array_equal(old[0], new[0]) and len(got) == len(old)
+        assert all(np.array_equal(a, b) for a, b in zip(got[:cut], old[:cut]))
+        assert all(np.array_equal(a, b) for a, b in zip(got[cut:], new[cut:]))
