@@ -35,10 +35,8 @@ class EnergyForces:
         real = dict(dtype=self.dtype, device=self.device)
         self.energy_sorted = torch.empty(n_atoms, **real)
         self.mol_energy = torch.zeros(n_mols, **real)
-        if not self.f64:      # what the tensor-core kernels hand from one to the next
+        if not self.f64:
             self.ones = torch.ones(n_atoms, **real)
-            self.dacts = [torch.empty((n_atoms, w), **real) for w in (128, 128, 64)]
-            self.dzs = [torch.empty((n_atoms, w), **real) for w in (128, 128, 64)]
         self.n_atoms_cap, self.n_mols_cap = n_atoms, n_mols
 
     def _fixed_args(self, packed):
@@ -49,9 +47,6 @@ class EnergyForces:
         if not self.f64:
             a.split_precision = int(self.split)
             a.grad_energy_sorted = self.ones.data_ptr()
-            for name, bufs in (("dact", self.dacts), ("dz", self.dzs)):
-                for k, t in enumerate(bufs):
-                    setattr(a, f"{name}{k + 1}", t.data_ptr())
         for t, ann in enumerate(self.model.anns):
             for k, (w, b) in enumerate(zip(ann.Ws, ann.bs)):
                 getattr(a, f"w{k + 1}")[t], getattr(a, f"b{k + 1}")[t] = w.data_ptr(), b.data_ptr()

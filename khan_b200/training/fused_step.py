@@ -115,13 +115,6 @@ class FusedTrainStep:
         sb.run_sort(stream)
         sb.run_featurize(stream)
 
-    def featurize_pass(self, sb: StagedBatch) -> None:
-        """The same as ``featurize`` through the one-call entry point (one argument block, one call)."""
-        self._check(sb)
-        a = self._pass_args(sb)
-        a.phases = _lib.PASS_FEATURIZE
-        _lib.check(_lib.lib().ani_network_pass_f32(ctypes.byref(a), self._stream()), "ani_network_pass_f32")
-
     def networks(self, sb: StagedBatch, labels: torch.Tensor, feature_grad: bool = True) -> None:
         """Weight packing, networks forward, molecule energies + MSE gradient, networks backward.
         Afterwards ``self.l2s[:n_mols]`` holds the squared errors, the dz buffers the layer

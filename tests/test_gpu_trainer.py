@@ -515,3 +515,14 @@ def test_weights_may_change_between_two_molecules_of_a_pass(precision, change):
         assert not np.array_equal(old[0], new[0]) and len(got) == len(old)
         assert all(np.array_equal(a, b) for a, b in zip(got[:cut], old[:cut]))
         assert all(np.array_equal(a, b) for a, b in zip(got[cut:], new[cut:]))
+
+
+def test_an_evaluator_holds_no_activations():
+    """Energies and forces keep what lies between the layers on the chip: per atom an energy and a seed, no more."""
+    import torch
+    from khan_b200.inference import EnergyForces
+    from khan_b200.model.nn import MoleculeNN
+    model = MoleculeNN(device="cuda:0", seed=3)
+    before = torch.cuda.memory_allocated()
+    ev = EnergyForces(model, 100000, 4000, device="cuda:0")
+    assert torch.cuda.memory_allocated() - before <= 100000 * 2 * 4 + 4000 * 4 + 4096 and ev.n_atoms_cap == 100000
