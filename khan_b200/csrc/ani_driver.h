@@ -219,24 +219,21 @@ class Driver {
         if (!started_) {
             started_ = true;
             have_ = feeder.next(&now_);
-            if (have_ > 0) rc = featurize(feeder, now_, 0);
-            if (have_ < 0 || rc) return rc ? rc : have_;
+            if (have_ > 0 && (rc = featurize(feeder, now_, 0))) return rc;
         }
-        if (!have_) return 0;
+        if (have_ <= 0) return have_;        // the pass is over, or failed behind the batch of the step before
         if (cudaStreamWaitEvent(main, side_done_, 0) != cudaSuccess) return ANI_ERR_CUDA;      // this batch's features
         // The next batch's features first, so that they run beside this one's networks; but the GPU does not wait
         // for a batch that is still being packed.
         ani_feeder_batch next;
         const int which = (int)(index_ & 1);
         int more = feeder.next(&next, false);
-        if (more > 0 && more != Feeder::kNotYet) rc = featurize(feeder, next, 1 - which);
-        if (more < 0 || rc) return rc ? rc : more;
+        if (more > 0 && more != Feeder::kNotYet && (rc = featurize(feeder, next, 1 - which))) return rc;
         if ((rc = update(now_, which, main))) return rc;
         if ((rc = feeder.release(now_.slot, main))) return rc;
         if (more == Feeder::kNotYet) {
             more = feeder.next(&next);
-            if (more > 0) rc = featurize(feeder, next, 1 - which);
-            if (more < 0 || rc) return rc ? rc : more;
+            if (more > 0 && (rc = featurize(feeder, next, 1 - which))) return rc;
         }
         *out = now_;
         now_ = next;
@@ -319,7 +316,7 @@ class Driver {
     cudaEvent_t side_done_ = nullptr, main_done_ = nullptr, ring_done_[kRing] = {};
     ani_feeder_batch now_{};
     bool started_ = false;
-    int have_ = 0;
+    int have_ = 0;             // of now_: what feeder.next() said
     long long index_ = 0, molecules_ = 0;
 };
 

@@ -526,3 +526,24 @@ def test_an_evaluator_holds_no_activations():
     before = torch.cuda.memory_allocated()
     ev = EnergyForces(model, 100000, 4000, device="cuda:0")
     assert torch.cuda.memory_allocated() - before <= 100000 * 2 * 4 + 4000 * 4 + 4096 and ev.n_atoms_cap == 100000
+
+
+def test_training_stops_behind_the_last_good_batch():
+    """A molecule with a negative size in batch 5: the batches before it are trained on, then the pass raises -- however
+    far the thread that prepares the batches is ahead."""
+    import torch
+    from khan_b200 import RawDataset, TrainerMultiTower, _lib
+    from khan_b200.data.feeder import PackedDataset
+    mols = syn.gdb_like_batch(400, seed=5).molecules()
+    tr = TrainerMultiTower(None, [torch.device("cuda", 0)], layer_sizes=(128, 128, 64, 1), seed=3)
+    tr.set_learning_rate(1e-6)
+    ds = RawDataset(mols, list(np.zeros(len(mols))))
+    packed = PackedDataset.from_raw(ds)
+    packed.capacity(40)                                   # before the table is damaged
+    packed.ptr[206] = packed.ptr[205] - 1
+    for _ in range(40):
+        before, rows = tr.global_step, 0
+        with pytest.raises(_lib.AniError):
+            for _ in tr.feed_dataset(ds, False, [tr.train_op], 40):
+                rows += 1
+        assert rows == 5 and tr.global_step == before + 5
