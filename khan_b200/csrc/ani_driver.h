@@ -183,8 +183,10 @@ class Driver {
         if ((forces || index_ < 2) && cudaStreamWaitEvent(stream, main_done_, 0) != cudaSuccess) return ANI_ERR_CUDA;
         if ((rc = feeder.wait(out->slot, stream))) return rc;
         if ((rc = pass(which, *out, ANI_PASS_FEATURIZE | ANI_PASS_FORWARD | ANI_PASS_ENERGY | ANI_PASS_TRANSIENT |
-                                        (forces ? ANI_PASS_BACKWARD | ANI_PASS_COORD_GRAD : 0), stream)))
+                                        (forces ? ANI_PASS_BACKWARD | ANI_PASS_COORD_GRAD : 0), stream))) {
+            feeder.used(out->slot, stream);
             return rc;
+        }
         if ((rc = feeder.release(out->slot, stream))) return rc;
         cudaError_t e = cudaSuccess;
         if (forces && out->n_atoms > 0)
@@ -245,7 +247,9 @@ class Driver {
         cudaStream_t side = streams_[0];
         if (cudaStreamWaitEvent(side, main_done_, 0) != cudaSuccess) return ANI_ERR_CUDA;
         if (int rc = feeder.wait(b.slot, side)) return rc;
-        if (int rc = pass(which, b, ANI_PASS_FEATURIZE, side)) return rc;
+        const int rc = pass(which, b, ANI_PASS_FEATURIZE, side);
+        const int used = feeder.used(b.slot, side);
+        if (rc || used) return rc ? rc : used;
         return cudaEventRecord(side_done_, side) == cudaSuccess ? ANI_OK : ANI_ERR_CUDA;
     }
     int update(const ani_feeder_batch& b, int which, cudaStream_t main)

@@ -158,6 +158,17 @@ public:
         return cudaStreamWaitEvent(stream, slots_[slot].uploaded, 0) == cudaSuccess ? ANI_OK : ANI_ERR_CUDA;
     }
 
+    // Work that reads the slot's device arena has been enqueued on `stream`, and the consumer keeps the slot.  Should the
+    // pass end before the slot is handed back, the next pass's copy into the arena waits for that work.
+    int used(int slot, cudaStream_t stream)
+    {
+        if (slot < 0 || slot >= (int)slots_.size()) return ANI_ERR_BAD_INDEX;
+        if (device_ < 0) return ANI_OK;
+        if (cudaEventRecord(slots_[slot].consumed, stream) != cudaSuccess) return ANI_ERR_CUDA;
+        slots_[slot].has_consumed = true;
+        return ANI_OK;
+    }
+
     // Hands the slot back: the next copy into its device arena is ordered behind the work enqueued on
     // `stream` so far.
     int release(int slot, cudaStream_t stream)

@@ -428,29 +428,34 @@ class TrainerMultiTower:
                 optimizer.step()
                 return fed.n_mols, fed.index
 
-        for _ in range(it.packed.num_batches(it.batch_size)):
-            if hooks:
-                self._run_hooks(hooks)
-            with torch.cuda.device(dev), torch.no_grad():
-                done = advance()
-                if done is None:
-                    return
-                n_mols, index = done
-                self.global_step += 1
-                row = []
-                for n in names:
-                    if n.startswith("train_op"):
-                        row.append(None)
-                    elif n in ("unordered_l2s", "tower_l2s"):
-                        row.append([step.l2s[:n_mols].cpu().numpy()])
-                    elif n == "_device_l2s":
-                        row.append([step.l2s[:n_mols].clone()])
-                    elif n == "tower_exp_loss":
-                        rmse = self._rmse_buf if loss_kind else step.l2s[:n_mols].mean().sqrt().clamp_min(1e-30)
-                        row.append([float(torch.exp(rmse.double()))])
-                    elif n == "tower_bids":
-                        row.append([np.array(index)])
-            yield row
+        try:
+            for _ in range(it.packed.num_batches(it.batch_size)):
+                if hooks:
+                    self._run_hooks(hooks)
+                with torch.cuda.device(dev), torch.no_grad():
+                    done = advance()
+                    if done is None:
+                        return
+                    n_mols, index = done
+                    self.global_step += 1
+                    row = []
+                    for n in names:
+                        if n.startswith("train_op"):
+                            row.append(None)
+                        elif n in ("unordered_l2s", "tower_l2s"):
+                            row.append([step.l2s[:n_mols].cpu().numpy()])
+                        elif n == "_device_l2s":
+                            row.append([step.l2s[:n_mols].clone()])
+                        elif n == "tower_exp_loss":
+                            rmse = self._rmse_buf if loss_kind else step.l2s[:n_mols].mean().sqrt().clamp_min(1e-30)
+                            row.append([float(torch.exp(rmse.double()))])
+                        elif n == "tower_bids":
+                            row.append([np.array(index)])
+                yield row
+        finally:
+            if it.native is not None:      # given up or failed: the features of the next batch may still be on their way
+                with torch.cuda.device(dev):
+                    driver.join()
 
     def _force_rounds(self, it, names, capacity, before_hooks):
         """Force training on one device without autograd (``ForceFitStep``)."""

@@ -547,3 +547,34 @@ def test_training_stops_behind_the_last_good_batch():
             for _ in tr.feed_dataset(ds, False, [tr.train_op], 40):
                 rows += 1
         assert rows == 5 and tr.global_step == before + 5
+
+
+def test_a_training_pass_given_up_keeps_its_arena_until_it_has_been_read():
+    """The features of the next batch are computed ahead.  When the pass is given up there, the next pass takes over the
+    ring: its uploads must not reach the arena that those features still have to be computed from."""
+    import torch
+    from khan_b200 import RawDataset, TrainerMultiTower
+    mols = syn.config4(seed=3, n_mols=20, n_min=12, n_max=12).molecules()      # equal sizes: the passes share a ring
+    other = [m * np.array([1.0, 0.7, 0.7, 0.7]) for m in mols]
+    tr = TrainerMultiTower(None, [torch.device("cuda", 0)], layer_sizes=(128, 128, 64, 1), seed=3)
+    data = RawDataset(mols, list(np.zeros(len(mols))))
+    for _ in tr.feed_dataset(data, False, [tr.train_op], 4):                    # buffers exist from here on
+        pass
+    tr.predict(RawDataset(other), batch_size=4)
+    torch.cuda.synchronize()
+
+    def given_up(behind):
+        steps = tr.feed_dataset(data, False, [tr.train_op], 4, before_hooks=behind)
+        for _ in range(4):                                                     # the arena of the fifth batch is the first
+            next(steps)
+        steps.close()
+        if behind is None:
+            torch.cuda.synchronize()
+        energies = tr.predict(RawDataset(other), batch_size=4)
+        torch.cuda.synchronize()
+        return tr._fused[1][0].features[:48].cpu().numpy(), energies            # the fifth batch, in the first buffers
+
+    want, energies = given_up(None)
+    got, again = given_up(lambda: torch.cuda._sleep(100_000_000))              # 50 ms: nothing of a step starts before
+    assert np.array_equal(got, want)
+    assert np.isfinite(energies).all() and np.isfinite(again).all()
