@@ -326,7 +326,7 @@ class _NativeHandle:
                    "ani_feeder_create")
 
     def __del__(self):
-        if self.ptr:
+        if self.ptr and _lib is not None:      # None: the interpreter is going down, and with it the process
             _lib.lib().ani_feeder_destroy(self.ptr)
             self.ptr = ctypes.c_void_p()
 
@@ -435,7 +435,7 @@ class BatchDriver:
         _lib.check(_lib.lib().ani_driver_wait(self._ptr, place), "ani_driver_wait")
 
     def __del__(self):
-        if getattr(self, "_ptr", None):
+        if getattr(self, "_ptr", None) and _lib is not None:
             _lib.lib().ani_driver_destroy(self._ptr)
             self._ptr = ctypes.c_void_p()
 

@@ -259,3 +259,15 @@ def test_a_negative_molecule_size_in_a_perturbed_pass_is_an_error():
         "    print('raised behind', got)\n")
     done = subprocess.run([sys.executable, "-c", program], cwd=ROOT, capture_output=True, text=True, timeout=120)
     assert done.returncode == 0 and "raised behind [0]" in done.stdout, done.stderr[-500:]
+
+
+def test_a_kept_feeder_goes_quietly_with_the_interpreter(monkeypatch):
+    """The rings of finished passes live as long as the module, whose imports may go first at exit."""
+    from khan_b200.data import feeder as module
+    ds = _dataset(9, with_grads=False)
+    feeder = BatchFeeder(PackedDataset.from_raw(ds), 4, False)
+    assert len(list(feeder)) == 3
+    with monkeypatch.context() as m:
+        m.setattr(module, "_lib", None)
+        feeder.native["owner"].__del__()
+    assert len(list(BatchFeeder(PackedDataset.from_raw(ds), 4, False))) == 3
