@@ -12,8 +12,10 @@
 // distributed shared memory, one cluster barrier per layer.  Inside a CTA a product is 2 x 2 register tiles
 // over four or eight slices of K, summed through shared memory.
 //
-// Double precision has no other kernel: there the tiles simply queue up (16 atoms of f64 cost
-// 2 x 16 x 81 k multiply-adds, 0.3 us of the device's FP64 rate).
+// Double precision has no other kernel: there the tiles simply queue up, each fetching the weights of its element from
+// L2 again.  Measured, forward / with backward: 891 atoms 40 / 68 us, 3.6 k 137 / 244, 14 k 516 / 939, 28 k 1034 / 1879:
+// 37 / 67 ns an atom, 4.4 TFLOP/s, an eighth of the FP64 rate.  (Before it, dense products: coordinate gradients of a data
+// set of 8,192 molecules 33.6 ms, 8.6 with it; energies 5.5 and 4.8.)
 #pragma once
 
 #include "ani_common.cuh"

@@ -302,7 +302,7 @@ def test_gradient_vs_oracle(gpu, oracle_mod, case, dt):
 @pytest.mark.parametrize("n_mols", [140, 310, 600, 1100])
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 def test_small_molecules_at_every_split(gpu, oracle_mod, n_mols, dt):
-    """Central atoms per warp (features), warps per molecule and size classes (gradient) depend on the batch size."""
+    """Central atoms per warp (features), warps per molecule and the order of the molecules (gradient) depend on the batch size."""
     b = _concat(syn.gdb_like_batch(n_mols, 21), CASES["large_among_small"](), CASES["dense_small"]())
     si, gi, ac = oracle_mod.ani_sort(b.atomic_numbers)
     up = syn.upstream_grads(b, ac, dtype=dt)
