@@ -242,11 +242,12 @@ int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, cons
     if (small_molecules(n_atoms, n_mols) && all_aligned16({oh, oc, on, oo}) &&
         (long long)n_mols * kMolMaxAtoms <= 0x7fffffffLL) {
         // As few central atoms per warp as still find all warps resident at once (28 per SM in float, 20 in double): with
-        // four, the scans and triplets of one warp are a chain of 12 us (float; double 22 us), however small the batch.
+        // four, the scans and triplets of one warp are a chain of 12 us (float; double 25 us), however small the batch.
         // Few atoms per warp cost more instructions (load, sort and table per round), so not beyond that.  Microseconds
-        // with 4 / 2 / 1 atoms in float, 64 molecules 13.6 / 10.3 / 8.3, 256: 16.5 / 13.3 / 13.2, 512: 19.8 / 17.4 / 20.5,
-        // 1024: 24.9 / 26.5 / 39.0; in double, 64: 25 / 18 / 15, 512: 39 / 41 / 47.  (32 float warps are resident, but with
-        // that line 1024 molecules take three atoms per warp: 27.3 instead of 25.2, and 1.5 more a batch with eight streams.)
+        // with 4 / 2 / 1 atoms in float, 64 molecules 12.9 / 9.8 / 8.3, 256: 16.0 / 12.8 / 12.0, 512: 18.7 / 16.0 / 18.9,
+        // 1024: 24.0 / 25.3 / 31.1, 8192: 118 / 153 / 238; in double, 64: 26 / 19 / 17, 256: 34 / 27 / 31, 512: 39 / 41 /
+        // 49, 1024: 60 / 64 / 84.  (32 float warps are resident, but with that line 1024 molecules take three atoms per
+        // warp: 27.3 us when four took 25.2, and 1.5 more a batch with eight streams.)
         const int resident = kSms * (sizeof(T) == 4 ? 28 : 20);
         const int per_round = (int)std::min<long long>((n_atoms + resident - 1) / resident, kMolCentrals);
         const int rounds = (kMolMaxAtoms + per_round - 1) / per_round;
@@ -335,9 +336,10 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
                                   acs_host[2], acs_host[3], sums));
             return ANI_OK;
         };
-        // Eight warps a molecule shorten its chain of scans and pair passes (64 molecules 14.8 -> 10.6 us, 512: 27.4 ->
-        // 20.4, double 38 -> 25 and 68 -> 58), four keep more of the lanes and the SM busy once there are several
-        // molecules per SM (1024: 32.2 against 34.5, 8192: 159 against 222; double 78 against 107).
+        // Eight warps a molecule shorten its chain of scans and pair passes (64 molecules 19.0 -> 14.2 us, 512: 29.3 ->
+        // 19.8, double 47 -> 33 and 67 -> 51), four keep more of the lanes and the SM busy once there are several
+        // molecules per SM (2048: 49 against 58, 8192: 156 against 219; double, 888: 75 against 85, 1024: 81 against 97).
+        // In float 1024 molecules alone would take 31 us with eight and 35 with four, but more instructions.
         if (n_mols <= kSms * (sizeof(T) == 4 ? 6 : 4)) return launch(std::integral_constant<int, 8>{});
         return launch(std::integral_constant<int, 4>{});
     }
