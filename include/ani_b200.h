@@ -616,8 +616,8 @@ int ani_feeder_set_slots(ani_feeder* f, const ani_feeder_slot* slots, int n_slot
  * Training runs on `stream`, with the features of the next batch on streams[0]; the other two run batch b on
  * streams[b & 1], energies behind what `stream` held at the first step (the weights must not change during the pass),
  * gradients each batch behind what `stream` held at its own step, with the weights as they were then (copied to
- * weights[b % ANI_DRIVER_RING]): work enqueued between two steps may change them.  ani_driver_join makes `stream` wait
- * for all of it.
+ * weights[b % ANI_DRIVER_RING]): work enqueued between two steps may change them.  Without weights[] gradients are as
+ * energies.  ani_driver_join makes `stream` wait for all of it.
  * ring_host is pinned memory that the kernels write; ani_driver_wait(d, place) blocks until the results last
  * enqueued for a place are there, and the caller has waited for a place before the step that fills it again.
  * pass / pass64: the argument block of each of the two sets of buffers used in turn (pass64: double precision,
@@ -638,7 +638,6 @@ typedef struct ani_driver_args {
     void* streams[2];                /* training: the first only */
     void* energies;                  /* [all molecules] or NULL */
     void* ring_host[ANI_DRIVER_RING];
-    void* weights[ANI_DRIVER_RING];  /* gradients only: ani_driver_weights_bytes() each, 256-byte aligned */
     float *params, *grads, *m, *v, *ema;       /* training: ani_nadam_step_f32 (update != 0) */
     long long n_params;
     const float* hyper;
@@ -649,6 +648,7 @@ typedef struct ani_driver_args {
     int clip_n_rows;                 /* > 0: ani_clip_rows_f32 before the batch */
     const int *clip_row_offsets, *clip_row_lengths;
     float clip_max_norm;
+    void* weights[ANI_DRIVER_RING];  /* gradients: ani_driver_weights_bytes() each, 256-byte aligned, or all NULL */
 } ani_driver_args;
 typedef struct ani_driver ani_driver;
 size_t ani_driver_weights_bytes(int double_precision);

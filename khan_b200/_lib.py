@@ -130,12 +130,13 @@ class DriverArgs(ctypes.Structure):
     _fields_ = ([("mode", ctypes.c_int), ("n_slots", ctypes.c_int), ("slots", ctypes.POINTER(DriverSlot)),
                  ("pass_", ctypes.POINTER(PassArgs) * 2), ("pass64", ctypes.POINTER(EnergyArgs64) * 2),
                  ("streams", ctypes.c_void_p * 2), ("energies", ctypes.c_void_p),
-                 ("ring_host", ctypes.c_void_p * DRIVER_RING), ("weights", ctypes.c_void_p * DRIVER_RING)]
+                 ("ring_host", ctypes.c_void_p * DRIVER_RING)]
                 + [(n, ctypes.c_void_p) for n in ("params", "grads", "m", "v", "ema")]
                 + [("n_params", ctypes.c_longlong), ("hyper", ctypes.c_void_p), ("state", ctypes.c_void_p),
                    ("update", ctypes.c_int), ("loss_kind", ctypes.c_int), ("rmse", ctypes.c_void_p),
                    ("clip_n_rows", ctypes.c_int), ("clip_row_offsets", ctypes.c_void_p),
-                   ("clip_row_lengths", ctypes.c_void_p), ("clip_max_norm", ctypes.c_float)])
+                   ("clip_row_lengths", ctypes.c_void_p), ("clip_max_norm", ctypes.c_float),
+                   ("weights", ctypes.c_void_p * DRIVER_RING)])
 
 
 PASS_PACK, PASS_FEATURIZE, PASS_FORWARD, PASS_ENERGY, PASS_BACKWARD, PASS_WEIGHT_GRAD, PASS_COORD_GRAD, PASS_TRANSIENT = (

@@ -1180,7 +1180,7 @@ int ani_driver_create(const ani_driver_args* a, ani_driver** out)
             if (!p) return ANI_ERR_NULL_POINTER;
     if (a->mode == ANI_DRIVER_GRADIENTS)
         for (void* p : a->weights) {
-            if (!p) return ANI_ERR_NULL_POINTER;
+            if (!p != !a->weights[0]) return ANI_ERR_NULL_POINTER;
             if (reinterpret_cast<uintptr_t>(p) & 255) return ANI_ERR_MISALIGNED;
         }
     ani_driver* d = new (std::nothrow) ani_driver(*a);

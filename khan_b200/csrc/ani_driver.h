@@ -126,6 +126,8 @@ class Driver {
 
   private:
     static constexpr int kRing = ANI_DRIVER_RING;
+    // every batch has its own copy of the weights
+    bool copies() const { return a_.mode == ANI_DRIVER_GRADIENTS && a_.weights[0]; }
 
     // Where the energies of this batch go: an array of all molecules, the host ring, or (null) the pass's own array.
     void* energies(size_t size) const
@@ -175,12 +177,12 @@ class Driver {
         cudaStream_t stream = streams_[which];
         int rc = ANI_OK;
         const bool forces = a_.mode == ANI_DRIVER_GRADIENTS;
-        // energies: nobody else has a turn during the pass, so the weights are packed once
-        if (index_ == 0 && !forces && (rc = weights(main))) return rc;
+        // without copies nobody else may have a turn during the pass, and the weights are packed once
+        if (index_ == 0 && !copies() && (rc = weights(main))) return rc;
         const int more = feeder.next(out);
         if (more <= 0) return more;
-        if (forces && (rc = weights(main))) return rc;
-        if ((forces || index_ < 2) && cudaStreamWaitEvent(stream, main_done_, 0) != cudaSuccess) return ANI_ERR_CUDA;
+        if (copies() && (rc = weights(main))) return rc;
+        if ((copies() || index_ < 2) && cudaStreamWaitEvent(stream, main_done_, 0) != cudaSuccess) return ANI_ERR_CUDA;
         if ((rc = feeder.wait(out->slot, stream))) return rc;
         if ((rc = pass(which, *out, ANI_PASS_FEATURIZE | ANI_PASS_FORWARD | ANI_PASS_ENERGY | ANI_PASS_TRANSIENT |
                                         (forces ? ANI_PASS_BACKWARD | ANI_PASS_COORD_GRAD : 0), stream))) {
@@ -199,7 +201,7 @@ class Driver {
     // main_done_ may read them.
     int weights(cudaStream_t main)
     {
-        if (a_.mode == ANI_DRIVER_GRADIENTS) {
+        if (copies()) {
             // the batch that had this copy before has ended: the caller has read its results
             const cudaError_t e = a_.pass64[0] ? copy_weights<double>(*a_.pass64[0], main) : copy_weights<float>(*a_.pass[0], main);
             if (e != cudaSuccess) return ANI_ERR_CUDA;
@@ -293,7 +295,7 @@ class Driver {
     // Points the pass at the batch's copy of the weights, if it has one.
     template <typename P> void own_weights(P& p)
     {
-        if (a_.mode != ANI_DRIVER_GRADIENTS) return;
+        if (!copies()) return;
         using Real = std::remove_const_t<std::remove_pointer_t<decltype(p.xs)>>;
         char* copy = static_cast<char*>(a_.weights[index_ % kRing]);
         const Real* values = reinterpret_cast<const Real*>(copy);

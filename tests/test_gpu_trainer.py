@@ -578,3 +578,15 @@ def test_a_training_pass_given_up_keeps_its_arena_until_it_has_been_read():
     got, again = given_up(lambda: torch.cuda._sleep(100_000_000))              # 50 ms: nothing of a step starts before
     assert np.array_equal(got, want)
     assert np.isfinite(energies).all() and np.isfinite(again).all()
+
+
+def test_gradients_without_copies_of_the_weights(monkeypatch):
+    """``ani_driver_args.weights`` may be left out by a caller that does not change the weights during the pass."""
+    import torch
+    from khan_b200 import RawDataset, TrainerMultiTower
+    from khan_b200.inference import PassTools
+    ds = RawDataset(syn.gdb_like_batch(150, seed=5).molecules())
+    tr = TrainerMultiTower(None, [torch.device("cuda", 0)], layer_sizes=(128, 128, 64, 1), seed=3)
+    want = list(tr.coordinate_gradients(ds, batch_size=16))
+    monkeypatch.setattr(PassTools, "weight_copies", lambda self: ())
+    assert all(np.array_equal(a, b) for a, b in zip(tr.coordinate_gradients(ds, batch_size=16), want))
