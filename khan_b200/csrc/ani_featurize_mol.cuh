@@ -41,8 +41,8 @@
 //
 // What bounds it: instruction issue, with as many one-warp CTAs per SM as shared memory allows.  That is allotted in
 // steps of 1 KB (other kernels of the library align theirs to that): 6 KB + 1 KB reserved let 32 in, 7 + 1 let in 28.
-// A group table without gaps brought it from the one to the other: 1024 molecules 26.0 -> 25.2 us alone, 14.45 -> 14.2
-// a batch with eight in flight (a division less per warp among it).
+// From the one to the other 1024 molecules went from 26.0 to 25.2 us alone, from 14.45 to 14.2 a batch with eight in
+// flight (a division less per warp among it).
 //
 // Computes what featurize_cpu of the reference computes (gpu_featurizer/kernel_cpu.cpp:406-537).
 #pragma once
@@ -57,7 +57,7 @@ namespace ani {
 constexpr int kMolMaxAtoms = 32;       // molecules up to this size take the fast path
 constexpr int kMolCentrals = 4;        // central atoms per round
 constexpr int kMolCapA = kMolMaxAtoms - 1;   // angular neighbours of a central atom
-constexpr int kMolGroups = kMolCentrals * kPairBuckets;   // group id = element-pair bucket * 4 + central slot
+constexpr int kMolGroupStride = 16;    // group id = central slot * 16 + element-pair bucket
 constexpr int kMolNoGroup = 0xff;      // id of the quads behind the last group
 constexpr int kMolSlotsPerLane = 1;    // slots a lane evaluates per pass B (2 was measured: no gain)
 constexpr int kMolChunk = kMolSlotsPerLane * kWarp;   // slots per pass B / C
@@ -96,7 +96,7 @@ template <typename T, int POOL, int MAXA> struct MolAngularShared {
     T ang_fc[POOL];                       // f_C(r_ij, A_Rc)
     alignas(16) T A[kNumThetas][kMolChunkStride];
     alignas(16) T BF[kNumARs][kMolChunkStride];
-    MolGroupInfo tab[kMolGroups];
+    MolGroupInfo tab[kMolCentrals * kMolGroupStride];
     T* row[kMolCentrals];                     // feature row of each central atom of the round
     alignas(16) int cnt_a[kMolCentrals * kTypes];   // angular neighbours per element, per central atom
     alignas(8) unsigned char quad_gid[mol_quad_bytes(MAXA, POOL)];

@@ -39,7 +39,7 @@
             e.packed = (first + pick4(stv, ta)) | ((first + pick4(stv, tb)) << 8) | (nb << 16) |
                        ((ta == tb ? 1 : 0) << 24);
             e.recip = (unsigned)(65536.0f * __frcp_rn((float)nb)) + 1u;   // in [2^16 / nb, 2^16 / nb + 1.01)
-            const int gid = bk * kMolCentrals + g;
+            const int gid = g * kMolGroupStride + bk;
             ws.ang.tab[gid] = e;
             for (int q = off >> 2; q < (off + pad) >> 2; q++) ws.ang.quad_gid[q] = (unsigned char)gid;
         }
@@ -111,8 +111,8 @@
 #endif
             if ((ends >> q) & 1u) {
                 const unsigned id = ids[q];
-                T* row = ws.ang.row[id & (kMolCentrals - 1)];
-                row[kRadial + (id / kMolCentrals) * kTS + lane] = (acc0.x + acc0.y) + (acc1.x + acc1.y);
+                T* row = ws.ang.row[id >> 4];
+                row[kRadial + (id & 15u) * kTS + lane] = (acc0.x + acc0.y) + (acc1.x + acc1.y);
                 acc0 = Pair<T>{(T)0, (T)0};
                 acc1 = Pair<T>{(T)0, (T)0};
             }
