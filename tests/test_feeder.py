@@ -219,7 +219,7 @@ def test_a_batch_that_fails_behind_others_raises_in_its_place(fuzz):
     outcomes = []
 
     def passes():
-        for _ in range(2000 if fuzz is None else 300):
+        for _ in range(800 if fuzz is None else 200):
             got = []
             with pytest.raises(_lib.AniError):
                 for fed in BatchFeeder(packed, 40, False, fuzz, depth=3, hold=1):
@@ -229,7 +229,7 @@ def test_a_batch_that_fails_behind_others_raises_in_its_place(fuzz):
 
     worker = threading.Thread(target=passes, daemon=True)
     worker.start()
-    worker.join(60)
+    worker.join(240)
     assert outcomes and outcomes[-1] == "done", f"a pass neither ended nor raised after {len(outcomes)} passes"
     assert all(got == [0, 1, 2, 3, 4] for got in outcomes[:-1])
 
