@@ -158,6 +158,9 @@ def test_train_schedule_halves_the_rate_and_keeps_the_best_weights(tmp_path):
     tr = TrainerMultiTower(None, [torch.device("cuda", 0)], layer_sizes=(128, 128, 64, 1), seed=3)
     before = tr.eval_abs_rmse(test)
     lines = []
+    # shuffle and perturbation come from numpy's global generator: of 60 seeds two (9 and 31) never get below the error of the
+    # untrained weights within the budget of two epochs, and the epoch count then ends at 1, as the schedule has it
+    np.random.seed(0)
     best = tr.train(str(tmp_path), train, test, batch_size=16, max_local_epoch_count=2,
                     max_batch_size=16 + 128 + 1, max_global_epoch_count=6, log=lines.append)
     assert best <= before
