@@ -302,7 +302,7 @@ template <typename T>
 int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types, const int* mos,
                         const int* macs, int n_mols, const int* sis, const T* gh, const T* gc,
                         const T* gn, const T* go, T* gx, T* gy, T* gz, const int* acs_host,
-                        void* stream, const MolEnergySums<T>& sums = MolEnergySums<T>{})
+                        void* stream, const MolEnergySums<T>& sums = MolEnergySums<T>{}, bool early_inputs = false)
 {
     long long n_atoms = 0;
     if (int rc = check_acs(acs_host, &n_atoms)) return rc;
@@ -319,7 +319,7 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
             if (acs_host[t] > 0 && !gin[t]) return ANI_ERR_NULL_POINTER;
         auto launch = [&](auto warps) -> int {
             constexpr int NW = decltype(warps)::value;
-            constexpr size_t smem = mol_grad_smem_bytes<T, NW>();
+            constexpr size_t smem = sizeof(MolGradShared<T, NW>);
             static thread_local int configured_dev = -1;     // one per NW
             int dev = 0;
             ANI_CUDA(cudaGetDevice(&dev));
@@ -327,21 +327,23 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
                 if (int rc = set_smem(featurize_grad_mol_kernel<T, NW>, smem)) return rc;
                 configured_dev = dev;
             }
-            // More molecules than are resident at once: the larger ones start first (figures at kMolGradOrder).
-            const bool in_order = (long long)n_mols * NW > (long long)kSms * (sizeof(T) == 4 ? 20 : 12);
-            constexpr int kOrder = kMolGradOrder<T, NW>;
-            const dim3 grid = in_order ? dim3((n_mols + kOrder - 1) / kOrder, kOrder) : dim3(n_mols);
+            // more molecules than are resident at once: the larger ones start first (figures at kMolGradOrder)
+            const bool in_order = n_mols > kSms * MolGradCfg<T, NW>::kCtas;
+            const dim3 grid = in_order ? dim3((n_mols + kMolGradOrder - 1) / kMolGradOrder, kMolGradOrder) : dim3(n_mols);
             ANI_CUDA(launch_chain(featurize_grad_mol_kernel<T, NW>, grid, NW * kWarp, smem, st, 1, xs, ys, zs, types, mos,
                                   macs, n_mols, (int)n_atoms, sis, gh, gc, gn, go, gx, gy, gz, acs_host[0], acs_host[1],
-                                  acs_host[2], acs_host[3], sums));
+                                  acs_host[2], acs_host[3], sums, early_inputs));
             return ANI_OK;
         };
-        // Eight warps a molecule shorten its chain of scans and pair passes (64 molecules 19.0 -> 14.2 us, 512: 29.3 ->
-        // 19.8, double 47 -> 33 and 67 -> 51), four keep more of the lanes and the SM busy once there are several
-        // molecules per SM (2048: 49 against 58, 8192: 156 against 219; double, 888: 75 against 85, 1024: 81 against 97).
-        // In float 1024 molecules alone would take 31 us with eight and 35 with four, but more instructions.
-        if (n_mols <= kSms * (sizeof(T) == 4 ? 6 : 4)) return launch(std::integral_constant<int, 8>{});
-        return launch(std::integral_constant<int, 4>{});
+        // Few molecules: all of an SM for one, the whole molecule in its tables.  Microseconds alone with 12 warps (one CTA
+        // per SM) / 10 (two) / 8 (four) in float: 148 molecules 12.2 / 14.1 / 18.6, 296: 16.0 / 16.5 / 21.0, 444: 22.7 / 17.7 /
+        // 23.2, 740: 35 / 23.8 / 25.9, 900: 42 / 28.1 / 28.5; with eight streams in flight 148: 6.5 / 4.6 / 4.4, 740: 32 /
+        // 19.8 / 15.2, so the wide ones only as far as they gain.  In double with 12 / 8 (two): 296: 28.5 / 41.5, 512: 41.2 /
+        // 45.7, 592: 47.5 / 47.0, 700: 54 / 50.
+        if (n_mols <= kSms * (sizeof(T) == 8 ? 4 : 1)) return launch(std::integral_constant<int, 12>{});
+        if constexpr (sizeof(T) == 4)
+            if (n_mols <= 5 * kSms) return launch(std::integral_constant<int, 10>{});
+        return launch(std::integral_constant<int, 8>{});
     }
     {
         const int threads = 256;
@@ -1479,13 +1481,16 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
         if (int rc = ani_mlp_weight_grad_f32(&w, acs, a->split_precision, stream)) return rc;
     }
     if (a->phases & ANI_PASS_COORD_GRAD) {
+        // the kernel before is one of the networks', launched above: it has waited for what came before it
+        const bool after_networks = backward_done && n_atoms > 0 && !(a->phases & ANI_PASS_WEIGHT_GRAD) &&
+                                    ((a->phases & ANI_PASS_ENERGY) == 0 || sums_with_grads);
         MolEnergySums<float> sums = {};
         if (sums_with_grads) sums = {a->energy_sorted, a->gather_idxs, a->mol_energy};
         if (int rc = featurize_grad_impl<float>(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
                                                 a->n_mols, a->scatter_idxs, rows(a->feature_grads, 0, kTotal),
                                                 rows(a->feature_grads, 1, kTotal), rows(a->feature_grads, 2, kTotal),
                                                 rows(a->feature_grads, 3, kTotal), a->x_grads, a->y_grads, a->z_grads,
-                                                acs, stream, sums))
+                                                acs, stream, sums, after_networks))
             return rc;
     }
     return ANI_OK;
@@ -1537,7 +1542,8 @@ int ani_energy_pass_f64(const ani_energy_args_f64* a, void* stream)
         if (sums_with_grads) sums = {a->energy_sorted, a->gather_idxs, a->mol_energy};
         if (int rc = featurize_grad_impl<double>(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
                                                  a->n_mols, a->scatter_idxs, grad_rows[0], grad_rows[1], grad_rows[2],
-                                                 grad_rows[3], a->x_grads, a->y_grads, a->z_grads, acs, stream, sums))
+                                                 grad_rows[3], a->x_grads, a->y_grads, a->z_grads, acs, stream, sums,
+                                                 (a->phases & ANI_PASS_FORWARD) && ((a->phases & ANI_PASS_ENERGY) == 0 || sums_with_grads)))
             return rc;
     }
     return ANI_OK;

@@ -85,7 +85,8 @@ template <typename T> __device__ __forceinline__ void angular_factors_dev(T cosv
     const T s = Num<T>::sqrt_(Num<T>::max_((T)0, (T)1 - c * c));
     T b[kNumThetas];
 #pragma unroll
-    for (int t = 0; t < kNumThetas; t++) b[t] = c * theta_cos<T>(t) + (s * theta_sin<T>(t) + (T)1);
+    for (int t = 0; t < kNumThetas; t++)      // the first shift is 0
+        b[t] = t == 0 ? c + (T)1 : c * theta_cos<T>(t) + (s * theta_sin<T>(t) + (T)1);
 #pragma unroll
     for (int t = 0; t < kNumThetas; t += 2) {
         const Pair<T> b1{b[t], b[t + 1]};
@@ -186,7 +187,7 @@ template <typename T>
 __device__ __forceinline__ void angular_vjp_dev(T cosv, T sin2, T rij, T rik, T fcj, T dfcj, T fck, T dfck,
                                                 const T* g, T* dc, T* drj, T* drk)
 {
-    const T c = Num<T>::max_((T)-1, Num<T>::min_((T)1, cosv));
+    const T c = cosv;                 // in [-1, 1]
     const T s2 = Num<T>::min_((T)1, sin2);
     const T s = Num<T>::sqrt_(s2);
     const bool bent = s2 > (T)1e-12;  // sin(theta) > 1e-6
@@ -222,7 +223,8 @@ __device__ __forceinline__ void angular_vjp_dev(T cosv, T sin2, T rij, T rik, T 
     }
     T b[kNumThetas];
 #pragma unroll
-    for (int t = 0; t < kNumThetas; t++) b[t] = c * theta_cos<T>(t) + (s * theta_sin<T>(t) + (T)1);
+    for (int t = 0; t < kNumThetas; t++)      // the first shift is 0
+        b[t] = t == 0 ? c + (T)1 : c * theta_cos<T>(t) + (s * theta_sin<T>(t) + (T)1);
     Pair<T> s0p{(T)0, (T)0}, s2p{(T)0, (T)0};
     T sc = (T)0, ss = (T)0;
 #pragma unroll
@@ -236,7 +238,7 @@ __device__ __forceinline__ void angular_vjp_dev(T cosv, T sin2, T rij, T rik, T 
         s2p = pfma(a, vt, s2p);
         const Pair<T> b7u = pmul(b7, ut);
         sc += b7u.x * theta_cos<T>(t) + b7u.y * theta_cos<T>(t + 1);
-        ss += b7u.x * theta_sin<T>(t) + b7u.y * theta_sin<T>(t + 1);
+        ss += t == 0 ? b7u.y * theta_sin<T>(1) : b7u.x * theta_sin<T>(t) + b7u.y * theta_sin<T>(t + 1);
     }
     const T s0 = s0p.x + s0p.y, s2sum = s2p.x + s2p.y;
     const T f = (T)kA_pref * fcj * fck;

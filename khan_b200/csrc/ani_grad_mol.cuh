@@ -1,25 +1,27 @@
 // Coordinate-gradient kernel for batches of small molecules (at most 32 atoms each).
 //
-// One CTA per molecule, NW warps.  The central atoms of the molecule, in element order (see
-// load_sorted_molecule), are dealt to the warps in turn; a warp walks its share in ROUNDS of three
-// atoms and keeps the molecule in registers, lane = atom.  Per round:
-//   - the 384 upstream values of each of its central atoms are copied global -> shared memory
-//     with asynchronous 16-byte copies (cp.async), all requested at the start of the round, so
-//     the copies run under the arithmetic and cost three instructions per lane and row;
-//   - A. per central atom c: one distance per lane; a lane whose atom j is within R_Rc contracts
-//     the 16 upstream values of radial block type(j) with the radial derivatives and WRITES the
-//     force on j into the molecule's force table part[c][j]; neighbours within A_Rc are
-//     appended to the warp's neighbour list;
-//   - B. when the list is full (or the round is in), the neighbour pairs of ALL central atoms in
-//     the list are walked together in circulant order: the neighbours of a central atom with k
-//     neighbours occupy k consecutive lanes, lane a handles the pair (a, a + d mod k) for
-//     d = 1 .. k/2, keeps the force on a in registers and hands the force on b to its owner
-//     with one shuffle.  Spare lanes run further offsets d at the same time;
-//   - the lanes then add their neighbour's force to part[c][a].
-// After one __syncthreads the molecule's gradient is column sum minus row sum of the table
-// (every term depends on coordinate differences only, so the central atom gets minus what it
-// handed out): each output value is written once, nothing is accumulated with atomics, the
-// outputs need no zero fill and the result is bit-reproducible.
+// One CTA per molecule, NW warps that share every step evenly, whatever the molecule's neighbourhoods look like:
+//   - the upstream values come with 16-byte asynchronous copies (cp.async), requested as soon as elements and rows are known:
+//     the radial ones of every atom, the angular ones of as many central atoms as a batch may have;
+//   - pairs of atoms: lane = unordered pair.  The radial derivatives of both directions are one contraction with the SUM of
+//     the two atoms' upstream values, and the pairs within A_Rc set a bit in both atoms' neighbour masks;
+//   - the central atoms go in BATCHES (limits in MolGradCfg; most molecules are one batch).  Per batch:
+//       entries  lane = (central atom, neighbour): unit vector, distance and cutoff into the list;
+//       pairs    lane = (central atom, neighbours a and b), all pairs of the batch in one numbering, so that all lanes of
+//                all warps work but for the last 32 pairs: the 32 upstream values contract to (dL/dcos, dL/dr_a, dL/dr_b);
+//       forces   lane = entry: sums over the k - 1 pairs it is in, in a fixed order;
+//       sums     lane = atom: what the central atoms hand to it less what it hands out.
+// Every output value is written once, nothing is accumulated with atomics, the outputs need no zero fill and the result is
+// bit-reproducible.
+//
+// Before, a warp took central atoms of its own, three at a time, with a lane per neighbour: 73 % of the lanes busy in the
+// pairs, and the warps of a large molecule (a cost that grows with the cube of its size) went on alone.  The busiest warp
+// scheduler issued 1.78 times the average on 1024 molecules, 1.17 times now.  Microseconds alone, before -> now: float, 1
+// molecule 8.9 -> 8.6, 64: 14.9 -> 11.7, 256: 19.4 -> 15.5, 512: 20.3 -> 18.2, 1024: 34.5 -> 29.5, 2048: 48.9 -> 44.5;
+// double, 1: 19.0 -> 16.4, 64: 35.2 -> 24.6, 256: 41.4 -> 28.3, 512: 51.6 -> 41.2, 1024: 81.6 -> 66.5, 2048: 130 -> 123.  With
+// eight streams in flight 1024 molecules in float take 20.4 instead of 19.6 and in double 59.9 instead of 61.0.  What
+// bounds it: issue at 0.6 instructions a cycle and scheduler, held up by shared memory (half of its wavefronts, the upstream
+// values of 32 lanes with different element pairs) and, for one molecule, by the chain of eight steps.
 //
 // A molecule with more than 32 atoms met by this kernel goes through the streaming routines
 // (zero fill by its own CTA, then global atomics, all inside the CTA).
@@ -34,8 +36,6 @@
 
 namespace ani {
 
-constexpr int kMolGradPitch = kMolMaxAtoms + 1;   // odd: rows and columns of the force table are both conflict-free
-
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
@@ -47,11 +47,6 @@ template <int N> __device__ __forceinline__ void cp_async_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Central atoms per round = upstream rows a warp holds in shared memory.
-template <typename T> struct MolGradCfg {
-    static constexpr int kRowBufs = 3;
-};
-
 template <typename T> struct alignas(16) MolGradNeighbor {
     Vec4<T> u;         // (x_c - x_j) / r, r
     T inv_r, fc, dfc;  // 1 / r, f_C(r, A_Rc) and its derivative
@@ -59,16 +54,42 @@ template <typename T> struct alignas(16) MolGradNeighbor {
                        // neighbours of that central atom << 12 | row buffer << 18 | lane of the central atom << 20
 };
 
-template <typename T> struct MolGradWarpShared {
-    alignas(16) T g[MolGradCfg<T>::kRowBufs][kGradRowWords];   // upstream rows, blocks of 32 at stride 36
-    MolGradNeighbor<T> nb[kWarp];
-    MolSortShared sort;
+constexpr int kMolGradPitch = kMolMaxAtoms + 1;
+constexpr int kMolGradRow = kPairBuckets * kGradBucketStride;
+
+// Warps of a CTA, and what its tables hold of a batch: upstream rows, list entries, neighbour pairs.  A batch takes at least
+// one atom with 31 neighbours, so kEntries >= 31 and kSlots >= 465.  With more than eight warps the tables are for the
+// whole molecule (one CTA fills an SM, or two); with eight, four (float) or two (double) fit an SM.  More batches cost
+// barriers and pairs short of 32: 1024 molecules in float take 29.5 us with these tables and 43 with 8 rows, 160 entries and
+// 512 pairs and four warps.
+template <typename T, int NW> struct MolGradCfg {
+    static constexpr bool kFloat = sizeof(T) == 4;
+    static constexpr int kCtas = NW == 12 ? 1 : (NW == 10 || !kFloat ? 2 : 4);      // resident per SM
+    static constexpr int kRows = NW == 12 ? (kFloat ? 32 : 24) : NW == 10 ? 24 : (kFloat ? 14 : 12);
+    static constexpr int kEntries = NW == 12 ? 512 : NW == 10 ? 384 : (kFloat ? 224 : 256);
+    static constexpr int kSlots = NW == 12 ? (kFloat ? 3072 : 2048) : NW == 10 ? 2560 : 1024;
+    static constexpr int kRadPitch = kRadial + 16 / (int)sizeof(T);   // rows of 64 values, conflict-free in 16-byte reads
+    static_assert(kRows >= 1 && kEntries >= kMolMaxAtoms - 1 && kEntries < 1 << 12 && kSlots < 1 << 13 &&
+                  kSlots >= (kMolMaxAtoms - 1) * (kMolMaxAtoms - 2) / 2, "any atom fits a batch");
 };
 
-template <typename T, int NW> constexpr size_t mol_grad_smem_bytes()
-{
-    return NW * sizeof(MolGradWarpShared<T>) + 3 * kMolMaxAtoms * kMolGradPitch * sizeof(T);
-}
+template <typename T, int NW> struct MolGradShared {
+    using Cfg = MolGradCfg<T, NW>;
+    alignas(16) T g[Cfg::kRows][kMolGradRow];     // angular upstream values, blocks of 32 at stride 36
+    // row d of a central atom with k neighbours, place a: dL/dcos(theta) and the part along bond a of the pairs
+    // (a, a + d) and (a - d, a)
+    alignas(32) Vec2<T> pair[2 * Cfg::kSlots];
+    Vec4<T> u[Cfg::kEntries], w[Cfg::kEntries];   // unit vector and r; 1 / r, f_C, f_C', element
+    T force[3][Cfg::kRows][kMolGradPitch];        // of a central atom of the batch on an atom
+    T radial[kMolMaxAtoms][kMolGradPitch];        // dL/dr / r of two atoms
+    T xyz[3][kMolMaxAtoms];
+    int type[kMolMaxAtoms];
+    unsigned near[kMolMaxAtoms];                  // atoms within A_Rc
+    unsigned char list[kMolMaxAtoms][kMolMaxAtoms];   // the same as a list
+    // the radial upstream values lie over the pairs and what follows: they have been used before the first entry
+    __device__ __forceinline__ T* rad(int c) { return &pair[0].x + c * Cfg::kRadPitch; }
+    static_assert(sizeof(T) * kMolMaxAtoms * Cfg::kRadPitch <= sizeof(pair) + sizeof(u) + sizeof(w) + sizeof(force), "radial rows");
+};
 
 // Bucket of the element pair (ta, tb), four bits per entry of the 4 x 4 table.
 constexpr unsigned long long kBucketLut =
@@ -126,33 +147,59 @@ template <typename T> struct MolEnergySums {
     T* mol_energy;
 };
 
-// Molecules whose CTAs are put into order of size.  Microseconds alone with 4 / 8 / 16 / 32, and in two classes with two
-// CTAs per molecule as it was: eight warps, float, 600 molecules 22.6 / 21.0 / 20.2 / 20.6, 22.3; four warps, float, 1024:
-// 34.9 / 34.2 / 32.8 / 33.7, 35.6, 2048: 49.3 / 47.8 / 45.6 / 44.1, 48.8; double, 1024: 88 / 83 / 81 / 81, 86, 2048: 143 /
-// 139 / 131 / 126, 138.  But the order costs instructions, and with eight streams in flight, where it gains nothing, 1024
-// molecules in float take 18.3 / 18.5 / 18.9, in two classes 19.2 and without any order 18.2 (37.7 alone).
-template <typename T, int NW> constexpr int kMolGradOrder = sizeof(T) == 4 && NW == 4 ? 4 : 16;
+// early_inputs: nothing less than two kernels back writes coordinates, elements, rows or the molecule table: they are read,
+// and the distances formed, ahead of the kernel before this one, whose upstream values come last.  Energies + forces of one
+// molecule 32.3 -> 31.0 us.
+// Molecules whose CTAs are put into order of size, when not all molecules are resident at once: 1024 molecules in float
+// take 34.9 us without the order, in double 83.6 instead of 64.1; with eight streams in flight the order gains nothing
+// (19.9 without, 20.4 with it).
+constexpr int kMolGradOrder = 16;
+
+__device__ __forceinline__ float bits_as(float, int v) { return __int_as_float(v); }
+__device__ __forceinline__ double bits_as(double, int v) { return __hiloint2double(0, v); }
+__device__ __forceinline__ int as_bits(float v) { return __float_as_int(v); }
+__device__ __forceinline__ int as_bits(double v) { return __double2loint(v); }
+
+// length_and_inverse with one Newton step on the SFU's reciprocal root in float: the distances are computed once per pair
+// of atoms here, and their error is what the Gaussians enlarge most.
+__device__ __forceinline__ void refined_length_and_inverse(float d2, float* r, float* inv)
+{
+    const float rs = d2 > 0.0f ? sfu_rsqrt(d2) : 0.0f;
+    const float h = d2 * rs;
+    const float e = fmaf(-h, rs, 1.0f);             // 1 - d2 rs^2
+    *inv = fmaf(0.5f * rs, e, rs);
+    *r = fmaf(0.5f * h, e, h);
+}
+__device__ __forceinline__ void refined_length_and_inverse(double d2, double* r, double* inv) { length_and_inverse(d2, r, inv); }
+
+// The lane (central atom) among `members` whose range of a prefix sum holds `first + lane`; off = where the range of this
+// lane's atom starts.  All lanes call it; `first + lane` must lie inside the total.
+__device__ __forceinline__ int owner_of(unsigned members, int off, int first, int index)
+{
+    const bool member = (members >> lane_id()) & 1u;
+    const int lo = 31 - __clz(__ballot_sync(kFull, member && off <= first));
+    const int hi = 31 - __clz(__ballot_sync(kFull, member && off <= first + kWarp - 1));
+    int c = lo;
+    for (int q = lo + 1; q <= hi; q++) c += index >= __shfl_sync(kFull, off, q) ? 1 : 0;
+    return c;
+}
 
 template <typename T, int NW>
-__global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
+__global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
     featurize_grad_mol_kernel(const T* __restrict__ xs, const T* __restrict__ ys, const T* __restrict__ zs,
                               const int* __restrict__ types, const int* __restrict__ mol_offsets,
                               const int* __restrict__ mol_counts, int n_mols, int n_atoms,
                               const int* __restrict__ scatter, const T* __restrict__ gh,
                               const T* __restrict__ gc, const T* __restrict__ gn, const T* __restrict__ go,
                               T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3,
-                              const MolEnergySums<T> sums)
+                              const MolEnergySums<T> sums, bool early_inputs)
 {
-    constexpr int GR = MolGradCfg<T>::kRowBufs;   // central atoms per round
+    using Cfg = MolGradCfg<T, NW>;
+    constexpr int kThreads = NW * kWarp;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    using WarpShared = MolGradWarpShared<T>;
+    MolGradShared<T, NW>& sh = *reinterpret_cast<MolGradShared<T, NW>*>(smem_raw);
     const int lane = lane_id(), warp = warp_id();
-    pdl_wait();
-    WarpShared& ws = reinterpret_cast<WarpShared*>(smem_raw)[warp];
-    T* part = reinterpret_cast<T*>(smem_raw + NW * sizeof(WarpShared));
-    auto part_at = [part](int plane, int c, int j) -> T& {
-        return part[(plane * kMolMaxAtoms + c) * kMolGradPitch + j];
-    };
+    if (!early_inputs) pdl_wait();
 
     // In a grid of (X, Y) CTAs the molecules i, i + X, i + 2 X ... share the CTAs (i, 0), (i, 1), (i, 2) ... in order of
     // their sizes: CTAs start in index order, so the expensive molecules start first and the cheap ones fill the SMs
@@ -163,27 +210,36 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
     if (gridDim.y == 1) {
         usable = load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol);
     } else {
-        constexpr int kLast = kMolGradOrder<T, NW> - 1;
-        const int mine = blockIdx.x + (lane & kLast) * gridDim.x;
-        const int size = mine < n_mols ? mol_counts[mine] : -1, first = mine < n_mols ? mol_offsets[mine] : 0;
-        int rank = 0;
+        const int mine = blockIdx.x + lane * gridDim.x;
+        const bool there = lane < kMolGradOrder && mine < n_mols;
+        const int size = there ? mol_counts[mine] : 0, first = there ? mol_offsets[mine] : 0;
+        // the blockIdx.y-th largest, bit by bit (all above 32 atoms alike)
+        const int key = min(max(size, 0), 63);
+        unsigned left = __ballot_sync(kFull, there);
+        int y = blockIdx.y;
+        if (y >= __popc(left)) return;
 #pragma unroll
-        for (int d = 1; d <= kLast; d++) {
-            const int other = __shfl_xor_sync(kFull, size, d), other_lane = (lane ^ d) & kLast;
-            rank += other > size || (other == size && other_lane < (lane & kLast)) ? 1 : 0;
+        for (int bit = 5; bit >= 0; bit--) {
+            const unsigned with = __ballot_sync(kFull, (key >> bit) & 1) & left;
+            const int c = __popc(with);
+            if (y < c) left = with;
+            else {
+                y -= c;
+                left &= ~with;
+            }
         }
-        const int src = __ffs(__ballot_sync(kFull, rank == (int)blockIdx.y)) - 1;
-        m = blockIdx.x + (src & kLast) * gridDim.x;
-        if (m >= n_mols) return;
+        const int src = __ffs(__ballot_sync(kFull, ((left >> lane) & 1u) && __popc(left & lanemask_lt()) == y)) - 1;
+        m = blockIdx.x + src * gridDim.x;
         usable = check_molecule(__shfl_sync(kFull, size, src), __shfl_sync(kFull, first, src), n_atoms, &mol);
     }
     if (!usable) {
+        pdl_wait();
         if (sums.mol_energy && threadIdx.x == 0) sums.mol_energy[m] = (T)0;
         return;
     }
     const int n = mol.n, base = mol.base;
 
-    T energy = (T)0;
+    T energy = (T)0;      // of the molecule, summed by the last warp and written at the end
     auto load_energy = [&] {
         if (!sums.mol_energy || warp != NW - 1) return;
         for (int i = lane; i < n; i += kWarp) {
@@ -198,17 +254,19 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
         for (int o = 16; o > 0; o >>= 1) energy += __shfl_xor_sync(kFull, energy, o);
         if (lane == 0) sums.mol_energy[m] = energy;
     };
-    // requested early; in double, where the registers are all in use, only at the end
-    if (sizeof(T) == 4 || n > kMolMaxAtoms) load_energy();
 
     if (n > kMolMaxAtoms) {   // a large molecule in a batch of small ones
+        pdl_wait();
+        load_energy();
         write_energy();
-        for (int j = threadIdx.x; j < n; j += NW * kWarp) {
+        for (int j = threadIdx.x; j < n; j += kThreads) {
             gx[base + j] = (T)0;
             gy[base + j] = (T)0;
             gz[base + j] = (T)0;
         }
         __syncthreads();
+        T* g = reinterpret_cast<T*>(smem_raw) + warp * kGradRowWords;
+        static_assert(NW * kGradRowWords * sizeof(T) <= sizeof(MolGradShared<T, NW>), "a row per warp");
         for (int i = warp; i < n; i += NW) {
             const int gi = base + i;
             const int ti = checked_type(types[gi]);
@@ -219,7 +277,6 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
                 continue;
             }
             const T* grow = (ti == 0 ? gh : (ti == 1 ? gc : (ti == 2 ? gn : go))) + (size_t)srow * kTotal;
-            T* g = ws.g[0];
             g[lane] = grow[lane];
             g[32 + lane] = grow[32 + lane];
             for (int bk = 0; bk < kPairBuckets; bk++)
@@ -232,127 +289,257 @@ __global__ void __launch_bounds__(NW* kWarp, sizeof(T) == 4 ? 20 / NW : 12 / NW)
         return;
     }
 
-    // every warp needs the sort for the last step, also one without a round of its own
-    MolLanes<T> ml;
-    load_sorted_molecule<T>(xs, ys, zs, types, scatter, base, n, &ws.sort, &ml);
+    // ---- the molecule: lane = atom in every warp (element and row), coordinates in shared memory ----
+    int my_type = 0, my_row = -1;
+    if (lane < n) {
+        my_type = types[base + lane];
+        my_row = scatter[base + lane];
+    }
+    if (threadIdx.x < n) {      // warp 0
+        sh.xyz[0][lane] = xs[base + lane];
+        sh.xyz[1][lane] = ys[base + lane];
+        sh.xyz[2][lane] = zs[base + lane];
+        sh.near[lane] = 0u;
+        sh.radial[lane][lane] = (T)0;
+    }
+    if (my_type < 0 || my_type >= kTypes) my_type = warp == 0 ? checked_type(my_type) : my_type & 3;
+    {
+        const int cap = my_type == 0 ? acs0 : (my_type == 1 ? acs1 : (my_type == 2 ? acs2 : acs3));
+        if (lane < n && (my_row < 0 || my_row >= cap)) {
+            if (warp == 0) report(ANI_ERR_BAD_INDEX);
+            my_row = -1;
+        }
+    }
+    if (threadIdx.x < n) sh.type[lane] = my_type;
+    const unsigned ok_mask = __ballot_sync(kFull, my_row >= 0);   // atoms that have an upstream row
+    const unsigned long long my_src = reinterpret_cast<unsigned long long>(
+        (my_type == 0 ? gh : (my_type == 1 ? gc : (my_type == 2 ? gn : go))) + (my_row >= 0 ? (size_t)my_row * kTotal : 0));
 
-    // Warp w takes the central atoms w, w + NW, w + 2 NW, ... (element order) and walks them in rounds
-    // of GR: every warp gets the same number of atoms (no idle warps) AND the same mix of light and heavy
-    // ones -- the cost of a central atom grows with the square of its neighbour count, and consecutive
-    // atoms are of one element.  Which warp starts with atom 0 rotates with the molecule: a warp's
-    // scheduler is fixed by its index, and the last warps have one atom less.
-    const int w0 = (warp + m) % NW;
-    const int K = w0 < n ? (n - w0 + NW - 1) / NW : 0;   // central atoms of this warp
-    for (int k_first = 0; k_first < K; k_first += GR) {
-        const int G = min(GR, K - k_first);
-        // ---- upstream rows of the round: one commit group per row slot ----
+    // upstream values, 16 bytes per copy: the radial ones of every atom, the angular ones of the rows [r0, r1)
+    constexpr int kPiece = 16 / (int)sizeof(T), kRadPieces = kRadial / kPiece, kPieces = kTotal / kPiece;
+    auto row_of = [&](int c) -> const T* {
+        return reinterpret_cast<const T*>(__shfl_sync(kFull, my_src, c));
+    };
+    auto request_angular = [&](const T* src, T* dst) {
 #pragma unroll
-        for (int g = 0; g < GR; g++) {
-            const int c = min(w0 + (k_first + g) * NW, n - 1);
-            const int ti = __shfl_sync(kFull, ml.type, c), sr = ws.sort.srow[c];
-            const int cap = ti == 0 ? acs0 : (ti == 1 ? acs1 : (ti == 2 ? acs2 : acs3));
-            if (g < G && sr >= 0 && sr < cap) {
-                const T* grow = (ti == 0 ? gh : (ti == 1 ? gc : (ti == 2 ? gn : go))) + (size_t)sr * kTotal;
-                T* dst = ws.g[g];
-                constexpr int V = 16 / (int)sizeof(T);   // values per 16-byte copy
+        for (int s = 0; s < (kPieces - kRadPieces + kWarp - 1) / kWarp; s++) {
+            const int v = (lane + s * kWarp) * kPiece;
+            if (v < kAngular) cp_async16(dst + (v >> 5) * kGradBucketStride + (v & 31), src + kRadial + v);
+        }
+    };
+    int r0 = 0, r1 = min(n, Cfg::kRows);
+    auto request_first = [&] {
+        for (int c = warp; c < n; c += NW) {
+            const T* src = row_of(c);
+            if (lane < kRadPieces) {
+                if ((ok_mask >> c) & 1u) cp_async16(sh.rad(c) + lane * kPiece, src + lane * kPiece);
+                else
 #pragma unroll
-                for (int s = 0; s < kTotal / V / kWarp; s++) {
-                    const int v = (lane + s * kWarp) * V;
-                    const int d = v < kRadial
-                                      ? v
-                                      : kRadial + ((v - kRadial) >> 5) * kGradBucketStride + ((v - kRadial) & 31);
-                    cp_async16(dst + d, grow + v);
+                    for (int q = 0; q < kPiece; q++) sh.rad(c)[lane * kPiece + q] = (T)0;
+            }
+            if (c < r1 && ((ok_mask >> c) & 1u)) request_angular(src, sh.g[c]);
+        }
+        cp_async_commit();
+    };
+    if (!early_inputs) request_first();
+    __syncthreads();
+
+    // ---- every two atoms once: pair p of n (n - 1) / 2 is (i, i + d mod n), d = 1, 2 ... ----
+    constexpr int kMaxPairs = (kMolMaxAtoms * (kMolMaxAtoms - 1) / 2 + kThreads - 1) / kThreads;
+    const int n_pairs = n * (n - 1) / 2;
+    const unsigned recip = (unsigned)(65536.0f * __frcp_rn((float)n)) + 1u;
+    T pr[kMaxPairs], pinv[kMaxPairs];
+    int pij[kMaxPairs];
+#pragma unroll
+    for (int s = 0; s < kMaxPairs; s++) {
+        const int p = s * kThreads + threadIdx.x;
+        if (p < n_pairs) {
+            const int d0 = (int)(((unsigned)p * recip) >> 16), i = p - d0 * n;
+            int j = i + d0 + 1;
+            if (j >= n) j -= n;
+            const T dx = sh.xyz[0][i] - sh.xyz[0][j], dy = sh.xyz[1][i] - sh.xyz[1][j], dz = sh.xyz[2][i] - sh.xyz[2][j];
+            refined_length_and_inverse(dx * dx + dy * dy + dz * dz, &pr[s], &pinv[s]);
+            pij[s] = i | (j << 8);
+            if (pr[s] < (T)kA_Rc) {
+                atomicOr(&sh.near[i], 1u << j);
+                atomicOr(&sh.near[j], 1u << i);
+            }
+        }
+    }
+    if (early_inputs) {
+        pdl_wait();
+        request_first();
+    }
+    load_energy();      // (the last warp has no pair of atoms in most molecules)
+    cp_async_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < kMaxPairs; s++) {
+        const int p = s * kThreads + threadIdx.x;
+        if (p < n_pairs) {
+            const int i = pij[s] & 0xff, j = pij[s] >> 8;
+            T force = (T)0;
+            if (pr[s] < (T)kR_Rc) {
+                T fc, dfc;
+                cutoff<T>(pr[s], (T)kR_Rc, &fc, &dfc);
+                const T *wi = sh.rad(i) + sh.type[j] * kNumRs, *wj = sh.rad(j) + sh.type[i] * kNumRs;
+                T w[kNumRs], v[4];
+#pragma unroll
+                for (int q = 0; q < kNumRs; q += 4) {
+                    load4(wi + q, w + q);
+                    load4(wj + q, v);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) w[q + k] += v[k];
                 }
+                force = radial_vjp_dev<T>(pr[s], fc, dfc, w) * pinv[s];
+            }
+            sh.radial[i][j] = force;
+            sh.radial[j][i] = force;
+            if (pr[s] < (T)kA_Rc) {
+                sh.list[i][__popc(sh.near[i] & ((1u << j) - 1u))] = (unsigned char)j;
+                sh.list[j][__popc(sh.near[j] & ((1u << i) - 1u))] = (unsigned char)i;
+            }
+        }
+    }
+    // lane = central atom: its neighbours and pairs, and where they start in the molecule's numbering
+    const unsigned my_near = lane < n ? sh.near[lane] : 0u;
+    const int my_k = (ok_mask >> lane) & 1u ? __popc(my_near) : 0, my_pairs = my_k * (my_k - 1) / 2;
+    int incl = my_k | (my_pairs << 12);      // at most 992 neighbours
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int excl = incl - (my_k | (my_pairs << 12));
+    const int k_first = excl & 0xfff, p_first = excl >> 12, k_end = incl & 0xfff, p_end = incl >> 12;
+    const unsigned k_recip = (unsigned)(65536.0f * __frcp_rn((float)max(my_k, 1))) + 1u;
+    __syncthreads();
+
+    T sum = (T)0;      // warps 0 .. 2: one component of the gradient of atom `lane`
+    int c0 = 0;
+    auto batch_end = [&](int from) {
+        const int k0 = __shfl_sync(kFull, k_first, from), p0 = __shfl_sync(kFull, p_first, from);
+        const bool fits = lane >= from && lane < n && lane - from < Cfg::kRows && k_end - k0 <= Cfg::kEntries &&
+                          p_end - p0 <= Cfg::kSlots;
+        return from + __popc(__ballot_sync(kFull, fits));
+    };
+    int c1 = batch_end(0);
+    while (true) {
+        const unsigned members = low_lanes(c1) & ~low_lanes(c0);
+        const int k0 = __shfl_sync(kFull, k_first, c0), p0 = __shfl_sync(kFull, p_first, c0);
+        const int n_entries = __shfl_sync(kFull, k_end, c1 - 1) - k0, n_slots = __shfl_sync(kFull, p_end, c1 - 1) - p0;
+        const int my_entry = k_first - k0, my_slot = p_first - p0, my_at = my_slot | (my_k << 13) | (my_entry << 19);
+        // ---- list entries of the batch, lane = entry ----
+        for (int first = warp * kWarp; first < n_entries; first += kThreads) {
+            const int e = min(first + lane, n_entries - 1);
+            const int c = owner_of(members, my_entry, first, e);
+            const int a = e - __shfl_sync(kFull, my_entry, c), j = sh.list[c][a];
+            const T dx = sh.xyz[0][c] - sh.xyz[0][j], dy = sh.xyz[1][c] - sh.xyz[1][j], dz = sh.xyz[2][c] - sh.xyz[2][j];
+            T r, inv, fc, dfc;
+            refined_length_and_inverse(dx * dx + dy * dy + dz * dz, &r, &inv);
+            cutoff<T>(r, (T)kA_Rc, &fc, &dfc);
+            sh.u[e] = Vec4<T>{dx * inv, dy * inv, dz * inv, r};
+            sh.w[e] = Vec4<T>{inv, fc, dfc, bits_as((T)0, sh.type[j])};
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+        // ---- neighbour pairs of the batch, lane = pair; the pairs of a central atom with k neighbours in circulant order:
+        // pair q is (a, a + d mod k) with d = 1 + q / k, a = q mod k ----
+        for (int first = ((warp + NW - 3) % NW) * kWarp; first < n_slots; first += kThreads) {
+            const int p = min(first + lane, n_slots - 1);
+            const int c = owner_of(members, my_slot, first, p);
+            const int at = __shfl_sync(kFull, my_at, c);
+            const unsigned rk = __shfl_sync(kFull, k_recip, c);
+            const int q = p - (at & 0x1fff), k = (at >> 13) & 0x3f, list = at >> 19;
+            const int d0 = (int)(((unsigned)q * rk) >> 16), a = q - d0 * k;
+            int b = a + d0 + 1;
+            if (b >= k) b -= k;
+            const Vec4<T> ua = sh.u[list + a], ub = sh.u[list + b], wa = sh.w[list + a], wb = sh.w[list + b];
+            T cosv = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
+            cosv = Num<T>::max_((T)-1, Num<T>::min_((T)1, cosv));
+            const T s2 = sin2_from_cross<T>(ua.x, ua.y, ua.z, ub.x, ub.y, ub.z);
+            T gl[kTS];
+            const T* gsrc = sh.g[c - r0] + bucket_of(as_bits(wa.w), as_bits(wb.w)) * kGradBucketStride;
+#pragma unroll
+            for (int i = 0; i < kTS; i += 4) load4(gsrc + i, gl + i);
+            T dc, dra, drb;
+            angular_vjp_dev<T>(cosv, s2, ua.w, ub.w, wa.y, wa.z, wb.y, wb.z, gl, &dc, &dra, &drb);
+            Vec2<T>* out = sh.pair + 2 * (p - a);
+            out[2 * a] = Vec2<T>{dc, cosv * dc * wa.x - dra};
+            out[2 * (2 * (d0 + 1) == k ? a : b) + 1] = Vec2<T>{dc, cosv * dc * wb.x - drb};
+        }
+        __syncthreads();
+        // ---- the next batch's rows, if they are not here ----
+        const int c2 = c1 < n ? batch_end(c1) : c1;
+        if (c2 > r1) {
+            r0 = c1;
+            r1 = min(r0 + Cfg::kRows, n);
+            for (int c = r0 + warp; c < r1; c += NW) {
+                const T* src = row_of(c);
+                if ((ok_mask >> c) & 1u) request_angular(src, sh.g[c - r0]);
             }
             cp_async_commit();
         }
-
-        int g = 0;
-        while (g < G) {
-            // ---- A: scan central atoms into the neighbour list until it is full ----
-            int used = 0, max_half = 0, taken = 0;
-            while (g < G) {
-                const int c = w0 + (k_first + g) * NW;
-                const T xi = __shfl_sync(kFull, ml.x, c), yi = __shfl_sync(kFull, ml.y, c),
-                        zi = __shfl_sync(kFull, ml.z, c);
-                const int ti = __shfl_sync(kFull, ml.type, c), sr = ws.sort.srow[c];
-                const int cap = ti == 0 ? acs0 : (ti == 1 ? acs1 : (ti == 2 ? acs2 : acs3));
-                const bool ok = sr >= 0 && sr < cap;
-                const T dx = xi - ml.x, dy = yi - ml.y, dz = zi - ml.z;
-                T r, inv;
-                length_and_inverse(dx * dx + dy * dy + dz * dz, &r, &inv);
-                const bool in_rad = ok && lane < n && lane != c && r < (T)kR_Rc;
-                const bool in_ang = in_rad && r < (T)kA_Rc;
-                const unsigned mA = __ballot_sync(kFull, in_ang);
-                const int nA = __popc(mA);
-                if (taken > 0 && used + nA > kWarp) break;   // this central atom opens the next pass
-
-                // row slot g has landed when at most GR - 1 - g younger groups are pending
-                if (g == 0) cp_async_wait<GR - 1>();
-                else if (g == 1) cp_async_wait<(GR > 2 ? GR - 2 : 0)>();
-                else if (g == 2) cp_async_wait<(GR > 3 ? GR - 3 : 0)>();
-                else cp_async_wait<0>();
-                __syncwarp();
-                if (!ok && lane == 0) report(ANI_ERR_BAD_INDEX);
-                const T* grow = ws.g[g];
-                const T ux = dx * inv, uy = dy * inv, uz = dz * inv;
-                T fx = (T)0, fy = (T)0, fz = (T)0;
-                if (in_rad) {
-                    T fc, dfc;
-                    cutoff<T>(r, (T)kR_Rc, &fc, &dfc);
-                    T w[kNumRs];
-#pragma unroll
-                    for (int q = 0; q < kNumRs; q += 4) load4(grow + ml.type * kNumRs + q, w + q);
-                    const T d = radial_vjp_dev<T>(r, fc, dfc, w);
-                    fx = d * ux; fy = d * uy; fz = d * uz;
-                }
-                if (lane < n) {   // force on atom j from the radial terms of central atom c (0 out of range)
-                    part_at(0, c, lane) = -fx;
-                    part_at(1, c, lane) = -fy;
-                    part_at(2, c, lane) = -fz;
-                }
-                if (in_ang) {
-                    MolGradNeighbor<T> e;
-                    e.u = Vec4<T>{ux, uy, uz, r};
-                    e.inv_r = inv;
-                    cutoff<T>(r, (T)kA_Rc, &e.fc, &e.dfc);
-                    e.info = ml.type | (lane << 2) | (used << 7) | (nA << 12) | (g << 18) | (c << 20);
-                    ws.nb[used + __popc(mA & lanemask_lt())] = e;
-                }
-                used += nA;
-                taken++;
-                max_half = max(max_half, nA >> 1);
-                g++;
+        // ---- lane = entry: the force on it from the pairs that it is in ----
+        for (int first = warp * kWarp; first < n_entries; first += kThreads) {
+            const int e = min(first + lane, n_entries - 1);
+            const int c = owner_of(members, my_entry, first, e);
+            const int at = __shfl_sync(kFull, my_at, c);
+            const int k = (at >> 13) & 0x3f, list = at >> 19, a = e - list;
+            const Vec4<T>*u = sh.u + list, *row = reinterpret_cast<const Vec4<T>*>(sh.pair) + (at & 0x1fff) + a;
+            T fx = (T)0, fy = (T)0, fz = (T)0, along = (T)0;
+            int b = a, z = a;
+            for (int left = k; left > 2; left -= 2, row += k) {
+                b = b + 1 >= k ? 0 : b + 1;
+                z = z == 0 ? k - 1 : z - 1;
+                const Vec4<T> ub = u[b], uz = u[z], q = *row;
+                along += q.y + q.w;
+                fx += q.x * ub.x + q.z * uz.x;
+                fy += q.x * ub.y + q.z * uz.y;
+                fz += q.x * ub.z + q.z * uz.z;
             }
-            __syncwarp();
-
-            // ---- B: neighbour pairs of every central atom in the list, circulant order ----
-            if (max_half > 0) {
-#include "ani_grad_pair_pass.inl"
-                if (lane < used) {
-                    const int cen = (ea.info >> 20) & 31, at = (ea.info >> 2) & 31;
-                    part_at(0, cen, at) += fax;
-                    part_at(1, cen, at) += fay;
-                    part_at(2, cen, at) += faz;
-                }
+            if (!(k & 1)) {      // the last row of an even k has k / 2 pairs; a + k / 2 = a - k / 2 (mod k)
+                b = b + 1 >= k ? 0 : b + 1;
+                const Vec4<T> ub = u[b];
+                const Vec2<T> q = reinterpret_cast<const Vec2<T>*>(row)[a < (k >> 1) ? 0 : 1 - k];
+                along += q.y;
+                fx += q.x * ub.x;
+                fy += q.x * ub.y;
+                fz += q.x * ub.z;
             }
-            __syncwarp();
+            const Vec4<T> ua = u[a];
+            const T inv = sh.w[e].x;
+            const int j = sh.list[c][a];
+            sh.force[0][c - c0][j] = along * ua.x - inv * fx;
+            sh.force[1][c - c0][j] = along * ua.y - inv * fy;
+            sh.force[2][c - c0][j] = along * ua.z - inv * fz;
         }
-        cp_async_wait<0>();   // row slots of a short round are empty groups; nothing may stay pending
+        __syncthreads();
+        // ---- warps 0 .. 2, lane = atom: what the batch's central atoms hand to it, less what it hands out ----
+        if (warp < 3) {
+            const T(*f)[kMolGradPitch] = sh.force[warp];
+            const unsigned from = my_near & ok_mask;
+            for (int q = c0; q < c1; q++)
+                if ((from >> q) & 1u) sum += f[q - c0][lane];
+            if ((members & ok_mask) >> lane & 1u)
+                for (int q = 0; q < n; q++)
+                    if ((my_near >> q) & 1u) sum -= f[lane - c0][q];
+        }
+        if (c1 >= n) break;
+        c0 = c1;
+        c1 = c2;
     }
     pdl_trigger();
-    __syncthreads();
-    if (sizeof(T) == 8) load_energy();
     write_energy();
-    // gradient of atom j = what the central atoms handed to j (column j) - what j handed out (row j)
-    for (int plane = warp; plane < 3; plane += NW) {
-        if (lane < n) {
-            T col = (T)0, rw = (T)0;
-            for (int c = 0; c < n; c++) col += part_at(plane, c, lane);
-            for (int j = 0; j < n; j++) rw += part_at(plane, lane, j);
-            T* dst = plane == 0 ? gx : (plane == 1 ? gy : gz);
-            dst[base + ws.sort.src[lane]] = col - rw;
+    if (warp < 3 && lane < n) {
+        const T* x = sh.xyz[warp];
+        const T xi = x[lane];
+#pragma unroll 4
+        for (int j = 0; j < n; j++) {
+            const T f = sh.radial[lane][j];
+            if (f != (T)0) sum += f * (xi - x[j]);
         }
+        (warp == 0 ? gx : (warp == 1 ? gy : gz))[base + lane] = sum;
     }
 }
 

@@ -359,6 +359,33 @@ def test_atoms_at_the_end_of_the_angular_list(gpu, oracle_mod, n_mols, n, dt):
         assert normwise(out, ref) < FTOL[dt]
 
 
+@pytest.mark.parametrize("n_mols", [2, 148, 149, 593, 741])
+@pytest.mark.parametrize("radius", [1.54, 2.2])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_gradient_in_batches_of_central_atoms(gpu, oracle_mod, n_mols, radius, dt):
+    """Molecules of every size up to 32 atoms, most atoms within A_Rc of one another (31 neighbours and 465 pairs an
+    atom): batches that end at each of their three limits, rows that two batches share, in every split of the gradient
+    kernel.  An atom whose row index is refused hands out nothing, and still gets what the others hand to it."""
+    sizes = (32, 16) if n_mols == 2 else range(1, 33)
+    b = _concat(*[_dense_blobs(1, n, radius, n) for n in sizes])
+    if n_mols > 32:
+        b = _concat(b, syn.gdb_like_batch(n_mols - 32, 4))
+    si, gi, ac = oracle_mod.ani_sort(b.atomic_numbers)
+    up = syn.upstream_grads(b, ac, dtype=dt)
+    refused = int(b.mol_offsets[1])
+    up[b.atomic_numbers[refused]].reshape(-1, 384)[si[refused]] = 0      # what the oracle takes for no row
+    args = [v.astype(np.float64) for v in b.coords(dt)] + [b.atomic_numbers, b.mol_offsets, b.mol_atom_counts, si, ac]
+    ref = oracle_mod.featurize_grad(*args, *[u.astype(np.float64) for u in up], impl="port", threads=8)
+    for row in (si[refused], -1):
+        rows = si.copy()
+        rows[refused] = row
+        x, y, z, a, mo, mac = gpu.batch_tensors(b, dt)
+        out = gpu.ani_mod.featurize_grad(x, y, z, a, mo, mac, gpu.to_dev(rows), ac, *[gpu.to_dev(u.astype(dt)) for u in up])
+        for k in range(3):
+            assert normwise(out[k].cpu().numpy(), ref[k]) < FTOL[dt], (row, k)
+        assert (gpu.ani_mod.device_status() != 0) == (row < 0)
+
+
 @pytest.mark.parametrize("n_mols", [1, 30, 75])
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 def test_large_molecules_at_every_split(gpu, oracle_mod, n_mols, dt):
