@@ -224,7 +224,7 @@ int check_acs(const int* acs_host, long long* n_atoms)
 template <typename T, int CAPT = kCapT, int CAPR = kCapR>
 int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, const int* mos,
                    const int* macs, int n_mols, const int* sis, T* oh, T* oc, T* on, T* oo,
-                   const int* acs_host, void* stream)
+                   const int* acs_host, void* stream, bool after_sort = false)
 {
     long long n_atoms = 0;
     if (int rc = check_acs(acs_host, &n_atoms)) return rc;
@@ -253,7 +253,7 @@ int featurize_impl(const T* xs, const T* ys, const T* zs, const int* types, cons
         const int rounds = (kMolMaxAtoms + per_round - 1) / per_round;
         ANI_CUDA(launch_chain(featurize_mol_kernel<T>, n_mols * rounds, kWarp, 0, (cudaStream_t)stream, 1, xs, ys, zs,
                               types, mos, macs, n_mols, (int)n_atoms, sis, oh, oc, on, oo, acs_host[0], acs_host[1],
-                              acs_host[2], acs_host[3], per_round, 65536 / per_round + 1));
+                              acs_host[2], acs_host[3], per_round, 65536 / per_round + 1, after_sort));
         return ANI_OK;
     }
 
@@ -590,7 +590,8 @@ int energy_launch(const T* atom_energy_sorted, const int* gather, const int* mos
 template <typename T>
 int mlp_small_launch(const T* feat, const int* acs, const T* const* w1, const T* const* b1, const T* const* w2,
                      const T* const* b2, const T* const* w3, const T* const* b3, const T* const* w4, const T* const* b4,
-                     const T* grad_energy, T* energy, T* grad_feat, int activation, bool early_weights, cudaStream_t st)
+                     const T* grad_energy, T* energy, T* grad_feat, int activation, bool early_weights, cudaStream_t st,
+                     const MlpPackParams* pack = nullptr)
 {
     if (activation < 0 || activation > 3) return ANI_ERR_BAD_SIZE;
     MlpSmallParams<T> p;
@@ -627,7 +628,9 @@ int mlp_small_launch(const T* feat, const int* acs, const T* const* w1, const T*
         if (int rc = set_smem(kernel, smem)) return rc;
         configured_dev = dev;
     }
-    ANI_CUDA(launch_chain(kernel, tiles * kSmallCtas, kSmallThreads, smem, st, kSmallCtas, p));
+    static_assert(kPackChunks * kTypes % kSmallCtas == 0, "whole clusters pack");
+    ANI_CUDA(launch_chain(kernel, tiles * kSmallCtas + (pack ? kPackChunks * kTypes : 0), kSmallThreads, smem, st, kSmallCtas, p,
+                          pack ? *pack : MlpPackParams{}));
     return ANI_OK;
 }
 
@@ -1358,11 +1361,19 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
     auto rows = [&](float* base, int t, int width) -> float* {
         return base && acs[t] > 0 ? base + start[t] * (size_t)width : nullptr;
     };
-    bool sorted = false;
+    const bool transient = (a->phases & ANI_PASS_TRANSIENT) != 0;
+    const bool small_networks = (a->phases & ANI_PASS_FORWARD) && transient && few_atoms(acs) &&
+                                !(a->phases & ANI_PASS_WEIGHT_GRAD) && !a->labels;
+    bool sorted = false, pack_later = false;
+    MlpPackParams p = {};
     if (a->phases & ANI_PASS_PACK) {
-        MlpPackParams p;
         bool any = false;
         if (int rc = pack_params(a->w1, a->w2, a->w3, a->packed, &p, &any)) return rc;
+        // networks of few atoms do not read the packed weights: packed beside them, on SMs that have nothing to do
+        if (any && small_networks && n_atoms > 0) {
+            pack_later = true;
+            any = false;
+        }
         // with a sort of one launch in the same pass: both in one kernel
         if (any && (a->phases & ANI_PASS_FEATURIZE) && n_atoms > 0 && n_atoms <= kSortSingleLaunchMax) {
             if (!a->atomic_numbers || !a->scatter_idxs || !a->gather_idxs || !a->atom_counts) return ANI_ERR_NULL_POINTER;
@@ -1379,21 +1390,21 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
         if (!sorted)
             if (int rc = ani_sort(a->atomic_numbers, a->n_atoms, a->scatter_idxs, a->gather_idxs, a->atom_counts, stream))
                 return rc;
-        if (int rc = ani_featurize_f32(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
-                                       a->n_mols, a->scatter_idxs, rows(a->features, 0, kTotal),
-                                       rows(a->features, 1, kTotal), rows(a->features, 2, kTotal),
-                                       rows(a->features, 3, kTotal), acs, stream))
+        if (int rc = featurize_impl<float>(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
+                                           a->n_mols, a->scatter_idxs, rows(a->features, 0, kTotal),
+                                           rows(a->features, 1, kTotal), rows(a->features, 2, kTotal),
+                                           rows(a->features, 3, kTotal), acs, stream, n_atoms <= kSortSingleLaunchMax))
             return rc;
     }
-    const bool transient = (a->phases & ANI_PASS_TRANSIENT) != 0;
     bool backward_done = false;
-    if ((a->phases & ANI_PASS_FORWARD) && transient && few_atoms(acs) && !(a->phases & ANI_PASS_WEIGHT_GRAD) && !a->labels) {
+    if (small_networks) {
         const bool backward = (a->phases & ANI_PASS_BACKWARD) && a->feature_grads;
         if (n_atoms > 0)
             if (int rc = mlp_small_launch<float>(a->features, acs, a->w1, a->b1, a->w2, a->b2, a->w3, a->b3, a->w4, a->b4,
                                                  a->grad_energy_sorted, a->energy_sorted,
                                                  backward ? a->feature_grads : nullptr, a->activation,
-                                                 (a->phases & ANI_PASS_FEATURIZE) != 0, (cudaStream_t)stream))
+                                                 (a->phases & ANI_PASS_FEATURIZE) != 0, (cudaStream_t)stream,
+                                                 pack_later ? &p : nullptr))
                 return rc;
         backward_done = true;
     } else if ((a->phases & ANI_PASS_FORWARD) && (a->phases & ANI_PASS_BACKWARD) && transient && a->feature_grads &&
@@ -1514,8 +1525,9 @@ int ani_energy_pass_f64(const ani_energy_args_f64* a, void* stream)
     if (a->phases & ANI_PASS_FEATURIZE) {
         if (int rc = ani_sort(a->atomic_numbers, a->n_atoms, a->scatter_idxs, a->gather_idxs, a->atom_counts, stream))
             return rc;
-        if (int rc = ani_featurize_f64(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts, a->n_mols,
-                                       a->scatter_idxs, rows[0], rows[1], rows[2], rows[3], acs, stream))
+        if (int rc = featurize_impl<double>(a->xs, a->ys, a->zs, a->atomic_numbers, a->mol_offsets, a->mol_atom_counts,
+                                            a->n_mols, a->scatter_idxs, rows[0], rows[1], rows[2], rows[3], acs, stream,
+                                            n_atoms <= kSortSingleLaunchMax))
             return rc;
     }
     if ((a->phases & ANI_PASS_FORWARD) && n_atoms > 0) {

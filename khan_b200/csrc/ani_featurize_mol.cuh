@@ -125,15 +125,16 @@ template <typename T>
 __device__ __forceinline__ void load_sorted_molecule(const T* __restrict__ xs, const T* __restrict__ ys,
                                                      const T* __restrict__ zs, const int* __restrict__ types,
                                                      const int* __restrict__ scatter, int base, int n,
-                                                     MolSortShared* sh, MolLanes<T>* out)
+                                                     MolSortShared* sh, MolLanes<T>* out, bool scatter_is_new = false)
 {
     unsigned char* inv = sh->src;
     const int lane = lane_id();
     const bool live = lane < n;
     const int gj = base + (live ? lane : 0);
     const T x0 = xs[gj], y0 = ys[gj], z0 = zs[gj];
-    const int s0 = scatter[gj];
     const int t0 = live ? checked_type(types[gj]) : kTypes;
+    if (scatter_is_new) pdl_wait();
+    const int s0 = scatter[gj];
     const unsigned m0 = __ballot_sync(kFull, t0 == 0), m1 = __ballot_sync(kFull, t0 == 1),
                    m2 = __ballot_sync(kFull, t0 == 2), m3 = __ballot_sync(kFull, t0 == 3);
     const int c0 = __popc(m0), c1 = __popc(m1), c2 = __popc(m2);
@@ -180,19 +181,21 @@ __device__ __forceinline__ bool decode_slot(const MolGroupInfo* tab, const unsig
     return valid;
 }
 
+// after_sort: the kernel before is the sort of the same call, which writes `scatter` only (of what is read here): the
+// molecule is read ahead of it.
 template <typename T>
 __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     featurize_mol_kernel(const T* __restrict__ xs, const T* __restrict__ ys, const T* __restrict__ zs,
                          const int* __restrict__ types, const int* __restrict__ mol_offsets,
                          const int* __restrict__ mol_counts, int n_mols, int n_atoms,
                          const int* __restrict__ scatter, T* out_h, T* out_c, T* out_n, T* out_o,
-                         int acs0, int acs1, int acs2, int acs3, int per_round, int per_round_recip)
+                         int acs0, int acs1, int acs2, int acs3, int per_round, int per_round_recip, bool after_sort)
 {
     __shared__ MolFwdWarpShared<T> ws;
     using Granule = Vec4<float>;                      // 16 bytes of zeros, whatever T is
     constexpr int kPerGranule = 16 / (int)sizeof(T);  // values in a granule
     const int lane = lane_id();
-    pdl_wait();
+    if (!after_sort) pdl_wait();
 
     // Round-major order of the grid: all first rounds (every molecule has one), then all second rounds, ...
     // so the work that exists starts first and is spread evenly over the SMs, and the CTAs of rounds that
@@ -204,6 +207,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     const int n = mol.n, base = mol.base;
 
     if (n > kMolMaxAtoms) {   // a large molecule in a batch of small ones: its CTAs take one atom at a time
+        pdl_wait();
         for (int i = round; i < n; i += gridDim.x / n_mols) {
             const int gi = base + i;
             const int ti = checked_type(types[gi]);
@@ -227,7 +231,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     const int G = (n - round + n_rounds - 1) / n_rounds;
 
     MolLanes<T> ml;
-    load_sorted_molecule<T>(xs, ys, zs, types, scatter, base, n, &ws.sort, &ml);
+    load_sorted_molecule<T>(xs, ys, zs, types, scatter, base, n, &ws.sort, &ml, after_sort);
 
     // Padding slots read entry 0 of the angular list, possibly before anything was written there.
     if (lane == 0) {

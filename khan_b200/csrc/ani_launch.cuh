@@ -5,8 +5,9 @@
 // set up while its predecessor drains; pdl_wait() holds it until everything before it in the stream has
 // finished and is visible.  Rules that every kernel of this library launched this way keeps:
 //   * pdl_wait() comes before the first access to memory that an earlier kernel of the stream may write,
-//     and before the first store; weights may be read ahead of it where the kernel before is known not to
-//     write any (the flag early_weights of mlp_small_kernel);
+//     and before the first store; weights and the geometry may be read ahead of it where the kernel before is one of
+//     the same call and known not to write any (early_weights of the network kernels, after_sort of the features,
+//     early_inputs of the gradient);
 //   * pdl_trigger() comes after pdl_wait(), so whatever lies two kernels back has finished when a kernel
 //     starts; a kernel that writes weights never triggers;
 //   * the kernels that fill the device with small molecules, and the sort in front of them, do not trigger at once.

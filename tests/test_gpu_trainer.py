@@ -225,6 +225,32 @@ def test_energy_forces_evaluator_matches_the_trainer():
     assert torch.equal(sb.grads[:, :b.n_atoms], keep_g)
 
 
+@pytest.mark.parametrize("n_mols", [1, 30])
+def test_a_pass_over_few_atoms_refreshes_the_packed_weights(n_mols):
+    """Networks of few atoms do not read the packed weights, but their pass refreshes them for a larger one."""
+    import torch
+    from khan_b200.inference import EnergyForces
+    from khan_b200.model.nn import MoleculeNN
+    from khan_b200.staged import HostBatch, StagedBatch
+    model = MoleculeNN(device="cuda:0", seed=2)
+
+    def staged(b):
+        sb = StagedBatch(b.n_atoms, b.n_mols)
+        sb.upload(HostBatch(b, None, pin=False), non_blocking=False, with_upstream=False)
+        return sb, EnergyForces(model, b.n_atoms, b.n_mols)
+    (few, ev_few), (many, ev_many) = staged(syn.config1(n_mols=n_mols)), staged(syn.config1(n_mols=200))
+    ev_few.run(few)                                   # allocates the packed copy
+    with torch.no_grad():
+        for p in model.get_parameters():
+            p.mul_(1.25)
+    ev_few.run(few)
+    ev_many.run(many, pack=False)
+    got = ev_many.mol_energy[:many.n_mols].clone()
+    ev_many.run(many)
+    torch.cuda.synchronize()
+    assert torch.equal(got, ev_many.mol_energy[:many.n_mols])
+
+
 def test_fused_train_step_matches_the_autograd_step():
     """FusedTrainStep (C ABI only) against the same step driven by torch autograd: same loss,
     same weight gradients, same coordinate gradients, same weights after the update."""
