@@ -96,7 +96,7 @@ class ForceFitArgs(ctypes.Structure):
     _fields_ = ([("pass_", PassArgs)]
                 + [(n, ctypes.c_void_p) for n in ("fx", "fy", "fz", "vx", "vy", "vz", "feature_rates", "r1", "r2", "adot1",
                                                   "adot2", "adot3", "q1", "q2", "q3", "partial", "rmse", "z1", "z2", "z3", "z_ready")]
-                + [("part", ctypes.c_int)])
+                + [("part", ctypes.c_int), ("side_stream", ctypes.c_void_p), ("features_ready", ctypes.c_void_p)])
 
 
 class EnergyArgs64(ctypes.Structure):
@@ -183,7 +183,6 @@ SIGNATURES = {
     "ani_host_pack_batch": (_i, [_vp]),
     "ani_network_pass_f32": (_i, [ctypes.POINTER(PassArgs), _vp]),
     "ani_force_fit_pass_f32": (_i, [ctypes.POINTER(ForceFitArgs), _vp]),
-    "ani_bias_celu_f32": (_i, [_vp, _vp, _vp, c_int_p, _i, _vp]),
     "ani_energy_pass_f64": (_i, [ctypes.POINTER(EnergyArgs64), _vp]),
     "ani_request": (_i, [ctypes.POINTER(RequestArgs), _vp]),
     "ani_feeder_create": (_i, [_i, _vp, _i, ctypes.POINTER(_vp)]),
@@ -261,7 +260,7 @@ def build_ops(force: bool = False) -> str:
         import numpy
         cmd += ["-I" + d for d in cpp_extension.include_paths("cuda") + [sysconfig.get_paths()["include"], numpy.get_include()]]
         cmd += ["-L" + d for d in cpp_extension.library_paths("cuda")]
-        cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lcudart", "-lcublas"]
+        cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lcudart"]
         out = subprocess.run(cmd, capture_output=True, text=True)
         if out.returncode != 0:
             raise RuntimeError("g++ failed building _torch_ops.so:\n" + out.stderr)
@@ -278,8 +277,7 @@ def torch_ops():
             raise RuntimeError(f"{OPS_PATH} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
         from . import _torch_ops as mod
         mod.bind(*(ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in (
-            "ani_sort", "ani_featurize_f32", "ani_featurize_f64", "ani_featurize_grad_f32", "ani_featurize_grad_f64",
-            "ani_bias_celu_f32")))
+            "ani_sort", "ani_featurize_f32", "ani_featurize_f64", "ani_featurize_grad_f32", "ani_featurize_grad_f64")))
         _ops = mod
     return _ops
 

@@ -634,6 +634,43 @@ int mlp_small_launch(const T* feat, const int* acs, const T* const* w1, const T*
     return ANI_OK;
 }
 
+// Pre-activations of the hidden layers with celu, in plain float32 products.
+int celu_preactivations_launch(const ani_pass_args* a, const int* acs, float* z1, float* z2, float* z3, cudaStream_t st)
+{
+    CeluPreParams p = {};
+    p.feat = a->features;
+    p.z[0] = z1; p.z[1] = z2; p.z[2] = z3;
+    p.aligned = all_aligned16({a->features});
+    int tiles = 0, row = 0;
+    for (int t = 0; t < kTypes; t++) {
+        const float* const w[3] = {a->w1[t], a->w2[t], a->w3[t]};
+        const float* const b[3] = {a->b1[t], a->b2[t], a->b3[t]};
+        for (int l = 0; l < 3; l++) {
+            if (acs[t] > 0 && (!w[l] || !b[l])) return ANI_ERR_NULL_POINTER;
+            p.aligned = p.aligned && (acs[t] == 0 || all_aligned16({w[l]}));
+            p.w[l][t] = w[l];
+            p.bias[l][t] = b[l];
+        }
+        p.count[t] = acs[t];
+        p.row_start[t] = row;
+        p.tile_start[t] = tiles;
+        row += acs[t];
+        tiles += (acs[t] + kCeluRows - 1) / kCeluRows;
+    }
+    p.tile_start[kTypes] = tiles;
+    if (tiles == 0) return ANI_OK;
+    if (!all_aligned16({z1, z2, z3})) return ANI_ERR_MISALIGNED;
+    static thread_local int configured_dev = -1;
+    int dev = 0;
+    ANI_CUDA(cudaGetDevice(&dev));
+    if (configured_dev != dev) {
+        if (int rc = set_smem(celu_preactivations_kernel, sizeof(CeluPreShared))) return rc;
+        configured_dev = dev;
+    }
+    ANI_CUDA(launch_chain(celu_preactivations_kernel, tiles, kCeluThreads, sizeof(CeluPreShared), st, 1, p));
+    return ANI_OK;
+}
+
 // True when every element that has atoms comes with packed weights.
 bool all_packed(const void* const* packed, const int* acs)
 {
@@ -1572,31 +1609,6 @@ int ani_request(const ani_request_args* a, void* stream)
     return ANI_OK;
 }
 
-int ani_bias_celu_f32(float* z, float* a, const float* const* bias, const int* acs_host, int width, void* stream)
-{
-    long long n_atoms = 0;
-    if (int rc = check_acs(acs_host, &n_atoms)) return rc;
-    if (width <= 0 || (width & 3) || n_atoms * width > 0x7fffffffLL) return ANI_ERR_BAD_SIZE;
-    if (n_atoms == 0) return ANI_OK;
-    if (!z || !bias) return ANI_ERR_NULL_POINTER;
-    BiasCeluParams p;
-    p.z = z;
-    p.a = a;
-    p.rows = (int)n_atoms;
-    p.width = width;
-    int row = 0;
-    for (int t = 0; t < kTypes; t++) {
-        if (acs_host[t] > 0 && !bias[t]) return ANI_ERR_NULL_POINTER;
-        if (!all_aligned16({bias[t]})) return ANI_ERR_MISALIGNED;
-        p.bias[t] = bias[t];
-        row += acs_host[t];
-        p.row_end[t] = row;
-    }
-    if (!all_aligned16({z, a})) return ANI_ERR_MISALIGNED;
-    ANI_CUDA(launch_chain(bias_celu_kernel, (int)((n_atoms * (width / 4) + 255) / 256), 256, 0, (cudaStream_t)stream, 1, p));
-    return ANI_OK;
-}
-
 int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
 {
     if (!f) return ANI_ERR_NULL_POINTER;
@@ -1616,14 +1628,29 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
             return ANI_ERR_NULL_POINTER;
     if (!all_aligned16({f->feature_rates, f->r1, f->r2, f->adot1, f->adot2, f->adot3, f->q1, f->q2, f->q3}))
         return ANI_ERR_MISALIGNED;
+    const bool signs_here = f->side_stream && a->activation == kActCelu && f->z1 && f->z2 && f->z3;
+    if (signs_here && (!f->features_ready || !f->z_ready)) return ANI_ERR_NULL_POINTER;
     cudaStream_t st = (cudaStream_t)stream;
     const int n = (int)n_atoms;
 
     // coordinate gradients of the energy: the first-order pass, which also leaves dE/dA_l
     if (f->part != 2) {
         ani_pass_args first = *a;
-        first.phases = (a->phases & (ANI_PASS_PACK | ANI_PASS_FEATURIZE)) | ANI_PASS_FORWARD;
         first.labels = nullptr;
+        const int before = a->phases & (ANI_PASS_PACK | ANI_PASS_FEATURIZE);
+        if (signs_here) {
+            // beside the networks, on the stream that the caller keeps for it
+            first.phases = before;
+            if (int rc = ani_network_pass_f32(&first, stream)) return rc;
+            const cudaStream_t side = (cudaStream_t)f->side_stream;
+            ANI_CUDA(cudaEventRecord((cudaEvent_t)f->features_ready, st));
+            ANI_CUDA(cudaStreamWaitEvent(side, (cudaEvent_t)f->features_ready, 0));
+            if (int rc = celu_preactivations_launch(a, acs, const_cast<float*>(f->z1), const_cast<float*>(f->z2),
+                                                    const_cast<float*>(f->z3), side))
+                return rc;
+            ANI_CUDA(cudaEventRecord((cudaEvent_t)f->z_ready, side));
+        }
+        first.phases = (signs_here ? 0 : before) | ANI_PASS_FORWARD;
         if (int rc = ani_network_pass_f32(&first, stream)) return rc;
         {
             ani_mlp_backward_args b;

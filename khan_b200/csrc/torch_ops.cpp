@@ -10,7 +10,6 @@
 // refuses and calls again.  A negative status of the library is returned as an int.  The entry points are
 // handed over as addresses (bind), so that there is one copy of the library in the process.
 #include <ATen/cuda/CUDAContext.h>
-#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/core/LegacyTypeDispatch.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -21,9 +20,6 @@
 
 #include <stdint.h>
 
-#include <condition_variable>
-#include <mutex>
-#include <thread>
 #include <vector>
 
 namespace py = pybind11;
@@ -42,13 +38,8 @@ SortFn g_sort = nullptr;
 FeaturizeFn g_featurize[2] = {};   // f32, f64
 GradFn g_grad[2] = {};
 
-using BiasCeluFn = int (*)(float*, float*, const float* const*, const int*, int, void*);
-BiasCeluFn g_bias_celu = nullptr;
-
-void bind(uintptr_t sort, uintptr_t featurize_f32, uintptr_t featurize_f64, uintptr_t grad_f32, uintptr_t grad_f64,
-          uintptr_t bias_celu)
+void bind(uintptr_t sort, uintptr_t featurize_f32, uintptr_t featurize_f64, uintptr_t grad_f32, uintptr_t grad_f64)
 {
-    g_bias_celu = reinterpret_cast<BiasCeluFn>(bias_celu);
     g_sort = reinterpret_cast<SortFn>(sort);
     g_featurize[0] = reinterpret_cast<FeaturizeFn>(featurize_f32);
     g_featurize[1] = reinterpret_cast<FeaturizeFn>(featurize_f64);
@@ -191,132 +182,6 @@ py::object featurize_grad(const at::Tensor& x, const at::Tensor& y, const at::Te
     return py::make_tuple(out.as_strided({n}, {1}, 0), out.as_strided({n}, {1}, n), out.as_strided({n}, {1}, 2 * n));
 }
 
-// Pre-activations z[l] of the three hidden layers with celu, in plain float32 products: per element and layer one
-// library GEMM (the call that at::mm makes, without its 6 us of dispatch) and one kernel for bias and activation.
-//
-// The elements are independent chains, each on a stream of its own beside the caller's, and a GEMM call takes 10 us of
-// host time: one thread spent 133 us issuing the twelve (four streams from one thread: 172), more than the GPU needs for
-// them; four threads 90.  Four batches of 256 molecules 1100 -> 1016 us.  Three helper threads, which
-// live as long as the object, and the caller take the elements as they come.  Calls must not overlap.
-class CeluPreactivations {
-  public:
-    // weights / biases [layer * 4 + element]; z, a: [>= n, width] buffers per layer, a of the first two
-    CeluPreactivations(std::vector<at::Tensor> weights, std::vector<at::Tensor> biases, std::vector<at::Tensor> z,
-                       std::vector<at::Tensor> a)
-        : weights_(std::move(weights)), biases_(std::move(biases)), z_(std::move(z)), a_(std::move(a))
-    {
-        TORCH_CHECK(weights_.size() == 12 && biases_.size() == 12 && z_.size() == 3 && a_.size() == 2);
-        for (const auto* list : {&weights_, &biases_, &z_, &a_})
-            for (const at::Tensor& t : *list) TORCH_CHECK(fits(t, c10::kFloat, z_[0].device()));
-        for (int t = 0; t < 4; t++) streams_.push_back(c10::cuda::getStreamFromPool(false, z_[0].device().index()));
-        for (int t = 0; t < 3; t++) helpers_.emplace_back([this] { help(); });
-    }
-    ~CeluPreactivations()
-    {
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            stop_ = true;
-        }
-        cv_.notify_all();
-        for (std::thread& t : helpers_) t.join();
-    }
-    // The features (and the last reader of z) are among the work enqueued on the current stream so far.
-    void begin()
-    {
-        const c10::cuda::CUDAGuard device(z_[0].device());
-        started_.record(c10::cuda::getCurrentCUDAStream());
-    }
-    // features: [>= n, 384], element-sorted, as of begin()
-    int run(const at::Tensor& features, py::handle counts)
-    {
-        TORCH_CHECK(read_counts(counts.ptr(), acs_) && fits(features, c10::kFloat, z_[0].device()));
-        const c10::cuda::CUDAGuard device(features.device());
-        features_ = features.const_data_ptr<float>();
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            next_ = 0;
-            open_ = 4;
-            rc_ = 0;
-        }
-        cv_.notify_all();
-        std::unique_lock<std::mutex> lk(mu_);
-        while (take(lk)) {}
-        finished_.wait(lk, [this] { return open_ == 0; });
-        if (rc_) return rc_;
-        for (int t = 1; t < 4; t++)
-            if (acs_[t] > 0) element_done_[t].block(streams_[0]);
-        done_.record(streams_[0]);
-        return 0;
-    }
-    uintptr_t done() { return reinterpret_cast<uintptr_t>(done_.event()); }
-
-  private:
-    void help()
-    {
-        std::unique_lock<std::mutex> lk(mu_);
-        for (;;) {
-            cv_.wait(lk, [this] { return stop_ || next_ < 4; });
-            if (stop_) return;
-            take(lk);
-        }
-    }
-    // One element, if there is one left; `lk` holds mu_ before and after.
-    bool take(std::unique_lock<std::mutex>& lk)
-    {
-        if (next_ >= 4) return false;
-        const int t = next_++;
-        lk.unlock();
-        int rc = -3;       // ANI_ERR_CUDA
-        try {
-            rc = acs_[t] > 0 ? element(t) : 0;
-        } catch (const std::exception&) {
-        }
-        lk.lock();
-        if (rc) rc_ = rc;
-        if (--open_ == 0) finished_.notify_all();
-        return true;
-    }
-    int element(int t)
-    {
-        const c10::cuda::CUDAStreamGuard guard(streams_[t]);
-        started_.block(streams_[t]);
-        const int64_t inputs[3] = {kFeatures, 128, 128};
-        const float one = 1.0f, zero = 0.0f;
-        int64_t row = 0;
-        for (int u = 0; u < t; u++) row += acs_[u];
-        int only[4] = {};
-        only[t] = acs_[t];
-        const cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();
-        for (int l = 0; l < 3; l++) {
-            const int64_t k = inputs[l], n = z_[l].size(1);
-            const float* in = (l == 0 ? features_ : a_[l - 1].const_data_ptr<float>()) + row * k;
-            float* out = z_[l].mutable_data_ptr<float>() + row * n;
-            if (cublasSgemm(handle, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, acs_[t], (int)k, &one,
-                            weights_[l * 4 + t].const_data_ptr<float>(), (int)n, in, (int)k, &zero, out,
-                            (int)n) != CUBLAS_STATUS_SUCCESS)
-                return -3;
-            const float* bias[4] = {};
-            bias[t] = biases_[l * 4 + t].const_data_ptr<float>();
-            if (const int rc = g_bias_celu(out, l < 2 ? a_[l].mutable_data_ptr<float>() + row * n : nullptr, bias, only,
-                                           (int)n, streams_[t].stream()))
-                return rc;
-        }
-        element_done_[t].record(streams_[t]);
-        return 0;
-    }
-
-    std::vector<at::Tensor> weights_, biases_, z_, a_;
-    std::vector<c10::cuda::CUDAStream> streams_;      // per element
-    at::cuda::CUDAEvent started_, element_done_[4], done_;
-    const float* features_ = nullptr;
-    int acs_[4] = {};
-    std::vector<std::thread> helpers_;
-    std::mutex mu_;
-    std::condition_variable cv_, finished_;
-    int next_ = 4, open_ = 0, rc_ = 0;
-    bool stop_ = false;
-};
-
 // Row ranges [cuts[k] - cuts[0], cuts[k + 1] - cuts[0]) of a C-contiguous 2-d array as a list of views.  Cutting the
 // gradients of a batch into molecules is what coordinate_gradients spends its host time on: 1024 views take 160 us
 // through slice objects, 85 us here.
@@ -361,9 +226,4 @@ PYBIND11_MODULE(_torch_ops, m)
     m.def("featurize", &featurize);
     m.def("featurize_into", &featurize_into);
     m.def("featurize_grad", &featurize_grad);
-    py::class_<CeluPreactivations>(m, "CeluPreactivations")
-        .def(py::init<std::vector<at::Tensor>, std::vector<at::Tensor>, std::vector<at::Tensor>, std::vector<at::Tensor>>())
-        .def("begin", &CeluPreactivations::begin)
-        .def("run", &CeluPreactivations::run)
-        .def("done", &CeluPreactivations::done);
 }

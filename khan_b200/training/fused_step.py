@@ -231,11 +231,12 @@ class ForceFitStep(FusedTrainStep):
         self.partial = torch.empty(192, dtype=torch.float64, device=self.device)
         self.rmse = torch.zeros(1, **f32)
         self.celu = model.activation_fn is activations.celu
-        if self.celu:      # see bias_celu_kernel: the signs of the pre-activations come from plain float32 products
+        if self.celu:      # the signs of the pre-activations come from plain float32 products, beside the first-order pass
             self.z = [torch.empty((n_atoms, w), **f32) for w in (128, 128, 64)]
-            layers = [[t.detach() for t in ts] for ts in zip(*[ann.Ws[:3] + ann.bs[:3] for ann in model.anns])]
-            self.preactivations = _lib.torch_ops().CeluPreactivations(
-                sum(layers[:3], []), sum(layers[3:], []), self.z, [torch.empty((n_atoms, 128), **f32) for _ in range(2)])
+            self.side = torch.cuda.Stream(device=self.device)
+            self.events = [torch.cuda.Event(), torch.cuda.Event()]
+            for event in self.events:
+                event.record(self.side)              # creates it
 
         f = self._force_args = _lib.ForceFitArgs()      # a batch changes the pass and the targets only
         f.vx, f.vy, f.vz = (self.v[k].data_ptr() for k in range(3))
@@ -244,6 +245,8 @@ class ForceFitStep(FusedTrainStep):
             setattr(f, name, t.data_ptr())
         if self.celu:
             f.z1, f.z2, f.z3 = (z.data_ptr() for z in self.z)
+            f.side_stream = self.side.cuda_stream
+            f.features_ready, f.z_ready = (event.cuda_event for event in self.events)
 
     def weight_gradients_of_forces(self, sb: StagedBatch, forces: torch.Tensor) -> None:
         """``forces``: the batch's target forces ``[3, n_atoms]``.  Afterwards ``self.rmse`` holds the sum of
@@ -258,21 +261,10 @@ class ForceFitStep(FusedTrainStep):
         a.x_grads, a.y_grads, a.z_grads = g, g + cap * size, g + 2 * cap * size
         a.feature_grads, a.labels = sb.upstream.data_ptr(), None
         a.phases = _lib.PASS_PACK | _lib.PASS_FEATURIZE
-        f, call = self._force_args, _lib.lib().ani_force_fit_pass_f32
+        f = self._force_args
         f.fx, f.fy, f.fz = (forces[k].data_ptr() for k in range(3))
-        f.part = 0
-        if self.celu:
-            _lib.check(_lib.lib().ani_network_pass_f32(ctypes.byref(a), stream), "ani_network_pass_f32")
-            a.phases = 0
-            self.preactivations.begin()
         f.pass_ = a
-        if self.celu:
-            # the GPU has the first-order pass to work on while the host issues the library products
-            f.part = 1
-            _lib.check(call(ctypes.byref(f), stream), "ani_force_fit_pass_f32")
-            _lib.check(self.preactivations.run(sb.features, sb.acs_host), "CeluPreactivations")
-            f.z_ready, f.part = self.preactivations.done(), 2
-        _lib.check(call(ctypes.byref(f), stream), "ani_force_fit_pass_f32")
+        _lib.check(_lib.lib().ani_force_fit_pass_f32(ctypes.byref(f), stream), "ani_force_fit_pass_f32")
         self._args_key = None
 
 

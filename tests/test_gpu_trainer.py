@@ -494,6 +494,45 @@ def test_force_training_step_matches_the_autograd_path(act, n_mols):
         assert float((g.double() * scale - w).abs().max()) < 1e-4 * norm
 
 
+@pytest.mark.parametrize("elements", [(1, 0, 0, 0), (31, 32, 33, 0), (0, 5, 64, 97), (300, 1, 1, 1)])
+def test_celu_preactivations(elements):
+    """The pre-activations whose signs force training takes, against float64: tiles of 32 atoms per element, none, one,
+    a row less and a row more.  A float32 sum of 384 products is off by sqrt(384) half ulps of its largest terms, here
+    1.2e-6 of the largest value, which the layers behind it carry on."""
+    import torch
+    from khan_b200 import FlatNadam
+    from khan_b200.model.nn import MoleculeNN
+    from khan_b200.staged import StagedBatch
+    from khan_b200.training.fused_step import ForceFitStep
+    n = sum(elements)
+    rng = np.random.default_rng(n)
+    model = MoleculeNN(device="cuda:0", seed=1)
+    with torch.no_grad():
+        for p in model.get_parameters():
+            if p.dim() == 1:
+                p.copy_(torch.from_numpy(rng.normal(0.0, 0.1, p.shape).astype(np.float32)))
+    optimizer = FlatNadam(model.get_parameters(), lr=1e-5, clip_norm=5.0)
+    sb = StagedBatch(n, 1)
+    sb.set_shape(n, 1, np.array(elements, dtype=np.int32))
+    for to, v in zip((sb.x, sb.y, sb.z), rng.normal(0.0, 3.0 + 0.9 * n ** (1 / 3), (3, n))):
+        to.copy_(torch.from_numpy(v.astype(np.float32)))
+    sb.types.copy_(torch.from_numpy(np.repeat(np.arange(4), elements).astype(np.int32)))
+    sb.mol_offsets.zero_()
+    sb.mol_counts.fill_(n)
+    step = ForceFitStep(model, optimizer, n, 1)
+    step.weight_gradients_of_forces(sb, torch.zeros((3, n), device="cuda:0"))
+    torch.cuda.synchronize()
+    first = 0
+    for t, count in enumerate(elements):
+        a, ann = sb.features[first:first + count].double(), model.anns[t]
+        for l in range(3):
+            z = a @ ann.Ws[l].detach().double() + ann.bs[l].detach().double()
+            got = step.z[l][first:first + count].double()
+            assert count == 0 or float((got - z).abs().max()) < 2e-6 * float(z.abs().max()), (t, l)
+            a = torch.where(z >= 0, z, 0.1 * (torch.exp(10.0 * z) - 1.0))
+        first += count
+
+
 def test_passes_over_a_data_set_may_interleave_and_be_given_up():
     """Two passes at once, one of them abandoned after its first molecules, give what undisturbed passes give."""
     import torch
