@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_wgrad_kernel(const MlpW
 #pragma unroll
                 for (int ks = 0; ks < kPipeK / 8; ks++) {
                     const unsigned step = ks * 2 * kMlpLbo, col = ks * 8;
+                    // (hi hi and hi lo as one instruction of 256 columns, as in mlp_chain_kernel, was slower here: 19.6 us)
                     mma_tf32_ts(tmem + kTmemAcc, a_hi + col, pipe_desc(b_hi + step), idesc, !(c == 0 && ks == 0));
                     if (SPLIT) {
                         mma_tf32_ts(tmem + kTmemSmall, a_hi + col, pipe_desc(b_lo + step), idesc, !(c == 0 && ks == 0));
@@ -186,6 +187,45 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_wgrad_kernel(const MlpW
             tc_fence_before();
             mbar_arrive(&sh.full[g]);
         }
+        if (blk == 4 && p.dw4[e]) {
+            // output layer, done by the CTA with the lightest product while that comes to its end: dw4 = A3^T g and
+            // db4 = sum g over this range; no tensor cores involved.  Eight atoms' loads at once: one behind the other,
+            // and behind the product, they made the kernel 21.8 us long for 1024 molecules instead of 18.9.
+            const int q = tid & 15, a_in = tid >> 4;      // 16 column quads x 32 atoms per pass
+            const float* act = p.act3[e] + (size_t)first * kMlpH3 + 4 * q;
+            const float* up = p.grad_energy[e] ? p.grad_energy[e] + first : nullptr;
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            float gsum = 0.0f;
+            constexpr int kStep = kMlpThreads / 16;
+            for (int k0 = a_in; k0 < n_here; k0 += 8 * kStep) {
+                float4 v[8];
+                float ge[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int k = k0 + i * kStep;
+                    ge[i] = k < n_here ? (up ? up[k] : 1.0f) : 0.0f;
+                    v[i] = k < n_here ? *reinterpret_cast<const float4*>(act + (size_t)k * kMlpH3) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    acc.x += v[i].x * ge[i]; acc.y += v[i].y * ge[i]; acc.z += v[i].z * ge[i]; acc.w += v[i].w * ge[i];
+                    gsum += q == 0 ? ge[i] : 0.0f;
+                }
+            }
+            // the two halves of a warp hold the same columns
+            acc.x += __shfl_xor_sync(kFull, acc.x, 16);
+            acc.y += __shfl_xor_sync(kFull, acc.y, 16);
+            acc.z += __shfl_xor_sync(kFull, acc.z, 16);
+            acc.w += __shfl_xor_sync(kFull, acc.w, 16);
+            gsum += __shfl_xor_sync(kFull, gsum, 16);
+            if (lane < 16) {
+                atomicAdd(p.dw4[e] + 4 * q + 0, acc.x);
+                atomicAdd(p.dw4[e] + 4 * q + 1, acc.y);
+                atomicAdd(p.dw4[e] + 4 * q + 2, acc.z);
+                atomicAdd(p.dw4[e] + 4 * q + 3, acc.w);
+                if (q == 0 && p.db4[e]) atomicAdd(p.db4[e], gsum);
+            }
+        }
         bool ok = n_here > 0 && !timed_out;
         if (ok && !mbar_wait(&sh.done, 0u)) {
             ok = false;
@@ -211,32 +251,6 @@ __global__ void __launch_bounds__(kMlpAllThreads, 1) mlp_wgrad_kernel(const MlpW
                 warp_tile_to_global<true>(scratch, v, out + (size_t)tile_row0 * N + c0, N, 32);
             }
             if (bias_out && me < N && g < nchunks) atomicAdd(bias_out + me, colsum);
-        }
-        if (blk == 4 && p.dw4[e]) {
-            // output layer, done by the CTA with the lightest product: dw4 = A3^T g and db4 = sum g
-            // over this range; no tensor cores involved
-            const int q = tid & 15, a_in = tid >> 4;      // 16 column quads x 32 atoms per pass
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            float gsum = 0.0f;
-            for (int k = a_in; k < n_here; k += kMlpThreads / 16) {
-                const float ge = p.grad_energy[e] ? p.grad_energy[e][first + k] : 1.0f;
-                const float4 v = *reinterpret_cast<const float4*>(p.act3[e] + (size_t)(first + k) * kMlpH3 + 4 * q);
-                acc.x += v.x * ge; acc.y += v.y * ge; acc.z += v.z * ge; acc.w += v.w * ge;
-                gsum += q == 0 ? ge : 0.0f;
-            }
-            // the two halves of a warp hold the same columns
-            acc.x += __shfl_xor_sync(kFull, acc.x, 16);
-            acc.y += __shfl_xor_sync(kFull, acc.y, 16);
-            acc.z += __shfl_xor_sync(kFull, acc.z, 16);
-            acc.w += __shfl_xor_sync(kFull, acc.w, 16);
-            gsum += __shfl_xor_sync(kFull, gsum, 16);
-            if (lane < 16) {
-                atomicAdd(p.dw4[e] + 4 * q + 0, acc.x);
-                atomicAdd(p.dw4[e] + 4 * q + 1, acc.y);
-                atomicAdd(p.dw4[e] + 4 * q + 2, acc.z);
-                atomicAdd(p.dw4[e] + 4 * q + 3, acc.w);
-                if (q == 0 && p.db4[e]) atomicAdd(p.db4[e], gsum);
-            }
         }
     }
     tc_fence_before();
