@@ -24,8 +24,9 @@ namespace ani {
 //
 // One CTA takes 32 atoms of an element through the three hidden layers: their features stay in shared memory, the weights
 // come in chunks of 32 rows through two stages, a thread has 4 x 4 outputs (2 x 4 in layer 3), the rows of a warp are the
-// same for all its lanes.  Sums are taken chunk by chunk and then added up, which leaves them closer to float64 than one sum
-// of 384 products.  It runs beside the first-order pass, whose network kernels fill a fifth of the device for 256
+// same for all its lanes.  A sum runs over k = 0, 1, 2 ... in one accumulator, as in the library's float32 products, whose
+// bits it gives (sums of 32 products added up would be closer to float64, but every sign that they change moves single
+// gradients by a thousandth of their rms).  It runs beside the first-order pass, whose network kernels fill a fifth of the device for 256
 // molecules.  Before, these were twelve library GEMMs and twelve launches of bias and activation, issued by four threads:
 // 90 us of host time and 60 us at the end of the chain in a batch of 256 molecules, now one launch of 33 us beside the
 // networks: four such batches 990 -> 783 us.
@@ -80,7 +81,6 @@ __device__ __forceinline__ void celu_layer(CeluPreShared& sh, const float* a, in
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
-        float acc[R][4] = {};
 #pragma unroll
         for (int k = 0; k < 32; k += 4) {
             float v[R][4];
@@ -91,17 +91,13 @@ __device__ __forceinline__ void celu_layer(CeluPreShared& sh, const float* a, in
                 const float4 q = *reinterpret_cast<const float4*>(b + (k + i) * N);
 #pragma unroll
                 for (int r = 0; r < R; r++) {
-                    acc[r][0] = fmaf(v[r][i], q.x, acc[r][0]);
-                    acc[r][1] = fmaf(v[r][i], q.y, acc[r][1]);
-                    acc[r][2] = fmaf(v[r][i], q.z, acc[r][2]);
-                    acc[r][3] = fmaf(v[r][i], q.w, acc[r][3]);
+                    sum[r][0] = fmaf(v[r][i], q.x, sum[r][0]);
+                    sum[r][1] = fmaf(v[r][i], q.y, sum[r][1]);
+                    sum[r][2] = fmaf(v[r][i], q.z, sum[r][2]);
+                    sum[r][3] = fmaf(v[r][i], q.w, sum[r][3]);
                 }
             }
         }
-#pragma unroll
-        for (int r = 0; r < R; r++)
-#pragma unroll
-            for (int q = 0; q < 4; q++) sum[r][q] += acc[r][q];
         __syncthreads();      // the stage is free again
     }
 }

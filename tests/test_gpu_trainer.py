@@ -497,8 +497,8 @@ def test_force_training_step_matches_the_autograd_path(act, n_mols):
 @pytest.mark.parametrize("elements", [(1, 0, 0, 0), (31, 32, 33, 0), (0, 5, 64, 97), (300, 1, 1, 1)])
 def test_celu_preactivations(elements):
     """The pre-activations whose signs force training takes, against float64: tiles of 32 atoms per element, none, one,
-    a row less and a row more.  A float32 sum of 384 products is off by sqrt(384) half ulps of its largest terms, here
-    1.2e-6 of the largest value, which the layers behind it carry on."""
+    a row less and a row more.  A float32 sum of 384 products is off by about sqrt(384) half ulps (1.2e-6) of its largest
+    partial sum, which is up to three times the largest result; the layers behind carry that on."""
     import torch
     from khan_b200 import FlatNadam
     from khan_b200.model.nn import MoleculeNN
@@ -528,7 +528,7 @@ def test_celu_preactivations(elements):
         for l in range(3):
             z = a @ ann.Ws[l].detach().double() + ann.bs[l].detach().double()
             got = step.z[l][first:first + count].double()
-            assert count == 0 or float((got - z).abs().max()) < 2e-6 * float(z.abs().max()), (t, l)
+            assert count == 0 or float((got - z).abs().max()) < 4e-6 * float(z.abs().max()), (t, l)
             a = torch.where(z >= 0, z, 0.1 * (torch.exp(10.0 * z) - 1.0))
         first += count
 
