@@ -5,8 +5,8 @@
 //
 // The batch is cut into tiles of kSortTile consecutive atoms, one CTA per tile, one thread per
 // atom.  Inside a tile the rank is a warp-level split: each warp ranks its 32-atom segment
-// with one ballot per element and a popc of the lanes below, and the warp bases come from a
-// scan of the 32 per-warp counts by the first warp.  What differs between the two variants is
+// with one ballot per element and a popc of the lanes below, and a warp's base is the sum of the
+// counts of the warps in front of it.  What differs between the two variants is
 // where a tile learns how many atoms of each element precede it:
 //   * single launch (batches up to kSortSingleLaunchMax atoms): every CTA recounts the whole
 //     batch straight from the (L2-resident) input with wide, unrolled loads, so no scratch
@@ -31,43 +31,39 @@ struct Count4 {
     int c[kTypes];
 };
 
-__device__ __forceinline__ void tally(Count4& v, int t, bool on)
+// Counts travel as four fields of one or two words: bytes within a thread (at most 65 atoms each), 16-bit pairs of the
+// elements 0, 2 and 1, 3 within a warp, so that an atom costs a shift and an add and a sum over a warp one instruction a
+// word.  Element by element (a compare and an add each, five shuffles a sum, and a scan over the warps by the first one)
+// the kernel was a chain of shuffles and barriers: microseconds alone before -> now, 20 atoms 3.8 -> 1.9, 900 atoms 4.3 ->
+// 2.2, 14 thousand 5.9 -> 2.8, 28 thousand 8.7 -> 3.8, 55 thousand 13.3 -> 5.1.  What is left is a launch, two reads of
+// the L2 cache one behind the other and one barrier.
+struct Pair16 {
+    unsigned even, odd;      // elements 0 | 2 << 16 and 1 | 3 << 16
+};
+// 1 in the byte of the element (the funnel shift takes its distance modulo 32: elements modulo 4, as checked_type has them)
+__device__ __forceinline__ unsigned one_byte(int t) { return __funnelshift_l(0u, 1u, 8 * t); }
+__device__ __forceinline__ Pair16 widen(unsigned bytes) { return Pair16{bytes & 0x00ff00ffu, (bytes >> 8) & 0x00ff00ffu}; }
+__device__ __forceinline__ Pair16 warp_sum(Pair16 v)
 {
-    t = checked_type(t);
-#pragma unroll
-    for (int g = 0; g < kTypes; g++) v.c[g] += (on && t == g) ? 1 : 0;
+    return Pair16{__reduce_add_sync(kFull, v.even), __reduce_add_sync(kFull, v.odd)};
+}
+__device__ __forceinline__ Count4 unpack(Pair16 v)
+{
+    return Count4{{(int)(v.even & 0xffffu), (int)(v.odd & 0xffffu), (int)(v.even >> 16), (int)(v.odd >> 16)}};
 }
 
-// Sum of per-thread Count4 over the CTA; result valid in every thread.
-__device__ __forceinline__ Count4 block_sum(Count4 v, int (*red)[kTypes])
-{
-    const int lane = lane_id(), warp = warp_id();
-#pragma unroll
-    for (int g = 0; g < kTypes; g++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v.c[g] += __shfl_xor_sync(kFull, v.c[g], o);
-        if (lane == 0) red[warp][g] = v.c[g];
-    }
-    __syncthreads();
-    Count4 out;
-#pragma unroll
-    for (int g = 0; g < kTypes; g++) {
-        int s = lane < kSortWarps ? red[lane][g] : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-        out.c[g] = s;
-    }
-    __syncthreads();
-    return out;
-}
+struct SortShared {
+    uint4 counted[kSortWarps];     // per warp: what it counted in front of the tile and in all
+    Pair16 own[kSortWarps];        // per warp: its atoms of the tile
+};
 
-// Counts types[0, n) twice in one sweep: everything (`total`) and the part in front of
-// `split` (`before`).  `split` is a multiple of 4.  Loads are 16 bytes wide and issued four
+// Byte counts of types[0, n), n <= kSortSingleLaunchMax: everything (`total`) and the part in front of
+// `split` (`before`), a multiple of 4.  Loads are 16 bytes wide and issued four
 // at a time so that their L2 latencies overlap.
 __device__ __forceinline__ void count_two_ranges(const int* __restrict__ types, int n, int split,
-                                                 Count4* before, Count4* total)
+                                                 unsigned* before, unsigned* total)
 {
-    Count4 vb = {{0, 0, 0, 0}}, vt = {{0, 0, 0, 0}};
+    unsigned vb = 0u, vt = 0u, seen = 0u;
     const bool aligned = (reinterpret_cast<uintptr_t>(types) & 15u) == 0;
     const int nvec = aligned ? n / 4 : 0;
     const int4* p4 = reinterpret_cast<const int4*>(types);
@@ -82,80 +78,88 @@ __device__ __forceinline__ void count_two_ranges(const int* __restrict__ types, 
 #pragma unroll
         for (int u = 0; u < kUnroll; u++) {
             const int k = k0 + u * kSortThreads;
-            const bool on = k < nvec, front = on && 4 * k < split;
-            tally(vt, q[u].x, on); tally(vt, q[u].y, on); tally(vt, q[u].z, on); tally(vt, q[u].w, on);
-            tally(vb, q[u].x, front); tally(vb, q[u].y, front); tally(vb, q[u].z, front);
-            tally(vb, q[u].w, front);
+            const unsigned v = one_byte(q[u].x) + one_byte(q[u].y) + one_byte(q[u].z) + one_byte(q[u].w);
+            seen |= (unsigned)(q[u].x | q[u].y | q[u].z | q[u].w);
+            if (k < nvec) vt += v;
+            if (k < nvec && 4 * k < split) vb += v;
         }
     }
     for (int k = nvec * 4 + threadIdx.x; k < n; k += kSortThreads) {
         const int t = types[k];
-        tally(vt, t, true);
-        tally(vb, t, k < split);
+        seen |= (unsigned)t;
+        vt += one_byte(t);
+        if (k < split) vb += one_byte(t);
     }
+    if (seen >= (unsigned)kTypes) report(ANI_ERR_BAD_ELEMENT);
     *before = vb;
     *total = vt;
 }
 
-// Ranks the atoms of tile `tile` given the per-element counts in front of the tile (`before`)
-// and in the whole batch (`total`).
-__device__ __forceinline__ void rank_tile(const int* __restrict__ types, int n_atoms, int tile,
-                                          const Count4& before, const Count4& total,
-                                          int* __restrict__ scatter, int* __restrict__ gather,
-                                          int (*warp_counts)[kTypes])
+// An atom's rank among the atoms of its element in its warp, and the warp's counts.  t = -1: no atom.
+__device__ __forceinline__ int rank_in_warp(int t, Pair16* counts)
 {
-    const int lane = lane_id(), warp = warp_id();
-    const int i = tile * kSortTile + threadIdx.x;
-    const int t = i < n_atoms ? checked_type(types[i]) : -1;
-    int rank = 0;
+    unsigned m[kTypes], mine = 0u;
 #pragma unroll
     for (int g = 0; g < kTypes; g++) {
-        const unsigned m = __ballot_sync(kFull, t == g);
-        if (t == g) rank = __popc(m & lanemask_lt());
-        if (lane == 0) warp_counts[warp][g] = __popc(m);
+        m[g] = __ballot_sync(kFull, t == g);
+        if (t == g) mine = m[g];
     }
-    __syncthreads();
-    if (warp == 0) {  // exclusive scan over the warps, one element per step
+    *counts = Pair16{(unsigned)(__popc(m[0]) | __popc(m[2]) << 16), (unsigned)(__popc(m[1]) | __popc(m[3]) << 16)};
+    return __popc(mine & lanemask_lt());
+}
+
+// Atoms of each element in the warps of the tile in front of this one; `own` holds every warp's counts.
+__device__ __forceinline__ Count4 warps_in_front(const Pair16* own)
+{
+    const Pair16 v = own[lane_id()];
+    const bool front = lane_id() < warp_id();
+    return unpack(warp_sum(Pair16{front ? v.even : 0u, front ? v.odd : 0u}));
+}
+
+__device__ __forceinline__ void place_atom(int i, int t, int rank, const Count4& before, const Count4& in_tile,
+                                           const Count4& total, int* __restrict__ scatter, int* __restrict__ gather)
+{
+    int start = 0;
 #pragma unroll
-        for (int g = 0; g < kTypes; g++) {
-            const int v = warp_counts[lane][g];
-            int x = v;
-#pragma unroll
-            for (int o = 1; o < kWarp; o <<= 1) {
-                const int y = __shfl_up_sync(kFull, x, o);
-                if (lane >= o) x += y;
-            }
-            warp_counts[lane][g] = x - v;
+    for (int g = 0; g < kTypes; g++) {
+        if (t == g) {
+            const int r = before.c[g] + in_tile.c[g] + rank;
+            scatter[i] = r;
+            gather[i] = start + r;
         }
-    }
-    __syncthreads();
-    if (i < n_atoms) {
-        int start = 0;
-#pragma unroll
-        for (int g = 0; g < kTypes; g++) {
-            if (t == g) {
-                const int r = before.c[g] + warp_counts[warp][g] + rank;
-                scatter[i] = r;
-                gather[i] = start + r;
-            }
-            start += total.c[g];
-        }
+        start += total.c[g];
     }
 }
 
 // Tile `tile` of a single-launch sort.
 __device__ __forceinline__ void sort_tile(const int* __restrict__ types, int n_atoms, int tile, int* __restrict__ scatter,
-                                          int* __restrict__ gather, int* __restrict__ counts, int (*red)[kTypes])
+                                          int* __restrict__ gather, int* __restrict__ counts, SortShared& sh)
 {
-    Count4 vb, vt;
+    static_assert(kSortSingleLaunchMax / kSortThreads + 1 <= 255, "a byte per element and thread");
+    static_assert(kSortSingleLaunchMax - kSortTile < 1 << 16, "16 bits for what lies in front of a tile");
+    const int lane = lane_id(), warp = warp_id();
+    const int i = tile * kSortTile + threadIdx.x;
+    const int t = i < n_atoms ? types[i] & 3 : -1;      // (bad elements are reported where everything is counted)
+    unsigned vb, vt;
     count_two_ranges(types, n_atoms, tile * kSortTile, &vb, &vt);
-    const Count4 before = block_sum(vb, red);
-    const Count4 total = block_sum(vt, red);
+    Pair16 own;
+    const int rank = rank_in_warp(t, &own);
+    const Pair16 warp_before = warp_sum(widen(vb)), warp_total = warp_sum(widen(vt));
+    if (lane == 0) {
+        sh.counted[warp] = make_uint4(warp_before.even, warp_before.odd, warp_total.even, warp_total.odd);
+        sh.own[warp] = own;
+    }
+    __syncthreads();
+    const uint4 v = sh.counted[lane];
+    const Count4 before = unpack(warp_sum(Pair16{v.x, v.y})), in_tile = warps_in_front(sh.own);
+    Count4 total = unpack(Pair16{v.z, v.w});      // a whole batch of one element may be 2^16 atoms
+#pragma unroll
+    for (int g = 0; g < kTypes; g++) total.c[g] = __reduce_add_sync(kFull, total.c[g]);
     if (tile == 0 && threadIdx.x == 0) {
 #pragma unroll
         for (int g = 0; g < kTypes; g++) counts[g] = total.c[g];
     }
-    rank_tile(types, n_atoms, tile, before, total, scatter, gather, red);
+    if (t >= 0) place_atom(i, t, rank, before, in_tile, total, scatter, gather);
 }
 
 // Single launch: grid = number of tiles.
@@ -163,9 +167,9 @@ __global__ void __launch_bounds__(kSortThreads)
     sort_single_kernel(const int* __restrict__ types, int n_atoms, int* __restrict__ scatter,
                        int* __restrict__ gather, int* __restrict__ counts)
 {
-    __shared__ int red[kSortWarps][kTypes];
+    __shared__ SortShared sh;
     pdl_wait();
-    sort_tile(types, n_atoms, blockIdx.x, scatter, gather, counts, red);
+    sort_tile(types, n_atoms, blockIdx.x, scatter, gather, counts, sh);
     pdl_trigger();
 }
 
@@ -175,29 +179,32 @@ __global__ void __launch_bounds__(kSortThreads)
     sort_and_pack_kernel(const int* __restrict__ types, int n_atoms, int n_tiles, int* __restrict__ scatter,
                          int* __restrict__ gather, int* __restrict__ counts, const MlpPackParams pack)
 {
-    __shared__ int red[kSortWarps][kTypes];
+    __shared__ SortShared sh;
     pdl_wait();     // no early trigger: the kernel writes weights
     if ((int)blockIdx.x >= n_tiles) {
         const int c = (int)blockIdx.x - n_tiles;
         pack_chunk(pack, c % kPackChunks, c / kPackChunks);
         return;
     }
-    sort_tile(types, n_atoms, blockIdx.x, scatter, gather, counts, red);
+    sort_tile(types, n_atoms, blockIdx.x, scatter, gather, counts, sh);
 }
 
 // Large batches, first: per-tile element counts into scratch[tile][4].
 __global__ void __launch_bounds__(kSortThreads)
     sort_histogram_kernel(const int* __restrict__ types, int n_atoms, int* __restrict__ tile_counts)
 {
-    __shared__ int red[kSortWarps][kTypes];
-    const int tile = blockIdx.x;
-    const int i = tile * kSortTile + threadIdx.x;
-    Count4 v = {{0, 0, 0, 0}};
-    if (i < n_atoms) tally(v, types[i], true);
-    const Count4 c = block_sum(v, red);
-    if (threadIdx.x == 0) {
+    __shared__ Pair16 red[kSortWarps];
+    const int tile = blockIdx.x, i = tile * kSortTile + threadIdx.x;
+    Pair16 own;
+    rank_in_warp(i < n_atoms ? checked_type(types[i]) : -1, &own);
+    if (lane_id() == 0) red[warp_id()] = own;
+    __syncthreads();
+    if (warp_id() == 0) {
+        const Count4 c = unpack(warp_sum(red[lane_id()]));
+        if (threadIdx.x == 0) {
 #pragma unroll
-        for (int g = 0; g < kTypes; g++) tile_counts[tile * kTypes + g] = c.c[g];
+            for (int g = 0; g < kTypes; g++) tile_counts[tile * kTypes + g] = c.c[g];
+        }
     }
 }
 
@@ -250,8 +257,9 @@ __global__ void __launch_bounds__(kSortThreads)
                      const int* __restrict__ tile_counts, int n_tiles, int* __restrict__ scatter,
                      int* __restrict__ gather, int* __restrict__ counts)
 {
-    __shared__ int red[kSortWarps][kTypes];
-    const int tile = blockIdx.x;
+    __shared__ Pair16 red[kSortWarps];
+    const int tile = blockIdx.x, i = tile * kSortTile + threadIdx.x;
+    const int t = i < n_atoms ? types[i] & 3 : -1;      // (bad elements were reported by the histogram)
     Count4 before, total;
 #pragma unroll
     for (int g = 0; g < kTypes; g++) {
@@ -262,7 +270,12 @@ __global__ void __launch_bounds__(kSortThreads)
 #pragma unroll
         for (int g = 0; g < kTypes; g++) counts[g] = total.c[g];
     }
-    rank_tile(types, n_atoms, tile, before, total, scatter, gather, red);
+    Pair16 own;
+    const int rank = rank_in_warp(t, &own);
+    if (lane_id() == 0) red[warp_id()] = own;
+    __syncthreads();
+    const Count4 in_tile = warps_in_front(red);
+    if (t >= 0) place_atom(i, t, rank, before, in_tile, total, scatter, gather);
 }
 
 // n_atoms == 0: the reference still returns atom_counts = {0, 0, 0, 0}.

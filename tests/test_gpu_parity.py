@@ -66,6 +66,24 @@ def test_sort_single_element_and_sorted_inputs(gpu, oracle_mod):
         np.testing.assert_array_equal(gi, egi)
 
 
+@pytest.mark.parametrize("n", [1, 3, 1023, 1025, 64513, 65535, 65536, 65537])
+@pytest.mark.parametrize("element", [0, 1, 2, 3])
+def test_sort_counts_at_the_limits_of_their_fields(gpu, element, n):
+    """All atoms of one element (65,536 of them do not fit 16 bits), but the last; read 16 bytes at a time and not."""
+    import torch
+    a = np.full(n, element, np.int32)
+    a[-1] = 3 - element
+    scatter, gather, counts = _host_sort(a)
+    for shift in (0, 1):
+        dev = torch.zeros(n + 4, dtype=torch.int32, device=gpu.DEV)[shift:shift + n]
+        dev.copy_(gpu.to_dev(a))
+        assert (dev.data_ptr() & 15 == 0) == (shift == 0)
+        for got, want in zip(gpu.ani_mod.ani_sort(dev), (scatter, gather, counts)):
+            np.testing.assert_array_equal(got.cpu().numpy(), want)
+        dev.copy_(gpu.to_dev(np.full(n, element, np.int32)))
+        np.testing.assert_array_equal(gpu.ani_mod.ani_sort(dev)[2].cpu().numpy(), np.where(np.arange(4) == element, n, 0))
+
+
 def _host_sort(a):
     order = np.argsort(a, kind="stable")
     gather = np.empty(a.size, np.int64)
