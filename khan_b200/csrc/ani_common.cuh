@@ -143,6 +143,12 @@ __device__ __forceinline__ int checked_type(int t)
     return t;
 }
 
+// An int carried in a floating-point field, and back.
+__device__ __forceinline__ float bits_as(float, int v) { return __int_as_float(v); }
+__device__ __forceinline__ double bits_as(double, int v) { return __hiloint2double(0, v); }
+__device__ __forceinline__ int as_bits(float v) { return __float_as_int(v); }
+__device__ __forceinline__ int as_bits(double v) { return __double2loint(v); }
+
 template <typename T> struct alignas(sizeof(T) * 4) Vec4 {
     T x, y, z, w;
 };

@@ -6,22 +6,26 @@
 // lane = slot over the groups of ALL central atoms of the round, contraction with lane = (theta,
 // shift)) are the very same code, ani_featurize_round_passes.inl -- but the molecule does not fit the lanes,
 // so the scan differs:
-//   A. the molecule is read from global memory 32 candidates at a time, once per round; every lane
-//      tests its candidate against the (up to) four central atoms, whose coordinates all lanes hold, by squared
-//      distance.  Radial neighbours go to the central atom's radial list in arrival order with their element,
-//      angular neighbours to its angular list (32 at most);
-//   L. lengths and cutoffs of the radial lists, lane = entry (in the scan 3 of 32 lanes had work for them);
-//   S. each angular list gets its lengths and cutoffs and is put into element order by one ballot sort (lane = entry), which is what
-//      pass T needs; the per-element counts fall out of the same ballots;
+//   A. the molecule is read from global memory 32 candidates at a time, once per round; every lane tests its candidate
+//      against the (up to) four central atoms, whose coordinates all lanes hold, by squared distance, and keeps no more
+//      than the ballots: lane = (central atom, one of eight groups of 32 candidates).  Then every lane writes the indices of
+//      its set bits to the central atom's radial list;
+//   L. lane = list entry: length and cutoff from the neighbour's coordinates (in the scan 3 of 32 lanes had work for them);
+//      angular neighbours go to the angular list (32 at most) in arrival order;
 //   R. radial features of the whole round, lane = (central atom, pair of shifts): every lane walks
-//      the radial list of its central atom and adds to the sum of the neighbour's element.
-// When a radial list is full (64 entries), pass R works it off and the scan goes on; a central atom with more
+//      the radial list of its central atom and adds to the sum of the neighbour's element;
+//   S. each angular list is put into element order by one ballot sort (lane = entry), which is what
+//      pass T needs; the per-element counts fall out of the same ballots.
+// When a radial list is full (64 entries), pass R works it off and the scan goes on behind the last whole group of 32; a
+// central atom with more
 // than 32 angular neighbours goes through the streaming routine of ani_featurize.cuh.  A CTA takes the rounds r, r + R0, r + 2 R0, ... of its molecule
 // (R0 rounds per molecule in the grid, chosen by the host from the mean molecule size), so molecules
 // of any size are covered.  Nothing is accumulated with atomics; rows need no zero fill by the caller.
 //
-// 256 molecules of 64 to 256 atoms: 95 us (float, as before), double 341 -> 256 (lengths and cutoffs off the scan);
-// 8 molecules 41 -> 21 us with one central atom per warp instead of four.
+// Bound by instruction issue.  With neighbours written to both lists inside the scan (ballots, counts and stores for every
+// 32 candidates of every central atom) and sums over all four elements added to for every neighbour, microseconds alone
+// before -> now: 256 molecules of 64 to 256 atoms 97 -> 82 (79.5 -> 72.8 a batch with eight streams in flight), 64: 43 -> 36,
+// 8: 21.3 -> 18.5; double, 256: 257 -> 247.
 //
 // Computes what featurize_cpu of the reference computes (gpu_featurizer/kernel_cpu.cpp:406-537).
 #pragma once
@@ -35,10 +39,23 @@ namespace ani {
 
 constexpr int kLargeCapR = 64;   // radial neighbours kept per central atom
 constexpr int kLargeCapA = 32;   // angular neighbours kept per central atom (one ballot sort covers 32 entries)
+constexpr int kLargeBlock = 8 * kWarp;   // candidates of a scan: eight masks of 32 for each of four central atoms
+
+__device__ __forceinline__ void add_where(bool on, Pair<float> v, Pair<float>* sum)      // one packed add, predicated
+{
+    unsigned long long s = pack2(sum->x, sum->y);
+    asm("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\n@p add.rn.f32x2 %0, %0, %1;\n}" : "+l"(s) : "l"(pack2(v.x, v.y)), "r"((int)on));
+    *sum = unpack2(s);
+}
+__device__ __forceinline__ void add_where(bool on, Pair<double> v, Pair<double>* sum)
+{
+    sum->x += on ? v.x : 0.0;
+    sum->y += on ? v.y : 0.0;
+}
 
 template <typename T> struct LargeFwdWarpShared {
     MolAngularShared<T, kMolCentrals * kLargeCapA, kLargeCapA> ang;
-    Vec2<T> rad[kMolCentrals][kLargeCapR];           // squared distance; from step L on (r, f_C(r, R_Rc))
+    Vec2<T> rad[kMolCentrals][kLargeCapR];           // index of the neighbour; from step L on (r, f_C(r, R_Rc))
     unsigned char rad_t[kMolCentrals][kLargeCapR];   // element of that neighbour
     unsigned char ang_t[kMolCentrals * kLargeCapA];    // element of each angular neighbour before the sort
     int cnt_r[kMolCentrals];
@@ -106,83 +123,80 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 22 : 1)
             }
         }
 
-        // ---- A: scan, 32 candidates at a time against all central atoms of the round ----
-        int cA[kMolCentrals] = {0, 0, 0, 0}, cR[kMolCentrals] = {0, 0, 0, 0};
+        // ---- A: scan, up to kLargeBlock candidates against all central atoms of the round ----
+        int cA[kMolCentrals] = {0, 0, 0, 0}, cR[kMolCentrals];
         int j0 = 0;
         bool again = false;   // pass R has written the rows once: it adds from now on
         do {
-        T qx, qy, qz;   // the next 32 candidates are requested before this chunk's arithmetic
-        int qt;
-        {
-            const int gj = base + (j0 + lane < n ? j0 + lane : 0);
-            qx = xs[gj]; qy = ys[gj]; qz = zs[gj];
-            qt = types[gj];
-        }
-        for (; j0 < n; j0 += kWarp) {
-            const int had_r[kMolCentrals] = {cR[0], cR[1], cR[2], cR[3]};
-            const int had_a[kMolCentrals] = {cA[0], cA[1], cA[2], cA[3]};
-            const int j = j0 + lane;
-            const bool live = j < n;
-            const T px = qx, py = qy, pz = qz;
-            const int tj = checked_type(qt);
-            if (j0 + kWarp < n) {
-                const int gj = base + (j + kWarp < n ? j + kWarp : 0);
-                qx = xs[gj]; qy = ys[gj]; qz = zs[gj];
-                qt = types[gj];
-            }
 #pragma unroll
-            for (int g = 0; g < kMolCentrals; g++) {
-                if ((skip >> g) & 1u) continue;   // warp-uniform
-                const T dx = xi[g] - px, dy = yi[g] - py, dz = zi[g] - pz;
-                const T d2 = dx * dx + dy * dy + dz * dz;
-                const bool in_rad = live && j != ci[g] && d2 < (T)(kR_Rc * kR_Rc);
-                const bool in_ang = in_rad && d2 < (T)(kA_Rc * kA_Rc);
-                const unsigned mR = __ballot_sync(kFull, in_rad);
-                if (mR == 0) continue;
-                const unsigned mA = __ballot_sync(kFull, in_ang);
-                if (in_rad) {
-                    const int pos = cR[g] + __popc(mR & lanemask_lt());
-                    if (pos < kLargeCapR) {
-                        ws.rad[g][pos].x = d2;
-                        ws.rad_t[g][pos] = (unsigned char)tj;
-                    }
-                }
-                if (in_ang) {
-                    const int pos = cA[g] + __popc(mA & lanemask_lt());
-                    if (pos < kLargeCapA) {
-                        const int p = g * kLargeCapA + pos;
-                        ws.ang.ang_u[p] = Vec4<T>{dx, dy, dz, d2};
-                        ws.ang_t[p] = (unsigned char)tj;
-                    }
-                }
-                cR[g] += __popc(mR);
-                cA[g] += __popc(mA);
-            }
-            if (max(max(cR[0], cR[1]), max(cR[2], cR[3])) > kLargeCapR) {   // this chunk comes again after pass R
+        for (int g = 0; g < kMolCentrals; g++) cR[g] = 0;
+        bool full = false;
+        while (j0 < n && !full) {
+            // lane 8 g + k: which of the candidates j0 + 32 k + (0 .. 31) are within R_Rc of central atom g
+            unsigned mask = 0u;
+#pragma unroll
+            for (int k = 0; k < kLargeBlock / kWarp; k++) {
+                const int j = j0 + k * kWarp + lane;
+                if (j0 + k * kWarp >= n) break;
+                const int gj = base + (j < n ? j : 0);
+                const T px = xs[gj], py = ys[gj], pz = zs[gj];
 #pragma unroll
                 for (int g = 0; g < kMolCentrals; g++) {
-                    cR[g] = had_r[g];
-                    cA[g] = had_a[g];
+                    if ((skip >> g) & 1u) continue;   // warp-uniform
+                    const T dx = xi[g] - px, dy = yi[g] - py, dz = zi[g] - pz;
+                    const unsigned m = __ballot_sync(kFull, j < n && j != ci[g] && dx * dx + dy * dy + dz * dz < (T)(kR_Rc * kR_Rc));
+                    if (lane == 8 * g + k) mask = m;
                 }
-                break;
             }
+            // as many groups of 32 candidates as the lists have room for; the rest comes again after pass R
+            int incl = __popc(mask);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const int y = __shfl_up_sync(kFull, incl, o, 8);
+                if ((lane & 7) >= o) incl += y;
+            }
+            int at = pick4(cR, lane >> 3) + incl - __popc(mask);
+            unsigned over = __ballot_sync(kFull, pick4(cR, lane >> 3) + incl > kLargeCapR);
+            over |= over >> 16;
+            over = (over | over >> 8) & 0xffu;
+            const int taken = over ? __ffs(over) - 1 : 8;
+            full = over != 0u;
+            if ((lane & 7) < taken)
+                for (; mask; mask &= mask - 1)
+                    ws.rad[lane >> 3][at++].x = bits_as((T)0, j0 + 32 * (lane & 7) + __ffs(mask) - 1);
+            if (taken > 0)
+#pragma unroll
+                for (int g = 0; g < kMolCentrals; g++) cR[g] += __shfl_sync(kFull, incl, 8 * g + taken - 1);
+            j0 += kWarp * taken;
         }
         __syncwarp();
+        if (lane < kMolCentrals) ws.cnt_r[lane] = pick4(cR, lane);
 
-        if (lane < kMolCentrals) ws.cnt_r[lane] = 0;
-        __syncwarp();
+        // ---- L: lane = list entry: length and cutoff; angular neighbours to their own list ----
 #pragma unroll
         for (int g = 0; g < kMolCentrals; g++)
-            if (lane == 0 && !((skip >> g) & 1u)) ws.cnt_r[g] = cR[g];
-        __syncwarp();
-
-        // ---- L: lengths and cutoffs, lane = list entry ----
-#pragma unroll
-        for (int g = 0; g < kMolCentrals; g++)
-            for (int p = lane; p < ws.cnt_r[g]; p += kWarp) {
+            for (int p0 = 0; p0 < cR[g]; p0 += kWarp) {
+                const int p = p0 + lane;
+                const bool have = p < cR[g];
+                const int gj = base + (have ? as_bits(ws.rad[g][p].x) : 0);
+                const T dx = xi[g] - xs[gj], dy = yi[g] - ys[gj], dz = zi[g] - zs[gj];
+                const int tj = checked_type(types[gj]);
+                const T d2 = dx * dx + dy * dy + dz * dz;
                 T r, inv;
-                length_and_inverse(ws.rad[g][p].x, &r, &inv);
-                ws.rad[g][p] = Vec2<T>{r, cutoff_value<T>(r, (T)kR_Rc)};
+                length_and_inverse(d2, &r, &inv);
+                const bool in_ang = have && d2 < (T)(kA_Rc * kA_Rc);
+                const unsigned mA = __ballot_sync(kFull, in_ang);
+                if (have) {
+                    ws.rad[g][p] = Vec2<T>{r, cutoff_value<T>(r, (T)kR_Rc)};
+                    ws.rad_t[g][p] = (unsigned char)tj;
+                }
+                const int pos = cA[g] + __popc(mA & lanemask_lt());
+                if (in_ang && pos < kLargeCapA) {
+                    const int q = g * kLargeCapA + pos;
+                    ws.ang.ang_u[q] = Vec4<T>{dx * inv, dy * inv, dz * inv, r};
+                    ws.ang_t[q] = (unsigned char)tj;
+                }
+                cA[g] += __popc(mA);
             }
         __syncwarp();
 
@@ -201,10 +215,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 22 : 1)
                 const Pair<T> d2 = pmul(d, d);
                 const Pair<T> v{Num<T>::exp_neg((T)kR_eta, d2.x) * e.y, Num<T>::exp_neg((T)kR_eta, d2.y) * e.y};
 #pragma unroll
-                for (int k = 0; k < kTypes; k++) {
-                    acc[k].x += t == k ? v.x : (T)0;
-                    acc[k].y += t == k ? v.y : (T)0;
-                }
+                for (int k = 0; k < kTypes; k++) add_where(t == k, v, &acc[k]);
             }
             if (!((skip >> g) & 1u)) {
                 T* row = ws.ang.row[g];
@@ -217,8 +228,6 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 22 : 1)
             }
         }
         again = true;
-#pragma unroll
-        for (int g = 0; g < kMolCentrals; g++) cR[g] = 0;
         __syncwarp();
         } while (j0 < n);
 
@@ -235,8 +244,6 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 22 : 1)
             const bool have = lane < cA[g];
             const int p = g * kLargeCapA + (have ? lane : 0);
             const Vec4<T> v = ws.ang.ang_u[p];
-            T r, inv;
-            length_and_inverse(v.w, &r, &inv);
             const int t = have ? ws.ang_t[p] : kTypes;
             const unsigned m0 = __ballot_sync(kFull, t == 0), m1 = __ballot_sync(kFull, t == 1),
                            m2 = __ballot_sync(kFull, t == 2), m3 = __ballot_sync(kFull, t == 3);
@@ -246,8 +253,8 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 22 : 1)
             __syncwarp();   // every entry has been read
             if (have) {
                 const int q = g * kLargeCapA + start + __popc(mine & lanemask_lt());
-                ws.ang.ang_u[q] = Vec4<T>{v.x * inv, v.y * inv, v.z * inv, r};
-                ws.ang.ang_fc[q] = cutoff_value<T>(r, (T)kA_Rc);
+                ws.ang.ang_u[q] = v;
+                ws.ang.ang_fc[q] = cutoff_value<T>(v.w, (T)kA_Rc);
             }
             if (lane == 0)
                 *reinterpret_cast<int4*>(&ws.ang.cnt_a[g * kTypes]) = make_int4(c0, c1, c2, __popc(m3));

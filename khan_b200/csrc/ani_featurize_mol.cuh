@@ -162,13 +162,13 @@ __device__ __forceinline__ void load_sorted_molecule(const T* __restrict__ xs, c
 // padding slot (a and b then point at entry 0 of the list, which always holds finite values).
 // Slot number q inside a group: different elements, q = ia * nb + ib; one element, q = (d - 1) * nb + a
 // with b = a + d mod nb (d <= nb / 2; the last row of an even nb holds only a < nb / 2).
-__device__ __forceinline__ bool decode_slot(const MolGroupInfo* tab, const unsigned char* quad_gid, int p,
+__device__ __forceinline__ bool decode_slot(const MolGroupInfo* tab, const unsigned char* quad_gid, int p, int end,
                                             int* a, int* b)
 {
     const int gid = quad_gid[p >> 2];
     const MolGroupInfo e = tab[gid == kMolNoGroup ? 0 : gid];
     const int q = p - e.off;
-    const bool valid = gid != kMolNoGroup && q < e.cnt;
+    const bool valid = p < end && q < e.cnt;
     const int nb = (e.packed >> 16) & 0xff;
     const bool same = (e.packed >> 24) != 0;
     const int hi = (int)(((unsigned)q * e.recip) >> 16);   // q / nb

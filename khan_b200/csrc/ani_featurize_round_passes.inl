@@ -10,8 +10,10 @@
 {
     // ---- T: one table for the groups (central atom, element pair) of the round.  Lane = (central
     // atom, bucket) covers the first eight buckets in one pass; N-O and O-O pairs (buckets 8, 9)
-    // are rare and get a second, short pass only when they occur. ----
+    // are rare and get a second, short pass only when they occur.  (Both written out: as a loop 1024 small molecules took
+    // 24.1 us instead of 23.6, 256 large ones 90 instead of 82.) ----
     int total = 0;
+#pragma unroll
     for (int pass = 0; pass < 2; pass++) {
         const int g = pass == 0 ? lane >> 3 : (lane >> 1) & 3;
         const int bk = pass == 0 ? lane & 7 : 8 + (lane & 1);
@@ -36,8 +38,7 @@
             e.off = off;
             e.cnt = cnt;
             const int first = ws.ang.first(g);
-            e.packed = (first + pick4(stv, ta)) | ((first + pick4(stv, tb)) << 8) | (nb << 16) |
-                       ((ta == tb ? 1 : 0) << 24);
+            e.packed = (first + pick4(stv, ta)) | ((first + pick4(stv, tb)) << 8) | (nb << 16) | ((ta == tb ? 1 : 0) << 24);
             e.recip = (unsigned)(65536.0f * __frcp_rn((float)nb)) + 1u;   // in [2^16 / nb, 2^16 / nb + 1.01)
             const int gid = g * kMolGroupStride + bk;
             ws.ang.tab[gid] = e;
@@ -63,7 +64,7 @@
 #pragma unroll
         for (int u = 0; u < kMolSlotsPerLane; u++) {
             int a, b;
-            const bool valid = decode_slot(ws.ang.tab, ws.ang.quad_gid, c0 + u * kWarp + lane, &a, &b);
+            const bool valid = decode_slot(ws.ang.tab, ws.ang.quad_gid, c0 + u * kWarp + lane, total, &a, &b);
             const Vec4<T> ua = ws.ang.ang_u[a], ub = ws.ang.ang_u[b];
             const T cosv = ua.x * ub.x + ua.y * ub.y + ua.z * ub.z;
             const T rbar = (T)0.5 * (ua.w + ub.w);
@@ -93,7 +94,7 @@
         constexpr int kQuads = kMolChunk / 4;
         const unsigned my_id = ids[lane & (kQuads - 1)];
         const unsigned ends =
-            __ballot_sync(kFull, lane < kQuads && my_id != kMolNoGroup && my_id != ids[(lane & (kQuads - 1)) + 1]);
+            __ballot_sync(kFull, lane < kQuads && c0 + 4 * lane < total && my_id != ids[(lane & (kQuads - 1)) + 1]);
         __syncwarp();
         // C: lane = (theta, shift).  Slots behind the last group hold BF = 0.
 #pragma unroll

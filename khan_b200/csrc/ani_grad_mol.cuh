@@ -155,11 +155,6 @@ template <typename T> struct MolEnergySums {
 // (19.9 without, 20.4 with it).
 constexpr int kMolGradOrder = 16;
 
-__device__ __forceinline__ float bits_as(float, int v) { return __int_as_float(v); }
-__device__ __forceinline__ double bits_as(double, int v) { return __hiloint2double(0, v); }
-__device__ __forceinline__ int as_bits(float v) { return __float_as_int(v); }
-__device__ __forceinline__ int as_bits(double v) { return __double2loint(v); }
-
 // length_and_inverse with one Newton step on the SFU's reciprocal root in float: the distances are computed once per pair
 // of atoms here, and their error is what the Gaussians enlarge most.
 __device__ __forceinline__ void refined_length_and_inverse(float d2, float* r, float* inv)
