@@ -421,14 +421,18 @@ def test_large_molecules_at_every_split(gpu, oracle_mod, n_mols, dt):
 
 @pytest.mark.parametrize("n", [64, 255, 256, 257, 289, 520])
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
-def test_large_molecule_features_across_scan_blocks(gpu, oracle_mod, n, dt):
-    """Candidates are scanned 256 at a time into lists of 64: at 0.2 atoms per cubic Angstrom most atoms have more
-    neighbours within R_Rc, so lists fill up in the middle of a block, and around its end."""
+def test_large_molecules_across_scan_blocks(gpu, oracle_mod, n, dt):
+    """Candidates are scanned 256 at a time, for the features into lists of 64: at 0.2 atoms per cubic Angstrom most atoms
+    have more neighbours within R_Rc, so lists fill up in the middle of a block, and around its end."""
     b = _dense_blobs(2, n, (3.0 * n / (4.0 * np.pi * 0.2)) ** (1.0 / 3.0), n)
     si, gi, ac = oracle_mod.ani_sort(b.atomic_numbers)
     args = [v.astype(np.float64) for v in b.coords(dt)] + [b.atomic_numbers, b.mol_offsets, b.mol_atom_counts, si, ac]
     for out, ref in zip(gpu.gpu_featurize(b, dt), oracle_mod.featurize(*args, impl="port", threads=8)):
         assert normwise(out, ref) < FTOL[dt]
+    up = syn.upstream_grads(b, ac, dtype=dt)
+    ref = oracle_mod.featurize_grad(*args, *[u.astype(np.float64) for u in up], impl="port", threads=8)
+    for k, out in enumerate(gpu.gpu_featurize_grad(b, dt, up)):
+        assert normwise(out, ref[k]) < FTOL[dt]
 
 
 def test_float32_gradient_vs_the_float32_reference_where_it_is_finite(gpu, oracle_mod, ref_impl):
