@@ -392,12 +392,20 @@ int featurize_grad_inverse_impl(const T* xs, const T* ys, const T* zs, const int
     for (int t = 0; t < kTypes; t++)
         if (acs_host[t] > 0 && !outs[t]) return ANI_ERR_NULL_POINTER;
 
-    // small molecules with outputs that take 16-byte stores: rounds of four central atoms per warp
+    // small molecules with outputs that take 16-byte stores: rounds of one to four central atoms per warp, as few as still
+    // find all warps resident at once, as in the features.  Microseconds with 4 / 3 / 2 / 1 in float, 32 molecules 14.6 /
+    // 13.0 / 10.9 / 8.8, 128: 17.2 / 15.6 / 13.3 / 11.5, 256: 22.5 / 19.1 / 16.2 / 18.0, 512: 25.1 / 25.8 / 24.5 / 29.9,
+    // 1024: 39.7 / 39.8 / 43.8 / 57.3; in double, 64: 36 / 34 / 26 / 20, 256: 42 / 36 / 40 / 44, 1024: 92 / 95 / 110 / 143.
+    // Three lose to four in float where the rule would take them, and do in both types with eight streams in flight.
     if (small_molecules(n_atoms, n_mols) && all_aligned16({oh, oc, on, oo}) &&
-        (long long)n_mols * kMolRounds <= 0x7fffffffLL) {
-        ANI_CUDA(launch_chain(featurize_tangent_mol_kernel<T>, n_mols * kMolRounds, kWarp, 0, (cudaStream_t)stream, 1, xs, ys,
+        (long long)n_mols * kMolMaxAtoms <= 0x7fffffffLL) {
+        const int resident = kSms * (sizeof(T) == 4 ? 16 : 10);
+        int per_round = (int)std::min<long long>((n_atoms + resident - 1) / resident, kMolCentrals);
+        if (sizeof(T) == 4 && per_round == 3) per_round = 4;
+        const int rounds = (kMolMaxAtoms + per_round - 1) / per_round;
+        ANI_CUDA(launch_chain(featurize_tangent_mol_kernel<T>, n_mols * rounds, kWarp, 0, (cudaStream_t)stream, 1, xs, ys,
                               zs, types, mos, macs, n_mols, (int)n_atoms, sis, vx, vy, vz, oh, oc, on, oo, acs_host[0],
-                              acs_host[1], acs_host[2], acs_host[3]));
+                              acs_host[1], acs_host[2], acs_host[3], per_round, 65536 / per_round + 1));
         return ANI_OK;
     }
 

@@ -62,7 +62,6 @@ constexpr int kMolNoGroup = 0xff;      // id of the quads behind the last group
 constexpr int kMolSlotsPerLane = 1;    // slots a lane evaluates per pass B (2 was measured: no gain)
 constexpr int kMolChunk = kMolSlotsPerLane * kWarp;   // slots per pass B / C
 constexpr int kMolChunkStride = kMolChunk + 4;        // + 4 words: keeps the 16-byte reads of pass C conflict-free
-constexpr int kMolRounds = kMolMaxAtoms / kMolCentrals;   // rounds of the largest molecule of the fast path
 // padded slots of the central atoms worked on together, in quads: at most n (n - 1) / 2 pairs for n neighbours
 // and 3 per bucket, n <= cap each and <= pool in all (most pairs: as many lists of `cap` as fit)
 constexpr int mol_quad_bytes(int cap, int pool)

@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 16 : 10)
                                  const int* __restrict__ mol_counts, int n_mols, int n_atoms,
                                  const int* __restrict__ scatter, const T* __restrict__ vx, const T* __restrict__ vy,
                                  const T* __restrict__ vz, T* out_h, T* out_c, T* out_n, T* out_o, int acs0, int acs1,
-                                 int acs2, int acs3)
+                                 int acs2, int acs3, int per_round, int per_round_recip)
 {
     __shared__ TangentWarpShared<T> ws;
     using Granule = Vec4<float>;
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 16 : 10)
     const int n = mol.n, base = mol.base;
 
     if (n > kMolMaxAtoms) {
-        for (int i = round; i < n; i += kMolRounds) {
+        for (int i = round; i < n; i += gridDim.x / n_mols) {
             const int gi = base + i;
             const int ti = checked_type(types[gi]);
             const int srow = scatter[gi];
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 16 : 10)
         }
         return;
     }
-    const int n_rounds = (n + kMolCentrals - 1) / kMolCentrals;
+    const int n_rounds = ((n + per_round - 1) * per_round_recip) >> 16;   // / per_round; n is at most 32 here
     if (round >= n_rounds) return;
     const int G = (n - round + n_rounds - 1) / n_rounds;
 

@@ -56,6 +56,22 @@ def test_jvp_vs_oracle(gpu, oracle_mod, case, dt):
         assert normwise(got[t], ref[t]) < TOL[dt], (case, t)
 
 
+@pytest.mark.parametrize("n_mols", [1, 170, 260, 400, 560, 800])
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_jvp_at_every_split(gpu, oracle_mod, n_mols, dt):
+    """One to four central atoms per warp follow from the number of atoms; a molecule of more than 32 atoms among them."""
+    from test_gpu_parity import _concat
+    b = _concat(syn.gdb_like_batch(n_mols, 40 + n_mols), syn.config4(seed=3, n_mols=1, n_min=33, n_max=33)) if n_mols > 1 else \
+        syn.gdb_like_batch(1, 41)
+    si, gi, ac = oracle_mod.ani_sort(b.atomic_numbers)
+    rng = np.random.default_rng(23)
+    v = [rng.normal(size=b.n_atoms).astype(dt) for _ in range(3)]
+    ref = oracle_mod.featurize_grad_inverse(*(c.astype(np.float64) for c in b.coords(dt)), b.atomic_numbers, b.mol_offsets,
+                                            b.mol_atom_counts, si, ac, *[c.astype(np.float64) for c in v], threads=8)
+    for out, want in zip(_gpu_jvp(gpu, b, dt, v, si, ac), ref):
+        assert normwise(out, want) < TOL[dt]
+
+
 def test_jvp_is_the_transpose_of_the_vjp_on_the_gpu(gpu, oracle_mod):
     b = syn.config1(n_mols=64)
     si, gi, ac = oracle_mod.ani_sort(b.atomic_numbers)
