@@ -3,10 +3,17 @@
 // of a shuffled training pass from numpy's global stream without holding the interpreter lock.  (Drawn by
 // numpy in a Python submitter, the noise and the hand-over cost 0.6 ms a batch of 1024 molecules against
 // 0.15 ms of GPU work.)  A block of 624 words is advanced in three loops whose iterations are independent of
-// one another, so that the compiler vectorises them.
+// one another, so that the compiler vectorises them, with AVX2 where the machine has it: 41 thousand values, the noise of
+// 1024 molecules, which batches draw one after the other, 70 -> 47 us.  (Not with FMA: that would round once less.)
 #pragma once
 
 #include <cstdint>
+
+#if defined(__x86_64__) && defined(__GNUC__) && !defined(__clang__)
+#define ANI_HOST_SIMD __attribute__((target_clones("avx2", "default")))
+#else
+#define ANI_HOST_SIMD
+#endif
 
 namespace ani {
 
@@ -25,7 +32,7 @@ class Mt19937 {
         *pos = pos_;
     }
     // n doubles of low + range * u, u uniform in [0, 1) with 53 bits from two words each.
-    void uniform(double* out, long long n, double low, double range)
+    ANI_HOST_SIMD void uniform(double* out, long long n, double low, double range)
     {
         while (n > 0) {
             if (pos_ >= kN) refill();
@@ -56,7 +63,7 @@ class Mt19937 {
         const uint32_t y = (u & 0x80000000u) | (v & 0x7fffffffu);
         return (y >> 1) ^ ((0u - (v & 1u)) & 0x9908b0dfu);
     }
-    void refill()
+    ANI_HOST_SIMD void refill()
     {
         for (int i = 0; i < kN - kM; i++) key_[i] = key_[i + kM] ^ twist(key_[i], key_[i + 1]);
         for (int i = kN - kM; i < kN - 1; i++) key_[i] = key_[i + kM - kN] ^ twist(key_[i], key_[i + 1]);
@@ -64,7 +71,7 @@ class Mt19937 {
         pos_ = 0;
         temper();
     }
-    void temper()
+    ANI_HOST_SIMD void temper()
     {
         for (int i = 0; i < kN; i++) {
             uint32_t y = key_[i];
