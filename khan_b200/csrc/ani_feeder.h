@@ -119,8 +119,8 @@ public:
             ready_.clear();
             for (int s = 0; s < (int)slots_.size(); s++) free_.push_back(s);
         }
-        // Packing 1024 shuffled molecules takes a core 0.1 ms, their noise as much again, the GPU 0.15 ms: one thread
-        // could not keep up.  A second one is worth its start (30 us) from the third batch on.
+        // Packing 1024 shuffled molecules takes a core 0.1 ms, their noise half as much again, the GPU 0.1 ms: one thread
+        // could not keep up.  A second one is worth its start (30 us) from the third batch on; a third or fourth gains nothing.
         try {
             for (int t = 0; t < (n_batches_ > 2 ? 2 : 1); t++) threads_.emplace_back([this] { run(); });
         } catch (const std::system_error&) {     // no thread to be had; one is enough
