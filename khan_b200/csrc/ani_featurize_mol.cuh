@@ -123,8 +123,8 @@ template <typename T> struct MolLanes {
 template <typename T>
 __device__ __forceinline__ void load_sorted_molecule(const T* __restrict__ xs, const T* __restrict__ ys,
                                                      const T* __restrict__ zs, const int* __restrict__ types,
-                                                     const int* __restrict__ scatter, int base, int n,
-                                                     MolSortShared* sh, MolLanes<T>* out, bool scatter_is_new = false)
+                                                     const int* scatter, int base, int n, MolSortShared* sh,
+                                                     MolLanes<T>* out, bool scatter_is_new = false)
 {
     unsigned char* inv = sh->src;
     const int lane = lane_id();
@@ -133,7 +133,7 @@ __device__ __forceinline__ void load_sorted_molecule(const T* __restrict__ xs, c
     const T x0 = xs[gj], y0 = ys[gj], z0 = zs[gj];
     const int t0 = live ? checked_type(types[gj]) : kTypes;
     if (scatter_is_new) pdl_wait();
-    const int s0 = scatter[gj];
+    const int s0 = load_fresh(scatter + gj);
     const unsigned m0 = __ballot_sync(kFull, t0 == 0), m1 = __ballot_sync(kFull, t0 == 1),
                    m2 = __ballot_sync(kFull, t0 == 2), m3 = __ballot_sync(kFull, t0 == 3);
     const int c0 = __popc(m0), c1 = __popc(m1), c2 = __popc(m2);
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     featurize_mol_kernel(const T* __restrict__ xs, const T* __restrict__ ys, const T* __restrict__ zs,
                          const int* __restrict__ types, const int* __restrict__ mol_offsets,
                          const int* __restrict__ mol_counts, int n_mols, int n_atoms,
-                         const int* __restrict__ scatter, T* out_h, T* out_c, T* out_n, T* out_o,
+                         const int* scatter, T* out_h, T* out_c, T* out_n, T* out_o,
                          int acs0, int acs1, int acs2, int acs3, int per_round, int per_round_recip, bool after_sort)
 {
     __shared__ MolFwdWarpShared<T> ws;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
         for (int i = round; i < n; i += gridDim.x / n_mols) {
             const int gi = base + i;
             const int ti = checked_type(types[gi]);
-            const int srow = scatter[gi];
+            const int srow = load_fresh(scatter + gi);
             const int cap = ti == 0 ? acs0 : (ti == 1 ? acs1 : (ti == 2 ? acs2 : acs3));
             if (srow < 0 || srow >= cap) {
                 if (lane == 0) report(ANI_ERR_BAD_INDEX);

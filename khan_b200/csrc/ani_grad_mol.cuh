@@ -184,8 +184,7 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
     featurize_grad_mol_kernel(const T* __restrict__ xs, const T* __restrict__ ys, const T* __restrict__ zs,
                               const int* __restrict__ types, const int* __restrict__ mol_offsets,
                               const int* __restrict__ mol_counts, int n_mols, int n_atoms,
-                              const int* __restrict__ scatter, const T* __restrict__ gh,
-                              const T* __restrict__ gc, const T* __restrict__ gn, const T* __restrict__ go,
+                              const int* __restrict__ scatter, const T* gh, const T* gc, const T* gn, const T* go,
                               T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3,
                               const MolEnergySums<T> sums, bool early_inputs)
 {
@@ -239,7 +238,7 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
         if (!sums.mol_energy || warp != NW - 1) return;
         for (int i = lane; i < n; i += kWarp) {
             const int g = sums.gather[base + i];
-            if (g >= 0 && g < n_atoms) energy += sums.atom_energy_sorted[g];
+            if (g >= 0 && g < n_atoms) energy += load_fresh(sums.atom_energy_sorted + g);
             else report(ANI_ERR_BAD_INDEX);
         }
     };
@@ -272,10 +271,10 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
                 continue;
             }
             const T* grow = (ti == 0 ? gh : (ti == 1 ? gc : (ti == 2 ? gn : go))) + (size_t)srow * kTotal;
-            g[lane] = grow[lane];
-            g[32 + lane] = grow[32 + lane];
+            g[lane] = load_fresh(grow + lane);
+            g[32 + lane] = load_fresh(grow + 32 + lane);
             for (int bk = 0; bk < kPairBuckets; bk++)
-                g[kRadial + bk * kGradBucketStride + lane] = grow[kRadial + bk * kTS + lane];
+                g[kRadial + bk * kGradBucketStride + lane] = load_fresh(grow + kRadial + bk * kTS + lane);
             __syncwarp();
             grad_atom_streaming_radial<T>(xs, ys, zs, types, base, n, i, g, gx, gy, gz);
             grad_atom_streaming<T>(xs, ys, zs, types, base, n, i, g, gx, gy, gz);

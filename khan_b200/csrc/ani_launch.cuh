@@ -8,6 +8,9 @@
 //     and before the first store; weights and the geometry may be read ahead of it where the kernel before is one of
 //     the same call and known not to write any (early_weights of the network kernels, after_sort of the features,
 //     early_inputs of the gradient);
+//   * a kernel that reads anything ahead of pdl_wait() takes what the kernel before it writes through load_fresh() or
+//     asynchronous copies, never through a read-only (const __restrict__) pointer: such a load may be moved above the
+//     wait, and a line fetched for a neighbouring array ahead of the wait may still be in the first-level cache;
 //   * pdl_trigger() comes after pdl_wait(), so whatever lies two kernels back has finished when a kernel
 //     starts; a kernel that writes weights never triggers;
 //   * the kernels that fill the device with small molecules, and the sort in front of them, do not trigger at once.
@@ -25,6 +28,26 @@ namespace ani {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// What the kernel before may just have written: read in this place, from the second-level cache.
+__device__ __forceinline__ int load_fresh(const int* p)
+{
+    int v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float load_fresh(const float* p)
+{
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double load_fresh(const double* p)
+{
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // cluster = 1: no cluster.
 template <typename... P, typename... A>

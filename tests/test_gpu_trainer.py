@@ -251,6 +251,35 @@ def test_a_pass_over_few_atoms_refreshes_the_packed_weights(n_mols):
     assert torch.equal(got, ev_many.mol_energy[:many.n_mols])
 
 
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+def test_rows_directly_behind_the_elements(precision):
+    """A pass reads the elements while its sort still writes the rows: with both in one allocation, one behind the other in
+    the same 32 bytes, and other elements in every pass, the results are those of separate arrays."""
+    import torch
+    from khan_b200.inference import EnergyForces
+    from khan_b200.model.nn import MoleculeNN
+    from khan_b200.staged import HostBatch, StagedBatch
+    real = getattr(torch, precision)
+    b = syn.gdb_like_batch(41, seed=5)                 # an odd number of atoms: sectors with both
+    model = MoleculeNN(device="cuda:0", seed=3, precision=real)
+
+    def staged():
+        sb = StagedBatch(b.n_atoms, b.n_mols, real)
+        sb.upload(HostBatch(b, None, sb.x.cpu().numpy().dtype.type, pin=False), non_blocking=False, with_upstream=False)
+        return sb, EnergyForces(model, b.n_atoms, b.n_mols)
+    (apart, ev_apart), (joint, ev_joint) = staged(), staged()
+    both = torch.empty(2 * b.n_atoms, dtype=torch.int32, device="cuda:0")
+    joint.types, joint.scatter = both[:b.n_atoms], both[b.n_atoms:]
+    elements = [torch.from_numpy(np.random.default_rng(k).integers(0, 4, b.n_atoms).astype(np.int32)).cuda() for k in range(8)]
+    for k in range(64):
+        for sb, ev in ((apart, ev_apart), (joint, ev_joint)):
+            sb.types.copy_(elements[k % 8])
+            sb.set_shape(b.n_atoms, b.n_mols, np.bincount(elements[k % 8].cpu(), minlength=4))
+            ev.run(sb)
+        assert torch.equal(joint.scatter, apart.scatter)
+        assert torch.equal(ev_joint.mol_energy, ev_apart.mol_energy) and torch.equal(joint.grads, apart.grads), k
+
+
 def test_fused_train_step_matches_the_autograd_step():
     """FusedTrainStep (C ABI only) against the same step driven by torch autograd: same loss,
     same weight gradients, same coordinate gradients, same weights after the update."""
