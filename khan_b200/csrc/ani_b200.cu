@@ -1476,7 +1476,7 @@ int ani_network_pass_f32(const ani_pass_args* a, void* stream)
             c.grad_feat[t] = rows(a->feature_grads, t, kTotal);
         }
         c.tile_start[kTypes] = tiles;
-        c.early_weights = (a->phases & ANI_PASS_FEATURIZE) != 0;
+        c.early_weights = (a->phases & ANI_PASS_FEATURIZE) != 0 && a->n_mols > 0;     // the features lie behind the packing
         if (int rc = mlp_chain_act<kChainForces>(c, a->activation, a->split_precision != 0, (cudaStream_t)stream)) return rc;
         backward_done = true;
     } else if (a->phases & ANI_PASS_FORWARD) {

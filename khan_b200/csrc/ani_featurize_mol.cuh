@@ -202,7 +202,10 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 32 : 20)
     // without work then hold up the start.)
     const int round = blockIdx.x / n_mols, m = blockIdx.x - round * n_mols;
     MolRange mol;
-    if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) return;
+    if (!load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol)) {
+        pdl_wait();
+        return;
+    }
     const int n = mol.n, base = mol.base;
 
     if (n > kMolMaxAtoms) {   // a large molecule in a batch of small ones: its CTAs take one atom at a time

@@ -5,7 +5,8 @@
 // set up while its predecessor drains; pdl_wait() holds it until everything before it in the stream has
 // finished and is visible.  Rules that every kernel of this library launched this way keeps:
 //   * pdl_wait() comes before the first access to memory that an earlier kernel of the stream may write,
-//     and before the first store; weights and the geometry may be read ahead of it where the kernel before is one of
+//     and before the first store, and in some CTA of every launch, whatever the batch looks like (a kernel that ends
+//     without a wait may end before its predecessor, and the kernel behind would take both for finished); weights and the geometry may be read ahead of it where the kernel before is one of
 //     the same call and known not to write any (early_weights of the network kernels, after_sort of the features,
 //     early_inputs of the gradient);
 //   * a kernel that reads anything ahead of pdl_wait() takes what the kernel before it writes through load_fresh() or

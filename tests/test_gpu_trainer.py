@@ -280,6 +280,36 @@ def test_rows_directly_behind_the_elements(precision):
         assert torch.equal(ev_joint.mol_energy, ev_apart.mol_energy) and torch.equal(joint.grads, apart.grads), k
 
 
+@pytest.mark.parametrize("n_mols", [0, 3])
+@pytest.mark.parametrize("n_atoms", [40, 3000])
+def test_a_pass_without_molecules_uses_the_weights_of_its_own_packing(n_atoms, n_mols):
+    """Atoms, but no molecule with any: the kernels of such a pass keep their order (new weights, packed in the pass itself)
+    and the rows that nothing writes are evaluated as they are."""
+    import torch
+    from khan_b200.inference import EnergyForces
+    from khan_b200.model.nn import MoleculeNN
+    from khan_b200.staged import StagedBatch
+    model = MoleculeNN(device="cuda:0", seed=2)
+    sb, ev = StagedBatch(n_atoms, n_mols), EnergyForces(model, n_atoms, max(n_mols, 1))
+    sb.types.copy_(torch.arange(n_atoms) % 4)
+    sb.set_shape(n_atoms, n_mols, np.bincount(np.arange(n_atoms) % 4))
+    sb.xyz.normal_()
+    sb.mol_offsets.zero_()
+    sb.mol_counts.zero_()
+    sb.features.uniform_(0.0, 0.5)
+    for _ in range(20):
+        with torch.no_grad():
+            for p in model.get_parameters():
+                p.mul_(1.01)
+        ev.mol_energy.fill_(1.0)
+        ev.run(sb)
+        got = ev.energy_sorted.clone()
+        ev.run(sb, featurized=True)
+        torch.cuda.synchronize()
+        assert torch.isfinite(got).all() and torch.equal(got, ev.energy_sorted)
+        assert float(ev.mol_energy[:n_mols].abs().sum()) == 0.0
+
+
 def test_fused_train_step_matches_the_autograd_step():
     """FusedTrainStep (C ABI only) against the same step driven by torch autograd: same loss,
     same weight gradients, same coordinate gradients, same weights after the update."""

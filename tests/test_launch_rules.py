@@ -31,3 +31,10 @@ def test_what_the_kernel_in_front_writes_is_read_in_its_place(file, name, writte
     for array in written:
         assert not re.search(r"__restrict__\s+%s\b" % array, params), array
         assert not re.search(r"\b%s\s*\[" % array, body), array
+
+
+def test_a_batch_without_molecules_to_work_on_waits_too():
+    """All molecules without atoms: some CTA must wait all the same, or the kernel behind runs beside the one in front."""
+    for file, name, failed in (("ani_featurize_mol.cuh", "featurize_mol_kernel", r"if \(!load_molecule\([^;{]*\)\)"),
+                               ("ani_grad_mol.cuh", "featurize_grad_mol_kernel", r"if \(!usable\)")):
+        assert re.search(failed + r" \{\s*pdl_wait\(\);", function(file, name)[1]), name
