@@ -519,6 +519,9 @@ typedef struct ani_force_fit_args {
     void* features_ready;            /* cudaEvent_t */
 } ani_force_fit_args;
 int ani_force_fit_pass_f32(const ani_force_fit_args* args, void* stream);
+/* Between two dense layers: z[rows][width] += the bias of the row's element (rows element-sorted, acs_host of
+ * each), a = celu(z) unless a is NULL.  width a multiple of 4. */
+int ani_bias_celu_f32(float* z, float* a, const float* const* bias_host4, const int* acs_host, int width, void* stream);
 
 /* Energies, and energies + forces, in double precision (the precision the reference serves in,
  * energy_server.py): the phases FEATURIZE, FORWARD, ENERGY, BACKWARD and COORD_GRAD of the above for

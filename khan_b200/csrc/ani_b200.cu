@@ -1617,6 +1617,31 @@ int ani_request(const ani_request_args* a, void* stream)
     return ANI_OK;
 }
 
+int ani_bias_celu_f32(float* z, float* a, const float* const* bias, const int* acs_host, int width, void* stream)
+{
+    long long n_atoms = 0;
+    if (int rc = check_acs(acs_host, &n_atoms)) return rc;
+    if (width <= 0 || (width & 3) || n_atoms * width > 0x7fffffffLL) return ANI_ERR_BAD_SIZE;
+    if (n_atoms == 0) return ANI_OK;
+    if (!z || !bias) return ANI_ERR_NULL_POINTER;
+    BiasCeluParams p;
+    p.z = z;
+    p.a = a;
+    p.rows = (int)n_atoms;
+    p.width = width;
+    int row = 0;
+    for (int t = 0; t < kTypes; t++) {
+        if (acs_host[t] > 0 && !bias[t]) return ANI_ERR_NULL_POINTER;
+        if (!all_aligned16({bias[t]})) return ANI_ERR_MISALIGNED;
+        p.bias[t] = bias[t];
+        row += acs_host[t];
+        p.row_end[t] = row;
+    }
+    if (!all_aligned16({z, a})) return ANI_ERR_MISALIGNED;
+    ANI_CUDA(launch_chain(bias_celu_kernel, (int)((n_atoms * (width / 4) + 255) / 256), 256, 0, (cudaStream_t)stream, 1, p));
+    return ANI_OK;
+}
+
 int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
 {
     if (!f) return ANI_ERR_NULL_POINTER;

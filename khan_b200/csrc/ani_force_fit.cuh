@@ -151,6 +151,35 @@ __global__ void __launch_bounds__(kCeluThreads, 2) celu_preactivations_kernel(co
     finish(s2, 2, kMlpH3, nullptr);
 }
 
+// Between two dense layers that somebody else computes: z += bias of the row's element, a = celu(z).  rows x width values,
+// 4 per thread.
+struct BiasCeluParams {
+    float* z;
+    float* a;                       // or null: last layer
+    const float* bias[kTypes];
+    int row_end[kTypes];            // rows of elements 0 .. t end here
+    int rows, width;                // width: a multiple of 4
+};
+__global__ void __launch_bounds__(256) bias_celu_kernel(const BiasCeluParams p)
+{
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    const int per_row = p.width >> 2;
+    const int row = i / per_row, c = (i - row * per_row) * 4;
+    if (row >= p.rows) return;
+    const int e = (row >= p.row_end[0]) + (row >= p.row_end[1]) + (row >= p.row_end[2]);
+    const float4 b = *reinterpret_cast<const float4*>(p.bias[e] + c);
+    float4* zp = reinterpret_cast<float4*>(p.z + (size_t)row * p.width + c);
+    float4 z = *zp;
+    z.x += b.x; z.y += b.y; z.z += b.z; z.w += b.w;
+    *zp = z;
+    if (p.a)
+        *reinterpret_cast<float4*>(p.a + (size_t)row * p.width + c) =
+            make_float4(mlp_activation<kActCelu>(z.x), mlp_activation<kActCelu>(z.y), mlp_activation<kActCelu>(z.z),
+                        mlp_activation<kActCelu>(z.w));
+}
+
 // ---- the loss: exp(sum over the axes of the rmse between the forces and their targets), as the reference's
 // train_op_forces (khan/training/trainer_multi_tower.py:377-399) ----
 constexpr int kForceLossThreads = 256;

@@ -82,6 +82,18 @@ def test_weight_grad_rejects_misaligned_matrices_before_launching(handle):
     assert handle.ani_nadam_step_f32(None, None, None, None, None, 0, None, None, None) == 0
 
 
+def test_bias_and_celu_checks_need_no_gpu(handle):
+    acs = (ctypes.c_int * 4)(5, 0, 0, 2)
+    bias = (ctypes.c_void_p * 4)(0x10000, None, None, 0x20000)
+    call = handle.ani_bias_celu_f32
+    assert call(None, None, None, (ctypes.c_int * 4)(), 128, None) == 0
+    assert call(0x30000, None, bias, acs, 126, None) == call(0x30000, None, bias, acs, 0, None) == -2
+    assert call(None, None, bias, acs, 128, None) == call(0x30000, None, None, acs, 128, None) == -1
+    assert call(0x30004, None, bias, acs, 128, None) == call(0x30000, 0x40008, bias, acs, 128, None) == -9
+    bias[3] = None
+    assert call(0x30000, None, bias, acs, 128, None) == -1
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
     monkeypatch.setattr(_lib, "_lib", None)

@@ -1,6 +1,8 @@
 """The fused tensor-core atomic-network kernel against a plain float64 torch evaluation of the
 same four 384-128-128-64-1 stacks.  Tolerances (relative to the largest energy): 2e-5 with the
 split-precision products (float32-grade), 5e-3 with plain tf32."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -204,3 +206,25 @@ def test_few_atom_networks_match_the_autograd_path(precision, n_mols, heavy):
         e1, g1 = tr.energy_and_gradient(mols[0])
         assert abs(e1 - want_e[0]) <= tol * np.abs(want_e).max()
         assert np.abs(g1 - want_g[:len(mols[0])]).max() <= tol * np.abs(want_g).max()
+
+
+@pytest.mark.parametrize("counts,width", [((1, 0, 0, 0), 4), ((5, 0, 3, 70), 64), ((300, 31, 0, 1), 128)])
+def test_bias_and_celu_between_layers(counts, width):
+    """ani_bias_celu_f32 against float64: one addition (half an ulp of z) and exp in float32 (at most 1e-6 off, times 0.1)."""
+    import torch
+    from khan_b200 import _lib
+    n, rng = sum(counts), np.random.default_rng(width)
+    z0, b = rng.normal(size=(n, width)).astype(np.float32), rng.normal(size=(4, width)).astype(np.float32)
+    z, bias = torch.from_numpy(z0).cuda(), torch.from_numpy(b).cuda()
+    a = torch.empty_like(z)
+    where = (ctypes.c_void_p * 4)(*[bias[t].data_ptr() if counts[t] else None for t in range(4)])
+    acs = (ctypes.c_int * 4)(*counts)
+    _lib.check(_lib.lib().ani_bias_celu_f32(z.data_ptr(), a.data_ptr(), where, acs, width, None), "ani_bias_celu_f32")
+    want = z0.astype(np.float64) + np.repeat(b.astype(np.float64), counts, axis=0)
+    assert np.abs(z.cpu().numpy() - want).max() <= 6e-8 * np.abs(want).max()
+    zs = z.cpu().numpy().astype(np.float64)
+    celu = np.where(zs >= 0, zs, 0.1 * np.expm1(10.0 * np.minimum(zs, 0.0)))
+    assert np.abs(a.cpu().numpy() - celu).max() < 2e-7
+    last = torch.from_numpy(z0).cuda()                # without an activation
+    _lib.check(_lib.lib().ani_bias_celu_f32(last.data_ptr(), None, where, acs, width, None), "ani_bias_celu_f32")
+    assert torch.equal(last, z)
