@@ -514,11 +514,12 @@ typedef struct ani_force_fit_args {
                                         NULL: whose sign decides about celu's second derivative (other activations: unused) */
     void* z_ready;                   /* cudaEvent_t after which they may be read, or NULL */
     int part;                        /* 0: everything; 1: up to the feature rates, which need no z; 2: from there on */
-    void* side_stream;               /* cudaStream_t: the call forms z1, z2, z3 itself, there, beside the first-order pass (they
-                                        are written then; both events are needed and recorded), or NULL */
-    void* features_ready;            /* cudaEvent_t */
 } ani_force_fit_args;
 int ani_force_fit_pass_f32(const ani_force_fit_args* args, void* stream);
+/* The same with z1, z2, z3 formed by the call (by its part 0 or 1) instead of the caller: they are written then, on
+ * `side_stream`, beside the first-order pass.  Both events, features_ready and args->z_ready, are needed and are recorded.
+ * With an activation other than celu it is ani_force_fit_pass_f32. */
+int ani_force_fit_pass_beside_f32(const ani_force_fit_args* args, void* side_stream, void* features_ready, void* stream);
 /* Between two dense layers: z[rows][width] += the bias of the row's element (rows element-sorted, acs_host of
  * each), a = celu(z) unless a is NULL.  width a multiple of 4. */
 int ani_bias_celu_f32(float* z, float* a, const float* const* bias_host4, const int* acs_host, int width, void* stream);

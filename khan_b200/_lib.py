@@ -96,7 +96,7 @@ class ForceFitArgs(ctypes.Structure):
     _fields_ = ([("pass_", PassArgs)]
                 + [(n, ctypes.c_void_p) for n in ("fx", "fy", "fz", "vx", "vy", "vz", "feature_rates", "r1", "r2", "adot1",
                                                   "adot2", "adot3", "q1", "q2", "q3", "partial", "rmse", "z1", "z2", "z3", "z_ready")]
-                + [("part", ctypes.c_int), ("side_stream", ctypes.c_void_p), ("features_ready", ctypes.c_void_p)])
+                + [("part", ctypes.c_int)])
 
 
 class EnergyArgs64(ctypes.Structure):
@@ -183,6 +183,7 @@ SIGNATURES = {
     "ani_host_pack_batch": (_i, [_vp]),
     "ani_network_pass_f32": (_i, [ctypes.POINTER(PassArgs), _vp]),
     "ani_force_fit_pass_f32": (_i, [ctypes.POINTER(ForceFitArgs), _vp]),
+    "ani_force_fit_pass_beside_f32": (_i, [ctypes.POINTER(ForceFitArgs), _vp, _vp, _vp]),
     "ani_bias_celu_f32": (_i, [_vp, _vp, _vp, c_int_p, _i, _vp]),
     "ani_energy_pass_f64": (_i, [ctypes.POINTER(EnergyArgs64), _vp]),
     "ani_request": (_i, [ctypes.POINTER(RequestArgs), _vp]),

@@ -1642,9 +1642,8 @@ int ani_bias_celu_f32(float* z, float* a, const float* const* bias, const int* a
     return ANI_OK;
 }
 
-int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
+static int force_fit_pass(const ani_force_fit_args* f, void* side_stream, void* features_ready, void* stream)
 {
-    if (!f) return ANI_ERR_NULL_POINTER;
     const ani_pass_args* a = &f->pass;
     const int* acs = a->acs_host;
     long long n_atoms = 0;
@@ -1661,8 +1660,8 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
             return ANI_ERR_NULL_POINTER;
     if (!all_aligned16({f->feature_rates, f->r1, f->r2, f->adot1, f->adot2, f->adot3, f->q1, f->q2, f->q3}))
         return ANI_ERR_MISALIGNED;
-    const bool signs_here = f->side_stream && a->activation == kActCelu && f->z1 && f->z2 && f->z3;
-    if (signs_here && (!f->features_ready || !f->z_ready)) return ANI_ERR_NULL_POINTER;
+    const bool signs_here = side_stream && a->activation == kActCelu;      // else they are the caller's
+    if (signs_here && (!f->z1 || !f->z2 || !f->z3 || !features_ready || !f->z_ready)) return ANI_ERR_NULL_POINTER;
     cudaStream_t st = (cudaStream_t)stream;
     const int n = (int)n_atoms;
 
@@ -1675,9 +1674,9 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
             // beside the networks, on the stream that the caller keeps for it
             first.phases = before;
             if (int rc = ani_network_pass_f32(&first, stream)) return rc;
-            const cudaStream_t side = (cudaStream_t)f->side_stream;
-            ANI_CUDA(cudaEventRecord((cudaEvent_t)f->features_ready, st));
-            ANI_CUDA(cudaStreamWaitEvent(side, (cudaEvent_t)f->features_ready, 0));
+            const cudaStream_t side = (cudaStream_t)side_stream;
+            ANI_CUDA(cudaEventRecord((cudaEvent_t)features_ready, st));
+            ANI_CUDA(cudaStreamWaitEvent(side, (cudaEvent_t)features_ready, 0));
             if (int rc = celu_preactivations_launch(a, acs, const_cast<float*>(f->z1), const_cast<float*>(f->z2),
                                                     const_cast<float*>(f->z3), side))
                 return rc;
@@ -1760,6 +1759,16 @@ int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
     if (int rc = mlp_chain_act<kChainTangent>(p, a->activation, a->split_precision != 0, st)) return rc;
     if (a->zero_ptr && a->zero_bytes) ANI_CUDA(cudaMemsetAsync(a->zero_ptr, 0, a->zero_bytes, st));
     return wgrad_call(sets, acs, 2, a->split_precision, st);
+}
+
+int ani_force_fit_pass_f32(const ani_force_fit_args* f, void* stream)
+{
+    return f ? force_fit_pass(f, nullptr, nullptr, stream) : ANI_ERR_NULL_POINTER;
+}
+
+int ani_force_fit_pass_beside_f32(const ani_force_fit_args* f, void* side_stream, void* features_ready, void* stream)
+{
+    return f && side_stream ? force_fit_pass(f, side_stream, features_ready, stream) : ANI_ERR_NULL_POINTER;
 }
 
 }  // extern "C"

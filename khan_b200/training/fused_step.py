@@ -218,7 +218,8 @@ class FusedTrainStep:
 
 class ForceFitStep(FusedTrainStep):
     """The force-training step (``train_op_forces`` of the reference) on the C ABI only: weight gradients of
-    exp(force rmse) in one call (``ani_force_fit_pass_f32``), added into the flat buffer."""
+    exp(force rmse) in one call (``ani_force_fit_pass_beside_f32``, without celu ``ani_force_fit_pass_f32``), added into the
+    flat buffer."""
 
     def __init__(self, model, optimizer: FlatNadam, n_atoms: int, n_mols: int, device="cuda:0"):
         super().__init__(model, optimizer, n_atoms, n_mols, device)
@@ -245,8 +246,7 @@ class ForceFitStep(FusedTrainStep):
             setattr(f, name, t.data_ptr())
         if self.celu:
             f.z1, f.z2, f.z3 = (z.data_ptr() for z in self.z)
-            f.side_stream = self.side.cuda_stream
-            f.features_ready, f.z_ready = (event.cuda_event for event in self.events)
+            f.z_ready = self.events[1].cuda_event
 
     def weight_gradients_of_forces(self, sb: StagedBatch, forces: torch.Tensor) -> None:
         """``forces``: the batch's target forces ``[3, n_atoms]``.  Afterwards ``self.rmse`` holds the sum of
@@ -264,7 +264,11 @@ class ForceFitStep(FusedTrainStep):
         f = self._force_args
         f.fx, f.fy, f.fz = (forces[k].data_ptr() for k in range(3))
         f.pass_ = a
-        _lib.check(_lib.lib().ani_force_fit_pass_f32(ctypes.byref(f), stream), "ani_force_fit_pass_f32")
+        if self.celu:
+            _lib.check(_lib.lib().ani_force_fit_pass_beside_f32(ctypes.byref(f), self.side.cuda_stream, self.events[0].cuda_event,
+                                                                stream), "ani_force_fit_pass_beside_f32")
+        else:
+            _lib.check(_lib.lib().ani_force_fit_pass_f32(ctypes.byref(f), stream), "ani_force_fit_pass_f32")
         self._args_key = None
 
 

@@ -2,6 +2,7 @@
 import ctypes
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -80,6 +81,20 @@ def test_weight_grad_rejects_misaligned_matrices_before_launching(handle):
     assert handle.ani_mlp_backward_f32(ctypes.byref(bwd), one, 1, None) == -9
     assert handle.ani_nadam_step_f32(None, None, None, None, None, 10, None, None, None) == -1
     assert handle.ani_nadam_step_f32(None, None, None, None, None, 0, None, None, None) == 0
+
+
+def test_force_training_block_ends_with_part(tmp_path):
+    """A caller's ``ani_force_fit_args`` ends with ``part``: the library reads nothing behind it, and the block of the ctypes
+    callers is laid out like the header's."""
+    source = tmp_path / "layout.c"
+    source.write_text('#include <stdio.h>\n#include <stddef.h>\n#include "ani_b200.h"\nint main(void) {\n'
+                      'printf("%zu %zu %zu\\n", sizeof(ani_force_fit_args), offsetof(ani_force_fit_args, part),'
+                      ' sizeof(ani_pass_args)); return 0; }\n')
+    subprocess.run(["gcc", "-I", os.path.join(ROOT, "include"), "-o", str(tmp_path / "layout"), str(source)], check=True)
+    size, part, block = map(int, subprocess.run([str(tmp_path / "layout")], capture_output=True, check=True).stdout.split())
+    # 21 pointers between the pass and part; the int is padded to eight bytes
+    assert part == block + 21 * 8 and size == part + 8
+    assert ctypes.sizeof(_lib.ForceFitArgs) == size and _lib.ForceFitArgs.part.offset == part
 
 
 def test_bias_and_celu_checks_need_no_gpu(handle):

@@ -592,6 +592,95 @@ def test_celu_preactivations(elements):
         first += count
 
 
+@pytest.fixture
+def force_batch():
+    """A batch that ForceFitStep has worked on once: (step, its batch, weight gradients, the argument block of that call)."""
+    import torch
+    from khan_b200 import FlatNadam
+    from khan_b200.model.nn import MoleculeNN
+    from khan_b200.staged import HostBatch, StagedBatch
+    from khan_b200.training.fused_step import ForceFitStep
+    b = syn.gdb_like_batch(60, seed=5)
+    model = MoleculeNN(device="cuda:0", seed=1)
+    optimizer = FlatNadam(model.get_parameters(), lr=1e-5, clip_norm=5.0)
+    sb = StagedBatch(b.n_atoms, b.n_mols)
+    sb.upload(HostBatch(b, None, pin=False), non_blocking=False, with_upstream=False)
+    step = ForceFitStep(model, optimizer, b.n_atoms, b.n_mols)
+    forces = torch.from_numpy(np.random.default_rng(1).normal(0.0, 0.05, (3, b.n_atoms)).astype(np.float32)).cuda()
+    step.weight_gradients_of_forces(sb, forces)
+    torch.cuda.synchronize()
+    step.targets = forces                                # the block points there
+    return step, sb, optimizer.flat_grads.clone(), step._force_args
+
+
+@pytest.mark.parametrize("route", ["whole", "parts", "parts, z last", "parts, beside"])
+def test_routes_of_a_force_training_batch(force_batch, route):
+    """ani_force_fit_pass_f32 with pre-activations that the caller brings, in one call or two, and the two parts of the call
+    that forms them itself, against that call as a whole.  The weight gradients are added with atomics, so not bit for bit."""
+    import ctypes
+    import torch
+    from khan_b200 import _lib
+    step, sb, want, f = force_batch
+    stream, other = torch.cuda.current_stream(), torch.cuda.Stream()
+    call, beside = _lib.lib().ani_force_fit_pass_f32, _lib.lib().ani_force_fit_pass_beside_f32
+    z, ready = [t.clone() for t in step.z], torch.cuda.Event()
+
+    def part(k, entry=call, *more):
+        f.part = k
+        _lib.check(entry(ctypes.byref(f), *more, stream.cuda_stream), "force training")
+    if route == "parts, beside":
+        for t in step.z:
+            t.fill_(float("nan"))
+        part(1, beside, step.side.cuda_stream, step.events[0].cuda_event)
+        part(2, beside, step.side.cuda_stream, step.events[0].cuda_event)
+    else:
+        f.z1, f.z2, f.z3 = (t.data_ptr() for t in z)
+        f.z_ready = None
+        if route == "whole":
+            part(0)
+        else:
+            if route == "parts, z last":                 # formed on a stream of the caller's while part 1 runs
+                keep = [t.clone() for t in z]
+                for t in z:
+                    t.fill_(float("nan"))
+                ready.record(other)
+                f.z_ready = ready.cuda_event
+            part(1)
+            if route == "parts, z last":
+                other.wait_stream(stream)
+                with torch.cuda.stream(other):
+                    for to, v in zip(z, keep):
+                        to.copy_(v)
+                    ready.record(other)
+            part(2)
+    torch.cuda.synchronize()
+    got = step.optimizer.flat_grads
+    assert float((got - want).norm()) < 1e-5 * float(want.norm())
+    if route == "whole":                                 # they are what decides: other signs give something else
+        for t in z:
+            t.neg_()
+        part(0)
+        torch.cuda.synchronize()
+        assert float((got - want).norm()) > 1e-2 * float(want.norm())
+
+
+def test_force_training_refuses_what_its_entries_cannot_do(force_batch):
+    import ctypes
+    from khan_b200 import _lib
+    step, _, _, f = force_batch
+    call, beside = _lib.lib().ani_force_fit_pass_f32, _lib.lib().ani_force_fit_pass_beside_f32
+    side, ready = step.side.cuda_stream, step.events[0].cuda_event
+    assert beside(ctypes.byref(f), None, ready, None) == beside(ctypes.byref(f), side, None, None) == -1
+    assert call(None, None) == beside(None, side, ready, None) == -1
+    for k in (-1, 3):
+        f.part = k
+        assert call(ctypes.byref(f), None) == beside(ctypes.byref(f), side, ready, None) == -2
+    f.part, f.z_ready = 0, None
+    assert beside(ctypes.byref(f), side, ready, None) == -1
+    f.z_ready, f.z2 = step.events[1].cuda_event, None
+    assert beside(ctypes.byref(f), side, ready, None) == -1
+
+
 def test_passes_over_a_data_set_may_interleave_and_be_given_up():
     """Two passes at once, one of them abandoned after its first molecules, give what undisturbed passes give."""
     import torch
