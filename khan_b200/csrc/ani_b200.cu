@@ -1642,6 +1642,17 @@ int ani_bias_celu_f32(float* z, float* a, const float* const* bias, const int* a
     return ANI_OK;
 }
 
+// Work on a side stream that a call has not waited for yet: where the call gives up, the caller's stream waits for it all the
+// same, so that the caller may take back the buffers in the order of its own stream.
+struct SideWork {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t done = nullptr;
+    ~SideWork()
+    {
+        if (done) cudaStreamWaitEvent(stream, done, 0);
+    }
+};
+
 static int force_fit_pass(const ani_force_fit_args* f, void* side_stream, void* features_ready, void* stream)
 {
     const ani_pass_args* a = &f->pass;
@@ -1664,6 +1675,7 @@ static int force_fit_pass(const ani_force_fit_args* f, void* side_stream, void* 
     if (signs_here && (!f->z1 || !f->z2 || !f->z3 || !features_ready || !f->z_ready)) return ANI_ERR_NULL_POINTER;
     cudaStream_t st = (cudaStream_t)stream;
     const int n = (int)n_atoms;
+    SideWork in_flight;
 
     // coordinate gradients of the energy: the first-order pass, which also leaves dE/dA_l
     if (f->part != 2) {
@@ -1681,6 +1693,8 @@ static int force_fit_pass(const ani_force_fit_args* f, void* side_stream, void* 
                                                     const_cast<float*>(f->z3), side))
                 return rc;
             ANI_CUDA(cudaEventRecord((cudaEvent_t)f->z_ready, side));
+            in_flight.stream = st;
+            in_flight.done = (cudaEvent_t)f->z_ready;
         }
         first.phases = (signs_here ? 0 : before) | ANI_PASS_FORWARD;
         if (int rc = ani_network_pass_f32(&first, stream)) return rc;
@@ -1754,6 +1768,7 @@ static int force_fit_pass(const ani_force_fit_args* f, void* side_stream, void* 
                                                     a->n_mols, a->scatter_idxs, f->vx, f->vy, f->vz, rates[0], rates[1],
                                                     rates[2], rates[3], acs, stream))
             return rc;
+    in_flight.done = nullptr;      // part 2 waits
     if (f->part == 1) return ANI_OK;
     if (f->z_ready) ANI_CUDA(cudaStreamWaitEvent(st, (cudaEvent_t)f->z_ready, 0));
     if (int rc = mlp_chain_act<kChainTangent>(p, a->activation, a->split_precision != 0, st)) return rc;

@@ -681,6 +681,24 @@ def test_force_training_refuses_what_its_entries_cannot_do(force_batch):
     assert beside(ctypes.byref(f), side, ready, None) == -1
 
 
+def test_a_force_training_batch_given_up_leaves_nothing_behind_on_its_side_stream(force_batch):
+    """A call that is refused half way (no rows for the coordinate gradients) has work in flight on the side stream: what the
+    caller enqueues afterwards on its own stream comes behind it."""
+    import ctypes
+    import torch
+    from khan_b200 import _lib
+    step, _, _, f = force_batch
+    f.pass_.phases, f.pass_.scatter_idxs = 0, None
+    with torch.cuda.stream(step.side):
+        torch.cuda._sleep(100_000_000)                   # 50 ms: nothing there is done when the call returns
+    stream = torch.cuda.current_stream().cuda_stream
+    assert _lib.lib().ani_force_fit_pass_beside_f32(ctypes.byref(f), step.side.cuda_stream, step.events[0].cuda_event, stream) == -1
+    for z in step.z:
+        z.fill_(7.0)
+    torch.cuda.synchronize()
+    assert all(bool((z == 7.0).all()) for z in step.z)
+
+
 def test_passes_over_a_data_set_may_interleave_and_be_given_up():
     """Two passes at once, one of them abandoned after its first molecules, give what undisturbed passes give."""
     import torch
