@@ -24,9 +24,9 @@ namespace ani {
 //
 // One CTA takes 32 atoms of an element through the three hidden layers: their features stay in shared memory, the weights
 // come in chunks of 32 rows through two stages, a thread has 4 x 4 outputs (2 x 4 in layer 3), the rows of a warp are the
-// same for all its lanes.  A sum runs over k = 0, 1, 2 ... in one accumulator, as in the library's float32 products, whose
-// bits it gives (sums of 32 products added up would be closer to float64, but every sign that they change moves single
-// gradients by a thousandth of their rms).  It runs beside the first-order pass, whose network kernels fill a fifth of the device for 256
+// same for all its lanes.  A pre-activation is one chain of fused multiply-adds in float32 over k = 0, 1, 2 ..., from 0, and
+// the bias added to its result: the same bits whatever the batch.  (Sums of 32 products added up would be closer to
+// float64, but every sign that another order changes moves single gradients by a thousandth of their rms.)  It runs beside the first-order pass, whose network kernels fill a fifth of the device for 256
 // molecules.  Before, these were twelve library GEMMs and twelve launches of bias and activation, issued by four threads:
 // 90 us of host time and 60 us at the end of the chain in a batch of 256 molecules, now one launch of 33 us beside the
 // networks: four such batches 990 -> 783 us.

@@ -569,7 +569,9 @@ def test_force_training_step_matches_the_autograd_path(act, n_mols):
 def test_celu_preactivations(elements):
     """The pre-activations whose signs force training takes, against float64: tiles of 32 atoms per element, none, one,
     a row less and a row more.  A float32 sum of 384 products is off by about sqrt(384) half ulps (1.2e-6) of its largest
-    partial sum, which is up to three times the largest result; the layers behind carry that on."""
+    partial sum, which is up to three times the largest result; the layers behind carry that on.  The first layer, whose
+    inputs are known to the bit, is what the kernel is defined to be: a chain of fused multiply-adds in order of k, then
+    the bias (80-bit sums round to float32 as an exact sum does, but for one in 2^39)."""
     import torch
     from khan_b200 import FlatNadam
     from khan_b200.model.nn import MoleculeNN
@@ -599,6 +601,12 @@ def test_celu_preactivations(elements):
         for l in range(3):
             z = a @ ann.Ws[l].detach().double() + ann.bs[l].detach().double()
             got = step.z[l][first:first + count].double()
+            if l == 0:
+                x, w = (v.cpu().numpy().astype(np.longdouble) for v in (a, ann.Ws[0].detach()))
+                chain = np.zeros((count, 128), np.float32)
+                for k in range(384):
+                    chain = (x[:, k:k + 1] * w[k] + chain).astype(np.float32)
+                assert np.array_equal(got.cpu().numpy(), (chain + ann.bs[0].detach().cpu().numpy()).astype(np.float64))
             assert count == 0 or float((got - z).abs().max()) < 4e-6 * float(z.abs().max()), (t, l)
             a = torch.where(z >= 0, z, 0.1 * (torch.exp(10.0 * z) - 1.0))
         first += count
