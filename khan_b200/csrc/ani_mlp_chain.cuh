@@ -7,8 +7,9 @@
 // for weights that are not packed.  The second-order pass is described in ani_force_fit.cuh.
 //
 // A tile is three products forward (K = 384, 128, 128) and five backward (K = 64, 128, 3 x 128), 38 chunks of 32
-// values of K, each 8 instructions = 0.43 us of the tensor core (three tf32 products, two of them as one of 256 columns);
-// the rest has to hide behind that.  The previous kernels took 1-2 us a chunk and 2-3 us between two products.  Here
+// values of K, three tf32 products each: 8 instructions, two of the products being one of 256 columns (12 in layer 3, which
+// has 64 columns), at the tensor core's nominal rate 0.43 us (a chunk of layer 1 was measured at 0.52); the rest has to
+// hide behind that.  The previous kernels took 1-2 us a chunk and 2-3 us between two products.  Here
 //   * one thread streams the weights through a ring of stages, ahead over the whole chain, also across epilogues;
 //   * every A operand is in tensor memory: an epilogue reads the accumulator, splits the new activations into
 //     their tf32 parts and stores those to TMEM, where the next product takes them (columns: accumulators 0-127 for
@@ -313,6 +314,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) mlp_chain_kernel(const MlpCh
                 for (int ks = 0; ks < kPipeK / 8; ks++) {
                     const unsigned step = ks * 2 * kMlpLbo, col = ks * 8;
                     const bool add = !(first && ks == 0);
+                    static_assert(kPipeOperandBytes == (kMlpTile / 8) * kPipeSbo && kTmemSmall == kTmemAcc + kMlpTile,
+                                  "the low part of B is rows 128 to 255 of the high part, and so are the accumulators' columns");
                     if (SPLIT && N == 128) {
                         // hi hi and hi lo as one instruction of 256 columns (the two parts of B lie behind one another, and so
                         // do the two accumulators): a chunk of layer 1 takes 0.52 us instead of 0.64, forward + backward of
