@@ -317,33 +317,40 @@ int featurize_grad_impl(const T* xs, const T* ys, const T* zs, const int* types,
         if (!xs || !ys || !zs || !types || !mos || !macs || !sis) return ANI_ERR_NULL_POINTER;
         for (int t = 0; t < kTypes; t++)
             if (acs_host[t] > 0 && !gin[t]) return ANI_ERR_NULL_POINTER;
-        auto launch = [&](auto warps) -> int {
-            constexpr int NW = decltype(warps)::value;
-            constexpr size_t smem = sizeof(MolGradShared<T, NW>);
-            static thread_local int configured_dev = -1;     // one per NW
+        auto launch = [&](auto warps, auto ctas) -> int {
+            constexpr int NW = decltype(warps)::value, CTAS = decltype(ctas)::value;
+            constexpr size_t smem = sizeof(MolGradShared<T, NW, CTAS>);
+            static thread_local int configured_dev = -1;     // one per variant
             int dev = 0;
             ANI_CUDA(cudaGetDevice(&dev));
             if (configured_dev != dev) {
-                if (int rc = set_smem(featurize_grad_mol_kernel<T, NW>, smem)) return rc;
+                if (int rc = set_smem(featurize_grad_mol_kernel<T, NW, CTAS>, smem)) return rc;
                 configured_dev = dev;
             }
             // more molecules than are resident at once: the larger ones start first (figures at kMolGradOrder)
-            const bool in_order = n_mols > kSms * MolGradCfg<T, NW>::kCtas;
+            const bool in_order = n_mols > kSms * CTAS;
             const dim3 grid = in_order ? dim3((n_mols + kMolGradOrder - 1) / kMolGradOrder, kMolGradOrder) : dim3(n_mols);
-            ANI_CUDA(launch_chain(featurize_grad_mol_kernel<T, NW>, grid, NW * kWarp, smem, st, 1, xs, ys, zs, types, mos,
+            ANI_CUDA(launch_chain(featurize_grad_mol_kernel<T, NW, CTAS>, grid, NW * kWarp, smem, st, 1, xs, ys, zs, types, mos,
                                   macs, n_mols, (int)n_atoms, sis, gh, gc, gn, go, gx, gy, gz, acs_host[0], acs_host[1],
                                   acs_host[2], acs_host[3], sums, early_inputs));
             return ANI_OK;
         };
-        // Few molecules: all of an SM for one, the whole molecule in its tables.  Microseconds alone with 12 warps (one CTA
-        // per SM) / 10 (two) / 8 (four) in float: 148 molecules 12.2 / 14.1 / 18.6, 296: 16.0 / 16.5 / 21.0, 444: 22.7 / 17.7 /
-        // 23.2, 740: 35 / 23.8 / 25.9, 900: 42 / 28.1 / 28.5; with eight streams in flight 148: 6.5 / 4.6 / 4.4, 740: 32 /
-        // 19.8 / 15.2, so the wide ones only as far as they gain.  In double with 12 / 8 (two): 296: 28.5 / 41.5, 512: 41.2 /
-        // 45.7, 592: 47.5 / 47.0, 700: 54 / 50.
-        if (n_mols <= kSms * (sizeof(T) == 8 ? 4 : 1)) return launch(std::integral_constant<int, 12>{});
-        if constexpr (sizeof(T) == 4)
-            if (n_mols <= 5 * kSms) return launch(std::integral_constant<int, 10>{});
-        return launch(std::integral_constant<int, 8>{});
+        // Few molecules: all of an SM for one (molecules for every other SM at most: the next batch's find a free SM then),
+        // or half of one.  Microseconds alone / with two / with eight streams in flight, float, one CTA of twelve warps per SM |
+        // two of them | four of eight: 64 molecules 10.6 / 5.4 / 2.6 | 11.7 / 6.0 / 2.1 | -, 148: 11.3 / 6.7 / 5.5 | 12.5 /
+        // 7.1 / 3.6 | -, 296: - | 15.8 / 8.8 / 7.3 | 19.8 / 11.2 / 5.5, 592: - | 18.9 / 14.6 / 14.6 | 24.3 / 14.0 / 10.5, 740: - |
+        // 22.3 / 18.0 / 18.1 | 23.8 / 14.2 / 13.5.  The second line is drawn where a batch alone stops gaining.  (With central
+        // atoms dealt to warps, as it was once, 14.6 / 7.5 / 2.5, 17.1 / 9.2 / 4.0, 19.2 / 10.7 /
+        // 8.1, 20.5 / 16.0 / 16.1 and 24.1 / 19.8 / 20.0.)  Double, one of twelve | two of eight: 296: 27.4 / 21.1 / 21.2 | 40.7 /
+        // 22.2 / 16.5, 512: 40.2 / 35.4 / 35.5 | 42.4 / 28.3 / 28.2, 592: 46.2 / 40.9 / 41.0 | 43.7 / 32.5 / 32.5.
+        using One = std::integral_constant<int, 1>;
+        using Two = std::integral_constant<int, 2>;
+        using Twelve = std::integral_constant<int, 12>;
+        using Eight = std::integral_constant<int, 8>;
+        if constexpr (sizeof(T) == 8) return 2 * n_mols <= 7 * kSms ? launch(Twelve{}, One{}) : launch(Eight{}, Two{});
+        if (2 * n_mols <= kSms) return launch(Twelve{}, One{});
+        if (n_mols <= 5 * kSms) return launch(Twelve{}, Two{});
+        return launch(Eight{}, std::integral_constant<int, 4>{});
     }
     {
         const int threads = 256;

@@ -15,13 +15,16 @@
 // bit-reproducible.
 //
 // Before, a warp took central atoms of its own, three at a time, with a lane per neighbour: 73 % of the lanes busy in the
-// pairs, and the warps of a large molecule (a cost that grows with the cube of its size) went on alone.  The busiest warp
-// scheduler issued 1.78 times the average on 1024 molecules, 1.17 times now.  Microseconds alone, before -> now: float, 1
-// molecule 8.9 -> 8.6, 64: 14.9 -> 11.7, 256: 19.4 -> 15.5, 512: 20.3 -> 18.2, 1024: 34.5 -> 29.5, 2048: 48.9 -> 44.5;
-// double, 1: 19.0 -> 16.4, 64: 35.2 -> 24.6, 256: 41.4 -> 28.3, 512: 51.6 -> 41.2, 1024: 81.6 -> 66.5, 2048: 130 -> 123.  With
-// eight streams in flight 1024 molecules in float take 20.4 instead of 19.6 and in double 59.9 instead of 61.0.  What
-// bounds it: issue at 0.6 instructions a cycle and scheduler, held up by shared memory (half of its wavefronts, the upstream
-// values of 32 lanes with different element pairs) and, for one molecule, by the chain of eight steps.
+// pairs, and the warps of a large molecule (a cost that grows with the cube of its size) went on alone.  Microseconds alone,
+// before -> now: float, 1 molecule 8.5 -> 7.0, 64: 14.6 -> 10.6, 592: 20.5 -> 18.9, 1024: 34.3 -> 27.1, 2048: 49.1 -> 41.4;
+// double, 1: 18.8 -> 13.7, 64: 34.9 -> 23.5, 500: 50.8 -> 39.6, 1024: 78.3 -> 62.2.  Beside other launches (eight streams)
+// 1024 molecules 18.5 -> 18.5, 2048: 37.0 -> 36.8, 148: 4.0 -> 3.6; double, 1024: 59.7 -> 56.4.  There it was slower at
+// first (1024 molecules 19.9, 2048: 39.7): every warp sought the molecule of its CTA, which the first warp now does for all
+// (0.2 us), and the central atom of every list entry, which is now written with the entry (0.75 us); and the sums at the
+// end tested every place of their tables, which are now without gaps and read four values at a time, the radial part beside
+// the forces of the first batch (0.5 us).  What bounds it: instruction issue (1009 an atom, in a cold capture 0.52 a cycle
+// and scheduler, the busiest 1.32 times the average), held up by shared memory (half of its wavefronts, the upstream values
+// of 32 lanes with different element pairs) and barriers, and, for one molecule, the chain of eight steps.
 //
 // A molecule with more than 32 atoms met by this kernel goes through the streaming routines
 // (zero fill by its own CTA, then global atomics, all inside the CTA).
@@ -54,41 +57,42 @@ template <typename T> struct alignas(16) MolGradNeighbor {
                        // neighbours of that central atom << 12 | row buffer << 18 | lane of the central atom << 20
 };
 
-constexpr int kMolGradPitch = kMolMaxAtoms + 1;
+constexpr int kMolGradPitch = kMolMaxAtoms + 4;      // rows in 16-byte reads, rows and columns conflict-free
 constexpr int kMolGradRow = kPairBuckets * kGradBucketStride;
 
-// Warps of a CTA, and what its tables hold of a batch: upstream rows, list entries, neighbour pairs.  A batch takes at least
-// one atom with 31 neighbours, so kEntries >= 31 and kSlots >= 465.  With more than eight warps the tables are for the
-// whole molecule (one CTA fills an SM, or two); with eight, four (float) or two (double) fit an SM.  More batches cost
-// barriers and pairs short of 32: 1024 molecules in float take 29.5 us with these tables and 43 with 8 rows, 160 entries and
-// 512 pairs and four warps.
-template <typename T, int NW> struct MolGradCfg {
+// CTAS of them fit an SM.  What the tables of one hold of a batch: upstream rows, list entries, neighbour pairs.  A batch
+// takes at least one atom with 31 neighbours, so kEntries >= 31 and kSlots >= 465.  With twelve warps the tables are for the
+// whole molecule, but for the largest; with eight, for most.  More batches cost
+// barriers and pairs short of 32: 1024 molecules in float take 27 us with these tables, and 43 (when it was 29.5 with them)
+// with 8 rows, 160 entries and 512 pairs and four warps.  (One CTA in double: with 512 entries its 197 KB leave less of the
+// first-level cache, 500 molecules 41.7 us instead of 39.6.)
+template <typename T, int NW, int CTAS> struct MolGradCfg {
     static constexpr bool kFloat = sizeof(T) == 4;
-    static constexpr int kCtas = NW == 12 ? 1 : (NW == 10 || !kFloat ? 2 : 4);      // resident per SM
-    static constexpr int kRows = NW == 12 ? (kFloat ? 32 : 24) : NW == 10 ? 24 : (kFloat ? 14 : 12);
-    static constexpr int kEntries = NW == 12 ? 512 : NW == 10 ? 384 : (kFloat ? 224 : 256);
-    static constexpr int kSlots = NW == 12 ? (kFloat ? 3072 : 2048) : NW == 10 ? 2560 : 1024;
+    static constexpr int kRows = NW == 12 ? (kFloat ? (CTAS == 1 ? 32 : 28) : 24) : (kFloat ? 14 : 12);
+    static constexpr int kEntries = NW == 12 ? (kFloat ? (CTAS == 1 ? 512 : 384) : 448) : (kFloat ? 224 : 256);
+    static constexpr int kSlots = NW == 12 ? (kFloat ? (CTAS == 1 ? 3072 : 2560) : 2048) : 1024;
     static constexpr int kRadPitch = kRadial + 16 / (int)sizeof(T);   // rows of 64 values, conflict-free in 16-byte reads
     static_assert(kRows >= 1 && kEntries >= kMolMaxAtoms - 1 && kEntries < 1 << 12 && kSlots < 1 << 13 &&
                   kSlots >= (kMolMaxAtoms - 1) * (kMolMaxAtoms - 2) / 2, "any atom fits a batch");
 };
 
-template <typename T, int NW> struct MolGradShared {
-    using Cfg = MolGradCfg<T, NW>;
+template <typename T, int NW, int CTAS> struct MolGradShared {
+    using Cfg = MolGradCfg<T, NW, CTAS>;
     alignas(16) T g[Cfg::kRows][kMolGradRow];     // angular upstream values, blocks of 32 at stride 36
     // row d of a central atom with k neighbours, place a: dL/dcos(theta) and the part along bond a of the pairs
     // (a, a + d) and (a - d, a)
     alignas(32) Vec2<T> pair[2 * Cfg::kSlots];
     Vec4<T> u[Cfg::kEntries], w[Cfg::kEntries];   // unit vector and r; 1 / r, f_C, f_C', element
-    T force[3][Cfg::kRows][kMolGradPitch];        // of a central atom of the batch on an atom
-    T radial[kMolMaxAtoms][kMolGradPitch];        // dL/dr / r of two atoms
-    T xyz[3][kMolMaxAtoms];
+    alignas(16) T force[Cfg::kRows][3][kMolGradPitch];        // of a central atom of the batch on an atom (0: not within A_Rc)
+    alignas(16) T radial[kMolMaxAtoms][kMolGradPitch];        // dL/dr / r of two atoms
+    alignas(16) T xyz[3][kMolMaxAtoms];
+    int4 molecule;                                // number (< 0: none), atoms, first atom, usable
     int type[kMolMaxAtoms];
     unsigned near[kMolMaxAtoms];                  // atoms within A_Rc
-    unsigned char list[kMolMaxAtoms][kMolMaxAtoms];   // the same as a list
-    // the radial upstream values lie over the pairs and what follows: they have been used before the first entry
+    unsigned short list[kMolMaxAtoms * (kMolMaxAtoms - 1)];   // the same as a list of all of them: atom | neighbour << 8
+    // the radial upstream values lie over the pairs: they have been used before the first pair
     __device__ __forceinline__ T* rad(int c) { return &pair[0].x + c * Cfg::kRadPitch; }
-    static_assert(sizeof(T) * kMolMaxAtoms * Cfg::kRadPitch <= sizeof(pair) + sizeof(u) + sizeof(w) + sizeof(force), "radial rows");
+    static_assert(sizeof(T) * kMolMaxAtoms * Cfg::kRadPitch <= sizeof(pair), "radial rows");
 };
 
 // Bucket of the element pair (ta, tb), four bits per entry of the 4 x 4 table.
@@ -147,12 +151,9 @@ template <typename T> struct MolEnergySums {
     T* mol_energy;
 };
 
-// early_inputs: nothing less than two kernels back writes coordinates, elements, rows or the molecule table: they are read,
-// and the distances formed, ahead of the kernel before this one, whose upstream values come last.  Energies + forces of one
-// molecule 32.3 -> 31.0 us.
-// Molecules whose CTAs are put into order of size, when not all molecules are resident at once: 1024 molecules in float
-// take 34.9 us without the order, in double 83.6 instead of 64.1; with eight streams in flight the order gains nothing
-// (19.9 without, 20.4 with it).
+// Molecules whose CTAs are put into order of size, when not all molecules are resident at once.  Without the order 1024
+// molecules in float take 32.5 us alone instead of 27.1, in double 78.6 instead of 62.2; with eight streams in flight, where
+// other batches fill the gaps, 18.0 instead of 18.5 and 55.6 instead of 56.4.
 constexpr int kMolGradOrder = 16;
 
 // length_and_inverse with one Newton step on the SFU's reciprocal root in float: the distances are computed once per pair
@@ -179,8 +180,11 @@ __device__ __forceinline__ int owner_of(unsigned members, int off, int first, in
     return c;
 }
 
-template <typename T, int NW>
-__global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
+// early_inputs: nothing less than two kernels back writes coordinates, elements, rows or the molecule table: they are read,
+// and the distances formed, ahead of the kernel before this one, whose upstream values come last.  Energies + forces of one
+// molecule 32.3 -> 31.0 us.
+template <typename T, int NW, int CTAS>
+__global__ void __launch_bounds__(NW* kWarp, CTAS)
     featurize_grad_mol_kernel(const T* __restrict__ xs, const T* __restrict__ ys, const T* __restrict__ zs,
                               const int* __restrict__ types, const int* __restrict__ mol_offsets,
                               const int* __restrict__ mol_counts, int n_mols, int n_atoms,
@@ -188,43 +192,55 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
                               T* gx, T* gy, T* gz, int acs0, int acs1, int acs2, int acs3,
                               const MolEnergySums<T> sums, bool early_inputs)
 {
-    using Cfg = MolGradCfg<T, NW>;
+    using Cfg = MolGradCfg<T, NW, CTAS>;
     constexpr int kThreads = NW * kWarp;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    MolGradShared<T, NW>& sh = *reinterpret_cast<MolGradShared<T, NW>*>(smem_raw);
+    MolGradShared<T, NW, CTAS>& sh = *reinterpret_cast<MolGradShared<T, NW, CTAS>*>(smem_raw);
     const int lane = lane_id(), warp = warp_id();
     if (!early_inputs) pdl_wait();
 
     // In a grid of (X, Y) CTAs the molecules i, i + X, i + 2 X ... share the CTAs (i, 0), (i, 1), (i, 2) ... in order of
     // their sizes: CTAs start in index order, so the expensive molecules start first and the cheap ones fill the SMs
-    // behind them.  Every CTA finds its molecule from the Y sizes; only those behind the end of the batch have none.
+    // behind them.  The first warp of a CTA finds its molecule from the Y sizes; only the CTAs behind the end of the
+    // batch have none.
     int m = blockIdx.x;
     MolRange mol;
     bool usable;
     if (gridDim.y == 1) {
         usable = load_molecule(mol_offsets, mol_counts, m, n_atoms, &mol);
     } else {
-        const int mine = blockIdx.x + lane * gridDim.x;
-        const bool there = lane < kMolGradOrder && mine < n_mols;
-        const int size = there ? mol_counts[mine] : 0, first = there ? mol_offsets[mine] : 0;
-        // the blockIdx.y-th largest, bit by bit (all above 32 atoms alike)
-        const int key = min(max(size, 0), 63);
-        unsigned left = __ballot_sync(kFull, there);
-        int y = blockIdx.y;
-        if (y >= __popc(left)) return;
+        if (warp == 0) {
+            const int mine = blockIdx.x + lane * gridDim.x;
+            const bool there = lane < kMolGradOrder && mine < n_mols;
+            const int size = there ? mol_counts[mine] : 0, first = there ? mol_offsets[mine] : 0;
+            // the blockIdx.y-th largest, bit by bit (all above 32 atoms alike)
+            const int key = min(max(size, 0), 63);
+            unsigned left = __ballot_sync(kFull, there);
+            int y = blockIdx.y;
+            const bool exists = y < __popc(left);
 #pragma unroll
-        for (int bit = 5; bit >= 0; bit--) {
-            const unsigned with = __ballot_sync(kFull, (key >> bit) & 1) & left;
-            const int c = __popc(with);
-            if (y < c) left = with;
-            else {
-                y -= c;
-                left &= ~with;
+            for (int bit = 5; bit >= 0; bit--) {
+                const unsigned with = __ballot_sync(kFull, (key >> bit) & 1) & left;
+                const int c = __popc(with);
+                if (y < c) left = with;
+                else {
+                    y -= c;
+                    left &= ~with;
+                }
             }
+            if (exists && ((left >> lane) & 1u) && __popc(left & lanemask_lt()) == y) {
+                usable = check_molecule(size, first, n_atoms, &mol);
+                sh.molecule = make_int4(mine, mol.n, mol.base, usable ? 1 : 0);
+            }
+            if (!exists && lane == 0) sh.molecule = make_int4(-1, 0, 0, 0);
         }
-        const int src = __ffs(__ballot_sync(kFull, ((left >> lane) & 1u) && __popc(left & lanemask_lt()) == y)) - 1;
-        m = blockIdx.x + src * gridDim.x;
-        usable = check_molecule(__shfl_sync(kFull, size, src), __shfl_sync(kFull, first, src), n_atoms, &mol);
+        __syncthreads();
+        const int4 found = sh.molecule;
+        m = found.x;
+        mol.n = found.y;
+        mol.base = found.z;
+        usable = found.w != 0;
+        if (m < 0) return;
     }
     if (!usable) {
         pdl_wait();
@@ -260,7 +276,7 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
         }
         __syncthreads();
         T* g = reinterpret_cast<T*>(smem_raw) + warp * kGradRowWords;
-        static_assert(NW * kGradRowWords * sizeof(T) <= sizeof(MolGradShared<T, NW>), "a row per warp");
+        static_assert(NW * kGradRowWords * sizeof(T) <= sizeof(MolGradShared<T, NW, CTAS>), "a row per warp");
         for (int i = warp; i < n; i += NW) {
             const int gi = base + i;
             const int ti = checked_type(types[gi]);
@@ -295,6 +311,7 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
         sh.xyz[2][lane] = zs[base + lane];
         sh.near[lane] = 0u;
         sh.radial[lane][lane] = (T)0;
+        for (int j = n; j & 3; j++) sh.radial[lane][j] = (T)0;      // rows are read four values at a time
     }
     if (my_type < 0 || my_type >= kTypes) my_type = warp == 0 ? checked_type(my_type) : my_type & 3;
     {
@@ -336,6 +353,11 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
         cp_async_commit();
     };
     if (!early_inputs) request_first();
+    auto clear_forces = [&] {
+        for (int i = threadIdx.x; i < min(n, Cfg::kRows) * (int)(sizeof(sh.force[0]) / 16); i += kThreads)
+            reinterpret_cast<Vec4<float>*>(sh.force)[i] = Vec4<float>{0.f, 0.f, 0.f, 0.f};
+    };
+    clear_forces();
     __syncthreads();
 
     // ---- every two atoms once: pair p of n (n - 1) / 2 is (i, i + d mod n), d = 1, 2 ... ----
@@ -367,11 +389,24 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
     load_energy();      // (the last warp has no pair of atoms in most molecules)
     cp_async_wait<0>();
     __syncthreads();
+    // lane = central atom: its neighbours and pairs, and where they start in the molecule's numbering
+    const unsigned my_near = lane < n ? sh.near[lane] : 0u;
+    const int my_k = (ok_mask >> lane) & 1u ? __popc(my_near) : 0, my_pairs = my_k * (my_k - 1) / 2;
+    int incl = my_k | (my_pairs << 12);      // at most 992 neighbours
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int excl = incl - (my_k | (my_pairs << 12));
+    const int k_first = excl & 0xfff, p_first = excl >> 12, k_end = incl & 0xfff, p_end = incl >> 12;
 #pragma unroll
     for (int s = 0; s < kMaxPairs; s++) {
         const int p = s * kThreads + threadIdx.x;
+        if (s * kThreads + warp * kWarp >= n_pairs) break;
+        const int i = p < n_pairs ? pij[s] & 0xff : 0, j = p < n_pairs ? pij[s] >> 8 : 0;
+        const int at_i = __shfl_sync(kFull, k_first, i), at_j = __shfl_sync(kFull, k_first, j);
         if (p < n_pairs) {
-            const int i = pij[s] & 0xff, j = pij[s] >> 8;
             T force = (T)0;
             if (pr[s] < (T)kR_Rc) {
                 T fc, dfc;
@@ -390,26 +425,17 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
             sh.radial[i][j] = force;
             sh.radial[j][i] = force;
             if (pr[s] < (T)kA_Rc) {
-                sh.list[i][__popc(sh.near[i] & ((1u << j) - 1u))] = (unsigned char)j;
-                sh.list[j][__popc(sh.near[j] & ((1u << i) - 1u))] = (unsigned char)i;
+                if ((ok_mask >> i) & 1u) sh.list[at_i + __popc(sh.near[i] & ((1u << j) - 1u))] = (unsigned short)(i | j << 8);
+                if ((ok_mask >> j) & 1u) sh.list[at_j + __popc(sh.near[j] & ((1u << i) - 1u))] = (unsigned short)(j | i << 8);
             }
         }
     }
-    // lane = central atom: its neighbours and pairs, and where they start in the molecule's numbering
-    const unsigned my_near = lane < n ? sh.near[lane] : 0u;
-    const int my_k = (ok_mask >> lane) & 1u ? __popc(my_near) : 0, my_pairs = my_k * (my_k - 1) / 2;
-    int incl = my_k | (my_pairs << 12);      // at most 992 neighbours
-#pragma unroll
-    for (int o = 1; o < kWarp; o <<= 1) {
-        const int y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-    }
-    const int excl = incl - (my_k | (my_pairs << 12));
-    const int k_first = excl & 0xfff, p_first = excl >> 12, k_end = incl & 0xfff, p_end = incl >> 12;
     const unsigned k_recip = (unsigned)(65536.0f * __frcp_rn((float)max(my_k, 1))) + 1u;
     __syncthreads();
 
-    T sum = (T)0;      // warps 0 .. 2: one component of the gradient of atom `lane`
+    // the last three warps, lane = atom: one component of its gradient.  The radial part first, beside the first batch's forces
+    const int plane = warp - (NW - 3);
+    T sum = (T)0;
     int c0 = 0;
     auto batch_end = [&](int from) {
         const int k0 = __shfl_sync(kFull, k_first, from), p0 = __shfl_sync(kFull, p_first, from);
@@ -426,8 +452,7 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
         // ---- list entries of the batch, lane = entry ----
         for (int first = warp * kWarp; first < n_entries; first += kThreads) {
             const int e = min(first + lane, n_entries - 1);
-            const int c = owner_of(members, my_entry, first, e);
-            const int a = e - __shfl_sync(kFull, my_entry, c), j = sh.list[c][a];
+            const int at = sh.list[k0 + e], c = at & 0xff, j = at >> 8;
             const T dx = sh.xyz[0][c] - sh.xyz[0][j], dy = sh.xyz[1][c] - sh.xyz[1][j], dz = sh.xyz[2][c] - sh.xyz[2][j];
             T r, inv, fc, dfc;
             refined_length_and_inverse(dx * dx + dy * dy + dz * dz, &r, &inv);
@@ -437,6 +462,7 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
         }
         cp_async_wait<0>();
         __syncthreads();
+        if (c0 > 0) clear_forces();
         // ---- neighbour pairs of the batch, lane = pair; the pairs of a central atom with k neighbours in circulant order:
         // pair q is (a, a + d mod k) with d = 1 + q / k, a = q mod k ----
         for (int first = ((warp + NW - 3) % NW) * kWarp; first < n_slots; first += kThreads) {
@@ -474,10 +500,22 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
             }
             cp_async_commit();
         }
+        if (plane >= 0 && c0 == 0 && lane < n) {
+            const T* x = sh.xyz[plane];
+            const T xi = x[lane];
+            for (int j = 0; j < n; j += 4) {
+                T f[4], xj[4];
+                load4(&sh.radial[lane][j], f);
+                load4(x + j, xj);
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (f[q] != (T)0) sum += f[q] * (xi - xj[q]);
+            }
+        }
         // ---- lane = entry: the force on it from the pairs that it is in ----
         for (int first = warp * kWarp; first < n_entries; first += kThreads) {
             const int e = min(first + lane, n_entries - 1);
-            const int c = owner_of(members, my_entry, first, e);
+            const int whose = sh.list[k0 + e], c = whose & 0xff;
             const int at = __shfl_sync(kFull, my_at, c);
             const int k = (at >> 13) & 0x3f, list = at >> 19, a = e - list;
             const Vec4<T>*u = sh.u + list, *row = reinterpret_cast<const Vec4<T>*>(sh.pair) + (at & 0x1fff) + a;
@@ -503,21 +541,22 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
             }
             const Vec4<T> ua = u[a];
             const T inv = sh.w[e].x;
-            const int j = sh.list[c][a];
-            sh.force[0][c - c0][j] = along * ua.x - inv * fx;
-            sh.force[1][c - c0][j] = along * ua.y - inv * fy;
-            sh.force[2][c - c0][j] = along * ua.z - inv * fz;
+            const int j = whose >> 8;
+            sh.force[c - c0][0][j] = along * ua.x - inv * fx;
+            sh.force[c - c0][1][j] = along * ua.y - inv * fy;
+            sh.force[c - c0][2][j] = along * ua.z - inv * fz;
         }
         __syncthreads();
-        // ---- warps 0 .. 2, lane = atom: what the batch's central atoms hand to it, less what it hands out ----
-        if (warp < 3) {
-            const T(*f)[kMolGradPitch] = sh.force[warp];
-            const unsigned from = my_near & ok_mask;
-            for (int q = c0; q < c1; q++)
-                if ((from >> q) & 1u) sum += f[q - c0][lane];
-            if ((members & ok_mask) >> lane & 1u)
-                for (int q = 0; q < n; q++)
-                    if ((my_near >> q) & 1u) sum -= f[lane - c0][q];
+        // ---- what the batch's central atoms hand to an atom, less what it hands out ----
+        if (plane >= 0) {
+#pragma unroll 4
+            for (int q = 0; q < c1 - c0; q++) sum += sh.force[q][plane][lane];
+            if ((members >> lane) & 1u)
+                for (int q = 0; q < n; q += 4) {
+                    T v[4];
+                    load4(&sh.force[lane - c0][plane][q], v);
+                    sum -= v[0]; sum -= v[1]; sum -= v[2]; sum -= v[3];
+                }
         }
         if (c1 >= n) break;
         c0 = c1;
@@ -525,16 +564,7 @@ __global__ void __launch_bounds__(NW* kWarp, MolGradCfg<T, NW>::kCtas)
     }
     pdl_trigger();
     write_energy();
-    if (warp < 3 && lane < n) {
-        const T* x = sh.xyz[warp];
-        const T xi = x[lane];
-#pragma unroll 4
-        for (int j = 0; j < n; j++) {
-            const T f = sh.radial[lane][j];
-            if (f != (T)0) sum += f * (xi - x[j]);
-        }
-        (warp == 0 ? gx : (warp == 1 ? gy : gz))[base + lane] = sum;
-    }
+    if (plane >= 0 && lane < n) (plane == 0 ? gx : (plane == 1 ? gy : gz))[base + lane] = sum;
 }
 
 }  // namespace ani

@@ -377,7 +377,7 @@ def test_atoms_at_the_end_of_the_angular_list(gpu, oracle_mod, n_mols, n, dt):
         assert normwise(out, ref) < FTOL[dt]
 
 
-@pytest.mark.parametrize("n_mols", [2, 148, 149, 593, 741])
+@pytest.mark.parametrize("n_mols", [2, 74, 75, 148, 149, 518, 519, 593, 741])
 @pytest.mark.parametrize("radius", [1.54, 2.2])
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 def test_gradient_in_batches_of_central_atoms(gpu, oracle_mod, n_mols, radius, dt):
