@@ -37,9 +37,16 @@ constexpr int kLargeGradPool = 96;
 constexpr int kLargeGradNoPlace = 63;              // not in the angular list
 constexpr int kLargeGradMaxAtoms = 1 << 22;        // index bits of a pool entry
 
+template <typename T> struct alignas(16) LargeGradNeighbor {
+    Vec4<T> u;         // (x_c - x_j) / r, r
+    T inv_r, fc, dfc;  // 1 / r, f_C(r, A_Rc) and its derivative
+    int info;          // element | lane of j << 2 | first list entry of its central atom << 7 |
+                       // neighbours of that central atom << 12 | row buffer << 18 | lane of the central atom << 20
+};
+
 template <typename T> struct LargeGradWarpShared {
     alignas(16) T g[kLargeGradCentrals][kGradRowWords];   // upstream rows, blocks of 32 at stride 36
-    MolGradNeighbor<T> nb[kWarp];
+    LargeGradNeighbor<T> nb[kWarp];
     Vec4<T> pool[kLargeGradPool];        // distance vector and its square; from step R on the force on the neighbour
     unsigned info[kLargeGradPool];       // element | central atom << 2 | place in the angular list << 4 | atom << 10
     int list[kLargeGradCentrals];        // of a central atom: first angular entry << 7 | angular neighbours << 12 | row << 18
@@ -179,7 +186,7 @@ __global__ void __launch_bounds__(kWarp, sizeof(T) == 4 ? 20 : 12)
                 const T d = -radial_vjp_dev<T>(r, fc, dfc, w);
                 ws.pool[p] = Vec4<T>{d * ux, d * uy, d * uz, (T)0};
                 if (q != kLargeGradNoPlace) {
-                    MolGradNeighbor<T> e;
+                    LargeGradNeighbor<T> e;
                     e.u = Vec4<T>{ux, uy, uz, r};
                     e.inv_r = inv;
                     cutoff<T>(r, (T)kA_Rc, &e.fc, &e.dfc);

@@ -22,8 +22,8 @@
 // first (1024 molecules 19.9, 2048: 39.7): every warp sought the molecule of its CTA, which the first warp now does for all
 // (0.2 us), and the central atom of every list entry, which is now written with the entry (0.75 us); and the sums at the
 // end tested every place of their tables, which are now without gaps and read four values at a time, the radial part beside
-// the forces of the first batch (0.5 us).  What bounds it: instruction issue (1009 an atom, in a cold capture 0.52 a cycle
-// and scheduler, the busiest 1.32 times the average), held up by shared memory (half of its wavefronts, the upstream values
+// the forces of the first batch (0.5 us).  What bounds it: instruction issue (1002 an atom, in a cold capture 0.55 a cycle
+// and scheduler, the busiest 1.36 times the average), held up by shared memory (half of its wavefronts, the upstream values
 // of 32 lanes with different element pairs) and barriers, and, for one molecule, the chain of eight steps.
 //
 // A molecule with more than 32 atoms met by this kernel goes through the streaming routines
@@ -49,13 +49,6 @@ template <int N> __device__ __forceinline__ void cp_async_wait()
 {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-
-template <typename T> struct alignas(16) MolGradNeighbor {
-    Vec4<T> u;         // (x_c - x_j) / r, r
-    T inv_r, fc, dfc;  // 1 / r, f_C(r, A_Rc) and its derivative
-    int info;          // element | lane of j << 2 | first list entry of its central atom << 7 |
-                       // neighbours of that central atom << 12 | row buffer << 18 | lane of the central atom << 20
-};
 
 constexpr int kMolGradPitch = kMolMaxAtoms + 4;      // rows in 16-byte reads, rows and columns conflict-free
 constexpr int kMolGradRow = kPairBuckets * kGradBucketStride;

@@ -1,10 +1,10 @@
-// The pair pass of the gradient kernels, as a fragment that is included inside a kernel (the function
+// The pair pass of featurize_grad_large_kernel, as a fragment that is included inside it (the function
 // form of such code compiled measurably worse): the neighbour pairs of every central atom in the warp's
 // neighbour list, in circulant order.  The k neighbours of a central atom occupy k consecutive list
 // entries = lanes; lane a handles the pair (a, a + d mod k) for d = 1 .. k / 2, keeps the force on a in
 // registers and hands the force on b to its owner with one shuffle; spare lanes run further offsets d
 // at the same time (`mult` copies of the list side by side).
-// Expects in scope: T, `ws` with nb[] (MolGradNeighbor<T>: info = element | ... | first entry of the
+// Expects in scope: T, `ws` with nb[] (LargeGradNeighbor<T>: info = element | ... | first entry of the
 // central atom's run << 7 | length of the run << 12 | upstream row buffer << 18 | ...) and g[][] (the
 // upstream rows), `lane`, `used` (entries in the list), `max_half` (largest k / 2 in the list, > 0).
 // Leaves: `ea` (the entry of this lane, lanes >= used hold a copy of another entry) and fax, fay, faz =
@@ -14,7 +14,7 @@
     const int copy = (lane >= used ? 1 : 0) + (lane >= 2 * used ? 1 : 0) + (lane >= 3 * used ? 1 : 0);
     const bool owner = copy < mult;
     const int l1 = owner ? lane - copy * used : 0;
-    const MolGradNeighbor<T> ea = ws.nb[l1];
+    const LargeGradNeighbor<T> ea = ws.nb[l1];
     const int ta = ea.info & 3, lb = (ea.info >> 7) & 31, na = (ea.info >> 12) & 63;
     const T* gblocks = ws.g[(ea.info >> 18) & 3] + kRadial;
     const int a = l1 - lb, hf = na >> 1;
@@ -29,7 +29,7 @@
         if (b >= na) b -= na;
         T gbx = (T)0, gby = (T)0, gbz = (T)0;
         if (valid) {
-            const MolGradNeighbor<T> eb = ws.nb[lb + b];
+            const LargeGradNeighbor<T> eb = ws.nb[lb + b];
             T c = ea.u.x * eb.u.x + ea.u.y * eb.u.y + ea.u.z * eb.u.z;
             c = Num<T>::max_((T)-1, Num<T>::min_((T)1, c));
             const T s2 = sin2_from_cross<T>(ea.u.x, ea.u.y, ea.u.z, eb.u.x, eb.u.y, eb.u.z);
